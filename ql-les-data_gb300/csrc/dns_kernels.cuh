@@ -16,9 +16,11 @@
 //   kx_fwd_band  x-axis forward c2c on the kept band, dealias mask, Leray projection
 //                (and the constant-power band coefficient of the stage field)
 //   k_rk_update  elementwise viscosity, extension terms and RK4 stage combination
-// The default explicit step has no elementwise pass: kx_fwd_band combines the stages
-// on the band in place, and the next stage's kx_inv scales every other mode by the
-// closed form of its linear decay (XLin, BandRk).
+// The default explicit step has no elementwise pass: in 2D and on small 3D grids
+// kx_stage (stage_kernels.cuh) takes the places of kx_fwd_band, k_rk_update and the next
+// stage's kx_inv; on larger 3D grids kx_fwd_band combines the stages on the band in place,
+// and the next stage's kx_inv scales every other mode by the closed form of its linear
+// decay (XLin, BandRk).
 // Intermediate fields never exist in physical space in HBM.
 #pragma once
 
@@ -115,14 +117,14 @@ __device__ __forceinline__ void band_coefficient(const float2* __restrict__ ub, 
 
 // Scale the outside-B modes of one x-pass column tile (a[c][e]: x row t + T e of column
 // m = mid * H + kh) to stage rk's field; the last stage stores their new state to S.
-template <int N, int DIM>
+template <int N>
 __device__ __forceinline__ void xlin_scale(float2 (&a)[3][Fft<N>::E], int t, int m, const XLin& xl, int batch,
                                            int* __restrict__ err) {
   constexpr int E = Fft<N>::E, T = Fft<N>::T, H = N / 2 + 1;
-  constexpr int MC = (DIM == 3 ? N : 1) * H;
-  const int mid = DIM == 3 ? m / H : 0;
+  constexpr int MC = N * H;
+  const int mid = m / H;
   const int kh = m - mid * H;
-  const int km = DIM == 3 ? kfull(mid, N) : 0;
+  const int km = kfull(mid, N);
   const unsigned ukd = 2u * (unsigned)xl.kd;
   const bool colband = (unsigned)(km + xl.kd) <= ukd && kh < xl.kt;
   const float nu = xl.nu_b[batch];
@@ -230,7 +232,7 @@ kx_inv(const float2* __restrict__ uh, long long cs, float2* __restrict__ w, long
     for (int e = 0; e < E; ++e)
       a[c][e] = ok ? uh[bofs + c * cs + (long long)(t + T * e) * MC + m] : make_float2(0.f, 0.f);
   if constexpr (LINF) {
-    if (ok && xl.rk > 0) xlin_scale<N, DIM>(a, t, m, xl, (int)blockIdx.y, err);
+    if (ok && xl.rk > 0) xlin_scale<N>(a, t, m, xl, (int)blockIdx.y, err);
   }
   kx_inv_fields<N, DIM, CURL, SKIPWX, XW>(a, t, m, ok, sm + p, w, (long long)blockIdx.y * NF * fs, fs, tw, wx,
                                           (long long)blockIdx.y * 2 * fs);
@@ -311,7 +313,7 @@ kx_inv_tma(const __grid_constant__ CUtensorMap umap, float2* __restrict__ w, lon
       issue(next);
     }
     if constexpr (LINF) {
-      if (xl.rk > 0) xlin_scale<N, 3>(a, t, tile * TW + p, xl, batch, err);
+      if (xl.rk > 0) xlin_scale<N>(a, t, tile * TW + p, xl, batch, err);
     }
     kx_inv_fields<N, 3, CURL, SKIPWX>(a, t, tile * TW + p, true, sm + p, w, (long long)batch * NF * fs, fs, tw,
                                       wx, (long long)batch * 2 * fs);
@@ -929,7 +931,7 @@ line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du,
       bulk_load(stg0, rows + 4 * fs, kPairBytes / 2, &bar[0]);
       bulk_load(stg0 + C::ROW2, rows + 5 * fs, kPairBytes / 2, &bar[0]);
     }
-    block_fft<N, E, kInv, 1, true, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
 #pragma unroll
     for (int e = 0; e < E; ++e) h1[e] = z[e];
     __syncwarp();
@@ -938,7 +940,7 @@ line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du,
       return;
     }
     c2r_pair_smem16<N>(stg1 + rsel, stg1 + C::ROW2 + rsel, t, z);  // u_z + i curl_x
-    block_fft<N, E, kInv, 1, true, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
 #pragma unroll
     for (int e = 0; e < E; ++e) h2[e] = z[e];
     __syncwarp();
@@ -947,7 +949,7 @@ line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du,
       return;
     }
     c2r_pair_smem16<N>(stg0 + rsel, stg0 + C::ROW2 + rsel, t, z);  // curl_y + i curl_z
-    block_fft<N, E, kInv, 1, true, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
     __syncwarp();
   } else {
     __shared__ float2 s_xs[C::LPC * C::XS];
@@ -955,17 +957,17 @@ line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du,
     float2* xs = s_x + (2 * warp + half) * C::XS;
     const float2* src = wb + line * H;
     c2r_pair_load16<N>(src, src + fs, t, z);  // u_x + i u_y
-    block_fft<N, E, kInv, 1, true, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
 #pragma unroll
     for (int e = 0; e < E; ++e) h1[e] = z[e];
     __syncwarp();
     c2r_pair_load16<N>(src + 2 * fs, src + 3 * fs, t, z);  // u_z + i curl_x
-    block_fft<N, E, kInv, 1, true, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
 #pragma unroll
     for (int e = 0; e < E; ++e) h2[e] = z[e];
     __syncwarp();
     c2r_pair_load16<N>(src + 4 * fs, src + 5 * fs, t, z);  // curl_y + i curl_z
-    block_fft<N, E, kInv, 1, true, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
     __syncwarp();
   }
   float2* xs = s_x + (2 * warp + half) * C::XS;
@@ -977,7 +979,7 @@ line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du,
     pz[e] = fmaf(ux, wy, -uy * wx);
     z[e] = make_float2(fmaf(uy, wz, -uz * wy), fmaf(uz, wx, -ux * wz));
   }
-  block_fft<N, E, kFwd, 1, true, true>(z, xs, t, ct16, 0);
+  block_fft<N, E, kFwd, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
   {
     float2 X[NE], Y[NE];
     r2c_pair_unpack16<N, NE>(z, t, s2, X, Y);

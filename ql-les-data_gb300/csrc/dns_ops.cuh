@@ -55,8 +55,36 @@ struct DnsOps {
       tma_ctas = persistent_ctas(kx_inv_tma<N, true, true>);
       tma_band_ctas = persistent_ctas(kx_fwd_band_tma<N>);
       tma_plain_ctas = persistent_ctas(kx_inv_tma<N, false>);
+    }
+    if constexpr (N >= kBandMin3d) {
       tma_lin_ctas = persistent_ctas(kx_inv_tma<N, true, true, true>);
       tma_band_fused_ctas = persistent_ctas(kx_fwd_band_tma<N, true>);
+    }
+    if constexpr (N >= 16) stage_attrs<2>();
+    if constexpr (N >= 16 && N <= kStageMax3d) stage_attrs<3>();
+  }
+
+  // kx_stage's shape: columns per CTA and values per thread in each transform
+  template <int DIM>
+  static constexpr int XS = DIM == 2 ? XN : TW;
+  template <int DIM>
+  static constexpr int ES = N <= (DIM == 2 ? 64 : 32) ? 4 : 8;
+  template <int DIM>
+  using Stage = XStageCfg<N, XS<DIM>, ES<DIM>>;
+
+  template <int DIM>
+  static void stage_attrs() {
+    if constexpr (Stage<DIM>::SMEM > 48 * 1024) {
+      auto set = [](auto kernel) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Stage<DIM>::SMEM);
+      };
+      set(kx_stage<N, DIM, XS<DIM>, ES<DIM>, -1, true>);
+      set(kx_stage<N, DIM, XS<DIM>, ES<DIM>, 0, true>);
+      set(kx_stage<N, DIM, XS<DIM>, ES<DIM>, 1, true>);
+      set(kx_stage<N, DIM, XS<DIM>, ES<DIM>, 2, true>);
+      set(kx_stage<N, DIM, XS<DIM>, ES<DIM>, 3, true>);
+      set(kx_stage<N, DIM, XS<DIM>, ES<DIM>, 3, false>);
+      cudaGetLastError();
     }
   }
 
@@ -96,74 +124,47 @@ struct DnsOps {
       if (c.sched.x_bulk && ctas > 0 && tma_encode(&map, us, 3, dims, strides, box)) {
         const int ntiles = (int)(mc / TW);
         const int gx = std::max(1, std::min(ntiles, ctas / c.batch));
-        if (xl)
-          L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                      kx_inv_tma<N, true, true, true><<<dim3(gx, c.batch), TX, KxTma<N>::SMEM, s>>>(
-                          map, c.W, c.fs, c.tw, ntiles, c.err, c.Wx, *xl));
-        else
-          L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                      kx_inv_tma<N, true, true><<<dim3(gx, c.batch), TX, KxTma<N>::SMEM, s>>>(
-                          map, c.W, c.fs, c.tw, ntiles, c.err, c.Wx, XLin{}));
+        if constexpr (N >= kBandMin3d)
+          if (xl) {
+            L3ES_LAUNCH(c, KK_X_INV, bytes, s,
+                        kx_inv_tma<N, true, true, true><<<dim3(gx, c.batch), TX, KxTma<N>::SMEM, s>>>(
+                            map, c.W, c.fs, c.tw, ntiles, c.err, c.Wx, *xl));
+            return;
+          }
+        L3ES_LAUNCH(c, KK_X_INV, bytes, s,
+                    kx_inv_tma<N, true, true><<<dim3(gx, c.batch), TX, KxTma<N>::SMEM, s>>>(
+                        map, c.W, c.fs, c.tw, ntiles, c.err, c.Wx, XLin{}));
         return;
       }
     }
     if constexpr (DIM == 2) {
       if (c.sched.x_bulk) {
         const dim3 gn((unsigned)((mc + XN - 1) / XN), c.batch);
-        if (xl)
-          L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                      kx_inv<N, 2, true, false, true, XN><<<gn, TXN, 0, s>>>(us, c.cs, c.W, c.fs, c.tw, c.Wx, *xl,
-                                                                            c.err));
-        else
-          L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                      kx_inv<N, 2, true, false, false, XN><<<gn, TXN, 0, s>>>(us, c.cs, c.W, c.fs, c.tw, c.Wx,
-                                                                             XLin{}, c.err));
+        L3ES_LAUNCH(c, KK_X_INV, bytes, s,
+                    kx_inv<N, 2, true, false, false, XN><<<gn, TXN, 0, s>>>(us, c.cs, c.W, c.fs, c.tw, c.Wx));
         return;
       }
     }
     const dim3 g((unsigned)((mc + TW - 1) / TW), c.batch);
-    if (xl)
-      L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                  kx_inv<N, DIM, true, DIM == 3, true><<<g, TX, 0, s>>>(us, c.cs, c.W, c.fs, c.tw, c.Wx, *xl, c.err));
-    else
-      L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                  kx_inv<N, DIM, true, DIM == 3><<<g, TX, 0, s>>>(us, c.cs, c.W, c.fs, c.tw, c.Wx));
+    if constexpr (DIM == 3 && N >= kBandMin3d)
+      if (xl) {
+        L3ES_LAUNCH(c, KK_X_INV, bytes, s,
+                    kx_inv<N, 3, true, true, true><<<g, TX, 0, s>>>(us, c.cs, c.W, c.fs, c.tw, c.Wx, *xl, c.err));
+        return;
+      }
+    L3ES_LAUNCH(c, KK_X_INV, bytes, s,
+                kx_inv<N, DIM, true, DIM == 3><<<g, TX, 0, s>>>(us, c.cs, c.W, c.fs, c.tw, c.Wx));
   }
 
-  // us: field the RHS is evaluated on; S: state; out: RK stage field (or du for rk=-1)
+  // W (u, curl u after the x inverse) -> DU (the nonlinear term before its x transform):
+  // y inverse, half-axis line pass, y forward
   template <int DIM>
-  static void stage_dim(const Ctx& c, const float2* us, float2* S, float2* out, int rk, const EpiParams& prm,
-                        cudaStream_t s) {
-    const long long mc = c.nmid * H;
+  static void nonlinear(const Ctx& c, cudaStream_t s) {
     const long long lines = c.nmid * N;
     const float scale = (float)(1.0 / (DIM == 3 ? (double)N * N * N : (double)N * N));
     const double B = c.batch, A = 8.0 * 3.0 * c.cs * B;  // bytes of one 3-component spectrum
     const double Adu = 8.0 * 3.0 * c.ds * B;               // bytes of the truncated DU field
     const double rows = DIM == 3 ? (2.0 * c.kd + 1.0) / N : 1.0;  // kept y rows
-    const double inv_n2d = 1.0 / (DIM == 3 ? std::pow((double)N, 6) : std::pow((double)N, 4));
-    // band-fused RK step (XLin): us == S; fb = the band's share of the modes
-    const bool fused = prm.band_rk && rk >= 0;
-    const double fb = (double)c.pcs / (double)c.cs;
-    XLin xl{};
-    if (fused) {
-      xl.S = S;
-      xl.cs = c.cs;
-      xl.nu_b = c.nu_b;
-      xl.drag = prm.drag;
-      xl.dt = prm.dt;
-      xl.kd = c.kd;
-      xl.kt = c.kt;
-      xl.rk = rk;
-      xl.band_kf = prm.band_kf2 > 0 ? c.kf : 0;
-      xl.inv_n2d = inv_n2d;
-      xl.eps_inj = c.eps_inj;
-      xl.band_scale = c.band;
-    }
-    // 3D: the x pass stores u_x, curl_y, curl_z in W and u_y, u_z in the side buffer
-    // Wx (curl_x is not stored); the y pass writes all six fields of W. The last
-    // band-fused stage also writes the new state outside the band.
-    x_inverse<DIM>(c, us, (DIM == 3 ? 8.0 : 9.0) / 3.0 * A + (fused && rk == 3 ? (1.0 - fb) * A : 0.0), s,
-                   fused ? &xl : nullptr);
     if (DIM == 3) y_inv_rhs(c, 11.0 / 3.0 * A, s);
     bool line_done = false;
     if constexpr (N >= 64 && N <= 256) {  // two real lines per complex FFT, persistent
@@ -200,16 +201,50 @@ struct DnsOps {
                   line_cross<N><<<dim3(line_blocks(lines), c.batch), L::THREADS, 0, s>>>(
                       c.W, c.fs, c.DU, c.ds, c.kt, c.kd, scale, c.tw, (int)lines));
     if (DIM == 3) y_pass<kFwd>(c, KK_Y_FWD, Adu * (1.0 + rows), c.DU, c.ds, c.kt, c.kd, 3 * c.batch, s);
+  }
+
+  // us: field the RHS is evaluated on; S: state; out: RK stage field (or du for rk=-1)
+  template <int DIM>
+  static void stage_dim(const Ctx& c, const float2* us, float2* S, float2* out, int rk, const EpiParams& prm,
+                        cudaStream_t s) {
+    const double B = c.batch, A = 8.0 * 3.0 * c.cs * B;  // bytes of one 3-component spectrum
+    const double Adu = 8.0 * 3.0 * c.ds * B;               // bytes of the truncated DU field
+    const double rows = DIM == 3 ? (2.0 * c.kd + 1.0) / N : 1.0;  // kept y rows
+    const double inv_n2d = 1.0 / (DIM == 3 ? std::pow((double)N, 6) : std::pow((double)N, 4));
+    // band-fused RK step (XLin): us == S; fb = the band's share of the modes
+    const bool fused = DIM == 3 && N >= kBandMin3d && prm.band_rk && rk >= 0;
+    const double fb = (double)c.pcs / (double)c.cs;
+    XLin xl{};
+    if (fused) {
+      xl.S = S;
+      xl.cs = c.cs;
+      xl.nu_b = c.nu_b;
+      xl.drag = prm.drag;
+      xl.dt = prm.dt;
+      xl.kd = c.kd;
+      xl.kt = c.kt;
+      xl.rk = rk;
+      xl.band_kf = prm.band_kf2 > 0 ? c.kf : 0;
+      xl.inv_n2d = inv_n2d;
+      xl.eps_inj = c.eps_inj;
+      xl.band_scale = c.band;
+    }
+    // 3D: the x pass stores u_x, curl_y, curl_z in W and u_y, u_z in the side buffer
+    // Wx (curl_x is not stored); the y pass writes all six fields of W. The last
+    // band-fused stage also writes the new state outside the band.
+    x_inverse<DIM>(c, us, (DIM == 3 ? 8.0 : 9.0) / 3.0 * A + (fused && rk == 3 ? (1.0 - fb) * A : 0.0), s,
+                   fused ? &xl : nullptr);
+    nonlinear<DIM>(c, s);
     // band x-FFT + projection into P, then the elementwise RK update
     const int nb = 2 * c.kd + 1;
     const double Ap = 8.0 * 3.0 * c.pcs * B;
-    if (fused) {
+    if constexpr (DIM == 3 && N >= kBandMin3d) if (fused) {
       // the stage combination on the band: rk 0 reads S and writes P (= u0) and S; rk 1
       // reads S, P and writes acc, S; rk 2 reads S, P, acc and writes acc, S; rk 3 reads
       // S, acc and writes S
       const BandRk br{S, c.C, c.cs, prm, c.band, c.nu_b, c.err};
       const double bb = Adu * rows + Ap * (rk == 0 ? 3.0 : rk == 1 ? 4.0 : rk == 2 ? 5.0 : 3.0);
-      if constexpr (DIM == 3 && N >= 64) {
+      {
         const bool bulk = c.sched.band_bulk < 0 ? N >= 256 : c.sched.band_bulk != 0;
         CUtensorMap map;
         const unsigned long long dims[4] = {(unsigned long long)c.kt, N, N, 3ull * c.batch};
@@ -224,14 +259,9 @@ struct DnsOps {
           return;
         }
       }
-      if (DIM == 2 && c.sched.x_bulk)
-        L3ES_LAUNCH(c, KK_X_EPI, bb, s,
-                    kx_fwd_band<N, DIM, true, XN><<<dim3(c.kt / XN, 1, c.batch), TXN, 0, s>>>(
-                        c.DU, c.ds, c.kt, c.kd, c.P, c.pcs, c.tw, us, c.cs, 0, inv_n2d, c.eps_inj, c.band, br));
-      else
-        L3ES_LAUNCH(c, KK_X_EPI, bb, s,
-                    kx_fwd_band<N, DIM, true><<<dim3(c.kt / TW, DIM == 3 ? nb : 1, c.batch), TX, 0, s>>>(
-                        c.DU, c.ds, c.kt, c.kd, c.P, c.pcs, c.tw, us, c.cs, 0, inv_n2d, c.eps_inj, c.band, br));
+      L3ES_LAUNCH(c, KK_X_EPI, bb, s,
+                  kx_fwd_band<N, 3, true><<<dim3(c.kt / TW, nb, c.batch), TX, 0, s>>>(
+                      c.DU, c.ds, c.kt, c.kd, c.P, c.pcs, c.tw, us, c.cs, 0, inv_n2d, c.eps_inj, c.band, br));
       return;
     }
     // (block 0 of each trajectory also computes the constant-power coefficient of us)
@@ -285,6 +315,59 @@ struct DnsOps {
       L3ES_LAUNCH(c, KK_RK_UPDATE, upd, s,
                   k_rk_update<N, DIM><<<ug, 256, 0, s>>>(c.P, c.pcs, c.kt, c.kd, us, S, c.C, out, S, c.cs, prm,
                                                           c.band, c.nu_b, c.err));
+  }
+
+  // One kx_stage launch: RK = -1 opens a step, RK = 0..3 closes that stage (XStage)
+  template <int DIM, int RK, bool INV>
+  static void x_stage(const Ctx& c, float2* S, const EpiParams& prm, cudaStream_t s) {
+    const double A = 8.0 * 3.0 * c.cs * c.batch;
+    // share of the columns (du is read there) and of the modes that the band holds
+    const double fc = (DIM == 3 ? (2.0 * c.kd + 1.0) / N : 1.0) * c.kt / H, fb = (double)c.pcs / (double)c.cs;
+    double b = INV ? (DIM == 3 ? 5.0 : 6.0) / 3.0 * A : 0.0;  // lines out
+    if (RK < 0) b += A;
+    if (RK == 0) b += (fc + 1.0 + fb) * A;              // du, S -> T
+    if (RK == 1) b += (fc + 1.0 + 3.0 * fb) * A;        // du, S, T -> T, C
+    if (RK == 2) b += (fc + 2.0 + 3.0 * fb) * A;        // du, S, T, C -> T, C, S outside the band
+    if (RK == 3) b += (fc + 3.0 * fb + (INV ? 1.0 - fb : 0.0)) * A;  // du, T, C -> S
+    if (RK >= 0 && prm.band_kf2 > 0) {
+      const double inv_n2d = 1.0 / std::pow((double)N, 2 * DIM);
+      L3ES_LAUNCH(c, KK_FORCE, 0.0, s,
+                  k_band_coefficient<DIM><<<c.batch, 256, 0, s>>>(RK == 0 ? S : c.Tb, c.cs, N, c.kf, inv_n2d, c.eps_inj,
+                                                                  c.band));
+    }
+    using K = Stage<DIM>;
+    const XStage st{c.cs, c.kd, c.kt, prm, c.band, c.nu_b, c.err};
+    const dim3 g((unsigned)((c.nmid * H + XS<DIM> - 1) / XS<DIM>), c.batch);
+    L3ES_LAUNCH(c, KK_X_STAGE, b, s,
+                kx_stage<N, DIM, XS<DIM>, ES<DIM>, RK, INV><<<g, K::THREADS, K::SMEM, s>>>(
+                    c.DU, c.ds, S, c.Tb, c.C, st, c.W, c.Wx, c.fs, c.tw));
+  }
+
+  // One RK4 step in place on S by kx_stage (stage_kernels.cuh). first: the x inverse of S
+  // is not in W yet; last: nothing follows that needs the new state's.
+  template <int DIM>
+  static void step_dim(const Ctx& c, float2* S, const EpiParams* prm, bool first, bool last, cudaStream_t s) {
+    if constexpr (N >= 16 && (DIM == 2 || N <= kStageMax3d)) {
+      if (first) x_stage<DIM, -1, true>(c, S, prm[0], s);
+      nonlinear<DIM>(c, s);
+      x_stage<DIM, 0, true>(c, S, prm[0], s);
+      nonlinear<DIM>(c, s);
+      x_stage<DIM, 1, true>(c, S, prm[1], s);
+      nonlinear<DIM>(c, s);
+      x_stage<DIM, 2, true>(c, S, prm[2], s);
+      nonlinear<DIM>(c, s);
+      if (last)
+        x_stage<DIM, 3, false>(c, S, prm[3], s);
+      else
+        x_stage<DIM, 3, true>(c, S, prm[3], s);
+    }
+  }
+
+  static void step(const Ctx& c, float2* S, const EpiParams* prm, bool first, bool last, cudaStream_t s) {
+    if (c.dim == 3)
+      step_dim<3>(c, S, prm, first, last, s);
+    else
+      step_dim<2>(c, S, prm, first, last, s);
   }
 
   static void stage(const Ctx& c, const float2* us, float2* S, float2* out, int rk, const EpiParams& prm,
@@ -405,6 +488,7 @@ DnsTable make_dns_table() {
   DnsOps<N>::init_attrs();
   DnsTable t;
   t.stage = &DnsOps<N>::stage;
+  t.step = &DnsOps<N>::step;
   t.irfftn = &DnsOps<N>::irfftn;
   t.rfftn = &DnsOps<N>::rfftn;
   t.vjp = &DnsOps<N>::vjp;

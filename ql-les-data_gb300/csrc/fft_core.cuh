@@ -155,19 +155,32 @@ __device__ __forceinline__ int xpad(int n) {
 template <int SS>
 __host__ __device__ constexpr int xpad_len(int n) { return SS == 1 ? n + 8 : n + n / 8; }
 
-template <bool WARP>
+// Scope of an FFT's exchange barriers: the whole CTA, one warp, or one group of
+// consecutive threads of a CTA that runs several FFTs side by side (group g of G threads
+// waits on named barrier 1 + g; G is a multiple of 32).
+constexpr int kSyncCta = 0, kSyncWarp = 1, kSyncGroup = 2;
+
+template <int G>
+__device__ __forceinline__ void group_sync() {
+  static_assert(G % 32 == 0, "named barriers count whole warps");
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / G), "n"(G) : "memory");
+}
+
+template <int SYNC, int G>
 __device__ __forceinline__ void fft_sync() {
-  if (WARP)
+  if constexpr (SYNC == kSyncWarp)
     __syncwarp();
+  else if constexpr (SYNC == kSyncGroup)
+    group_sync<G>();
   else
     __syncthreads();
 }
 
 // One Stockham stage. FIRST: inputs from registers; LAST: outputs to registers.
-// sm: exchange buffer, element n at sm[xpad<SS>(n) * SS]. WARP: all T threads of the
-// FFT are in one warp, so __syncwarp orders the exchanges.
+// sm: exchange buffer, element n at sm[xpad<SS>(n) * SS]. SYNC: the scope of the
+// exchange barriers (kSync*; a group holds the SS T threads of SS interleaved FFTs).
 // CT: tw is the compact table at this stage's offset (tws unused).
-template <int N, int E, int R, int NS, int DIR, int SS, bool WARP, bool FIRST, bool LAST, bool CT = false>
+template <int N, int E, int R, int NS, int DIR, int SS, int SYNC, bool FIRST, bool LAST, bool CT = false>
 __device__ __forceinline__ void stockham_stage(float2 (&v)[E], float2* sm, int t,
                                                const float2* __restrict__ tw, int tws) {
   constexpr int T = N / E;
@@ -181,7 +194,7 @@ __device__ __forceinline__ void stockham_stage(float2 (&v)[E], float2* sm, int t
       x[b][r] = FIRST ? v[b + r * BPT] : sm[xpad<SS, E>(j + r * (N / R)) * SS];
     }
   }
-  if (!FIRST && !LAST) fft_sync<WARP>();  // all reads done before the in-place writes
+  if (!FIRST && !LAST) fft_sync<SYNC, SS * (N / E)>();  // all reads done before the in-place writes
 #pragma unroll
   for (int b = 0; b < BPT; ++b) {
     const int j = t + T * b;
@@ -201,35 +214,35 @@ __device__ __forceinline__ void stockham_stage(float2 (&v)[E], float2* sm, int t
       for (int r = 0; r < R; ++r) sm[xpad<SS, E>(base + r * NS) * SS] = x[b][r];
     }
   }
-  if (!LAST) fft_sync<WARP>();
+  if (!LAST) fft_sync<SYNC, SS * (N / E)>();
 }
 
-template <int N, int E, int DIR, int SS, bool WARP, bool CT, int S, bool DONE = (S >= Sched<N, E>::kStages)>
+template <int N, int E, int DIR, int SS, int SYNC, bool CT, int S, bool DONE = (S >= Sched<N, E>::kStages)>
 struct Stages;
-template <int N, int E, int DIR, int SS, bool WARP, bool CT, int S>
-struct Stages<N, E, DIR, SS, WARP, CT, S, false> {
+template <int N, int E, int DIR, int SS, int SYNC, bool CT, int S>
+struct Stages<N, E, DIR, SS, SYNC, CT, S, false> {
   using Sc = Sched<N, E>;
   static __device__ __forceinline__ void run(float2 (&v)[E], float2* sm, int t,
                                              const float2* __restrict__ tw, int tws) {
-    stockham_stage<N, E, Sc::radix(S), Sc::ns(S), DIR, SS, WARP, S == 0, S == Sc::kStages - 1, CT>(
+    stockham_stage<N, E, Sc::radix(S), Sc::ns(S), DIR, SS, SYNC, S == 0, S == Sc::kStages - 1, CT>(
         v, sm, t, CT ? tw + Sc::ctoff(S) : tw, tws);
-    Stages<N, E, DIR, SS, WARP, CT, S + 1>::run(v, sm, t, tw, tws);
+    Stages<N, E, DIR, SS, SYNC, CT, S + 1>::run(v, sm, t, tw, tws);
   }
 };
-template <int N, int E, int DIR, int SS, bool WARP, bool CT, int S>
-struct Stages<N, E, DIR, SS, WARP, CT, S, true> {
+template <int N, int E, int DIR, int SS, int SYNC, bool CT, int S>
+struct Stages<N, E, DIR, SS, SYNC, CT, S, true> {
   static __device__ __forceinline__ void run(float2 (&)[E], float2*, int, const float2* __restrict__, int) {}
 };
 
-// N-point FFT by T = N/E threads; every thread of the CTA (WARP = false) or of the
-// warp (WARP = true) must call it, since it synchronises between stages. v[e] holds
+// N-point FFT by T = N/E threads; every thread of the CTA, warp or group (SYNC) must
+// call it, since it synchronises between stages. v[e] holds
 // element t + T*e on entry and on exit. tws: stride into the twiddle table (table
 // length / N); with CT, tw is the compact table of the N-point FFT instead. The exchange buffer is free on return only after the caller's next
 // barrier of the same scope.
-template <int N, int E, int DIR, int SS, bool WARP = false, bool CT = false>
+template <int N, int E, int DIR, int SS, int SYNC = kSyncCta, bool CT = false>
 __device__ __forceinline__ void block_fft(float2 (&v)[E], float2* sm, int t,
                                           const float2* __restrict__ tw, int tws) {
-  Stages<N, E, DIR, SS, WARP, CT, 0>::run(v, sm, t, tw, tws);
+  Stages<N, E, DIR, SS, SYNC, CT, 0>::run(v, sm, t, tw, tws);
 }
 
 // N-point FFT whose T = N/E threads sit in one warp (per-line buffers, SS = 1). For
@@ -244,11 +257,11 @@ __device__ __forceinline__ void warp_fft(float2 (&v)[E], float2* sm, int t, cons
   constexpr bool kTail2 = Sc::kStages == 3 && Sc::radix(0) == E && Sc::radix(1) == E && Sc::radix(2) == 2 &&
                           N / E == 2 * E && N / E <= 32;
   if constexpr (!kTail2) {
-    block_fft<N, E, DIR, 1, true, true>(v, sm, t, ct, 0);
+    block_fft<N, E, DIR, 1, kSyncWarp, true>(v, sm, t, ct, 0);
   } else {
     constexpr int T = N / E;
     // stage 0: radix E on the registers, out to shared memory
-    stockham_stage<N, E, E, 1, DIR, 1, true, true, false>(v, sm, t, ct, 0);
+    stockham_stage<N, E, E, 1, DIR, 1, kSyncWarp, true, false>(v, sm, t, ct, 0);
     // stage 1: radix E (Ns = E), one butterfly per thread, outputs stay in registers:
     // slot r holds element (t / E) N/2 + t % E + r E
     {

@@ -10,6 +10,7 @@
 #include "../../include/l3es_gb300.h"
 #include "adjoint_kernels.cuh"
 #include "dns_kernels.cuh"
+#include "stage_kernels.cuh"
 
 namespace l3es {
 
@@ -35,6 +36,7 @@ enum KernelKind {
   KK_ADJ_X_INV,     // kx_inv_adjproj (projected cotangent, x inverse, band terms)
   KK_ADJ_LINE,      // line_cross_adj (both adjoint products)
   KK_ADJ_EPI,       // k_adj_epi (vjp assembly + RK4 reverse recursion)
+  KK_X_STAGE,       // kx_stage (closes an RK stage on the x pencils, opens the next)
   KK_COUNT
 };
 const char* kernel_kind_name(int k);
@@ -157,9 +159,9 @@ struct Ctx {
   float* nu_b = nullptr;       // [batch] viscosity per trajectory
   int* err = nullptr;          // device error word: nonzero after a kernel wait timed out
   int step_form = 2;           // explicit RK4 step (run_steps): 0 per-mode update of the whole
-                               // spectrum, 1 closed-form stages outside the stage region, 2 the
-                               // stage combination fused into the band pass (l3es_plan_set_step_form;
-                               // plans start at 2 in 3D, 1 in 2D)
+                               // spectrum, 1 closed-form stages outside the stage region (3D;
+                               // in 2D as 2), 2 the stage combination inside the x passes
+                               // (l3es_plan_set_step_form; plans start at 2 in 3D, 1 in 2D)
   Schedule sched;              // kernel variants of the step
   int kf = 0;                  // forcing band 0 < |k|^2 <= kf^2
   double eps_inj = 0.0;        // constant-power injection rate
@@ -172,6 +174,9 @@ struct DnsTable {
   // `out`; rk = -1 writes the RHS itself to `out`
   void (*stage)(const Ctx&, const float2* us, float2* S, float2* out, int rk, const EpiParams& prm,
                 cudaStream_t s);
+  // one explicit RK4 step in place on S by kx_stage; prm: the four stages. first / last:
+  // whether the step opens with an x inverse of S / ends without one of the new state
+  void (*step)(const Ctx&, float2* S, const EpiParams* prm, bool first, bool last, cudaStream_t s);
   void (*irfftn)(const Ctx&, const float2* uh, float* u, cudaStream_t s);
   void (*rfftn)(const Ctx&, const float* u, float2* uh, cudaStream_t s);
   // vector-Jacobian product of the RHS at a.us with cotangent a.gscale * a.g, folded

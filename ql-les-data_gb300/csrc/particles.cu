@@ -95,7 +95,7 @@ line_c2c_re(const float2* __restrict__ g, float* __restrict__ gre, long long nli
   float2 v[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) v[e] = __ldg(g + line * NL + t + T * e);
-  block_fft<NL, E, kInv, 1, true>(v, s_x + q * XS, t, tw, 1);
+  block_fft<NL, E, kInv, 1, kSyncWarp>(v, s_x + q * XS, t, tw, 1);
   if (valid) {
 #pragma unroll
     for (int e = 0; e < E; ++e) gre[line * NL + t + T * e] = scale * v[e].x;
@@ -346,7 +346,7 @@ line_fft_real_fwd(const float* __restrict__ x, float2* __restrict__ g, long long
   float2 v[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) v[e] = make_float2(__ldg(x + line * NL + t + T * e), 0.f);
-  block_fft<NL, E, kFwd, 1, true>(v, s_x + q * XS, t, tw, 1);
+  block_fft<NL, E, kFwd, 1, kSyncWarp>(v, s_x + q * XS, t, tw, 1);
   if (valid) {
 #pragma unroll
     for (int e = 0; e < E; ++e) g[line * NL + t + T * e] = v[e];

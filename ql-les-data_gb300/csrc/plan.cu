@@ -33,7 +33,7 @@ const char* kernel_kind_name(int k) {
       "kx_inv_curl", "ky_pass_inv", "line_cross", "ky_pass_fwd", "kx_fwd_band",
       "force_ekin", "kx_inv", "line_c2r", "line_r2c", "kx_fwd", "reduce",
       "filter", "nufft_prep", "nufft_fft", "nufft_gather", "particle_sort", "rk_update",
-      "kx_inv_adjproj", "line_cross_adj", "adj_epilogue"};
+      "kx_inv_adjproj", "line_cross_adj", "adj_epilogue", "kx_stage"};
   return (k >= 0 && k < KK_COUNT) ? names[k] : "";
 }
 
@@ -237,9 +237,7 @@ int l3es_plan_create(const l3es_plan_desc* desc, l3es_plan** out) {
   c.kd = dealias_kd(n);
   c.kt = ((c.kd + 1 + TW - 1) / TW) * TW;
   if (n == 256) c.sched.line_pair = 3;  // the staged radix-16 line pass (measured best at 256)
-  // the band-fused step in 3D; a 2D band pass has one CTA per 8 half-axis columns (11 at
-  // 256^2), too few to hide its epilogue's loads (2D Kolmogorov 256^2 with particles:
-  // 104.5 us per step fused, 101.4 us with the elementwise update)
+  // the stage combination inside the x passes (in 2D forms 1 and 2 both are kx_stage)
   c.step_form = dim == 3 ? 2 : 1;
   c.nmid = dim == 3 ? n : 1;
   c.cs = c.nmid * n * c.h;
@@ -494,9 +492,11 @@ static void tune_cache_write(const char* path, const std::string& key, const int
   std::fclose(f);
 }
 
-// The four stages of one RK4 step of the state S in the plan's step form
-// (spectral_solver.py:65-80; the forcing rescale of ekin_tot follows in run_steps).
-static void rk4_stages(l3es_plan* plan, float2* S, cudaStream_t s) {
+// One RK4 step of the state S in the plan's step form (spectral_solver.py:65-80; the
+// forcing rescale of ekin_tot follows each step in run_steps). first / last: whether the
+// x inverse of S has to be made, and whether the one of the new state is left out; the
+// forms with an elementwise update do neither.
+static void rk4_step(l3es_plan* plan, float2* S, bool first, bool last, cudaStream_t s) {
   const Ctx& c = plan->ctx;
   const l3es_plan_desc& d = plan->desc;
   static const double a_rk4[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
@@ -506,40 +506,46 @@ static void rk4_stages(l3es_plan* plan, float2* S, cudaStream_t s) {
   const int kf_band = d.forcing == L3ES_FORCING_CONST_POWER ? d.kf : 0;
   const int lin_ok = c.step_form >= 1 && d.scheme != L3ES_SCHEME_INTEGRATING_FACTOR && kf_band <= c.kd &&
                      kf_band < c.kt && (d.kolm_k <= 0 || d.kolm_k < c.kt);
-  // the band-fused form: the band pass combines the stages on the band in place in S,
-  // the x inverse applies the closed form to every other mode; its accumulator lives in
-  // C in the band's compact layout (kt <= N/2 + 1, i.e. N >= 16, keeps that inside C)
-  const int band_rk = lin_ok && c.step_form >= 2 && c.kt <= c.h;
+  // the stage combination inside the x passes (form 2; in 2D, where the elementwise update
+  // is one launch of four per stage, form 1 as well); the band has to lie inside the half
+  // axis (kt <= N/2 + 1, i.e. N >= 16)
+  const bool band = lin_ok && c.step_form >= (c.dim == 3 ? 2 : 1) && c.kt <= c.h;
+  const bool one_visit = band && step_by_kx_stage(c.dim, c.n, c.batch);
+  EpiParams prm[4];
   for (int rk = 0; rk < 4; ++rk) {
-    EpiParams prm;
-    prm.a_dt = (float)(a_rk4[rk] * d.dt);
-    prm.b_dt = rk < 3 ? (float)(b_rk4[rk] * d.dt) : 0.f;
-    prm.nu = (float)d.nu;
-    prm.drag = (float)d.drag;
-    prm.kolm_amp = (float)d.kolm_amp;
-    prm.kolm_k = d.kolm_k;
-    prm.band_kf2 = d.forcing == L3ES_FORCING_CONST_POWER ? d.kf * d.kf : 0;
-    prm.rk = rk;
-    prm.if_h = d.scheme == L3ES_SCHEME_INTEGRATING_FACTOR ? (float)d.dt : 0.f;
-    prm.dt = (float)d.dt;
-    prm.lin = lin_ok;
-    prm.band_rk = band_rk;
-    if (band_rk)
-      plan->tab.stage(c, S, S, S, rk, prm, s);
-    else
-      plan->tab.stage(c, rk == 0 ? S : c.Tb, S, c.Tb, rk, prm, s);
+    EpiParams& q = prm[rk];
+    q.a_dt = (float)(a_rk4[rk] * d.dt);
+    q.b_dt = rk < 3 ? (float)(b_rk4[rk] * d.dt) : 0.f;
+    q.nu = (float)d.nu;
+    q.drag = (float)d.drag;
+    q.kolm_amp = (float)d.kolm_amp;
+    q.kolm_k = d.kolm_k;
+    q.band_kf2 = d.forcing == L3ES_FORCING_CONST_POWER ? d.kf * d.kf : 0;
+    q.rk = rk;
+    q.if_h = d.scheme == L3ES_SCHEME_INTEGRATING_FACTOR ? (float)d.dt : 0.f;
+    q.dt = (float)d.dt;
+    q.lin = lin_ok;
+    q.band_rk = band;
   }
+  if (one_visit) {
+    plan->tab.step(c, S, prm, first, last, s);
+    return;
+  }
+  // the band-fused stages (XLin, BandRk) work in place, the accumulator in C in the band's
+  // compact layout; the elementwise update keeps its stage field in T
+  for (int rk = 0; rk < 4; ++rk)
+    plan->tab.stage(c, band || rk == 0 ? S : c.Tb, S, band ? S : c.Tb, rk, prm[rk], s);
 }
 
 // mean milliseconds of one RK4 step in the plan's step form with its current schedule,
-// on the zeroed stage scratch T as the state (timing only: the explicit forms then alias
-// their stage field with the state; zeros stay finite through every term)
+// on the zeroed stage scratch T as the state (timing only: the steps then alias their
+// stage field with the state; zeros stay finite through every term)
 static float time_step(l3es_plan* p, cudaStream_t s, cudaEvent_t e0, cudaEvent_t e1) {
   const Ctx& c = p->ctx;
-  rk4_stages(p, c.Tb, s);
+  rk4_step(p, c.Tb, true, true, s);
   const int reps = c.cs * c.batch > (1 << 20) ? 2 : 5;
   cudaEventRecord(e0, s);
-  for (int i = 0; i < reps; ++i) rk4_stages(p, c.Tb, s);
+  for (int i = 0; i < reps; ++i) rk4_step(p, c.Tb, true, true, s);
   cudaEventRecord(e1, s);
   cudaEventSynchronize(e1);
   float ms = 0.f;
@@ -632,7 +638,9 @@ static int run_steps(l3es_plan* plan, void* u_hat, float* u_out, int32_t nsteps,
   const double inv_n2d = 1.0 / std::pow((double)c.n, 2 * c.dim);
   const double eps64 = 2.220446049250313e-16;  // jnp.finfo(float).eps, spectral_solver.py:23
   for (int st = 0; st < nsteps; ++st) {
-    rk4_stages(plan, S, s);
+    // the ekin_tot rescale changes the new state, so its x inverse cannot be part of the step
+    const bool apart = d.forcing == L3ES_FORCING_EKIN_TOT;
+    rk4_step(plan, S, st == 0 || apart, st == nsteps - 1 || apart, s);
     double* einj = e_inj_dev ? e_inj_dev + (long long)st * c.batch : c.einj;
     double* ke_final = (ke_dev && st == nsteps - 1) ? ke_dev : nullptr;
     // energy partials of the new state by the row-wise float-float pass (a separate

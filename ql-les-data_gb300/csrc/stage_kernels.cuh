@@ -1,0 +1,236 @@
+// The x pass of the explicit RK4 step for sm_103a: one kernel closes a stage and opens
+// the next one.
+//
+// On an x pencil (fixed middle and half-axis wavenumbers) the forward x FFT of the
+// nonlinear term, the dealias mask, the Leray projection, the RK4 stage combination and
+// the next stage's inverse x FFT of u and curl u all act on the same column of modes, so
+// kx_stage does them in one visit: the new stage field goes from the combination into
+// the inverse transform without a trip through memory, and a stage is two launches in 2D
+// (kx_stage, line pass) and four in 3D (kx_stage, y inverse, line pass, y forward).
+//
+// The band B = {|kx| <= kd, |kmid| <= kd (3D), khalf < kt} holds every nonlinear and
+// forcing term. Outside it du = -(nu k^2 + drag) u exactly, so a stage field there is a
+// polynomial in z = (nu k^2 + drag) dt times the step's initial value (lin_stage_factor):
+// those modes keep u0 in the state S until stage 2 replaces them by their new state, and
+// are read and scaled on the way into each inverse transform. On the band, S keeps u0
+// until stage 3 writes the new state, T holds the stage field and C the accumulator, all
+// in S's layout.
+#pragma once
+
+#include "dns_kernels.cuh"
+
+namespace l3es {
+
+// Where the explicit step takes kx_stage: every 2D grid, 3D grids below 64^3, and 64^3 up
+// to a batch of 4. There the passes are latency: few CTAs, each a chain of dependent
+// transforms, and the launches count. Measured per step against the separate passes:
+// 2D 256^2 98.3 -> 69.7 us, 128^2 x 8 98.4 -> 70.6 us, 512^2 122.9 -> 97.7 us, 3D 32^3
+// 120.9 -> 90.5 us, 64^3 132.1 -> 107.1 us, 64^3 x 3 172 -> 157 us. Once the chip is full
+// the three groups' barriers and the thread count (one or two CTAs per SM) cost more than
+// the saved round trip: 64^3 x 6 263 -> 281 us, 128^3 (one stage's x passes) 32.6 -> 38 us,
+// 256^3 195 -> 267 us. Larger 3D grids keep kx_inv and the band-fused kx_fwd_band.
+constexpr int kStageMax3d = 64;  // largest 3D grid with kx_stage kernels
+constexpr int kBandMin3d = 64;   // smallest 3D grid with band-fused kernels
+inline bool step_by_kx_stage(int dim, int n, int batch) {
+  return dim == 2 || n < kBandMin3d || (n <= kStageMax3d && batch <= 4);
+}
+
+// Parameters of one stage.
+struct XStage {
+  long long cs;
+  int kd, kt;
+  EpiParams prm;             // prm.rk is the kernel's RK
+  const double* band_scale;  // [batch] constant-power coefficient of the stage's input field
+  const float* nu_b;         // [batch] viscosities
+  int* err;
+};
+
+// XW columns per CTA and one thread group per velocity component, XW T threads each
+// (thread = (component g, x row t, column p), p fastest). A group transforms its own
+// component; the two contractions that mix components (projection, curl) read the other
+// two from shared memory. Against one group that walks through the components, the CTA
+// has three times the threads and a third of the registers per thread, and the chain of
+// dependent transforms is 3 instead of 8 (3D) or 9 (2D).
+template <int N, int XW, int EE>
+struct XStageCfg {
+  static constexpr int E = EE, T = N / E;
+  static constexpr int G = XW * T;                       // threads per component
+  static constexpr int THREADS = 3 * G;
+  static constexpr int SYNC = G % 32 == 0 ? kSyncGroup : kSyncCta;
+  static constexpr int XS = xpad_len<XW>(N) * XW;        // exchange slots per component
+  static constexpr int US = N * XW;                      // shared column values per component
+  static constexpr int SMEM = 3 * (XS + US) * (int)sizeof(float2);
+};
+
+// S: the state, T_: stage field, C: accumulator, [batch][3][cs] each.
+// RK = -1: opens a step: inverse transforms of S as it is. RK = 0..3: closes stage RK
+// from the y-transformed nonlinear term du; INV: also opens the next stage (RK < 3) or
+// the next step (RK = 3), else only the band of S is written.
+// 3D: u_x, curl_y, curl_z go to w (fields 0, 4, 5) and u_y, u_z to wx, as ky_inv_rhs
+// reads them; 2D: six fields to w.
+template <int N, int DIM, int XW, int EE, int RK, bool INV>
+__global__ void __launch_bounds__(XStageCfg<N, XW, EE>::THREADS)
+kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, float2* __restrict__ T_,
+         float2* __restrict__ C, const __grid_constant__ XStage st, float2* __restrict__ w, float2* __restrict__ wx,
+         long long fs, const float2* __restrict__ tw) {
+  using K = XStageCfg<N, XW, EE>;
+  constexpr int E = K::E, T = K::T, H = N / 2 + 1;
+  constexpr int NMID = DIM == 3 ? N : 1;
+  constexpr int MC = NMID * H;
+  extern __shared__ __align__(16) float2 s_stage[];
+  const int g = threadIdx.x / K::G, q = threadIdx.x % K::G;
+  const int p = q % XW, t = q / XW;
+  float2* su = s_stage;                           // [component][row][column]
+  float2* sx = s_stage + 3 * K::US + g * K::XS;   // this component's exchange buffer
+  const int m = blockIdx.x * XW + p;
+  const int batch = blockIdx.y;
+  const bool ok = m < MC;
+  const int mid = DIM == 3 ? m / H : 0;
+  const int kh = m - mid * H;
+  const int km = DIM == 3 ? kfull(mid, N) : 0;
+  const int kd = st.kd, kt = st.kt;
+  const unsigned ukd = 2u * (unsigned)kd;
+  const bool colband = RK >= 0 && ok && kh < kt && (DIM == 2 || (unsigned)(km + kd) <= ukd);
+  const long long so = ((long long)batch * 3 + g) * st.cs + m;  // + row * MC
+  const float nu = st.nu_b[batch];
+  float2 v[E];
+  if (RK >= 0) {
+    const bool tile_band = __syncthreads_or(colband);
+    if (!INV && !tile_band) return;
+    if (tile_band) {
+      // nonlinear term: x forward, dealias, Leray projection of this component
+      const float2* db = du + ((long long)batch * 3 + g) * dcs + (long long)mid * kt + kh;
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        v[e] = colband ? __ldg(db + (long long)(t + T * e) * NMID * kt) : make_float2(0.f, 0.f);
+      block_fft<N, E, kFwd, XW, K::SYNC>(v, sx + p, t, tw, 1);
+#pragma unroll
+      for (int e = 0; e < E; ++e) su[g * K::US + (t + T * e) * XW + p] = v[e];
+      __syncthreads();
+      const bool keep = kh <= kd;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int row = t + T * e;
+        const float2 z = make_float2(0.f, 0.f);
+        const float2 v0 = keep ? su[row * XW + p] : z;
+        const float2 v1 = keep ? su[K::US + row * XW + p] : z;
+        const float2 v2 = keep ? su[2 * K::US + row * XW + p] : z;
+        float k0, k1, k2;
+        const int kx = kfull(row, N);
+        kvec<DIM>(kx, km, kh, k0, k1, k2);
+        const int ik2 = kx * kx + km * km + kh * kh;
+        const float inv = 1.0f / (ik2 == 0 ? 1.0f : (float)ik2);
+        const float pr = (v0.x * k0 + v1.x * k1 + v2.x * k2) * inv;
+        const float pi_ = (v0.y * k0 + v1.y * k1 + v2.y * k2) * inv;
+        const float2 own = g == 0 ? v0 : g == 1 ? v1 : v2;
+        const float kg = g == 0 ? k0 : g == 1 ? k1 : k2;
+        v[e] = make_float2(own.x - pr * kg, own.y - pi_ * kg);
+      }
+      if (INV) __syncthreads();  // the products are read; su takes the new stage field
+    }
+  }
+  // stage combination on the band, closed form elsewhere: v becomes this component's
+  // field. Operands of four modes are loaded before the first of them is stored.
+  if constexpr (RK < 0) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = ok ? S[so + (long long)(t + T * e) * MC] : make_float2(0.f, 0.f);
+  } else {
+    EpiParams prm = st.prm;
+    prm.rk = RK;
+    prm.nu = nu;
+    const float fscale = prm.band_kf2 > 0 ? (float)st.band_scale[batch] : 0.f;
+    bool bad = false;
+    constexpr int CH = E < 4 ? E : 4;
+#pragma unroll
+    for (int e0 = 0; e0 < E; e0 += CH) {
+      float2 u0[CH], sv[CH], ac[CH];
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const int row = t + T * (e0 + i);
+        const bool band = colband && (unsigned)(kfull(row, N) + kd) <= ukd;
+        const long long o = so + (long long)row * MC;
+        const float2 z = make_float2(0.f, 0.f);
+        u0[i] = (band ? RK < 3 : INV && ok) ? S[o] : z;
+        sv[i] = RK > 0 && band ? T_[o] : z;
+        ac[i] = RK > 1 && band ? C[o] : z;
+      }
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const int e = e0 + i, row = t + T * e;
+        const int kx = kfull(row, N);
+        const long long o = so + (long long)row * MC;
+        const int ik2 = kx * kx + km * km + kh * kh;
+        float2 nv;
+        if (colband && (unsigned)(kx + kd) <= ukd) {
+          const float2 ra = rk_core_r<N, DIM, false>(row, mid, kh, ik2, g, v[e], RK == 0 ? u0[i] : sv[i], ac[i], u0[i],
+                                                     prm, fscale, nv);
+          if (RK == 1 || RK == 2) C[o] = ra;
+          if (RK == 3)
+            S[o] = nv;
+          else
+            T_[o] = nv;
+          if (RK == 3) bad |= !isfinite(nv.x + nv.y);
+          v[e] = nv;
+        } else if (RK == 3) {
+          v[e] = u0[i];  // the new state, written by stage 2
+        } else {
+          const float z = (nu * (float)ik2 + prm.drag) * prm.dt;
+          const float f = lin_stage_factor(RK, z);
+          if (RK == 2 && ok) {
+            const float gn = lin_stage_factor(3, z);
+            nv = make_float2(gn * u0[i].x, gn * u0[i].y);
+            S[o] = nv;
+            bad |= !isfinite(nv.x + nv.y);
+          }
+          v[e] = make_float2(f * u0[i].x, f * u0[i].y);
+        }
+      }
+    }
+    if (RK >= 2 && bad) atomicOr(st.err, kErrNonFinite);
+  }
+  if constexpr (INV) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) su[g * K::US + (t + T * e) * XW + p] = v[e];
+    __syncthreads();
+    block_fft<N, E, kInv, XW, K::SYNC>(v, sx + p, t, tw, 1);
+    if (ok) {
+      float2* dst = DIM == 3 && g > 0 ? wx + ((long long)batch * 2 + g - 1) * fs : w + ((long long)batch * 6 + g) * fs;
+#pragma unroll
+      for (int e = 0; e < E; ++e) dst[(long long)(t + T * e) * MC + m] = v[e];
+    }
+    // curl component g = i (k x u)_g; in 3D the y pass forms the x component itself
+    if (DIM == 3 && g == 0 && K::SYNC == kSyncGroup) return;
+    const int ga = g == 2 ? 0 : g + 1, gb = g == 0 ? 2 : g - 1;  // (k x u)_g = k_ga u_gb - k_gb u_ga
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int row = t + T * e;
+      float k0, k1, k2;
+      kvec<DIM>(kfull(row, N), km, kh, k0, k1, k2);
+      const float ka = g == 0 ? k1 : g == 1 ? k2 : k0, kb = g == 0 ? k2 : g == 1 ? k0 : k1;
+      const float2 ua = su[ga * K::US + row * XW + p], ub = su[gb * K::US + row * XW + p];
+      v[e] = mul_i<kInv>(make_float2(ka * ub.x - kb * ua.x, ka * ub.y - kb * ua.y));
+    }
+    if constexpr (K::SYNC == kSyncGroup)
+      group_sync<K::G>();  // the exchange buffer's last reads are done
+    else
+      __syncthreads();
+    block_fft<N, E, kInv, XW, K::SYNC>(v, sx + p, t, tw, 1);
+    if (ok && !(DIM == 3 && g == 0)) {
+      float2* dst = w + ((long long)batch * 6 + 3 + g) * fs;
+#pragma unroll
+      for (int e = 0; e < E; ++e) dst[(long long)(t + T * e) * MC + m] = v[e];
+    }
+  }
+}
+
+// Constant-power coefficient of a stage field (one CTA per trajectory): the low modes of
+// S (stage 0) or T.
+template <int DIM>
+__global__ void __launch_bounds__(256)
+k_band_coefficient(const float2* __restrict__ us, long long cs, int N, int kf, double inv_n2d, double eps_inj,
+                   double* __restrict__ band_scale) {
+  band_coefficient<DIM>(us + (long long)blockIdx.x * 3 * cs, cs, N, kf, inv_n2d, eps_inj, 1e-30,
+                        band_scale + blockIdx.x);
+}
+
+}  // namespace l3es
