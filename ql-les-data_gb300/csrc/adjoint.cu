@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(256)
 k_ekin_adj_coef(const float2* __restrict__ urk, const float2* __restrict__ lam, long long cs,
                 const double* __restrict__ partial, int npartial, const double* __restrict__ e0, int N, int kf,
                 double inv_n2d, double eps, double* __restrict__ coef) {
+  pdl_begin();
   const int batch = blockIdx.x;
   const float2* ub = urk + (long long)batch * 3 * cs;
   const float2* lb = lam + (long long)batch * 3 * cs;
@@ -87,6 +88,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256)
 k_ekin_adj_apply(float2* __restrict__ lam, const float2* __restrict__ urk, long long cs, int N, int kf,
                  const double* __restrict__ coef) {
+  pdl_begin();
   const int batch = blockIdx.y;
   const long long pairs = 3 * cs / 2;
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -250,13 +252,15 @@ int l3es_adjoint_step(l3es_plan* plan, const void* u_hat_n, void* lam, void* str
     const long long pairs = 3 * c.cs / 2;
     const dim3 eb((unsigned)((pairs + 255) / 256), c.batch);
     if (c.dim == 3) {
-      k_ekin_adj_coef<3><<<c.batch, 256, 0, s>>>(w.Wm, L1, c.cs, c.partial, nke, c.e0, c.n, d.kf, inv_n2d, eps64,
+      pdl_launch(k_ekin_adj_coef<3>, c.batch, 256, 0, s, w.Wm, L1, c.cs, c.partial, nke, c.e0, c.n, d.kf, inv_n2d,
+                 eps64,
                                                  w.ekin);
-      k_ekin_adj_apply<3><<<eb, 256, 0, s>>>(L1, w.Wm, c.cs, c.n, d.kf, w.ekin);
+      pdl_launch(k_ekin_adj_apply<3>, eb, 256, 0, s, L1, w.Wm, c.cs, c.n, d.kf, w.ekin);
     } else {
-      k_ekin_adj_coef<2><<<c.batch, 256, 0, s>>>(w.Wm, L1, c.cs, c.partial, nke, c.e0, c.n, d.kf, inv_n2d, eps64,
+      pdl_launch(k_ekin_adj_coef<2>, c.batch, 256, 0, s, w.Wm, L1, c.cs, c.partial, nke, c.e0, c.n, d.kf, inv_n2d,
+                 eps64,
                                                  w.ekin);
-      k_ekin_adj_apply<2><<<eb, 256, 0, s>>>(L1, w.Wm, c.cs, c.n, d.kf, w.ekin);
+      pdl_launch(k_ekin_adj_apply<2>, eb, 256, 0, s, L1, w.Wm, c.cs, c.n, d.kf, w.ekin);
     }
   }
   const float dt = (float)d.dt;

@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(TW * Fft<N>::T)
 kx_inv_adjproj(const float2* __restrict__ g, long long cs, float gscale, int kd, float2* __restrict__ w,
                long long fs, const float2* __restrict__ tw, const float2* __restrict__ us, int band_kf,
                double inv_n2d, double eps_inj, double* __restrict__ band_out) {
+  pdl_begin();
   constexpr int E = Fft<N>::E, T = Fft<N>::T, H = N / 2 + 1;
   constexpr int NMID = DIM == 3 ? N : 1;
   constexpr int MC = NMID * H;
@@ -138,6 +139,7 @@ template <int N>
 __global__ void __launch_bounds__(LineCfg<N>::THREADS, 3)
 line_cross_adj(const float2* __restrict__ wm, const float2* __restrict__ wuw, long long fs,
                float2* __restrict__ out, long long cs, float scale, const float2* __restrict__ twN, int nlines) {
+  pdl_begin();
   using C = LineCfg<N>;
   constexpr int M = C::M, H = N / 2 + 1, E = C::E, T = C::T, LPC = C::LPC;
   __shared__ float2 s_x[LPC * C::XS];
@@ -245,6 +247,7 @@ struct AdjEpi {
 template <int N, int DIM>
 __global__ void __launch_bounds__(256)
 k_adj_epi(const float2* __restrict__ y, long long cs, AdjEpi a, const float* __restrict__ nu_b) {
+  pdl_begin();
   constexpr unsigned H = N / 2 + 1;
   constexpr unsigned NMID = DIM == 3 ? N : 1;
   const int batch = blockIdx.y;

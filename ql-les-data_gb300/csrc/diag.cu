@@ -17,6 +17,7 @@ namespace l3es {
 // per block: max |u_c| for c = 0..2 and sum_c u_c^2, over ps values per component
 __global__ void __launch_bounds__(256)
 k_field_stats(const float* __restrict__ u, long long ps, int nblk, double* __restrict__ partial) {
+  pdl_begin();
   const int batch = blockIdx.y;
   const float* ub = u + (long long)batch * 3 * ps;
   float mx[3] = {0.f, 0.f, 0.f};
@@ -62,6 +63,7 @@ k_field_stats(const float* __restrict__ u, long long ps, int nblk, double* __res
 // out[batch*4 + {0,1,2}] = max |u_c|, out[batch*4 + 3] = 0.5 mean sum u^2
 __global__ void k_field_stats_final(const double* __restrict__ partial, int nblk, double inv_ps,
                                     double* __restrict__ out) {
+  pdl_begin();
   const int batch = blockIdx.x;
   if (threadIdx.x != 0) return;
   double m[3] = {0.0, 0.0, 0.0}, s = 0.0;
@@ -99,6 +101,7 @@ __device__ __forceinline__ void curl_at(const float2* __restrict__ ub, long long
 template <int DIM>
 __global__ void __launch_bounds__(256)
 k_diss_partial(const float2* __restrict__ uh, long long cs, int n, int nblk, double* __restrict__ partial) {
+  pdl_begin();
   const int batch = blockIdx.y;
   const float2* ub = uh + (long long)batch * 3 * cs;
   const int h = n / 2 + 1;
@@ -135,6 +138,7 @@ k_diss_partial(const float2* __restrict__ uh, long long cs, int n, int nblk, dou
 template <int DIM>
 __global__ void __launch_bounds__(256)
 k_spectrum(const float2* __restrict__ uh, long long cs, int n, int nblk, double scale, double* __restrict__ acc) {
+  pdl_begin();
   extern __shared__ double hist[];  // [2][n]
   const int batch = blockIdx.y;
   for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) hist[i] = 0.0;
@@ -175,6 +179,7 @@ k_spectrum(const float2* __restrict__ uh, long long cs, int n, int nblk, double 
 // sum of n partials per trajectory times scale
 __global__ void __launch_bounds__(256)
 k_diag_sum(const double* __restrict__ partial, int n, double scale, double* __restrict__ out) {
+  pdl_begin();
   __shared__ double red[32];
   const int batch = blockIdx.x;
   double s = 0.0;
@@ -190,6 +195,7 @@ k_diag_sum(const double* __restrict__ partial, int n, double scale, double* __re
 }
 
 __global__ void k_spectrum_final(const double* __restrict__ acc, int n, double eps, double* __restrict__ ek) {
+  pdl_begin();
   const int batch = blockIdx.y;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
@@ -210,9 +216,9 @@ int l3es_field_stats(l3es_plan* plan, const float* u, double* out_dev, void* str
   cudaStream_t s = (cudaStream_t)stream;
   const int nblk = (int)std::min<long long>(608, (c.ps + 255) / 256);
   L3ES_LAUNCH(c, KK_REDUCE, 4.0 * 3.0 * c.ps * c.batch, s,
-              k_field_stats<<<dim3(nblk, c.batch), 256, 0, s>>>(u, c.ps, nblk, c.partial));
+              pdl_launch(k_field_stats, dim3(nblk, c.batch), 256, 0, s, u, c.ps, nblk, c.partial));
   L3ES_LAUNCH(c, KK_REDUCE, 0.0, s,
-              k_field_stats_final<<<c.batch, 32, 0, s>>>(c.partial, nblk, 1.0 / (double)c.ps, out_dev));
+              pdl_launch(k_field_stats_final, c.batch, 32, 0, s, c.partial, nblk, 1.0 / (double)c.ps, out_dev));
   return cuda_check(cudaGetLastError(), "l3es_field_stats launch");
 }
 
@@ -224,13 +230,13 @@ int l3es_dissipation(l3es_plan* plan, const void* u_hat, double nu, double* out_
   const double scale = nu / std::pow((double)c.n, 2 * c.dim);
   if (c.dim == 3)
     L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
-                k_diss_partial<3><<<dim3(nblk, c.batch), 256, 0, s>>>((const float2*)u_hat, c.cs, c.n, nblk,
+                pdl_launch(k_diss_partial<3>, dim3(nblk, c.batch), 256, 0, s, (const float2*)u_hat, c.cs, c.n, nblk,
                                                                      c.partial));
   else
     L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
-                k_diss_partial<2><<<dim3(nblk, c.batch), 256, 0, s>>>((const float2*)u_hat, c.cs, c.n, nblk,
+                pdl_launch(k_diss_partial<2>, dim3(nblk, c.batch), 256, 0, s, (const float2*)u_hat, c.cs, c.n, nblk,
                                                                      c.partial));
-  L3ES_LAUNCH(c, KK_REDUCE, 0.0, s, k_diag_sum<<<c.batch, 256, 0, s>>>(c.partial, nblk, scale, out_dev));
+  L3ES_LAUNCH(c, KK_REDUCE, 0.0, s, pdl_launch(k_diag_sum, c.batch, 256, 0, s, c.partial, nblk, scale, out_dev));
   return cuda_check(cudaGetLastError(), "l3es_dissipation launch");
 }
 
@@ -247,14 +253,15 @@ int l3es_energy_spectrum(l3es_plan* plan, const void* u_hat, double mul_fac, dou
   const size_t smem = sizeof(double) * 2 * n;
   if (c.dim == 3)
     L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
-                k_spectrum<3><<<dim3(nblk, c.batch), 256, smem, s>>>((const float2*)u_hat, c.cs, n, nblk, scale,
+                pdl_launch(k_spectrum<3>, dim3(nblk, c.batch), 256, smem, s, (const float2*)u_hat, c.cs, n, nblk, scale,
                                                                     c.partial));
   else
     L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
-                k_spectrum<2><<<dim3(nblk, c.batch), 256, smem, s>>>((const float2*)u_hat, c.cs, n, nblk, scale,
+                pdl_launch(k_spectrum<2>, dim3(nblk, c.batch), 256, smem, s, (const float2*)u_hat, c.cs, n, nblk, scale,
                                                                     c.partial));
   L3ES_LAUNCH(c, KK_REDUCE, 0.0, s,
-              k_spectrum_final<<<dim3((n + 127) / 128, c.batch), 128, 0, s>>>(c.partial, n, 2.220446049250313e-16,
+              pdl_launch(k_spectrum_final, dim3((n + 127) / 128, c.batch), 128, 0, s, c.partial, n,
+                         2.220446049250313e-16,
                                                                               ek_dev));
   return cuda_check(cudaGetLastError(), "l3es_energy_spectrum launch");
 }

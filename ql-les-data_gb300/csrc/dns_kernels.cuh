@@ -25,6 +25,7 @@
 #pragma once
 
 #include "fft_core.cuh"
+#include "pdl.cuh"
 #include "tma.cuh"
 
 namespace l3es {
@@ -211,6 +212,7 @@ __global__ void __launch_bounds__(XW * Fft<N>::T)
 kx_inv(const float2* __restrict__ uh, long long cs, float2* __restrict__ w, long long fs,
        const float2* __restrict__ tw, float2* __restrict__ wx = nullptr, XLin xl = XLin{},
        int* __restrict__ err = nullptr) {
+  pdl_begin();
   constexpr int E = Fft<N>::E, T = Fft<N>::T, H = N / 2 + 1;
   constexpr int NMID = DIM == 3 ? N : 1;
   constexpr int MC = NMID * H;
@@ -258,6 +260,7 @@ __global__ void __launch_bounds__(TW * Fft<N>::T, TW * Fft<N>::T >= 512 ? 1 : 2)
 kx_inv_tma(const __grid_constant__ CUtensorMap umap, float2* __restrict__ w, long long fs,
            const float2* __restrict__ tw, int ntiles, int* __restrict__ err, float2* __restrict__ wx,
            const __grid_constant__ XLin xl) {
+  pdl_begin();
   using K = KxTma<N>;
   constexpr int E = Fft<N>::E, T = Fft<N>::T;
   constexpr int NF = CURL ? 6 : 3;
@@ -329,6 +332,7 @@ template <int N, int DIR, int V = 0>
 __global__ void __launch_bounds__(KyCfg<N, V>::THREADS)
 ky_pass(float2* __restrict__ w, long long fs, int row, int ncols, int kd_store,
         const float2* __restrict__ tw) {
+  pdl_begin();
   using C = KyCfg<N, V>;
   constexpr int E = C::E, T = C::T, TWY = C::TWY;
   __shared__ float2 sm[xpad_len<TWY>(N) * TWY];
@@ -362,6 +366,7 @@ ky_pass(float2* __restrict__ w, long long fs, int row, int ncols, int kd_store,
 template <int N, int V = 0>
 __global__ void __launch_bounds__(KyCfg<N, V>::THREADS)
 ky_inv_rhs(float2* __restrict__ w, const float2* __restrict__ wx, long long fs, const float2* __restrict__ tw) {
+  pdl_begin();
   using C = KyCfg<N, V>;
   constexpr int E = C::E, T = C::T, TWY = C::TWY, H = N / 2 + 1;
   __shared__ float2 sm[xpad_len<TWY>(N) * TWY];
@@ -496,6 +501,7 @@ template <int N>
 __global__ void __launch_bounds__(LineCfg<N>::THREADS, N <= 256 ? 4 : 3)
 line_cross(const float2* __restrict__ w, long long fs, float2* __restrict__ du, long long ds,
            int kt, int kd, float scale, const float2* __restrict__ twN, int nlines) {
+  pdl_begin();
   using C = LineCfg<N>;
   constexpr int M = C::M, H = N / 2 + 1, E = C::E, T = C::T, LPC = C::LPC;
   __shared__ float2 s_x[LPC * C::XS];
@@ -676,6 +682,7 @@ template <int N>
 __global__ void __launch_bounds__(Line2Cfg<N>::THREADS, 4)
 line_cross2(const float2* __restrict__ w, long long fs, float2* __restrict__ du, long long ds, int kt, int kd,
             float s2, const float2* __restrict__ ct, int nlines) {
+  pdl_begin();
   static_assert(N >= 64 && N <= 256, "two-for-one line pass: N in [64, 256]");
   using C = Line2Cfg<N>;
   constexpr int T = C::T, H = N / 2 + 1;
@@ -873,6 +880,7 @@ template <int N, bool STAGED>
 __global__ void __launch_bounds__(Line3Cfg<N>::THREADS, 3)
 line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du, long long ds, int kt, int kd,
             float s2, const float2* __restrict__ ct8, const float2* __restrict__ ct16, int nlines, int* err) {
+  pdl_begin();
   static_assert(N == 256, "radix-16 line pass: N = 256");
   using C = Line3Cfg<N>;
   constexpr int E = C::E, H = N / 2 + 1;
@@ -1023,6 +1031,7 @@ template <int N>
 __global__ void __launch_bounds__(LineCfg<N>::THREADS)
 line_c2r(const float2* __restrict__ w, long long fs, float* __restrict__ out, long long os,
          float scale, const float2* __restrict__ twN, int nlines) {
+  pdl_begin();
   using C = LineCfg<N>;
   constexpr int M = C::M, H = N / 2 + 1, E = C::E, T = C::T, LPC = C::LPC;
   __shared__ float2 s_x[LPC * C::XS];
@@ -1054,6 +1063,7 @@ template <int N>
 __global__ void __launch_bounds__(LineCfg<N>::THREADS)
 line_r2c(const float* __restrict__ in, long long is, float2* __restrict__ w, long long fs,
          const float2* __restrict__ twN, int nlines) {
+  pdl_begin();
   using C = LineCfg<N>;
   constexpr int M = C::M, H = N / 2 + 1, E = C::E, T = C::T, LPC = C::LPC;
   __shared__ float2 s_x[LPC * C::XS];
@@ -1089,6 +1099,7 @@ template <int N, int DIM>
 __global__ void __launch_bounds__(TW * Fft<N>::T)
 kx_fwd_plain(const float2* __restrict__ w, long long fs, float2* __restrict__ uh, long long cs,
              const float2* __restrict__ tw) {
+  pdl_begin();
   constexpr int E = Fft<N>::E, T = Fft<N>::T, H = N / 2 + 1;
   constexpr int NMID = DIM == 3 ? N : 1;
   constexpr int MC = NMID * H;
@@ -1446,6 +1457,7 @@ __global__ void __launch_bounds__(XW * Fft<N>::T)
 kx_fwd_band(const float2* __restrict__ du, long long dcs, int kt, int kd, float2* __restrict__ P, long long pcs,
             const float2* __restrict__ tw, const float2* __restrict__ us, long long cs, int band_kf,
             double inv_n2d, double eps_inj, double* __restrict__ band_scale, const BandRk br = BandRk{}) {
+  pdl_begin();
   constexpr int E = Fft<N>::E, T = Fft<N>::T;
   constexpr int NMID = DIM == 3 ? N : 1;
   __shared__ float2 sm[xpad_len<XW>(N) * XW];
@@ -1477,6 +1489,7 @@ kx_fwd_band_tma(const __grid_constant__ CUtensorMap dmap, int kt, int kd, float2
                 const float2* __restrict__ tw, const float2* __restrict__ us, long long cs, int band_kf,
                 double inv_n2d, double eps_inj, double* __restrict__ band_scale, int* __restrict__ err,
                 const __grid_constant__ BandRk br) {
+  pdl_begin();
   using K = KxTma<N>;
   constexpr int E = Fft<N>::E, T = Fft<N>::T;
   extern __shared__ __align__(128) float2 s_dyn[];
@@ -1606,6 +1619,7 @@ __global__ void __launch_bounds__(256)
 k_rk_update_lin(const float2* __restrict__ P, long long pcs, int kt, int kd, const float2* us, const float2* u0,
                 float2* acc, float2* out, float2* fin, long long cs, EpiParams prm,
                 const double* __restrict__ band_scale, const float* __restrict__ nu_b, int* __restrict__ err) {
+  pdl_begin();
   constexpr unsigned H = N / 2 + 1, NMID = DIM == 3 ? N : 1, CS = NMID * N * H;  // CS == cs
   const int batch = blockIdx.y;
   prm.nu = nu_b[batch];  // per-trajectory viscosity
@@ -1669,6 +1683,7 @@ __global__ void __launch_bounds__(256)
 k_rk_update(const float2* __restrict__ P, long long pcs, int kt, int kd, const float2* us, const float2* u0,
             float2* acc, float2* out, float2* fin, long long cs, EpiParams prm,
             const double* __restrict__ band_scale, const float* __restrict__ nu_b, int* __restrict__ err) {
+  pdl_begin();
   const int batch = blockIdx.y;
   prm.nu = nu_b[batch];  // per-trajectory viscosity
   const long long pairs = 3 * cs / 2;
@@ -1713,6 +1728,7 @@ __global__ void __launch_bounds__(256)
 k_force_ekin(float2* __restrict__ uh, long long cs, const double* __restrict__ partial,
              int npartial, const double* __restrict__ e0, double dt, int N, int kf,
              double inv_n2d, double eps, double* __restrict__ e_inj, double* __restrict__ ke_out) {
+  pdl_begin();
   const int batch = blockIdx.x;
   float2* ub = uh + (long long)batch * 3 * cs;
   __shared__ double red[32];

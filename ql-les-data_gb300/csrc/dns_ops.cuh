@@ -96,18 +96,20 @@ struct DnsOps {
     const dim3 g(ky_tiles(ncols), N, nz);
     if (c.sched.y_var == 1)
       L3ES_LAUNCH(c, kind, bytes, s,
-                  ky_pass<N, DIR, 1><<<g, KyCfg<N, 1>::THREADS, 0, s>>>(w, fs, ncols, ncols, kd_store, c.tw));
+                  pdl_launch(ky_pass<N, DIR, 1>, g, KyCfg<N, 1>::THREADS, 0, s, w, fs, ncols, ncols, kd_store, c.tw));
     else
-      L3ES_LAUNCH(c, kind, bytes, s, ky_pass<N, DIR, 0><<<g, KY::THREADS, 0, s>>>(w, fs, ncols, ncols, kd_store, c.tw));
+      L3ES_LAUNCH(c, kind, bytes, s, pdl_launch(ky_pass<N, DIR, 0>, g, KY::THREADS, 0, s, w, fs, ncols, ncols,
+                                                kd_store, c.tw));
   }
 
   // the RHS's y inverse (six one-FFT jobs per tile) in the plan's y schedule
   static void y_inv_rhs(const Ctx& c, double bytes, cudaStream_t s) {
     const dim3 g(6 * ky_tiles(H), N, c.batch);
     if (c.sched.y_var == 1)
-      L3ES_LAUNCH(c, KK_Y_INV, bytes, s, ky_inv_rhs<N, 1><<<g, KyCfg<N, 1>::THREADS, 0, s>>>(c.W, c.Wx, c.fs, c.tw));
+      L3ES_LAUNCH(c, KK_Y_INV, bytes, s, pdl_launch(ky_inv_rhs<N, 1>, g, KyCfg<N, 1>::THREADS, 0, s, c.W, c.Wx, c.fs,
+                                                    c.tw));
     else
-      L3ES_LAUNCH(c, KK_Y_INV, bytes, s, ky_inv_rhs<N, 0><<<g, KY::THREADS, 0, s>>>(c.W, c.Wx, c.fs, c.tw));
+      L3ES_LAUNCH(c, KK_Y_INV, bytes, s, pdl_launch(ky_inv_rhs<N, 0>, g, KY::THREADS, 0, s, c.W, c.Wx, c.fs, c.tw));
   }
 
   // x inverse pass with curl prologue: us -> W (6 fields); xl: the x inverse of a
@@ -127,13 +129,13 @@ struct DnsOps {
         if constexpr (N >= kBandMin3d)
           if (xl) {
             L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                        kx_inv_tma<N, true, true, true><<<dim3(gx, c.batch), TX, KxTma<N>::SMEM, s>>>(
-                            map, c.W, c.fs, c.tw, ntiles, c.err, c.Wx, *xl));
+                        pdl_launch(kx_inv_tma<N, true, true, true>, dim3(gx, c.batch), TX, KxTma<N>::SMEM, s, map,
+                                   c.W, c.fs, c.tw, ntiles, c.err, c.Wx, *xl));
             return;
           }
         L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                    kx_inv_tma<N, true, true><<<dim3(gx, c.batch), TX, KxTma<N>::SMEM, s>>>(
-                        map, c.W, c.fs, c.tw, ntiles, c.err, c.Wx, XLin{}));
+                    pdl_launch(kx_inv_tma<N, true, true>, dim3(gx, c.batch), TX, KxTma<N>::SMEM, s, map, c.W, c.fs,
+                               c.tw, ntiles, c.err, c.Wx, XLin{}));
         return;
       }
     }
@@ -141,7 +143,8 @@ struct DnsOps {
       if (c.sched.x_bulk) {
         const dim3 gn((unsigned)((mc + XN - 1) / XN), c.batch);
         L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                    kx_inv<N, 2, true, false, false, XN><<<gn, TXN, 0, s>>>(us, c.cs, c.W, c.fs, c.tw, c.Wx));
+                    pdl_launch(kx_inv<N, 2, true, false, false, XN>, gn, TXN, 0, s, us, c.cs, c.W, c.fs, c.tw, c.Wx,
+                               XLin{}, nullptr));
         return;
       }
     }
@@ -149,11 +152,13 @@ struct DnsOps {
     if constexpr (DIM == 3 && N >= kBandMin3d)
       if (xl) {
         L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                    kx_inv<N, 3, true, true, true><<<g, TX, 0, s>>>(us, c.cs, c.W, c.fs, c.tw, c.Wx, *xl, c.err));
+                    pdl_launch(kx_inv<N, 3, true, true, true>, g, TX, 0, s, us, c.cs, c.W, c.fs, c.tw, c.Wx, *xl,
+                               c.err));
         return;
       }
     L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                kx_inv<N, DIM, true, DIM == 3><<<g, TX, 0, s>>>(us, c.cs, c.W, c.fs, c.tw, c.Wx));
+                pdl_launch(kx_inv<N, DIM, true, DIM == 3>, g, TX, 0, s, us, c.cs, c.W, c.fs, c.tw, c.Wx, XLin{},
+                           nullptr));
   }
 
   // W (u, curl u after the x inverse) -> DU (the nonlinear term before its x transform):
@@ -175,13 +180,13 @@ struct DnsOps {
           const long long tiles = (lines + L3::LPC - 1) / L3::LPC;
           if (c.sched.line_pair == 3 && lc3_staged_ok && lines % L3::LPC == 0)
             L3ES_LAUNCH(c, KK_LINE_CROSS, 2.0 * A + Adu, s,
-                        line_cross3<N, true><<<dim3((unsigned)tiles, c.batch), L3::THREADS, L3::SMEM_STAGED, s>>>(
-                            c.W, c.fs, c.DU, c.ds, c.kt, c.kd, s2, c.tw + line2_ct_offset<N>(),
+                        pdl_launch(line_cross3<N, true>, dim3((unsigned)tiles, c.batch), L3::THREADS, L3::SMEM_STAGED,
+                                   s, c.W, c.fs, c.DU, c.ds, c.kt, c.kd, s2, c.tw + line2_ct_offset<N>(),
                             c.tw + line3_ct16_offset<N>(), (int)lines, c.err));
           else
             L3ES_LAUNCH(c, KK_LINE_CROSS, 2.0 * A + Adu, s,
-                        line_cross3<N, false><<<dim3((unsigned)tiles, c.batch), L3::THREADS, 0, s>>>(
-                            c.W, c.fs, c.DU, c.ds, c.kt, c.kd, s2, c.tw + line2_ct_offset<N>(),
+                        pdl_launch(line_cross3<N, false>, dim3((unsigned)tiles, c.batch), L3::THREADS, 0, s, c.W,
+                                   c.fs, c.DU, c.ds, c.kt, c.kd, s2, c.tw + line2_ct_offset<N>(),
                             c.tw + line3_ct16_offset<N>(), (int)lines, c.err));
           line_done = true;
         }
@@ -191,15 +196,15 @@ struct DnsOps {
         const float s2 = 0.5f * scale * scale;
         const long long tiles = (lines + L2::LPC - 1) / L2::LPC;
         L3ES_LAUNCH(c, KK_LINE_CROSS, 2.0 * A + Adu, s,
-                    line_cross2<N><<<dim3((unsigned)tiles, c.batch), L2::THREADS, 0, s>>>(
-                        c.W, c.fs, c.DU, c.ds, c.kt, c.kd, s2, c.tw + line2_ct_offset<N>(), (int)lines));
+                    pdl_launch(line_cross2<N>, dim3((unsigned)tiles, c.batch), L2::THREADS, 0, s, c.W, c.fs, c.DU,
+                               c.ds, c.kt, c.kd, s2, c.tw + line2_ct_offset<N>(), (int)lines));
         line_done = true;
       }
     }
     if (!line_done)
       L3ES_LAUNCH(c, KK_LINE_CROSS, 2.0 * A + Adu, s,
-                  line_cross<N><<<dim3(line_blocks(lines), c.batch), L::THREADS, 0, s>>>(
-                      c.W, c.fs, c.DU, c.ds, c.kt, c.kd, scale, c.tw, (int)lines));
+                  pdl_launch(line_cross<N>, dim3(line_blocks(lines), c.batch), L::THREADS, 0, s, c.W, c.fs, c.DU,
+                             c.ds, c.kt, c.kd, scale, c.tw, (int)lines));
     if (DIM == 3) y_pass<kFwd>(c, KK_Y_FWD, Adu * (1.0 + rows), c.DU, c.ds, c.kt, c.kd, 3 * c.batch, s);
   }
 
@@ -254,14 +259,14 @@ struct DnsOps {
           const int ntiles = (c.kt / TW) * nb;
           const int gx = std::max(1, std::min(ntiles, tma_band_fused_ctas / c.batch));
           L3ES_LAUNCH(c, KK_X_EPI, bb, s,
-                      kx_fwd_band_tma<N, true><<<dim3(gx, c.batch), TX, KxTma<N>::SMEM, s>>>(
-                          map, c.kt, c.kd, c.P, c.pcs, c.tw, us, c.cs, 0, inv_n2d, c.eps_inj, c.band, c.err, br));
+                      pdl_launch(kx_fwd_band_tma<N, true>, dim3(gx, c.batch), TX, KxTma<N>::SMEM, s, map, c.kt, c.kd,
+                                 c.P, c.pcs, c.tw, us, c.cs, 0, inv_n2d, c.eps_inj, c.band, c.err, br));
           return;
         }
       }
       L3ES_LAUNCH(c, KK_X_EPI, bb, s,
-                  kx_fwd_band<N, 3, true><<<dim3(c.kt / TW, nb, c.batch), TX, 0, s>>>(
-                      c.DU, c.ds, c.kt, c.kd, c.P, c.pcs, c.tw, us, c.cs, 0, inv_n2d, c.eps_inj, c.band, br));
+                  pdl_launch(kx_fwd_band<N, 3, true>, dim3(c.kt / TW, nb, c.batch), TX, 0, s, c.DU, c.ds, c.kt, c.kd,
+                             c.P, c.pcs, c.tw, us, c.cs, 0, inv_n2d, c.eps_inj, c.band, br));
       return;
     }
     // (block 0 of each trajectory also computes the constant-power coefficient of us)
@@ -278,22 +283,22 @@ struct DnsOps {
         const int ntiles = (c.kt / TW) * nb;
         const int gx = std::max(1, std::min(ntiles, tma_band_ctas / c.batch));
         L3ES_LAUNCH(c, KK_X_EPI, Adu * rows + Ap, s,
-                    kx_fwd_band_tma<N><<<dim3(gx, c.batch), TX, KxTma<N>::SMEM, s>>>(
-                        map, c.kt, c.kd, c.P, c.pcs, c.tw, us, c.cs, prm.band_kf2 > 0 ? c.kf : 0, inv_n2d,
+                    pdl_launch(kx_fwd_band_tma<N>, dim3(gx, c.batch), TX, KxTma<N>::SMEM, s, map, c.kt, c.kd, c.P,
+                               c.pcs, c.tw, us, c.cs, prm.band_kf2 > 0 ? c.kf : 0, inv_n2d,
                         c.eps_inj, c.band, c.err, BandRk{}));
         band_done = true;
       }
     }
     if (!band_done && DIM == 2 && c.sched.x_bulk)
       L3ES_LAUNCH(c, KK_X_EPI, Adu * rows + Ap, s,
-                  kx_fwd_band<N, DIM, false, XN><<<dim3(c.kt / XN, 1, c.batch), TXN, 0, s>>>(
-                      c.DU, c.ds, c.kt, c.kd, c.P, c.pcs, c.tw, us, c.cs, prm.band_kf2 > 0 ? c.kf : 0, inv_n2d,
-                      c.eps_inj, c.band));
+                  pdl_launch(kx_fwd_band<N, DIM, false, XN>, dim3(c.kt / XN, 1, c.batch), TXN, 0, s, c.DU, c.ds, c.kt,
+                             c.kd, c.P, c.pcs, c.tw, us, c.cs, prm.band_kf2 > 0 ? c.kf : 0, inv_n2d,
+                      c.eps_inj, c.band, BandRk{}));
     else if (!band_done)
       L3ES_LAUNCH(c, KK_X_EPI, Adu * rows + Ap, s,
-                  kx_fwd_band<N, DIM><<<dim3(c.kt / TW, DIM == 3 ? nb : 1, c.batch), TX, 0, s>>>(
-                      c.DU, c.ds, c.kt, c.kd, c.P, c.pcs, c.tw, us, c.cs, prm.band_kf2 > 0 ? c.kf : 0, inv_n2d,
-                      c.eps_inj, c.band));
+                  pdl_launch(kx_fwd_band<N, DIM>, dim3(c.kt / TW, DIM == 3 ? nb : 1, c.batch), TX, 0, s, c.DU, c.ds,
+                             c.kt, c.kd, c.P, c.pcs, c.tw, us, c.cs, prm.band_kf2 > 0 ? c.kf : 0, inv_n2d,
+                      c.eps_inj, c.band, BandRk{}));
     // rk -1: us -> du; 0: us -> out; 1: us, u0 -> acc, out; 2: us, u0, acc -> acc, out;
     // 3: us, acc -> fin
     double upd = Ap + A * (rk < 0 ? 2.0 : rk == 0 ? 2.0 : rk == 1 ? 4.0 : rk == 2 ? 5.0 : 3.0);
@@ -305,15 +310,17 @@ struct DnsOps {
     const dim3 ug((unsigned)((pairs + 255) / 256), c.batch);
     if (prm.lin && rk >= 0 && !(prm.if_h > 0.f))
       L3ES_LAUNCH(c, KK_RK_UPDATE, upd, s,
-                  k_rk_update_lin<N, DIM><<<ug, 256, 0, s>>>(c.P, c.pcs, c.kt, c.kd, us, S, c.C, out, S, c.cs, prm,
+                  pdl_launch(k_rk_update_lin<N, DIM>, ug, 256, 0, s, c.P, c.pcs, c.kt, c.kd, us, S, c.C, out, S, c.cs,
+                             prm,
                                                             c.band, c.nu_b, c.err));
     else if (prm.if_h > 0.f && rk >= 0)
       L3ES_LAUNCH(c, KK_RK_UPDATE, upd, s,
-                  k_rk_update<N, DIM, true><<<ug, 256, 0, s>>>(c.P, c.pcs, c.kt, c.kd, us, S, c.C, out, S, c.cs, prm,
+                  pdl_launch(k_rk_update<N, DIM, true>, ug, 256, 0, s, c.P, c.pcs, c.kt, c.kd, us, S, c.C, out, S,
+                             c.cs, prm,
                                                                 c.band, c.nu_b, c.err));
     else
       L3ES_LAUNCH(c, KK_RK_UPDATE, upd, s,
-                  k_rk_update<N, DIM><<<ug, 256, 0, s>>>(c.P, c.pcs, c.kt, c.kd, us, S, c.C, out, S, c.cs, prm,
+                  pdl_launch(k_rk_update<N, DIM>, ug, 256, 0, s, c.P, c.pcs, c.kt, c.kd, us, S, c.C, out, S, c.cs, prm,
                                                           c.band, c.nu_b, c.err));
   }
 
@@ -332,15 +339,16 @@ struct DnsOps {
     if (RK >= 0 && prm.band_kf2 > 0) {
       const double inv_n2d = 1.0 / std::pow((double)N, 2 * DIM);
       L3ES_LAUNCH(c, KK_FORCE, 0.0, s,
-                  k_band_coefficient<DIM><<<c.batch, 256, 0, s>>>(RK == 0 ? S : c.Tb, c.cs, N, c.kf, inv_n2d, c.eps_inj,
+                  pdl_launch(k_band_coefficient<DIM>, c.batch, 256, 0, s, RK == 0 ? S : c.Tb, c.cs, N, c.kf, inv_n2d,
+                             c.eps_inj,
                                                                   c.band));
     }
     using K = Stage<DIM>;
     const XStage st{c.cs, c.kd, c.kt, prm, c.band, c.nu_b, c.err};
     const dim3 g((unsigned)((c.nmid * H + XS<DIM> - 1) / XS<DIM>), c.batch);
     L3ES_LAUNCH(c, KK_X_STAGE, b, s,
-                kx_stage<N, DIM, XS<DIM>, ES<DIM>, RK, INV><<<g, K::THREADS, K::SMEM, s>>>(
-                    c.DU, c.ds, S, c.Tb, c.C, st, c.W, c.Wx, c.fs, c.tw));
+                pdl_launch(kx_stage<N, DIM, XS<DIM>, ES<DIM>, RK, INV>, g, K::THREADS, K::SMEM, s, c.DU, c.ds, S,
+                           c.Tb, c.C, st, c.W, c.Wx, c.fs, c.tw));
   }
 
   // One RK4 step in place on S by kx_stage (stage_kernels.cuh). first: the x inverse of S
@@ -394,19 +402,20 @@ struct DnsOps {
         const int ntiles = (int)(mc / TW);
         const int gx = std::max(1, std::min(ntiles, tma_plain_ctas / c.batch));
         L3ES_LAUNCH(c, KK_X_INV_PLAIN, 2.0 * A, s,
-                    kx_inv_tma<N, false><<<dim3(gx, c.batch), TX, KxTma<N>::SMEM, s>>>(map, c.W, c.fs, c.tw, ntiles,
+                    pdl_launch(kx_inv_tma<N, false>, dim3(gx, c.batch), TX, KxTma<N>::SMEM, s, map, c.W, c.fs, c.tw,
+                               ntiles,
                                                                                         c.err, nullptr, XLin{}));
         x_done = true;
       }
     }
     if (!x_done)
       L3ES_LAUNCH(c, KK_X_INV_PLAIN, 2.0 * A, s,
-                  kx_inv<N, DIM, false><<<dim3((unsigned)((mc + TW - 1) / TW), c.batch), TX, 0, s>>>(
-                      uh, c.cs, c.W, c.fs, c.tw));
+                  pdl_launch(kx_inv<N, DIM, false>, dim3((unsigned)((mc + TW - 1) / TW), c.batch), TX, 0, s, uh, c.cs,
+                             c.W, c.fs, c.tw, nullptr, XLin{}, nullptr));
     if (DIM == 3) y_pass<kInv>(c, KK_Y_INV, 2.0 * A, c.W, c.fs, H, N / 2, 3 * c.batch, s);
     L3ES_LAUNCH(c, KK_LINE_C2R, A + P, s,
-                line_c2r<N><<<dim3(line_blocks(lines), c.batch), L::THREADS, 0, s>>>(
-                    c.W, c.fs, u, c.ps, scale, c.tw, (int)lines));
+                pdl_launch(line_c2r<N>, dim3(line_blocks(lines), c.batch), L::THREADS, 0, s, c.W, c.fs, u, c.ps,
+                           scale, c.tw, (int)lines));
   }
 
   static void irfftn(const Ctx& c, const float2* uh, float* u, cudaStream_t s) {
@@ -422,12 +431,12 @@ struct DnsOps {
     const long long lines = c.nmid * N;
     const double A = 8.0 * 3.0 * c.cs * c.batch, P = 4.0 * 3.0 * c.ps * c.batch;
     L3ES_LAUNCH(c, KK_LINE_R2C, A + P, s,
-                line_r2c<N><<<dim3(line_blocks(lines), c.batch), L::THREADS, 0, s>>>(
-                    u, c.ps, c.W, c.fs, c.tw, (int)lines));
+                pdl_launch(line_r2c<N>, dim3(line_blocks(lines), c.batch), L::THREADS, 0, s, u, c.ps, c.W, c.fs, c.tw,
+                           (int)lines));
     if (DIM == 3) y_pass<kFwd>(c, KK_Y_FWD, 2.0 * A, c.W, c.fs, H, N / 2, 3 * c.batch, s);
     L3ES_LAUNCH(c, KK_X_FWD_PLAIN, 2.0 * A, s,
-                kx_fwd_plain<N, DIM><<<dim3((unsigned)((mc + TW - 1) / TW), c.batch), TX, 0, s>>>(
-                    c.W, c.fs, uh, c.cs, c.tw));
+                pdl_launch(kx_fwd_plain<N, DIM>, dim3((unsigned)((mc + TW - 1) / TW), c.batch), TX, 0, s, c.W, c.fs,
+                           uh, c.cs, c.tw));
   }
 
   static void rfftn(const Ctx& c, const float* u, float2* uh, cudaStream_t s) {
@@ -453,25 +462,25 @@ struct DnsOps {
     const float2* wuw = a.wlines ? a.wlines : c.W;
     if (!a.wlines) x_inverse<DIM>(c, a.us, (DIM == 3 ? 8.0 : 9.0) / 3.0 * A, s);
     L3ES_LAUNCH(c, KK_ADJ_X_INV, 2.0 * A, s,
-                kx_inv_adjproj<N, DIM><<<dim3(xb, c.batch), TX, 0, s>>>(
-                    a.g, c.cs, a.gscale, c.kd, Wm, c.fs, c.tw, a.us, a.band_kf2 > 0 ? c.kf : 0, inv_n2d,
+                pdl_launch(kx_inv_adjproj<N, DIM>, dim3(xb, c.batch), TX, 0, s, a.g, c.cs, a.gscale, c.kd, Wm, c.fs,
+                           c.tw, a.us, a.band_kf2 > 0 ? c.kf : 0, inv_n2d,
                     c.eps_inj, const_cast<double*>(a.band_adj)));
     if (DIM == 3) {
       if (!a.wlines) y_inv_rhs(c, 11.0 / 3.0 * A, s);
       y_pass<kInv>(c, KK_Y_INV, 2.0 * A, Wm, c.fs, H, N / 2, 3 * c.batch, s);
     }
     L3ES_LAUNCH(c, KK_ADJ_LINE, 5.0 * A, s,
-                line_cross_adj<N><<<dim3(line_blocks(lines), c.batch), L::THREADS, 0, s>>>(
-                    Wm, wuw, c.fs, Y6, c.cs, scale, c.tw, (int)lines));
+                pdl_launch(line_cross_adj<N>, dim3(line_blocks(lines), c.batch), L::THREADS, 0, s, Wm, wuw, c.fs, Y6,
+                           c.cs, scale, c.tw, (int)lines));
     if (DIM == 3) y_pass<kFwd>(c, KK_Y_FWD, 4.0 * A, Y6, c.cs, H, N / 2, 6 * c.batch, s);
     // Y6 (6 fields per trajectory) -> W, as 2 * batch groups of 3 fields
     L3ES_LAUNCH(c, KK_X_FWD_PLAIN, 4.0 * A, s,
-                kx_fwd_plain<N, DIM><<<dim3(xb, 2 * c.batch), TX, 0, s>>>(Y6, c.cs, c.W, c.fs, c.tw));
+                pdl_launch(kx_fwd_plain<N, DIM>, dim3(xb, 2 * c.batch), TX, 0, s, Y6, c.cs, c.W, c.fs, c.tw));
     const long long pairs = c.cs / 2;
     // reads: 2 product spectra, g, lam1, lam_in; writes: lam_out, g_out
     const double epi = (3.0 + (a.lam1 ? 1.0 : 0.0) + (a.lam_in ? 1.0 : 0.0) + 1.0 + (a.g_out ? 1.0 : 0.0)) * A;
     L3ES_LAUNCH(c, KK_ADJ_EPI, epi, s,
-                k_adj_epi<N, DIM><<<dim3((unsigned)((pairs + 255) / 256), c.batch), 256, 0, s>>>(c.W, c.cs, a,
+                pdl_launch(k_adj_epi<N, DIM>, dim3((unsigned)((pairs + 255) / 256), c.batch), 256, 0, s, c.W, c.cs, a,
                                                                                                  c.nu_b));
   }
 

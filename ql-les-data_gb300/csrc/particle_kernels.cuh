@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "fft_core.cuh"
+#include "pdl.cuh"
 
 namespace l3es {
 
@@ -43,6 +44,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256)
 k_crop(const float2* __restrict__ uh, long long cs, int N, float2* __restrict__ hh, long long hcs, int c,
        float scale) {
+  pdl_begin();
   const int hc = c / 2 + 1;
   const long long per = DIM == 3 ? (long long)c * c * hc : (long long)c * hc;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -82,6 +84,7 @@ template <int DIM>
 __global__ void __launch_bounds__(128)
 k_dft_interp(const float2* __restrict__ hh, long long hcs, int c, int ncomp, const double* __restrict__ r,
              long long np, double* __restrict__ u_r, double dt, double* __restrict__ r_out) {
+  pdl_begin();
   extern __shared__ float2 ph[];  // [DIM][c][128]
   const long long j_raw = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = j_raw < np;

@@ -30,6 +30,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256)
 k_nufft_prep(const float2* __restrict__ hh, long long hcs, int c, const float* __restrict__ inv_psi,
              float2* __restrict__ g, long long gcs, int n) {
+  pdl_begin();
   const long long per = DIM == 3 ? (long long)n * n * n : (long long)n * n;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int comp = blockIdx.y;
@@ -83,6 +84,7 @@ template <int NL>
 __global__ void __launch_bounds__(128)
 line_c2c_re(const float2* __restrict__ g, float* __restrict__ gre, long long nlines, const float2* __restrict__ tw,
             float scale) {
+  pdl_begin();
   constexpr int E = Fft<NL>::E, T = Fft<NL>::T;
   static_assert(T <= 32, "line inside one warp");
   constexpr int LPC = (32 / T) * 4;
@@ -123,6 +125,7 @@ __device__ __forceinline__ int particle_bin(const double* __restrict__ r, long l
 // r + b np dim, its bins at count / start + b nbins and its permutation at perm + b np.
 template <int DIM>
 __global__ void k_bin_count(const double* __restrict__ r, long long np, int nb, int nbins, int* __restrict__ count) {
+  pdl_begin();
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   r += (long long)blockIdx.y * np * DIM;
   count += (long long)blockIdx.y * nbins;
@@ -131,6 +134,7 @@ __global__ void k_bin_count(const double* __restrict__ r, long long np, int nb, 
 
 // exclusive scan of nbins counts by one CTA of 1024 threads (chunked)
 __global__ void __launch_bounds__(1024) k_bin_scan(const int* __restrict__ count, int nbins, int* __restrict__ start) {
+  pdl_begin();
   __shared__ int part[1024];
   count += (long long)blockIdx.x * nbins;
   start += (long long)blockIdx.x * nbins;
@@ -158,6 +162,7 @@ __global__ void __launch_bounds__(1024) k_bin_scan(const int* __restrict__ count
 template <int DIM>
 __global__ void k_bin_scatter(const double* __restrict__ r, long long np, int nb, int nbins, int* __restrict__ cursor,
                               int* __restrict__ perm) {
+  pdl_begin();
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   r += (long long)blockIdx.y * np * DIM;
   cursor += (long long)blockIdx.y * nbins;
@@ -182,6 +187,7 @@ __global__ void __launch_bounds__(128)
 k_nufft_gather(const float* __restrict__ gre, long long gcs, int n, int ncomp, float beta, double norm,
                const double* __restrict__ r, const int* __restrict__ perm, long long np, double* __restrict__ u_r,
                double dt, double* __restrict__ r_out) {
+  pdl_begin();
   static_assert(W <= kGatherLanes, "one support row per lane");
   {  // batched plans: trajectory blockIdx.y (its 3-field grid, positions, order, outputs)
     const long long b = blockIdx.y;
@@ -281,6 +287,7 @@ __global__ void __launch_bounds__(128)
 k_nufft_spread(float* __restrict__ gbar, long long gcs, int n, int ncomp, float beta, double norm,
                const double* __restrict__ r, const int* __restrict__ perm, long long np,
                const double* __restrict__ lam) {
+  pdl_begin();
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long i = gt / kGatherLanes;
   const int a = (int)(gt % kGatherLanes);
@@ -334,6 +341,7 @@ template <int NL>
 __global__ void __launch_bounds__(128)
 line_fft_real_fwd(const float* __restrict__ x, float2* __restrict__ g, long long nlines,
                   const float2* __restrict__ tw) {
+  pdl_begin();
   constexpr int E = Fft<NL>::E, T = Fft<NL>::T;
   static_assert(T <= 32, "line inside one warp");
   constexpr int LPC = (32 / T) * 4;
@@ -364,6 +372,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256)
 k_box_to_half_adj(const float2* __restrict__ G, long long gcs, int gn, int c, const float* __restrict__ inv_psi,
                   float scale, float2* __restrict__ hb, long long hcs) {
+  pdl_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int comp = blockIdx.y;
   if (i >= hcs) return;
@@ -406,6 +415,7 @@ k_box_to_half_adj(const float2* __restrict__ G, long long gcs, int gn, int c, co
 template <int DIM>
 __global__ void __launch_bounds__(256)
 k_herm_project(const float2* __restrict__ hb, long long hcs, int c, float cd, float2* __restrict__ V) {
+  pdl_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int comp = blockIdx.y;
   if (i >= hcs) return;
@@ -435,6 +445,7 @@ template <int DIM>
 __global__ void __launch_bounds__(128)
 k_p2g_dft(const double* __restrict__ r, const double* __restrict__ u_r, long long np, int ncomp, int n,
           float2* __restrict__ S, long long scs) {
+  pdl_begin();
   extern __shared__ float2 sh[];            // [128][DIM][n] phases
   __shared__ float su[128][3];              // velocities of the tile
   const long long modes = DIM == 3 ? (long long)n * n * n : (long long)n * n;
@@ -508,6 +519,7 @@ k_p2g_dft(const double* __restrict__ r, const double* __restrict__ u_r, long lon
 __global__ void k_rk4_particles(int stage, const double* __restrict__ r0, const double* __restrict__ v,
                                 double* __restrict__ acc, double* __restrict__ rs, double dt, long long n,
                                 double box) {
+  pdl_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double vi = v[i];
@@ -532,6 +544,7 @@ __global__ void k_rk4_particles(int stage, const double* __restrict__ r0, const 
 // shift_fn(r, dr) = (r + scale * dr) mod box (integrator.py:21-23), elementwise
 __global__ void k_shift(const double* __restrict__ r, const double* __restrict__ dr, long long n, double scale,
                         double box, double* __restrict__ out) {
+  pdl_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double x = r[i] + scale * dr[i];
@@ -554,6 +567,7 @@ __global__ void k_shift(const double* __restrict__ r, const double* __restrict__
 __global__ void __launch_bounds__(256)
 k_mse_resid(float* __restrict__ uc, const float* __restrict__ tgt, long long per, int ncomp, double inv_size,
             double* __restrict__ partial) {
+  pdl_begin();
   double acc = 0.0;
   const long long total = 3 * per;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -571,6 +585,7 @@ k_mse_resid(float* __restrict__ uc, const float* __restrict__ tgt, long long per
 
 __global__ void __launch_bounds__(256)
 k_mse_sum(const double* __restrict__ partial, int n, double inv_size, double* __restrict__ out) {
+  pdl_begin();
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) acc += partial[i];
   __shared__ double tot[1];
@@ -585,6 +600,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256)
 k_uncrop_grad(const float2* __restrict__ V, long long hcs, int c, int N, long long cs, int ncomp, float scale,
               float2* __restrict__ G) {
+  pdl_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int comp = blockIdx.y;
   if (i >= cs) return;
@@ -698,14 +714,15 @@ static void c2c_inverse_re(int dim, float2* g, float* gre, const float2* tw, flo
   constexpr int TX = KY::THREADS, TWY = KY::TWY;
   const long long per = dim == 3 ? (long long)NG * NG * NG : (long long)NG * NG;
   if (dim == 3) {
-    ky_pass<NG, kInv><<<dim3((NG * NG + TWY - 1) / TWY, 1, 3), TX, 0, s>>>(g, per, NG * NG, NG * NG, NG / 2, tw);
-    ky_pass<NG, kInv><<<dim3((NG + TWY - 1) / TWY, NG, 3), TX, 0, s>>>(g, per, NG, NG, NG / 2, tw);
+    pdl_launch(ky_pass<NG, kInv>, dim3((NG * NG + TWY - 1) / TWY, 1, 3), TX, 0, s, g, per, NG * NG, NG * NG, NG / 2,
+               tw);
+    pdl_launch(ky_pass<NG, kInv>, dim3((NG + TWY - 1) / TWY, NG, 3), TX, 0, s, g, per, NG, NG, NG / 2, tw);
   } else {
-    ky_pass<NG, kInv><<<dim3((NG + TWY - 1) / TWY, 1, 3), TX, 0, s>>>(g, per, NG, NG, NG / 2, tw);
+    pdl_launch(ky_pass<NG, kInv>, dim3((NG + TWY - 1) / TWY, 1, 3), TX, 0, s, g, per, NG, NG, NG / 2, tw);
   }
   const long long lines = 3 * per / NG;
   constexpr int LPC = (32 / Fft<NG>::T) * 4;
-  line_c2c_re<NG><<<(unsigned)((lines + LPC - 1) / LPC), 128, 0, s>>>(g, gre, lines, tw, scale);
+  pdl_launch(line_c2c_re<NG>, (unsigned)((lines + LPC - 1) / LPC), 128, 0, s, g, gre, lines, tw, scale);
 }
 
 // strided c2c passes of the NUFFT grid (inverse), via the ky_pass kernel
@@ -717,15 +734,16 @@ static void grid_passes(const l3es_interp_plan* p, cudaStream_t s) {
   const unsigned nf = 3u * (unsigned)p->batch;  // fields of every trajectory, one after another
   if (p->dim == 3) {
     // x: pencils of stride n^2, columns = (y, z) flattened
-    ky_pass<NG, kInv><<<dim3((NG * NG + TWY - 1) / TWY, 1, nf), TX, 0, s>>>(p->g, per, NG * NG, NG * NG, NG / 2, p->tw);
+    pdl_launch(ky_pass<NG, kInv>, dim3((NG * NG + TWY - 1) / TWY, 1, nf), TX, 0, s, p->g, per, NG * NG, NG * NG,
+               NG / 2, p->tw);
     // y: pencils of stride n inside each x-plane, columns = z
-    ky_pass<NG, kInv><<<dim3((NG + TWY - 1) / TWY, NG, nf), TX, 0, s>>>(p->g, per, NG, NG, NG / 2, p->tw);
+    pdl_launch(ky_pass<NG, kInv>, dim3((NG + TWY - 1) / TWY, NG, nf), TX, 0, s, p->g, per, NG, NG, NG / 2, p->tw);
   } else {
-    ky_pass<NG, kInv><<<dim3((NG + TWY - 1) / TWY, 1, nf), TX, 0, s>>>(p->g, per, NG, NG, NG / 2, p->tw);
+    pdl_launch(ky_pass<NG, kInv>, dim3((NG + TWY - 1) / TWY, 1, nf), TX, 0, s, p->g, per, NG, NG, NG / 2, p->tw);
   }
   const long long lines = (long long)nf * per / NG;
   constexpr int LPC = (32 / Fft<NG>::T) * 4;
-  line_c2c_re<NG><<<(unsigned)((lines + LPC - 1) / LPC), 128, 0, s>>>(p->g, p->gre, lines, p->tw, 1.0f);
+  pdl_launch(line_c2c_re<NG>, (unsigned)((lines + LPC - 1) / LPC), 128, 0, s, p->g, p->gre, lines, p->tw, 1.0f);
 }
 
 // forward c2c passes of the real NUFFT grid gre (the adjoint of the inverse passes):
@@ -737,12 +755,13 @@ static void grid_fwd_passes(const l3es_interp_plan* p, cudaStream_t s) {
   const long long per = p->gcs;
   const long long lines = 3 * per / NG;
   constexpr int LPC = (32 / Fft<NG>::T) * 4;
-  line_fft_real_fwd<NG><<<(unsigned)((lines + LPC - 1) / LPC), 128, 0, s>>>(p->gre, p->g, lines, p->tw);
+  pdl_launch(line_fft_real_fwd<NG>, (unsigned)((lines + LPC - 1) / LPC), 128, 0, s, p->gre, p->g, lines, p->tw);
   if (p->dim == 3) {
-    ky_pass<NG, kFwd><<<dim3((NG + TWY - 1) / TWY, NG, 3), TX, 0, s>>>(p->g, per, NG, NG, NG / 2, p->tw);
-    ky_pass<NG, kFwd><<<dim3((NG * NG + TWY - 1) / TWY, 1, 3), TX, 0, s>>>(p->g, per, NG * NG, NG * NG, NG / 2, p->tw);
+    pdl_launch(ky_pass<NG, kFwd>, dim3((NG + TWY - 1) / TWY, NG, 3), TX, 0, s, p->g, per, NG, NG, NG / 2, p->tw);
+    pdl_launch(ky_pass<NG, kFwd>, dim3((NG * NG + TWY - 1) / TWY, 1, 3), TX, 0, s, p->g, per, NG * NG, NG * NG,
+               NG / 2, p->tw);
   } else {
-    ky_pass<NG, kFwd><<<dim3((NG + TWY - 1) / TWY, 1, 3), TX, 0, s>>>(p->g, per, NG, NG, NG / 2, p->tw);
+    pdl_launch(ky_pass<NG, kFwd>, dim3((NG + TWY - 1) / TWY, 1, 3), TX, 0, s, p->g, per, NG, NG, NG / 2, p->tw);
   }
 }
 
@@ -887,9 +906,9 @@ int l3es_interp_set_spectrum(l3es_interp_plan* p, const void* u_hat_fine, void* 
   const unsigned blocks = (unsigned)((p->hcs + 255) / 256);
   const unsigned nf = 3u * (unsigned)p->batch;  // batched: [batch][3] fine spectra in, [batch][3] coarse out
   if (p->dim == 3)
-    k_crop<3><<<dim3(blocks, nf), 256, 0, s>>>((const float2*)u_hat_fine, cs, N, p->hh, p->hcs, c, scale);
+    pdl_launch(k_crop<3>, dim3(blocks, nf), 256, 0, s, (const float2*)u_hat_fine, cs, N, p->hh, p->hcs, c, scale);
   else
-    k_crop<2><<<dim3(blocks, nf), 256, 0, s>>>((const float2*)u_hat_fine, cs, N, p->hh, p->hcs, c, scale);
+    pdl_launch(k_crop<2>, dim3(blocks, nf), 256, 0, s, (const float2*)u_hat_fine, cs, N, p->hh, p->hcs, c, scale);
   return cuda_check(cudaGetLastError(), "l3es_interp_set_spectrum launch");
 }
 
@@ -923,10 +942,10 @@ static int dft_eval(l3es_interp_plan* p, const double* r, int64_t np, double* u_
   const size_t smem = sizeof(float2) * p->dim * p->c * 128;
   if (p->dim == 3) {
     cudaFuncSetAttribute(k_dft_interp<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_dft_interp<3><<<pb, 128, smem, s>>>(p->hh, p->hcs, p->c, ncomp, r, np, u_r, dt, r_out);
+    pdl_launch(k_dft_interp<3>, pb, 128, smem, s, p->hh, p->hcs, p->c, ncomp, r, np, u_r, dt, r_out);
   } else {
     cudaFuncSetAttribute(k_dft_interp<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_dft_interp<2><<<pb, 128, smem, s>>>(p->hh, p->hcs, p->c, ncomp, r, np, u_r, dt, r_out);
+    pdl_launch(k_dft_interp<2>, pb, 128, smem, s, p->hh, p->hcs, p->c, ncomp, r, np, u_r, dt, r_out);
   }
   return cuda_check(cudaGetLastError(), "l3es_interp (dft) launch");
 }
@@ -940,7 +959,7 @@ static int nufft_eval(l3es_interp_plan* p, const double* r, int64_t np, double* 
   const float beta = (float)p->beta;
   const dim3 gblk((unsigned)((np * kGatherLanes + 127) / 128), (unsigned)p->batch);
 #define L3ES_GATHER(D, W)                                                                                   \
-  k_nufft_gather<D, W><<<gblk, 128, 0, s>>>(p->gre, p->gcs, p->n, ncomp, beta, norm, r, p->perm, np, u_r, dt, \
+  pdl_launch(k_nufft_gather<D, W>, gblk, 128, 0, s, p->gre, p->gcs, p->n, ncomp, beta, norm, r, p->perm, np, u_r, dt, \
                                           r_out)
   if (p->dim == 3) {
     if (p->w == 6) L3ES_GATHER(3, 6);
@@ -992,7 +1011,7 @@ int l3es_interp_advect_rk4(l3es_interp_plan* p, const double* r, int64_t np, dou
     double* vel = stage == 0 ? u_r : p->rk_vel;  // u_r: the velocity at the old positions
     rc = backend == 0 ? nufft_eval(p, pos, np, vel, 0.0, nullptr, s) : dft_eval(p, pos, np, vel, 0.0, nullptr, s);
     if (rc != L3ES_OK) break;
-    k_rk4_particles<<<eb, 256, 0, s>>>(stage, r, vel, p->rk_acc, stage == 3 ? r_out : p->rk_pos, dt, n, box);
+    pdl_launch(k_rk4_particles, eb, 256, 0, s, stage, r, vel, p->rk_acc, stage == 3 ? r_out : p->rk_pos, dt, n, box);
     rc = cuda_check(cudaGetLastError(), "l3es_interp_advect_rk4 launch");
   }
   return rc;
@@ -1008,9 +1027,9 @@ static int nufft_grid(l3es_interp_plan* p, const double* r, int64_t np, cudaStre
   const unsigned gb = (unsigned)((p->gcs + 255) / 256);
   const unsigned nf = 3u * (unsigned)p->batch;
   if (p->dim == 3)
-    k_nufft_prep<3><<<dim3(gb, nf), 256, 0, s>>>(p->hh, p->hcs, p->c, p->inv_psi, p->g, p->gcs, p->n);
+    pdl_launch(k_nufft_prep<3>, dim3(gb, nf), 256, 0, s, p->hh, p->hcs, p->c, p->inv_psi, p->g, p->gcs, p->n);
   else
-    k_nufft_prep<2><<<dim3(gb, nf), 256, 0, s>>>(p->hh, p->hcs, p->c, p->inv_psi, p->g, p->gcs, p->n);
+    pdl_launch(k_nufft_prep<2>, dim3(gb, nf), 256, 0, s, p->hh, p->hcs, p->c, p->inv_psi, p->g, p->gcs, p->n);
   const int rc = run_grid_passes(p, s);
   return rc != L3ES_OK ? rc : bin_particles(p, r, np, s);
 }
@@ -1022,13 +1041,13 @@ static int bin_particles(l3es_interp_plan* p, const double* r, int64_t np, cudaS
   int rc = cuda_check(cudaMemsetAsync(p->count, 0, sizeof(int) * nbins * p->batch, s), "l3es_interp memset");
   if (rc != L3ES_OK) return rc;
   if (p->dim == 3) {
-    k_bin_count<3><<<pb, 128, 0, s>>>(r, np, p->nb, nbins, p->count);
-    k_bin_scan<<<p->batch, 1024, 0, s>>>(p->count, nbins, p->start);
-    k_bin_scatter<3><<<pb, 128, 0, s>>>(r, np, p->nb, nbins, p->start, p->perm);
+    pdl_launch(k_bin_count<3>, pb, 128, 0, s, r, np, p->nb, nbins, p->count);
+    pdl_launch(k_bin_scan, p->batch, 1024, 0, s, p->count, nbins, p->start);
+    pdl_launch(k_bin_scatter<3>, pb, 128, 0, s, r, np, p->nb, nbins, p->start, p->perm);
   } else {
-    k_bin_count<2><<<pb, 128, 0, s>>>(r, np, p->nb, nbins, p->count);
-    k_bin_scan<<<p->batch, 1024, 0, s>>>(p->count, nbins, p->start);
-    k_bin_scatter<2><<<pb, 128, 0, s>>>(r, np, p->nb, nbins, p->start, p->perm);
+    pdl_launch(k_bin_count<2>, pb, 128, 0, s, r, np, p->nb, nbins, p->count);
+    pdl_launch(k_bin_scan, p->batch, 1024, 0, s, p->count, nbins, p->start);
+    pdl_launch(k_bin_scatter<2>, pb, 128, 0, s, r, np, p->nb, nbins, p->start, p->perm);
   }
   return cuda_check(cudaGetLastError(), "l3es_interp grid launch");
 }
@@ -1056,12 +1075,12 @@ int l3es_interp_vjp(l3es_interp_plan* p, const double* r, int64_t np, const doub
     const float scale = (float)(1.0 / (double)modes);
     if (dim == 3) {
       cudaFuncSetAttribute(k_p2g_dft<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      k_p2g_dft<3><<<(unsigned)((modes + 127) / 128), 128, smem, s>>>(r, lam, np, 3, c, p->g, modes);
-      k_box_to_half_adj<3><<<dim3(hbk, 3), 256, 0, s>>>(p->g, modes, c, c, nullptr, scale, p->hb, p->hcs);
+      pdl_launch(k_p2g_dft<3>, (unsigned)((modes + 127) / 128), 128, smem, s, r, lam, np, 3, c, p->g, modes);
+      pdl_launch(k_box_to_half_adj<3>, dim3(hbk, 3), 256, 0, s, p->g, modes, c, c, nullptr, scale, p->hb, p->hcs);
     } else {
       cudaFuncSetAttribute(k_p2g_dft<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      k_p2g_dft<2><<<(unsigned)((modes + 127) / 128), 128, smem, s>>>(r, lam, np, 2, c, p->g, modes);
-      k_box_to_half_adj<2><<<dim3(hbk, 3), 256, 0, s>>>(p->g, modes, c, c, nullptr, scale, p->hb, p->hcs);
+      pdl_launch(k_p2g_dft<2>, (unsigned)((modes + 127) / 128), 128, smem, s, r, lam, np, 2, c, p->g, modes);
+      pdl_launch(k_box_to_half_adj<2>, dim3(hbk, 3), 256, 0, s, p->g, modes, c, c, nullptr, scale, p->hb, p->hcs);
     }
   } else {
     rc = bin_particles(p, r, np, s);
@@ -1071,7 +1090,7 @@ int l3es_interp_vjp(l3es_interp_plan* p, const double* r, int64_t np, const doub
     const float beta = (float)p->beta;
     const unsigned gblk = (unsigned)((np * kGatherLanes + 127) / 128);
 #define L3ES_SPREAD(D, W) \
-  k_nufft_spread<D, W><<<gblk, 128, 0, s>>>(p->gre, p->gcs, p->n, dim, beta, norm, r, p->perm, np, lam)
+  pdl_launch(k_nufft_spread<D, W>, gblk, 128, 0, s, p->gre, p->gcs, p->n, dim, beta, norm, r, p->perm, np, lam)
     if (dim == 3) {
       if (p->w == 6) L3ES_SPREAD(3, 6);
       else if (p->w == 8) L3ES_SPREAD(3, 8);
@@ -1085,20 +1104,20 @@ int l3es_interp_vjp(l3es_interp_plan* p, const double* r, int64_t np, const doub
     rc = run_grid_fwd_passes(p, s);
     if (rc != L3ES_OK) return rc;
     if (dim == 3)
-      k_box_to_half_adj<3><<<dim3(hbk, 3), 256, 0, s>>>(p->g, p->gcs, p->n, c, p->inv_psi, 1.f, p->hb, p->hcs);
+      pdl_launch(k_box_to_half_adj<3>, dim3(hbk, 3), 256, 0, s, p->g, p->gcs, p->n, c, p->inv_psi, 1.f, p->hb, p->hcs);
     else
-      k_box_to_half_adj<2><<<dim3(hbk, 3), 256, 0, s>>>(p->g, p->gcs, p->n, c, p->inv_psi, 1.f, p->hb, p->hcs);
+      pdl_launch(k_box_to_half_adj<2>, dim3(hbk, 3), 256, 0, s, p->g, p->gcs, p->n, c, p->inv_psi, 1.f, p->hb, p->hcs);
   }
   // coarse cotangent -> fine half spectrum (p->g is free again: V goes there)
   const float cd = (float)std::pow((double)c, dim);
   const float uscale = (float)(0.5 / std::pow((double)N, dim));
   const dim3 gb((unsigned)((cs + 255) / 256), 3);
   if (dim == 3) {
-    k_herm_project<3><<<dim3(hbk, 3), 256, 0, s>>>(p->hb, p->hcs, c, cd, p->g);
-    k_uncrop_grad<3><<<gb, 256, 0, s>>>(p->g, p->hcs, c, N, cs, 3, uscale, (float2*)grad_fine);
+    pdl_launch(k_herm_project<3>, dim3(hbk, 3), 256, 0, s, p->hb, p->hcs, c, cd, p->g);
+    pdl_launch(k_uncrop_grad<3>, gb, 256, 0, s, p->g, p->hcs, c, N, cs, 3, uscale, (float2*)grad_fine);
   } else {
-    k_herm_project<2><<<dim3(hbk, 3), 256, 0, s>>>(p->hb, p->hcs, c, cd, p->g);
-    k_uncrop_grad<2><<<gb, 256, 0, s>>>(p->g, p->hcs, c, N, cs, 2, uscale, (float2*)grad_fine);
+    pdl_launch(k_herm_project<2>, dim3(hbk, 3), 256, 0, s, p->hb, p->hcs, c, cd, p->g);
+    pdl_launch(k_uncrop_grad<2>, gb, 256, 0, s, p->g, p->hcs, c, N, cs, 2, uscale, (float2*)grad_fine);
   }
   return cuda_check(cudaGetLastError(), "l3es_interp_vjp launch");
 }
@@ -1116,10 +1135,10 @@ int l3es_interp_particles_to_grid(l3es_interp_plan* p, const double* r, const do
   if (smem > 200 * 1024) return fail(L3ES_EINVAL, "l3es_interp_particles_to_grid: grid too large");
   if (p->dim == 3) {
     cudaFuncSetAttribute(k_p2g_dft<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_p2g_dft<3><<<(unsigned)((modes + 127) / 128), 128, smem, s>>>(r, u_r, np, 3, c, p->g, modes);
+    pdl_launch(k_p2g_dft<3>, (unsigned)((modes + 127) / 128), 128, smem, s, r, u_r, np, 3, c, p->g, modes);
   } else {
     cudaFuncSetAttribute(k_p2g_dft<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_p2g_dft<2><<<(unsigned)((modes + 127) / 128), 128, smem, s>>>(r, u_r, np, 2, c, p->g, modes);
+    pdl_launch(k_p2g_dft<2>, (unsigned)((modes + 127) / 128), 128, smem, s, r, u_r, np, 2, c, p->g, modes);
   }
   // u_grid = real(ifftn(S)) (ifftn carries 1/c^dim)
   const float scale = (float)(1.0 / (double)modes);
@@ -1148,8 +1167,8 @@ int l3es_interp_coarse_mse(l3es_interp_plan* p, const void* u_hat_fine, const fl
   const long long per = p->dim == 3 ? (long long)c * c * c : (long long)c * c;
   const double inv_size = 1.0 / ((double)p->dim * per);
   const int nblk = (int)std::min<long long>(1024, (3 * per + 255) / 256);
-  k_mse_resid<<<nblk, 256, 0, s>>>(p->gre, target, per, p->dim, inv_size, p->red);
-  k_mse_sum<<<1, 256, 0, s>>>(p->red, nblk, inv_size, loss_dev);
+  pdl_launch(k_mse_resid, nblk, 256, 0, s, p->gre, target, per, p->dim, inv_size, p->red);
+  pdl_launch(k_mse_sum, 1, 256, 0, s, p->red, nblk, inv_size, loss_dev);
   rc = cuda_check(cudaGetLastError(), "l3es_interp_coarse_mse launch");
   if (rc != L3ES_OK || !grad) return rc;
   rc = l3es_rfftn(p->coarse, p->gre, p->g, stream);  // V = rfftn_c(residual)
@@ -1158,16 +1177,16 @@ int l3es_interp_coarse_mse(l3es_interp_plan* p, const void* u_hat_fine, const fl
   const float scale = (float)(0.5 / std::pow((double)N, p->dim));
   const dim3 gb((unsigned)((cs + 255) / 256), 3);
   if (p->dim == 3)
-    k_uncrop_grad<3><<<gb, 256, 0, s>>>(p->g, p->hcs, c, N, cs, 3, scale, (float2*)grad);
+    pdl_launch(k_uncrop_grad<3>, gb, 256, 0, s, p->g, p->hcs, c, N, cs, 3, scale, (float2*)grad);
   else
-    k_uncrop_grad<2><<<gb, 256, 0, s>>>(p->g, p->hcs, c, N, cs, 2, scale, (float2*)grad);
+    pdl_launch(k_uncrop_grad<2>, gb, 256, 0, s, p->g, p->hcs, c, N, cs, 2, scale, (float2*)grad);
   return cuda_check(cudaGetLastError(), "l3es_interp_coarse_mse launch");
 }
 
 int l3es_shift(const double* r, const double* dr, int64_t n, double scale, double box, double* out, void* stream) {
   if (!r || !dr || !out) return fail(L3ES_EINVAL, "l3es_shift: null argument");
   if (n <= 0) return n == 0 ? L3ES_OK : fail(L3ES_EINVAL, "l3es_shift: n < 0");
-  k_shift<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(r, dr, n, scale, box, out);
+  pdl_launch(k_shift, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, r, dr, n, scale, box, out);
   return cuda_check(cudaGetLastError(), "l3es_shift launch");
 }
 

@@ -142,6 +142,7 @@ static std::vector<float2> twiddles(int n) {
 // FP32 and accumulated in float-float (Ff), combined across warps and blocks in FP64.
 __global__ void __launch_bounds__(256)
 k_energy_partial(const float2* __restrict__ uh, long long cs, int h, int nblk, double* __restrict__ partial) {
+  pdl_begin();
   const int batch = blockIdx.y;
   const float4* ub = reinterpret_cast<const float4*>(uh + (long long)batch * 3 * cs);
   const unsigned pairs = (unsigned)(3 * cs / 2), uh_ = (unsigned)h;  // 3 cs < 2^32 for N <= 512
@@ -158,6 +159,7 @@ k_energy_partial(const float2* __restrict__ uh, long long cs, int h, int nblk, d
 
 __global__ void __launch_bounds__(256)
 k_sum_partials(const double* __restrict__ partial, int n, double scale, double* __restrict__ out) {
+  pdl_begin();
   __shared__ double red[32];
   const int batch = blockIdx.x;
   double s = 0.0;
@@ -620,7 +622,7 @@ int l3es::energy_partials(const Ctx& c, const float2* uh, cudaStream_t s) {
   // 8 blocks of 256 threads per SM of a 152-SM GB300, fewer when the field is small
   const int nblk = (int)std::min<long long>(std::min<long long>(c.npartial, 8 * 152), (3 * c.cs / 2 + 255) / 256);
   L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
-              k_energy_partial<<<dim3(nblk, c.batch), 256, 0, s>>>(uh, c.cs, c.h, nblk, c.partial));
+              pdl_launch(k_energy_partial, dim3(nblk, c.batch), 256, 0, s, uh, c.cs, c.h, nblk, c.partial));
   return nblk;
 }
 
@@ -650,16 +652,17 @@ static int run_steps(l3es_plan* plan, void* u_hat, float* u_out, int32_t nsteps,
     if (d.forcing == L3ES_FORCING_EKIN_TOT) {
       if (c.dim == 3)
         L3ES_LAUNCH(c, KK_FORCE, 0.0, s,
-                    k_force_ekin<3><<<c.batch, 256, 0, s>>>(S, c.cs, c.partial, nke, c.e0, d.dt, c.n, d.kf,
+                    pdl_launch(k_force_ekin<3>, c.batch, 256, 0, s, S, c.cs, c.partial, nke, c.e0, d.dt, c.n, d.kf,
                                                             inv_n2d, eps64, einj, ke_final));
       else
         L3ES_LAUNCH(c, KK_FORCE, 0.0, s,
-                    k_force_ekin<2><<<c.batch, 256, 0, s>>>(S, c.cs, c.partial, nke, c.e0, d.dt, c.n, d.kf,
+                    pdl_launch(k_force_ekin<2>, c.batch, 256, 0, s, S, c.cs, c.partial, nke, c.e0, d.dt, c.n, d.kf,
                                                             inv_n2d, eps64, einj, ke_final));
     } else {
       if (e_inj_dev) L3ES_TRY_CUDA(cudaMemsetAsync(einj, 0, sizeof(double) * c.batch, s), "l3es_step memset");
       if (ke_final)
-        L3ES_LAUNCH(c, KK_REDUCE, 0.0, s, k_sum_partials<<<c.batch, 256, 0, s>>>(c.partial, nke, 0.5 * inv_n2d, ke_final));
+        L3ES_LAUNCH(c, KK_REDUCE, 0.0, s, pdl_launch(k_sum_partials, c.batch, 256, 0, s, c.partial, nke,
+                                                     0.5 * inv_n2d, ke_final));
     }
   }
   if (nsteps == 0 && ke_dev) {
@@ -720,7 +723,7 @@ int l3es_kinetic_energy(l3es_plan* plan, const void* u_hat, double* out_dev, voi
   cudaStream_t s = (cudaStream_t)stream;
   const int nblk = energy_partials(c, (const float2*)u_hat, s);
   const double scale = 0.5 / std::pow((double)c.n, 2 * c.dim);
-  L3ES_LAUNCH(c, KK_REDUCE, 0.0, s, k_sum_partials<<<c.batch, 256, 0, s>>>(c.partial, nblk, scale, out_dev));
+  L3ES_LAUNCH(c, KK_REDUCE, 0.0, s, pdl_launch(k_sum_partials, c.batch, 256, 0, s, c.partial, nblk, scale, out_dev));
   return cuda_check(cudaGetLastError(), "l3es_kinetic_energy launch");
 }
 

@@ -86,6 +86,7 @@ template <int DIM>
 __global__ void __launch_bounds__(kSphThreads)
 k_sph_bin(const double* __restrict__ r, const double* __restrict__ u, double dt, long long np, SphGeom g,
           double* __restrict__ xw, int* __restrict__ cell, int* __restrict__ count) {
+  pdl_begin();
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= np) return;
   int ci[DIM];
@@ -106,6 +107,7 @@ k_sph_bin(const double* __restrict__ r, const double* __restrict__ u, double dt,
 // contiguous segment, the segment sums are scanned with warp shuffles
 __global__ void __launch_bounds__(1024)
 k_sph_scan(const int* __restrict__ count, int ncell, int* __restrict__ start, int* __restrict__ cursor) {
+  pdl_begin();
   __shared__ int warp_sum[32];
   const int seg = (ncell + 1023) / 1024;
   const int b = threadIdx.x * seg, e = min(ncell, b + seg);
@@ -141,6 +143,7 @@ k_sph_scan(const int* __restrict__ count, int ncell, int* __restrict__ start, in
 
 __global__ void __launch_bounds__(kSphThreads)
 k_sph_scatter(const int* __restrict__ cell, long long np, int* __restrict__ cursor, int* __restrict__ perm0) {
+  pdl_begin();
   const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (j < np) perm0[atomicAdd(cursor + cell[j], 1)] = (int)j;
 }
@@ -152,6 +155,7 @@ __global__ void __launch_bounds__(kSphThreads)
 k_sph_order(const int* __restrict__ perm0, const int* __restrict__ cell, const int* __restrict__ start,
             const double* __restrict__ xw, const double* __restrict__ u, long long np, SphGeom g,
             int* __restrict__ perm, float4* __restrict__ xs, float4* __restrict__ us) {
+  pdl_begin();
   const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= np) return;
   const int j = perm0[s];
@@ -240,6 +244,7 @@ __global__ void __launch_bounds__(kSphThreads)
 k_sph_density(const float4* __restrict__ xs, const int* __restrict__ start, const int* __restrict__ perm,
               const double* __restrict__ xw, long long np, SphGeom g, double m_sigma, double p_ref,
               float2* __restrict__ rp, double* __restrict__ rho_out) {
+  pdl_begin();
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long i = gt / kSphLanes;
   const int lane = (int)(gt % kSphLanes);
@@ -287,6 +292,7 @@ struct SphAccelArgs {
 // Relaxation acceleration = acc_p + acc_tvf / 2.
 template <int DIM, int MODE>
 __global__ void __launch_bounds__(kSphThreads) k_sph_accel(SphAccelArgs a, SphGeom g) {
+  pdl_begin();
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long i = gt / kSphLanes;
   const int lane = (int)(gt % kSphLanes);
@@ -401,17 +407,17 @@ static int sph_build(l3es_sph_plan* p, const double* r, const double* u_pred, do
   if (rc != L3ES_OK) return rc;
   const unsigned pb = (unsigned)((np + kSphThreads - 1) / kSphThreads);
   if (p->dim == 3) {
-    k_sph_bin<3><<<pb, kSphThreads, 0, s>>>(r, u_pred, dt, np, p->g, p->xw, p->cell, p->count);
+    pdl_launch(k_sph_bin<3>, pb, kSphThreads, 0, s, r, u_pred, dt, np, p->g, p->xw, p->cell, p->count);
   } else {
-    k_sph_bin<2><<<pb, kSphThreads, 0, s>>>(r, u_pred, dt, np, p->g, p->xw, p->cell, p->count);
+    pdl_launch(k_sph_bin<2>, pb, kSphThreads, 0, s, r, u_pred, dt, np, p->g, p->xw, p->cell, p->count);
   }
-  k_sph_scan<<<1, 1024, 0, s>>>(p->count, p->ncell, p->start, p->cursor);
-  k_sph_scatter<<<pb, kSphThreads, 0, s>>>(p->cell, np, p->cursor, p->perm0);
+  pdl_launch(k_sph_scan, 1, 1024, 0, s, p->count, p->ncell, p->start, p->cursor);
+  pdl_launch(k_sph_scatter, pb, kSphThreads, 0, s, p->cell, np, p->cursor, p->perm0);
   if (p->dim == 3)
-    k_sph_order<3><<<pb, kSphThreads, 0, s>>>(p->perm0, p->cell, p->start, p->xw, u, np, p->g, p->perm, p->xs,
+    pdl_launch(k_sph_order<3>, pb, kSphThreads, 0, s, p->perm0, p->cell, p->start, p->xw, u, np, p->g, p->perm, p->xs,
                                                u ? p->us : nullptr);
   else
-    k_sph_order<2><<<pb, kSphThreads, 0, s>>>(p->perm0, p->cell, p->start, p->xw, u, np, p->g, p->perm, p->xs,
+    pdl_launch(k_sph_order<2>, pb, kSphThreads, 0, s, p->perm0, p->cell, p->start, p->xw, u, np, p->g, p->perm, p->xs,
                                                u ? p->us : nullptr);
   return cuda_check(cudaGetLastError(), "l3es_sph cell list");
 }
@@ -420,10 +426,12 @@ static void sph_density(l3es_sph_plan* p, long long np, double p_ref, double* rh
   const unsigned pb = (unsigned)((np * kSphLanes + kSphThreads - 1) / kSphThreads);
   const double m_sigma = p->mass * p->sigma;
   if (p->dim == 3)
-    k_sph_density<3><<<pb, kSphThreads, 0, s>>>(p->xs, p->start, p->perm, p->xw, np, p->g, m_sigma, p_ref, p->rp,
+    pdl_launch(k_sph_density<3>, pb, kSphThreads, 0, s, p->xs, p->start, p->perm, p->xw, np, p->g, m_sigma, p_ref,
+               p->rp,
                                                  rho_out);
   else
-    k_sph_density<2><<<pb, kSphThreads, 0, s>>>(p->xs, p->start, p->perm, p->xw, np, p->g, m_sigma, p_ref, p->rp,
+    pdl_launch(k_sph_density<2>, pb, kSphThreads, 0, s, p->xs, p->start, p->perm, p->xw, np, p->g, m_sigma, p_ref,
+               p->rp,
                                                  rho_out);
 }
 
@@ -431,9 +439,9 @@ template <int MODE>
 static void sph_accel(l3es_sph_plan* p, SphAccelArgs& a, cudaStream_t s) {
   const unsigned pb = (unsigned)((a.np * kSphLanes + kSphThreads - 1) / kSphThreads);
   if (p->dim == 3)
-    k_sph_accel<3, MODE><<<pb, kSphThreads, 0, s>>>(a, p->g);
+    pdl_launch(k_sph_accel<3, MODE>, pb, kSphThreads, 0, s, a, p->g);
   else
-    k_sph_accel<2, MODE><<<pb, kSphThreads, 0, s>>>(a, p->g);
+    pdl_launch(k_sph_accel<2, MODE>, pb, kSphThreads, 0, s, a, p->g);
 }
 
 static SphAccelArgs sph_args(l3es_sph_plan* p, long long np, double u_ref) {

@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(XStageCfg<N, XW, EE>::THREADS)
 kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, float2* __restrict__ T_,
          float2* __restrict__ C, const __grid_constant__ XStage st, float2* __restrict__ w, float2* __restrict__ wx,
          long long fs, const float2* __restrict__ tw) {
+  pdl_begin();
   using K = XStageCfg<N, XW, EE>;
   constexpr int E = K::E, T = K::T, H = N / 2 + 1;
   constexpr int NMID = DIM == 3 ? N : 1;
@@ -229,6 +230,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256)
 k_band_coefficient(const float2* __restrict__ us, long long cs, int N, int kf, double inv_n2d, double eps_inj,
                    double* __restrict__ band_scale) {
+  pdl_begin();
   band_coefficient<DIM>(us + (long long)blockIdx.x * 3 * cs, cs, N, kf, inv_n2d, eps_inj, 1e-30,
                         band_scale + blockIdx.x);
 }
