@@ -33,8 +33,7 @@
 //    memory. A host whose device memory is spoken for should make that first call
 //    (a warm-up call with a small np) before it hands the device to its own pool,
 //    or run with CUDA_MODULE_LOADING=EAGER;
-//  - np is at most 128 (2^31 - 1) particles (one thread per particle, the grid-x
-//    limit).
+//  - np is at most 128 (2^31 - 1) particles.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -113,20 +112,11 @@ extern "C" int l3es_interp_dft_noalloc(int32_t dim, int32_t n_fine, int32_t ckp_
   const long long cs = dim == 3 ? (long long)N * N * (N / 2 + 1) : (long long)N * (N / 2 + 1);
   const float scale = (float)std::pow((double)c / N, dim);
   const unsigned blocks = (unsigned)((hcs + 255) / 256);
-  const unsigned pb = (unsigned)((np + 127) / 128);
-  const size_t smem = sizeof(float2) * dim * c * 128;
-  if (dim == 3) {
-    k_crop<3><<<dim3(blocks, 3), 256, 0, s>>>((const float2*)u_hat_fine, cs, N, hh, hcs, c, scale);
-    rc = cuda_check(cudaFuncSetAttribute(k_dft_interp<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                    "l3es_interp_dft_noalloc: shared memory attribute");
-    if (rc != L3ES_OK) return rc;
-    k_dft_interp<3><<<pb, 128, smem, s>>>(hh, hcs, c, 3, r, np, u_r, 0.0, nullptr);
-  } else {
-    k_crop<2><<<dim3(blocks, 3), 256, 0, s>>>((const float2*)u_hat_fine, cs, N, hh, hcs, c, scale);
-    rc = cuda_check(cudaFuncSetAttribute(k_dft_interp<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                    "l3es_interp_dft_noalloc: shared memory attribute");
-    if (rc != L3ES_OK) return rc;
-    k_dft_interp<2><<<pb, 128, smem, s>>>(hh, hcs, c, 2, r, np, u_r, 0.0, nullptr);
-  }
+  if (dim == 3)
+    pdl_launch(k_crop<3>, dim3(blocks, 3), 256, 0, s, (const float2*)u_hat_fine, cs, N, hh, hcs, c, scale);
+  else
+    pdl_launch(k_crop<2>, dim3(blocks, 3), 256, 0, s, (const float2*)u_hat_fine, cs, N, hh, hcs, c, scale);
+  rc = cuda_check(dft_launch(dim, hh, hcs, c, r, np, u_r, 0.0, nullptr, s), "l3es_interp_dft_noalloc launch");
+  if (rc != L3ES_OK) return rc;
   return cuda_check(cudaGetLastError(), "l3es_interp_dft_noalloc launch");
 }

@@ -937,17 +937,9 @@ int l3es_interp_coarse_spectrum(l3es_interp_plan* p, void* out, void* stream) {
 // Exact interpolation (dft backend) at r into u_r, with the fused Euler shift when r_out.
 static int dft_eval(l3es_interp_plan* p, const double* r, int64_t np, double* u_r, double dt, double* r_out,
                     cudaStream_t s) {
-  const int ncomp = p->dim;
-  const unsigned pb = (unsigned)((np + 127) / 128);
-  const size_t smem = sizeof(float2) * p->dim * p->c * 128;
-  if (p->dim == 3) {
-    cudaFuncSetAttribute(k_dft_interp<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    pdl_launch(k_dft_interp<3>, pb, 128, smem, s, p->hh, p->hcs, p->c, ncomp, r, np, u_r, dt, r_out);
-  } else {
-    cudaFuncSetAttribute(k_dft_interp<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    pdl_launch(k_dft_interp<2>, pb, 128, smem, s, p->hh, p->hcs, p->c, ncomp, r, np, u_r, dt, r_out);
-  }
-  return cuda_check(cudaGetLastError(), "l3es_interp (dft) launch");
+  if (!dft_supported(p->dim, p->c))
+    return fail(L3ES_ECUDA, "l3es_interp (dft) launch: ckp_N too large for the exact interpolation's phase tables");
+  return cuda_check(dft_launch(p->dim, p->hh, p->hcs, p->c, r, np, u_r, dt, r_out, s), "l3es_interp (dft) launch");
 }
 
 // NUFFT gather at r from the prepared fine grid (nufft_grid), visiting particles in the
