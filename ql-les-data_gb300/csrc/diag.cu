@@ -1,8 +1,7 @@
 // Diagnostics of the drivers (l3es/spectral_solver.py:123-127, :318-320;
 // l3es/utils.py:35-97, :300-315) with FP64 partial sums. Each point's or mode's
-// contribution is formed in FP32 and accumulated in float-float (Ff, ~48 bits) or FP64
-// (field statistics); FP64 arithmetic is scarce on this GPU. The spectral loops run one
-// warp per contiguous half-axis row, so no per-element index division is needed.
+// contribution is formed in FP32 and accumulated in float-float (Ff, ~48 bits); FP64
+// arithmetic is scarce on this GPU and only combines the threads' sums.
 //   l3es_field_stats      max |u_c| per component and 0.5 mean sum u^2 of a physical field
 //   l3es_dissipation      nu <|curl u|^2> by Parseval on the half spectrum
 //   l3es_energy_spectrum  shell sums E(k), shells int(|k| + 0.5)
@@ -14,7 +13,24 @@
 
 namespace l3es {
 
-// per block: max |u_c| for c = 0..2 and sum_c u_c^2, over ps values per component
+// Sum of M non-negative FP32 terms in FP64: float-float, or FP64 throughout where that is
+// not finite (its error terms turn an infinite or overflowing sum into NaN).
+template <int M>
+__device__ __forceinline__ double ff_sum(const float (&e)[M]) {
+  Ff a{e[0], 0.f};
+#pragma unroll
+  for (int i = 1; i < M; ++i) a = ff_add(a, e[i]);
+  double s = (double)a.hi + (double)a.lo;
+  if (!isfinite(a.hi)) {
+    s = 0.0;
+    for (int i = 0; i < M; ++i) s += (double)e[i];
+  }
+  return s;
+}
+
+// per block: max |u_c| for c = 0..2 and sum_c u_c^2, over ps values per component; four
+// points per thread in flight, summed in float-float before one FP64 addition (an FP64
+// addition per point and one point in flight took 68 us on a 256^3 field)
 __global__ void __launch_bounds__(256)
 k_field_stats(const float* __restrict__ u, long long ps, int nblk, double* __restrict__ partial) {
   pdl_begin();
@@ -22,15 +38,24 @@ k_field_stats(const float* __restrict__ u, long long ps, int nblk, double* __res
   const float* ub = u + (long long)batch * 3 * ps;
   float mx[3] = {0.f, 0.f, 0.f};
   double s = 0.0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ps; i += (long long)nblk * blockDim.x) {
-    float e = 0.f;
+  const long long step = (long long)nblk * blockDim.x;
+  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < ps; i0 += 4 * step) {
+    float v[4][3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const float v = ub[c * ps + i];
-      mx[c] = fmaxf(mx[c], fabsf(v));
-      e = fmaf(v, v, e);
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[q][c] = i0 + q * step < ps ? __ldg(ub + c * ps + i0 + q * step) : 0.f;
+    float e[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      e[q] = 0.f;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        mx[c] = fmaxf(mx[c], fabsf(v[q][c]));
+        e[q] = fmaf(v[q][c], v[q][c], e[q]);
+      }
     }
-    s += (double)e;
+    s += ff_sum(e);
   }
   __shared__ float smx[3][32];
   __shared__ double ss[32];
@@ -60,20 +85,36 @@ k_field_stats(const float* __restrict__ u, long long ps, int nblk, double* __res
   }
 }
 
-// out[batch*4 + {0,1,2}] = max |u_c|, out[batch*4 + 3] = 0.5 mean sum u^2
-__global__ void k_field_stats_final(const double* __restrict__ partial, int nblk, double inv_ps,
-                                    double* __restrict__ out) {
+// out[batch*4 + {0,1,2}] = max |u_c|, out[batch*4 + 3] = 0.5 mean sum u^2; one block per
+// trajectory (a single thread walking 608 partials took 163 us)
+__global__ void __launch_bounds__(256)
+k_field_stats_final(const double* __restrict__ partial, int nblk, double inv_ps, double* __restrict__ out) {
   pdl_begin();
   const int batch = blockIdx.x;
-  if (threadIdx.x != 0) return;
   double m[3] = {0.0, 0.0, 0.0}, s = 0.0;
-  for (int b = 0; b < nblk; ++b) {
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
     const double* p = partial + ((long long)batch * nblk + b) * 4;
     for (int c = 0; c < 3; ++c) m[c] = fmax(m[c], p[c]);
     s += p[3];
   }
-  for (int c = 0; c < 3; ++c) out[batch * 4 + c] = m[c];
-  out[batch * 4 + 3] = 0.5 * s * inv_ps;
+  __shared__ double red[8][4];
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    for (int c = 0; c < 3; ++c) m[c] = fmax(m[c], __shfl_xor_sync(0xffffffffu, m[c], o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    double* o = red[threadIdx.x >> 5];
+    o[0] = m[0];
+    o[1] = m[1];
+    o[2] = m[2];
+    o[3] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double t = red[0][threadIdx.x];
+    for (int w = 1; w < 8; ++w) t = threadIdx.x < 3 ? fmax(t, red[w][threadIdx.x]) : t + red[w][threadIdx.x];
+    out[batch * 4 + threadIdx.x] = threadIdx.x < 3 ? t : 0.5 * t * inv_ps;
+  }
 }
 
 // dissipation partials: Parseval sum of w |C|^2 over the half spectrum, C = k x u_hat
@@ -81,14 +122,10 @@ __global__ void k_field_stats_final(const double* __restrict__ partial, int nblk
 // kh = N/2 planes, and i C is not Hermitian there (kz = +N/2 for both partners), so
 // those planes use |(C(k) - conj C(-k)) / 2|^2 with weight 1 (utils.py:312-315).
 template <int DIM>
-__device__ __forceinline__ void curl_at(const float2* __restrict__ ub, long long cs, int n, int kxi, int mid, int kh,
-                                        float* re, float* im) {
-  const int h = n / 2 + 1;
-  const int nmid = DIM == 3 ? n : 1;
-  const long long i = ((long long)kxi * nmid + mid) * h + kh;
+__device__ __forceinline__ void curl_of(const float2* v, int n, int kxi, int mid, int kh, float* re, float* im) {
   float k0, k1, k2;
   kvec<DIM>(kfull(kxi, n), DIM == 3 ? kfull(mid, n) : 0, kh, k0, k1, k2);
-  const float2 a = ub[i], b = ub[cs + i], c = ub[2 * cs + i];
+  const float2 a = v[0], b = v[1], c = v[2];
   // (k x u)_x = k1 c - k2 b, (k x u)_y = k2 a - k0 c, (k x u)_z = k0 b - k1 a
   re[0] = k1 * c.x - k2 * b.x;
   im[0] = k1 * c.y - k2 * b.y;
@@ -98,26 +135,40 @@ __device__ __forceinline__ void curl_at(const float2* __restrict__ ub, long long
   im[2] = k0 * b.y - k1 * a.y;
 }
 
+// One mode per thread and turn over the flat half spectrum (a warp per 129-mode row left
+// every fifth turn to one lane), two modes in flight.
 template <int DIM>
 __global__ void __launch_bounds__(256)
 k_diss_partial(const float2* __restrict__ uh, long long cs, int n, int nblk, double* __restrict__ partial) {
   pdl_begin();
   const int batch = blockIdx.y;
   const float2* ub = uh + (long long)batch * 3 * cs;
-  const int h = n / 2 + 1;
-  const int nmid = DIM == 3 ? n : 1;
-  const long long rows = cs / h;
-  const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+  const unsigned h = (unsigned)(n / 2 + 1), nmid = DIM == 3 ? (unsigned)n : 1u, ucs = (unsigned)cs;  // cs < 2^31
+  const unsigned step = (unsigned)nblk * blockDim.x;
   Ff s{0.f, 0.f};
-  for (long long r = (long long)blockIdx.x * wpb + (threadIdx.x >> 5); r < rows; r += (long long)nblk * wpb) {
-    const int mid = (int)(r % nmid), kxi = (int)(r / nmid);
-    for (int kh = lane; kh < h; kh += 32) {
+  for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < ucs; i0 += 2 * step) {
+    float2 v[2][3];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const unsigned i = i0 + q * step;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[q][c] = i < ucs ? __ldg(ub + c * cs + i) : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const unsigned i = i0 + q * step;
+      if (i >= ucs) continue;
+      const unsigned row = i / h;
+      const int kh = (int)(i - row * h), mid = (int)(row % nmid), kxi = (int)(row / nmid);
       float re[3], im[3];
-      curl_at<DIM>(ub, cs, n, kxi, mid, kh, re, im);
+      curl_of<DIM>(v[q], n, kxi, mid, kh, re, im);
       float e = 0.f;
       if (kh == 0 || kh == n / 2) {
+        const int mx = (n - kxi) % n, mm = DIM == 3 ? (n - mid) % n : 0;
+        const long long o = ((long long)mx * nmid + mm) * h + kh;
+        const float2 w[3] = {ub[o], ub[cs + o], ub[2 * cs + o]};
         float re2[3], im2[3];
-        curl_at<DIM>(ub, cs, n, (n - kxi) % n, DIM == 3 ? (n - mid) % n : 0, kh, re2, im2);
+        curl_of<DIM>(w, n, mx, mm, kh, re2, im2);
         // Hermitian part of i C is i (C(k) - conj C(-k)) / 2
         for (int c = 0; c < 3; ++c) {
           const float hr = 0.5f * (re[c] - re2[c]), hi = 0.5f * (im[c] + im2[c]);
@@ -133,47 +184,80 @@ k_diss_partial(const float2* __restrict__ uh, long long cs, int n, int nblk, dou
   block_sum_store_ff(s, partial, batch * nblk + blockIdx.x);
 }
 
-// energy spectrum: per-block shared-memory histograms of (weight, weight*|u_hat|^2)
-// over shells int(|k| + 0.5) < n, merged with FP64 atomics into acc[batch][2][n]
+// Energy spectrum over shells int(|k| + 0.5) < n: per-block shared-memory histograms of
+// the mode count and of weight * |u_hat|^2, merged with FP64 atomics into
+// acc[batch][2][n]. The shell depends on the magnitudes of the wavenumbers only, so a warp
+// takes all rows (+-a, +-b) and (+-b, +-a) of one pair a >= b (2D: +-a) at once, sums a
+// mode's energies over them in float-float (up to 8 rows, 24 loads in flight per lane) and
+// makes one shared FP64 addition for the lot: those atomics are a compare-and-swap loop,
+// and two per mode took 289 us on a 256^3 spectrum. shell int(|k| + 0.5): |k|^2 is an
+// integer below 3 (n/2)^2, whose square root is never within 1/(8|k|) of a half integer,
+// far more than the FP32 rounding.
 template <int DIM>
 __global__ void __launch_bounds__(256)
 k_spectrum(const float2* __restrict__ uh, long long cs, int n, int nblk, double scale, double* __restrict__ acc) {
   pdl_begin();
-  extern __shared__ double hist[];  // [2][n]
+  extern __shared__ double hist[];  // [n] energies, then [n] counts (32-bit)
+  unsigned* cnt = reinterpret_cast<unsigned*>(hist + n);
   const int batch = blockIdx.y;
-  for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) hist[i] = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    hist[i] = 0.0;
+    cnt[i] = 0u;
+  }
   __syncthreads();
   const float2* ub = uh + (long long)batch * 3 * cs;
-  const int h = n / 2 + 1;
-  const int nmid = DIM == 3 ? n : 1;
-  const long long rows = cs / h;
+  const int h = n / 2 + 1, m = n / 2;
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-  for (long long r = (long long)blockIdx.x * wpb + (threadIdx.x >> 5); r < rows; r += (long long)nblk * wpb) {
-    const int kx = kfull((int)(r / nmid), n);
-    const int km = DIM == 3 ? kfull((int)(r % nmid), n) : 0;
-    const float2* row = ub + r * h;
-    for (int kh = lane; kh < h; kh += 32) {
-      // shell int(|k| + 0.5): |k|^2 is an integer below 3 (n/2)^2, whose square root is
-      // never within 1/(8|k|) of a half integer, far more than the FP32 rounding
-      const int k2 = kx * kx + km * km + kh * kh;
-      const int shell = (int)(sqrtf((float)k2) + 0.5f);
-      float e = 0.f;
+  const int tasks = DIM == 3 ? (m + 1) * (m + 2) / 2 : m + 1;
+  for (int t = blockIdx.x * wpb + (threadIdx.x >> 5); t < tasks; t += nblk * wpb) {
+    int a = t, b = 0;
+    if (DIM == 3) {  // t = a (a + 1) / 2 + b, 0 <= b <= a
+      a = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
+      while (a * (a + 1) / 2 > t) --a;
+      while ((a + 1) * (a + 2) / 2 <= t) ++a;
+      b = t - a * (a + 1) / 2;
+    }
+    // storage indices of +-a, +-b: 0 and n/2 stand once
+    const int na = a == 0 || a == m ? 1 : 2, nb = DIM == 2 ? 1 : b == 0 || b == m ? 1 : 2;
+    const int rows = na * nb * (DIM == 3 && a != b ? 2 : 1);
+    constexpr int R = DIM == 3 ? 8 : 2;
+    unsigned off[R];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float2 v = row[c * cs + kh];
-        e = fmaf(v.x, v.x, fmaf(v.y, v.y, e));
+    for (int r = 0; r < R; ++r) {
+      const int sw = r / (na * nb), rr = r - sw * (na * nb);
+      const int ia = rr % na == 0 ? a : n - a, ib = rr / na == 0 ? b : n - b;
+      const int x = sw ? ib : ia, y = sw ? ia : ib;
+      off[r] = r < rows ? (DIM == 3 ? (unsigned)(x * n + y) : (unsigned)x) * (unsigned)h : 0u;
+    }
+    for (int kh = lane; kh < h; kh += 32) {
+      float2 v[R][3];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[r][c] = r < rows ? __ldg(ub + c * cs + off[r] + kh) : make_float2(0.f, 0.f);
+      float e[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        e[r] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) e[r] = fmaf(v[r][c].x, v[r][c].x, fmaf(v[r][c].y, v[r][c].y, e[r]));
       }
+      const int k2 = a * a + b * b + kh * kh;
+      const int shell = (int)(sqrtf((float)k2) + 0.5f);
       if (shell < n) {
-        const double w = (kh == 0 || kh == n / 2) ? 1.0 : 2.0;
-        atomicAdd(&hist[shell], w);
-        atomicAdd(&hist[n + shell], w * scale * (double)e);
+        const int w = (kh == 0 || kh == n / 2) ? 1 : 2;
+        atomicAdd(cnt + shell, (unsigned)(w * rows));
+        atomicAdd(hist + shell, (w * scale) * ff_sum(e));
       }
     }
   }
   __syncthreads();
-  double* a = acc + (long long)batch * 2 * n;
-  for (int i = threadIdx.x; i < 2 * n; i += blockDim.x)
-    if (hist[i] != 0.0) atomicAdd(&a[i], hist[i]);
+  double* ab = acc + (long long)batch * 2 * n;
+  for (int i = threadIdx.x; i < n; i += blockDim.x)
+    if (cnt[i]) {
+      atomicAdd(&ab[i], (double)cnt[i]);
+      atomicAdd(&ab[n + i], hist[i]);
+    }
 }
 
 // sum of n partials per trajectory times scale
@@ -218,7 +302,7 @@ int l3es_field_stats(l3es_plan* plan, const float* u, double* out_dev, void* str
   L3ES_LAUNCH(c, KK_REDUCE, 4.0 * 3.0 * c.ps * c.batch, s,
               pdl_launch(k_field_stats, dim3(nblk, c.batch), 256, 0, s, u, c.ps, nblk, c.partial));
   L3ES_LAUNCH(c, KK_REDUCE, 0.0, s,
-              pdl_launch(k_field_stats_final, c.batch, 32, 0, s, c.partial, nblk, 1.0 / (double)c.ps, out_dev));
+              pdl_launch(k_field_stats_final, c.batch, 256, 0, s, c.partial, nblk, 1.0 / (double)c.ps, out_dev));
   return cuda_check(cudaGetLastError(), "l3es_field_stats launch");
 }
 
@@ -226,7 +310,7 @@ int l3es_dissipation(l3es_plan* plan, const void* u_hat, double nu, double* out_
   if (!plan || !u_hat || !out_dev) return fail(L3ES_EINVAL, "l3es_dissipation: null argument");
   const Ctx& c = plan_ctx(plan);
   cudaStream_t s = (cudaStream_t)stream;
-  const int nblk = (int)std::min<long long>(608, (c.cs / c.h + 7) / 8);  // one warp per row
+  const int nblk = (int)std::min<long long>(608, (c.cs + 511) / 512);
   const double scale = nu / std::pow((double)c.n, 2 * c.dim);
   if (c.dim == 3)
     L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
@@ -247,10 +331,12 @@ int l3es_energy_spectrum(l3es_plan* plan, const void* u_hat, double mul_fac, dou
   const int n = c.n;
   int rc = cuda_check(cudaMemsetAsync(c.partial, 0, sizeof(double) * 2 * n * c.batch, s), "l3es_energy_spectrum");
   if (rc != L3ES_OK) return rc;
-  const int nblk = (int)std::min<long long>(608, (c.cs / c.h + 7) / 8);  // one warp per row
+  // one warp per pair of wavenumber magnitudes, two blocks per SM
+  const long long tasks = c.dim == 3 ? (long long)c.h * (c.h + 1) / 2 : c.h;
+  const int nblk = (int)std::min<long long>(304, (tasks + 7) / 8);
   // |u_hat / n^dim|^2 * mul_fac (utils.py:82-86)
   const double scale = mul_fac / std::pow((double)n, 2 * c.dim);
-  const size_t smem = sizeof(double) * 2 * n;
+  const size_t smem = (sizeof(double) + sizeof(unsigned)) * n;
   if (c.dim == 3)
     L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
                 pdl_launch(k_spectrum<3>, dim3(nblk, c.batch), 256, smem, s, (const float2*)u_hat, c.cs, n, nblk, scale,
