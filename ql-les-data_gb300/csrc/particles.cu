@@ -4,9 +4,8 @@
 //
 // Data flow of one particle update (fused path of the combined loop):
 //   fine u_hat (N)  --k_crop-->  coarse half spectrum Hh (c)       [spectral_filtering]
-//   Hh --k_nufft_prep--> fine NUFFT grid G (n = 2c), deconvolved by the ES kernel's
-//   Fourier transform --3 c2c passes--> Re g (float) --k_nufft_gather--> u_r,
-//   advected r (particles binned by cell so warps gather neighbouring grid points)
+//   Hh --k_grid_x, _y, _z--> Re of the fine NUFFT grid (n = 2c), deconvolved by the ES
+//   kernel's Fourier transform --k_nufft_gather--> u_r, advected r
 // and, when the coarse field itself is wanted, irfftn(Hh) at c (write_u / plots).
 #include <cuda_runtime.h>
 
@@ -21,64 +20,146 @@
 namespace l3es {
 
 // ------------------------------------------------------------------------------
-// NUFFT grid: G(g) = Hhat(k) / (psi(kx) psi(ky) psi(kz)) at g = k mod n for k in
-// [-c/2, c/2-1]^dim (modes in fftshift order, as finufft receives them from
-// integrator.py:38-44), zero elsewhere. Hhat from the coarse half spectrum via
-// Hermitian symmetry. inv_psi: 1/psi_hat(k), k = -c/2..c/2-1.
+// NUFFT grid: Re of the inverse FFT over n^dim of G(g) = Hhat(k) / (psi(kx) psi(ky)
+// psi(kz)) at g = k mod n for k in [-c/2, c/2-1]^dim (modes in fftshift order, as finufft
+// receives them from integrator.py:38-44), zero elsewhere (n = 2c). Hhat from the coarse
+// half spectrum via Hermitian symmetry. inv_psi: 1/psi_hat(k), k = -c/2..c/2-1.
+// Three passes, none of which stores or reads the zeros: an axis not transformed yet
+// keeps its c modes in the order 0..c/2-1, -c/2..-1.
+//   grid_x  deconvolution + x transform of the c^(dim-1) columns -> [n][c][c] (2D [n][c])
+//   grid_y  (3D) y transform                                     -> [n][n][c]
+//   grid_z  half-axis transform, real part, components interleaved per grid point
+//           (float4 in 3D, float2 in 2D): one load per point and particle in the gather
 // ------------------------------------------------------------------------------
-template <int DIM>
-__global__ void __launch_bounds__(256)
-k_nufft_prep(const float2* __restrict__ hh, long long hcs, int c, const float* __restrict__ inv_psi,
-             float2* __restrict__ g, long long gcs, int n) {
+// index into an axis of c kept modes of FFT index g, or -1 where the padded axis is zero
+__device__ __forceinline__ int kept_mode(int g, int n, int c) {
+  return g < c / 2 ? g : g >= n - c / 2 ? g - (n - c) : -1;
+}
+
+// fields [blockIdx.y] = trajectory * DIM + component of hh ([trajectory][3][hcs])
+template <int DIM, int NG>
+__global__ void __launch_bounds__(KyCfg<NG>::THREADS)
+k_grid_x(const float2* __restrict__ hh, long long hcs, const float* __restrict__ inv_psi, float2* __restrict__ g,
+         const float2* __restrict__ tw) {
   pdl_begin();
-  const long long per = DIM == 3 ? (long long)n * n * n : (long long)n * n;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int comp = blockIdx.y;
-  if (i >= per) return;
-  int gx, gy, gz;
-  if (DIM == 3) {
-    gz = (int)(i % n);
-    gy = (int)((i / n) % n);
-    gx = (int)(i / ((long long)n * n));
-  } else {
-    gz = 0;
-    gy = (int)(i % n);
-    gx = (int)(i / n);
-  }
-  const int kx = gx < n / 2 ? gx : gx - n, ky = gy < n / 2 ? gy : gy - n, kz = gz < n / 2 ? gz : gz - n;
-  const int lo = -c / 2, hi = c / 2 - 1;
-  float2 out = make_float2(0.f, 0.f);
-  const bool in = kx >= lo && kx <= hi && ky >= lo && ky <= hi && (DIM == 2 || (kz >= lo && kz <= hi));
-  if (in) {
-    const int hc = c / 2 + 1;
-    const float2* h = hh + comp * hcs;
-    float2 v;
-    if (DIM == 3) {
-      if (kz >= 0) {
-        v = __ldg(h + ((long long)((kx + c) % c) * c + (ky + c) % c) * hc + kz);
-      } else {
-        const float2 t = __ldg(h + ((long long)((-kx + c) % c) * c + (-ky + c) % c) * hc + (-kz));
-        v = make_float2(t.x, -t.y);
-      }
-      const float s = inv_psi[kx + c / 2] * inv_psi[ky + c / 2] * inv_psi[kz + c / 2];
-      out = make_float2(v.x * s, v.y * s);
-    } else {
-      if (ky >= 0) {
-        v = __ldg(h + (long long)((kx + c) % c) * hc + ky);
-      } else {
-        const float2 t = __ldg(h + (long long)((-kx + c) % c) * hc + (-ky));
-        v = make_float2(t.x, -t.y);
-      }
-      const float s = inv_psi[kx + c / 2] * inv_psi[ky + c / 2];
-      out = make_float2(v.x * s, v.y * s);
+  using C = KyCfg<NG>;
+  constexpr int E = C::E, T = C::T, TWY = C::TWY, NC = NG / 2, HC = NC / 2 + 1;
+  constexpr int COLS = DIM == 3 ? NC * NC : NC;
+  __shared__ float2 sm[xpad_len<TWY>(NG) * TWY];
+  const int p = threadIdx.x % TWY, t = threadIdx.x / TWY;
+  const int col = blockIdx.x * TWY + p;
+  const bool ok = col < COLS;
+  const int f = blockIdx.y;
+  const float2* h = hh + (long long)(f / DIM * 3 + f % DIM) * hcs;
+  // wavenumbers of the other axes: my (3D), mz the half axis
+  const int yi = DIM == 3 ? col / NC : 0, zi = DIM == 3 ? col % NC : col;
+  const int my = yi < NC / 2 ? yi : yi - NC, mz = zi < NC / 2 ? zi : zi - NC;
+  const int sg = mz >= 0 ? 1 : -1;
+  const float sy = ok && DIM == 3 ? inv_psi[my + NC / 2] : 1.f, sz = ok ? inv_psi[mz + NC / 2] : 0.f;
+  float2 v[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int gx = t + T * e, xi = kept_mode(gx, NG, NC);
+    v[e] = make_float2(0.f, 0.f);
+    if (ok && xi >= 0) {
+      const int mx = xi < NC / 2 ? xi : xi - NC;
+      const int x = (sg * mx) & (NC - 1), y = (sg * my) & (NC - 1);
+      float2 a = __ldg(h + (DIM == 3 ? ((long long)x * NC + y) * HC : (long long)x * HC) + sg * mz);
+      if (sg < 0) a.y = -a.y;
+      const float s = DIM == 3 ? inv_psi[mx + NC / 2] * sy * sz : inv_psi[mx + NC / 2] * sz;
+      v[e] = make_float2(a.x * s, a.y * s);
     }
   }
-  g[comp * gcs + i] = out;
+  block_fft<NG, E, kInv, TWY>(v, sm + p, t, tw, 1);
+  if (ok) {
+    float2* o = g + (long long)f * NG * COLS + col;
+#pragma unroll
+    for (int e = 0; e < E; ++e) o[(long long)(t + T * e) * COLS] = v[e];
+  }
+}
+
+// in: [field][n][c][c], out: [field][n][n][c]; plane x = blockIdx.y, field = blockIdx.z
+template <int NG>
+__global__ void __launch_bounds__(KyCfg<NG>::THREADS)
+k_grid_y(const float2* __restrict__ in, float2* __restrict__ out, const float2* __restrict__ tw) {
+  pdl_begin();
+  using C = KyCfg<NG>;
+  constexpr int E = C::E, T = C::T, TWY = C::TWY, NC = NG / 2;
+  __shared__ float2 sm[xpad_len<TWY>(NG) * TWY];
+  const int p = threadIdx.x % TWY, t = threadIdx.x / TWY;
+  const int col = blockIdx.x * TWY + p;
+  const bool ok = col < NC;
+  const long long plane = (long long)blockIdx.z * NG + blockIdx.y;
+  const float2* src = in + plane * NC * NC + col;
+  float2 v[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int yi = kept_mode(t + T * e, NG, NC);
+    v[e] = ok && yi >= 0 ? __ldg(src + (long long)yi * NC) : make_float2(0.f, 0.f);
+  }
+  block_fft<NG, E, kInv, TWY>(v, sm + p, t, tw, 1);
+  if (ok) {
+    float2* o = out + plane * NG * NC + col;
+#pragma unroll
+    for (int e = 0; e < E; ++e) o[(long long)(t + T * e) * NC] = v[e];
+  }
+}
+
+// in: [trajectory][DIM][lines][c], out: [trajectory][lines][n] of DIM (padded to 4 in 3D)
+// real values; trajectory = blockIdx.y
+template <int DIM>
+struct GridVec {
+  using type = float4;
+};
+template <>
+struct GridVec<2> {
+  using type = float2;
+};
+
+template <int DIM, int NG>
+__global__ void __launch_bounds__(128)
+k_grid_z(const float2* __restrict__ in, typename GridVec<DIM>::type* __restrict__ out, int lines,
+         const float2* __restrict__ tw) {
+  pdl_begin();
+  constexpr int E = Fft<NG>::E, T = Fft<NG>::T, NC = NG / 2;
+  static_assert(T <= 32, "line inside one warp");
+  constexpr int LPC = (32 / T) * 4;
+  constexpr int XS = xpad_len<1>(NG);
+  __shared__ float2 s_x[LPC * XS];
+  const int q = threadIdx.x / T, t = threadIdx.x % T;
+  const int line_raw = blockIdx.x * LPC + q;
+  const bool valid = line_raw < lines;
+  const int line = valid ? line_raw : lines - 1;
+  float re[DIM][E];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    const float2* src = in + (((long long)blockIdx.y * DIM + d) * lines + line) * NC;
+    float2 v[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int zi = kept_mode(t + T * e, NG, NC);
+      v[e] = zi >= 0 ? __ldg(src + zi) : make_float2(0.f, 0.f);
+    }
+    block_fft<NG, E, kInv, 1, kSyncWarp>(v, s_x + q * XS, t, tw, 1);
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < E; ++e) re[d][e] = v[e].x;
+  }
+  if (valid) {
+    auto* o = out + ((long long)blockIdx.y * lines + line) * NG;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      if constexpr (DIM == 3)
+        o[t + T * e] = make_float4(re[0][e], re[1][e], re[2][e], 0.f);
+      else
+        o[t + T * e] = make_float2(re[0][e], re[1][e]);
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------
-// Last NUFFT grid pass: c2c inverse FFT of contiguous lines of n complex values,
-// writing only the real part (the interpolant of a real kernel needs no more).
+// c2c inverse FFT of contiguous lines of n complex values, writing only the real part
+// (the last pass of the particle -> grid transform).
 // ------------------------------------------------------------------------------
 template <int NL>
 __global__ void __launch_bounds__(128)
@@ -105,8 +186,8 @@ line_c2c_re(const float2* __restrict__ g, float* __restrict__ gre, long long nli
 }
 
 // ------------------------------------------------------------------------------
-// Particle binning by cell (counting sort) so that consecutive threads of the
-// gather work on neighbouring grid points. Bins: cubes of (n/nb)^dim fine cells.
+// Particle binning by cell (counting sort) so that consecutive threads of the spread
+// (and of the gather on grids beyond L2) work on neighbouring grid points. Bins: cubes of (n/nb)^dim fine cells.
 // ------------------------------------------------------------------------------
 template <int DIM>
 __device__ __forceinline__ int particle_bin(const double* __restrict__ r, long long j, int nb) {
@@ -176,97 +257,105 @@ __global__ void k_bin_scatter(const double* __restrict__ r, long long np, int nb
 //   r_out[j] = (r[j] + dt u_r[j]) mod 2 pi                 (integrator.py:21-23)
 // phi(z) = exp(beta (sqrt(1 - z^2) - 1)); w-point support per axis.
 // Eight lanes per particle (four particles per warp): lane q < W takes support index q
-// of the innermost (contiguous) axis and sums over the W^(dim-1) outer support rows, so
-// the group's loads of one row are W adjacent floats (one L1 wavefront instead of one
-// per particle); the group adds its partial sums by shuffles and lane 0 writes.
+// of the innermost (contiguous) axis and sums over the W^(dim-1) outer support rows, all
+// components of a grid point in one load, so the group's loads of one row are W adjacent
+// float4; the group adds its partial sums by shuffles. Lane d < dim forms axis d's grid
+// coordinate and lane q every axis' weight q (3 exponentials instead of 18 per lane);
+// the outer axes' weights reach the group by shuffle. Bound by the latency of those loads.
+// 32768 particles on 64^3 (w = 6), the whole update: 29 us; 80 us with planar components,
+// every lane forming all weights, a zero-filled grid and binned particles.
 // ------------------------------------------------------------------------------
 constexpr int kGatherLanes = 8;
 
 template <int DIM, int W>
 __global__ void __launch_bounds__(128)
-k_nufft_gather(const float* __restrict__ gre, long long gcs, int n, int ncomp, float beta, double norm,
+k_nufft_gather(const typename GridVec<DIM>::type* __restrict__ gre, long long gcs, int n, float beta, double norm,
                const double* __restrict__ r, const int* __restrict__ perm, long long np, double* __restrict__ u_r,
                double dt, double* __restrict__ r_out) {
   pdl_begin();
   static_assert(W <= kGatherLanes, "one support row per lane");
-  {  // batched plans: trajectory blockIdx.y (its 3-field grid, positions, order, outputs)
+  {  // batched plans: trajectory blockIdx.y (its grid, positions, order, outputs)
     const long long b = blockIdx.y;
-    gre += b * 3 * gcs;
+    gre += b * gcs;
     r += b * np * DIM;
     if (perm) perm += b * np;
-    u_r += b * np * ncomp;
+    u_r += b * np * DIM;
     if (r_out) r_out += b * np * DIM;
   }
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long i = gt / kGatherLanes;
   const int a = (int)(gt % kGatherLanes);
+  const int base = (threadIdx.x & 31) - a;  // the group's first lane
   const bool live = i < np;  // every lane stays for the group shuffles
   const long long j = live ? (perm ? perm[i] : i) : 0;
   const double two_pi = 2.0 * 3.14159265358979323846;
   const double inv_h = n / two_pi;
-  float wk[DIM][W];
-  int id[DIM][W];
+  // lane d: grid coordinate on axis d and its offset from the first support point in FP64
+  // (FP64 division is avoided: it is slow on this GPU); the kernel arguments
+  // z = (t - a) / (W/2) in FP32
+  const double xr = live && a < DIM ? r[j * DIM + a] : 0.0;
+  const double xs = xr * inv_h;
+  const double l0 = ceil(xs - 0.5 * W);
+  const int my_il0 = (int)l0;
+  const float my_t = (float)(xs - l0);
+  float wq[DIM];
+  int il0[DIM];
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
-    // grid coordinate and its offset from the first support point in FP64 (3 FP64
-    // operations per axis; FP64 division is avoided: it is slow on this GPU), the W
-    // kernel arguments z = (t - a) / (W/2) in FP32
-    const double xs = (live ? r[j * DIM + d] : 0.0) * inv_h;
-    const double l0 = ceil(xs - 0.5 * W);
-    const int il0 = (int)l0;
-    const float t = (float)(xs - l0);
+    il0[d] = __shfl_sync(0xffffffffu, my_il0, base + d);
+    const float t = __shfl_sync(0xffffffffu, my_t, base + d);
+    const float z = (t - (float)a) * (2.0f / W);
+    const float qq = 1.f - z * z;
+    wq[d] = qq > 0.f ? expf(beta * (sqrtf(qq) - 1.f)) : 0.f;
+  }
+  float w0[W], w1[W];  // weights of axis 0 and (3D) axis 1
 #pragma unroll
-    for (int q = 0; q < W; ++q) {
-      const float z = (t - (float)q) * (2.0f / W);
-      const float qq = 1.f - z * z;
-      wk[d][q] = qq > 0.f ? expf(beta * (sqrtf(qq) - 1.f)) : 0.f;
-      id[d][q] = (il0 + q) & (n - 1);  // n is a power of two; two's complement wraps negatives
-    }
+  for (int q = 0; q < W; ++q) {
+    w0[q] = __shfl_sync(0xffffffffu, wq[0], base + q);
+    if (DIM == 3) w1[q] = __shfl_sync(0xffffffffu, wq[1], base + q);
   }
   const bool col = live && a < W;
-  float wl = 0.f;  // this lane's innermost-axis weight and grid index
-  int il = 0;
+  float acc[DIM];
 #pragma unroll
-  for (int q = 0; q < W; ++q)
-    if (q == a) {
-      wl = wk[DIM - 1][q];
-      il = id[DIM - 1][q];
-    }
-  double ur[3] = {0.0, 0.0, 0.0};
+  for (int d = 0; d < DIM; ++d) acc[d] = 0.f;
+  if (col) {
+    // grid indices mod n (n is a power of two; two's complement wraps negatives)
+    const typename GridVec<DIM>::type* gc = gre + ((il0[DIM - 1] + a) & (n - 1));
 #pragma unroll
-  for (int comp = 0; comp < 3; ++comp) {
-    if (comp >= ncomp) break;
-    const float* gc = gre + comp * gcs + il;
-    float acc = 0.f;
-    if (col) {
-      if (DIM == 3) {
+    for (int q0 = 0; q0 < W; ++q0) {
+      const int x = ((il0[0] + q0) & (n - 1)) * n;
+      if constexpr (DIM == 3) {
+        float sb[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-        for (int q0 = 0; q0 < W; ++q0) {
-          float sb = 0.f;
-#pragma unroll
-          for (int q1 = 0; q1 < W; ++q1)
-            sb = fmaf(__ldg(gc + ((long long)id[0][q0] * n + id[1][q1]) * n), wk[1][q1], sb);
-          acc = fmaf(sb, wk[0][q0], acc);
+        for (int q1 = 0; q1 < W; ++q1) {
+          const float4 v = __ldg(gc + (long long)(x + ((il0[1] + q1) & (n - 1))) * n);
+          sb[0] = fmaf(v.x, w1[q1], sb[0]);
+          sb[1] = fmaf(v.y, w1[q1], sb[1]);
+          sb[2] = fmaf(v.z, w1[q1], sb[2]);
         }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) acc[d] = fmaf(sb[d], w0[q0], acc[d]);
       } else {
-#pragma unroll
-        for (int q0 = 0; q0 < W; ++q0) acc = fmaf(__ldg(gc + (long long)id[0][q0] * n), wk[0][q0], acc);
+        const float2 v = __ldg(gc + x);
+        acc[0] = fmaf(v.x, w0[q0], acc[0]);
+        acc[1] = fmaf(v.y, w0[q0], acc[1]);
       }
-      acc *= wl;
     }
 #pragma unroll
-    for (int o = kGatherLanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    ur[comp] = (double)acc * norm;
+    for (int d = 0; d < DIM; ++d) acc[d] *= wq[DIM - 1];
   }
-  if (!live || a != 0) return;
-  for (int comp = 0; comp < ncomp; ++comp) u_r[j * ncomp + comp] = ur[comp];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d)
+#pragma unroll
+    for (int o = kGatherLanes / 2; o > 0; o >>= 1) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
+  if (!live || a >= DIM) return;
+  const double ur = (double)(a == 0 ? acc[0] : a == 1 ? acc[1] : acc[DIM - 1]) * norm;
+  u_r[j * DIM + a] = ur;
   if (r_out) {
-    for (int d = 0; d < DIM; ++d) {
-      double x = r[j * DIM + d] + dt * ur[d];
-      x = x - two_pi * floor(x / two_pi);
-      if (x >= two_pi) x -= two_pi;  // Python % never returns the modulus itself
-      r_out[j * DIM + d] = x;
-    }
+    double x = xr + dt * ur;
+    x = x - two_pi * floor(x / two_pi);
+    if (x >= two_pi) x -= two_pi;  // Python % never returns the modulus itself
+    r_out[j * DIM + a] = x;
   }
 }
 
@@ -361,7 +450,7 @@ line_fft_real_fwd(const float* __restrict__ x, float2* __restrict__ g, long long
   }
 }
 
-// Adjoint of the reads of the coarse half spectrum by k_nufft_prep (inv_psi: its
+// Adjoint of the reads of the coarse half spectrum by k_grid_x (inv_psi: its
 // deconvolution factors) or by k_dft_interp (inv_psi == nullptr: factors 1): the box
 // mode k in [-c/2, c/2 - 1]^dim reads Hh(k) for a half-axis frequency >= 0 and
 // conj Hh(-k) below, so
@@ -671,7 +760,7 @@ struct l3es_interp_plan {
   float2* tw = nullptr;      // n-point twiddles
   float2* hh = nullptr;      // [3][coarse half spectrum]
   float2* g = nullptr;       // [3][n^dim]
-  float* gre = nullptr;      // [3][n^dim]
+  float* gre = nullptr;      // [n^dim] points of 4 (2D 2) interleaved components; also [3][n^dim]
   float* inv_psi = nullptr;  // [c]
   float2* twc = nullptr;     // c-point twiddles (particle -> grid inverse transform)
   int* count = nullptr;      // [nb^dim]
@@ -725,25 +814,35 @@ static void c2c_inverse_re(int dim, float2* g, float* gre, const float2* tw, flo
   pdl_launch(line_c2c_re<NG>, (unsigned)((lines + LPC - 1) / LPC), 128, 0, s, g, gre, lines, tw, scale);
 }
 
-// strided c2c passes of the NUFFT grid (inverse), via the ky_pass kernel
-template <int NG>
+// the NUFFT grid of every trajectory from the coarse spectra (k_grid_x / _y / _z); the two
+// intermediate arrays share p->g: [fields][n][c^(dim-1)] first (2^-(dim-1) of a full grid),
+// in 3D then [fields][n][n][c] (half of one) behind it
+template <int DIM, int NG>
 static void grid_passes(const l3es_interp_plan* p, cudaStream_t s) {
   using KY = KyCfg<NG>;
-  constexpr int TX = KY::THREADS, TWY = KY::TWY;
-  const long long per = p->gcs;
-  const unsigned nf = 3u * (unsigned)p->batch;  // fields of every trajectory, one after another
-  if (p->dim == 3) {
-    // x: pencils of stride n^2, columns = (y, z) flattened
-    pdl_launch(ky_pass<NG, kInv>, dim3((NG * NG + TWY - 1) / TWY, 1, nf), TX, 0, s, p->g, per, NG * NG, NG * NG,
-               NG / 2, p->tw);
-    // y: pencils of stride n inside each x-plane, columns = z
-    pdl_launch(ky_pass<NG, kInv>, dim3((NG + TWY - 1) / TWY, NG, nf), TX, 0, s, p->g, per, NG, NG, NG / 2, p->tw);
-  } else {
-    pdl_launch(ky_pass<NG, kInv>, dim3((NG + TWY - 1) / TWY, 1, nf), TX, 0, s, p->g, per, NG, NG, NG / 2, p->tw);
+  constexpr int NC = NG / 2, TX = KY::THREADS, TWY = KY::TWY;
+  constexpr int cols = DIM == 3 ? NC * NC : NC;
+  const unsigned nf = (unsigned)(DIM * p->batch);
+  pdl_launch(k_grid_x<DIM, NG>, dim3((cols + TWY - 1) / TWY, nf), TX, 0, s, p->hh, p->hcs, p->inv_psi, p->g, p->tw);
+  const float2* last = p->g;
+  if constexpr (DIM == 3) {
+    float2* g2 = p->g + (long long)nf * NG * cols;
+    pdl_launch(k_grid_y<NG>, dim3((NC + TWY - 1) / TWY, NG, nf), TX, 0, s, p->g, g2, p->tw);
+    last = g2;
   }
-  const long long lines = (long long)nf * per / NG;
+  const int lines = DIM == 3 ? NG * NG : NG;
   constexpr int LPC = (32 / Fft<NG>::T) * 4;
-  pdl_launch(line_c2c_re<NG>, (unsigned)((lines + LPC - 1) / LPC), 128, 0, s, p->g, p->gre, lines, p->tw, 1.0f);
+  using V = typename GridVec<DIM>::type;
+  pdl_launch(k_grid_z<DIM, NG>, dim3((lines + LPC - 1) / LPC, p->batch), 128, 0, s, last, reinterpret_cast<V*>(p->gre),
+             lines, p->tw);
+}
+
+template <int NG>
+static void grid_passes(const l3es_interp_plan* p, cudaStream_t s) {
+  if (p->dim == 3)
+    grid_passes<3, NG>(p, s);
+  else
+    grid_passes<2, NG>(p, s);
 }
 
 // forward c2c passes of the real NUFFT grid gre (the adjoint of the inverse passes):
@@ -826,7 +925,7 @@ int l3es_interp_plan_create_batch(int32_t dim, int32_t n_fine, int32_t ckp_n, in
   rc = rc ? rc : ip_alloc(p, (void**)&p->tw, sizeof(float2) * p->n, "twiddles");
   rc = rc ? rc : ip_alloc(p, (void**)&p->hh, sizeof(float2) * 3 * batch * p->hcs, "coarse spectrum");
   rc = rc ? rc : ip_alloc(p, (void**)&p->g, sizeof(float2) * 3 * batch * p->gcs, "nufft grid");
-  rc = rc ? rc : ip_alloc(p, (void**)&p->gre, sizeof(float) * 3 * batch * p->gcs, "nufft grid re");
+  rc = rc ? rc : ip_alloc(p, (void**)&p->gre, sizeof(float) * 4 * batch * p->gcs, "nufft grid re");
   rc = rc ? rc : ip_alloc(p, (void**)&p->inv_psi, sizeof(float) * ckp_n, "deconvolution");
   rc = rc ? rc : ip_alloc(p, (void**)&p->twc, sizeof(float2) * ckp_n, "coarse twiddles");
   rc = rc ? rc : ip_alloc(p, (void**)&p->count, sizeof(int) * batch * nbins, "bins");
@@ -942,17 +1041,25 @@ static int dft_eval(l3es_interp_plan* p, const double* r, int64_t np, double* u_
   return cuda_check(dft_launch(p->dim, p->hh, p->hcs, p->c, r, np, u_r, dt, r_out, s), "l3es_interp (dft) launch");
 }
 
-// NUFFT gather at r from the prepared fine grid (nufft_grid), visiting particles in the
-// bin order of the positions nufft_grid was given; fused Euler shift when r_out.
+// Whether the gather visits particles in bin order. While a trajectory's grid fits L2 the
+// input order is faster: the binning's four launches cost more than the gather's L1 misses
+// (32768 particles on 64^3 29 against 48 us, 60000 on 128^3 61 against 117, 2e6 on 128^3
+// 894 against 1054). On a 256^3 grid (268 MB) misses go to memory and many particles repay
+// the binning: 3e5 459 against 716 us, 2e6 1777 against 1537.
+static bool nufft_binned(const l3es_interp_plan* p, int64_t np) {
+  return p->dim == 3 && p->gcs * (long long)sizeof(float4) > (128LL << 20) && np >= (1LL << 20);
+}
+
+// NUFFT gather at r from the prepared fine grid (nufft_grid); fused Euler shift when r_out.
 static int nufft_eval(l3es_interp_plan* p, const double* r, int64_t np, double* u_r, double dt, double* r_out,
                       cudaStream_t s) {
-  const int ncomp = p->dim;
   const double norm = 1.0 / (std::pow((double)p->n, p->dim) * std::pow((double)p->c, p->dim));
   const float beta = (float)p->beta;
+  const int* perm = nufft_binned(p, np) ? p->perm : nullptr;
   const dim3 gblk((unsigned)((np * kGatherLanes + 127) / 128), (unsigned)p->batch);
-#define L3ES_GATHER(D, W)                                                                                   \
-  pdl_launch(k_nufft_gather<D, W>, gblk, 128, 0, s, p->gre, p->gcs, p->n, ncomp, beta, norm, r, p->perm, np, u_r, dt, \
-                                          r_out)
+#define L3ES_GATHER(D, W)                                                                                      \
+  pdl_launch(k_nufft_gather<D, W>, gblk, 128, 0, s, reinterpret_cast<const GridVec<D>::type*>(p->gre), p->gcs, \
+             p->n, beta, norm, r, perm, np, u_r, dt, r_out)
   if (p->dim == 3) {
     if (p->w == 6) L3ES_GATHER(3, 6);
     else if (p->w == 8) L3ES_GATHER(3, 8);
@@ -1011,19 +1118,13 @@ int l3es_interp_advect_rk4(l3es_interp_plan* p, const double* r, int64_t np, dou
 
 }  // extern "C"
 
-// Fine NUFFT grid of the plan's coarse spectrum (deconvolve, zero-pad, 3 c2c passes, Re)
-// and the bin order of the positions r.
+// Fine NUFFT grid of the plan's coarse spectrum and, where the gather uses it
+// (nufft_binned), the bin order of the positions r.
 static int bin_particles(l3es_interp_plan* p, const double* r, int64_t np, cudaStream_t s);
 
 static int nufft_grid(l3es_interp_plan* p, const double* r, int64_t np, cudaStream_t s) {
-  const unsigned gb = (unsigned)((p->gcs + 255) / 256);
-  const unsigned nf = 3u * (unsigned)p->batch;
-  if (p->dim == 3)
-    pdl_launch(k_nufft_prep<3>, dim3(gb, nf), 256, 0, s, p->hh, p->hcs, p->c, p->inv_psi, p->g, p->gcs, p->n);
-  else
-    pdl_launch(k_nufft_prep<2>, dim3(gb, nf), 256, 0, s, p->hh, p->hcs, p->c, p->inv_psi, p->g, p->gcs, p->n);
   const int rc = run_grid_passes(p, s);
-  return rc != L3ES_OK ? rc : bin_particles(p, r, np, s);
+  return rc != L3ES_OK || !nufft_binned(p, np) ? rc : bin_particles(p, r, np, s);
 }
 
 // counting sort of the particles by cell into p->perm
