@@ -237,13 +237,14 @@ __device__ __forceinline__ int3 slot_cell(long long i, const int* __restrict__ p
   return c;
 }
 
-// rho[slot] = m sigma sum_j w(r_ij / h); rp[slot] = (rho, p = p_ref (rho - 1)) in FP32
-// for the acceleration pass; rho_out[input index] when requested
+// rho[slot] = m sigma sum_j w(r_ij / h); rp[slot] = (rho, p = p_ref (rho - 1),
+// 1 / rho^2) in FP32 for the acceleration pass (the quotient once per particle: it was one
+// of three divisions per pair there); rho_out[input index] when requested
 template <int DIM>
 __global__ void __launch_bounds__(kSphThreads)
 k_sph_density(const float4* __restrict__ xs, const int* __restrict__ start, const int* __restrict__ perm,
               const double* __restrict__ xw, long long np, SphGeom g, double m_sigma, double p_ref,
-              float2* __restrict__ rp, double* __restrict__ rho_out) {
+              float4* __restrict__ rp, double* __restrict__ rho_out) {
   pdl_begin();
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long i = gt / kSphLanes;
@@ -261,7 +262,8 @@ k_sph_density(const float4* __restrict__ xs, const int* __restrict__ start, cons
   const double acc = lanes_sum((double)part.hi + (double)part.lo);
   if (!live || lane != 0) return;
   const double rho = m_sigma * acc;
-  rp[i] = make_float2((float)rho, (float)(p_ref * (rho - 1.0)));
+  const float rf = (float)rho;
+  rp[i] = make_float4(rf, (float)(p_ref * (rho - 1.0)), 1.f / (rf * rf), 0.f);
   if (rho_out) rho_out[perm[i]] = rho;
 }
 
@@ -272,7 +274,7 @@ struct SphAccelArgs {
   const int* start;
   const int* perm;
   const double* xw;     // wrapped (predicted) positions, input order
-  const float2* rp;     // (rho, p) per slot
+  const float4* rp;     // (rho, p, 1 / rho^2, -) per slot
   const float4* us;     // velocities per slot (forces only)
   long long np;
   float mass, grad_scale, p_ref, eps;  // grad_scale = sigma / h
@@ -300,15 +302,14 @@ __global__ void __launch_bounds__(kSphThreads) k_sph_accel(SphAccelArgs a, SphGe
   const long long is = live ? i : 0;
   const float4 xi = a.xs[is];
   const int3 ci = slot_cell<DIM>(is, a.perm, a.xw, g);
-  const float2 rpi = a.rp[is];
-  const float inv_ri2 = 1.f / (rpi.x * rpi.x);
+  const float4 rpi = a.rp[is];
   const float4 ui = MODE == kSphForces ? a.us[is] : make_float4(0.f, 0.f, 0.f, 0.f);
   Ff fp[3] = {}, ft[3] = {}, fv[3] = {};
   if (live) for_neighbours<DIM>(xi, ci, g, a.start, a.xs, lane, [&](int jj, float dx, float dy, float dz, float r2) {
-    const float2 rpj = a.rp[jj];
+    const float4 rpj = a.rp[jj];
     const float r = sqrtf(r2);
     const float dw = a.grad_scale * quintic_dw(r * g.inv_h);
-    const float pref = a.mass * (inv_ri2 + 1.f / (rpj.x * rpj.x));
+    const float pref = a.mass * (rpi.z + rpj.z);
     const float pij = (rpj.x * rpi.y + rpi.x * rpj.y) / (rpi.x + rpj.x);
     const float s = dw / (r + a.eps);
     if (MODE == kSphForces) {
@@ -381,7 +382,7 @@ struct l3es_sph_plan {
   int* perm = nullptr;     // [np_max] slot -> input index
   float4* xs = nullptr;    // [np_max] cell-local coordinates per slot
   float4* us = nullptr;    // [np_max] velocity per slot (forces)
-  float2* rp = nullptr;    // [np_max] (rho, p) per slot
+  float4* rp = nullptr;    // [np_max] (rho, p, 1 / rho^2, -) per slot
   std::vector<void*> allocs;
 };
 
@@ -504,7 +505,7 @@ int l3es_sph_plan_create(int32_t dim, int32_t n, double box, int64_t np_max, l3e
   if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->perm, sizeof(int) * npm, "perm");
   if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->xs, sizeof(float4) * npm, "xs");
   if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->us, sizeof(float4) * npm, "us");
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->rp, sizeof(float2) * npm, "rp");
+  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->rp, sizeof(float4) * npm, "rp");
   if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->count, sizeof(int) * p->ncell, "count");
   if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->cursor, sizeof(int) * p->ncell, "cursor");
   if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->start, sizeof(int) * (p->ncell + 1), "start");
