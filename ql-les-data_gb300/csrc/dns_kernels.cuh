@@ -255,11 +255,10 @@ struct KxTma {
   static constexpr unsigned BYTES = (unsigned)STAGE * sizeof(float2);
 };
 
-template <int N, bool CURL, bool SKIPWX = false, bool LINF = false>
+template <int N, bool CURL, bool SKIPWX = false>
 __global__ void __launch_bounds__(TW * Fft<N>::T, TW * Fft<N>::T >= 512 ? 1 : 2)
 kx_inv_tma(const __grid_constant__ CUtensorMap umap, float2* __restrict__ w, long long fs,
-           const float2* __restrict__ tw, int ntiles, int* __restrict__ err, float2* __restrict__ wx,
-           const __grid_constant__ XLin xl) {
+           const float2* __restrict__ tw, int ntiles, int* __restrict__ err, float2* __restrict__ wx) {
   pdl_begin();
   using K = KxTma<N>;
   constexpr int E = Fft<N>::E, T = Fft<N>::T;
@@ -270,11 +269,6 @@ kx_inv_tma(const __grid_constant__ CUtensorMap umap, float2* __restrict__ w, lon
   __shared__ uint64_t bar;
   const int p = threadIdx.x % TW, t = threadIdx.x / TW;
   const int batch = blockIdx.y;
-  if constexpr (LINF) {
-    if (xl.band_kf > 0 && blockIdx.x == 0)
-      band_coefficient<3>(xl.S + (long long)batch * 3 * xl.cs, xl.cs, N, xl.band_kf, xl.inv_n2d, xl.eps_inj, 1e-30,
-                          xl.band_scale + batch);
-  }
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
     mbar_init_fence();
@@ -314,9 +308,6 @@ kx_inv_tma(const __grid_constant__ CUtensorMap umap, float2* __restrict__ w, lon
     if (threadIdx.x == 0 && next < ntiles) {
       fence_proxy_async_smem();
       issue(next);
-    }
-    if constexpr (LINF) {
-      if (xl.rk > 0) xlin_scale<N>(a, t, tile * TW + p, xl, batch, err);
     }
     kx_inv_fields<N, 3, CURL, SKIPWX>(a, t, tile * TW + p, true, sm + p, w, (long long)batch * NF * fs, fs, tw,
                                       wx, (long long)batch * 2 * fs);

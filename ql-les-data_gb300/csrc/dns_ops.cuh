@@ -26,8 +26,7 @@ struct DnsOps {
 
   static inline int tma_band_ctas = 0;
   static inline int tma_plain_ctas = 0;  // x inverse without curl (irfftn)
-  static inline int tma_lin_ctas = 0;    // band-fused RK step: x inverse and band pass
-  static inline int tma_band_fused_ctas = 0;
+  static inline int tma_band_fused_ctas = 0;  // band pass of the band-fused RK step
 
   // resident CTAs (all SMs) of a persistent kernel with K::SMEM dynamic shared memory
   template <typename F>
@@ -57,7 +56,6 @@ struct DnsOps {
       tma_plain_ctas = persistent_ctas(kx_inv_tma<N, false>);
     }
     if constexpr (N >= kBandMin3d) {
-      tma_lin_ctas = persistent_ctas(kx_inv_tma<N, true, true, true>);
       tma_band_fused_ctas = persistent_ctas(kx_fwd_band_tma<N, true>);
     }
     if constexpr (N >= 16) stage_attrs<2>();
@@ -122,20 +120,14 @@ struct DnsOps {
       const unsigned long long dims[3] = {(unsigned long long)mc, N, 3ull * c.batch};
       const unsigned long long strides[2] = {8ull * mc, 8ull * c.cs};
       const unsigned box[3] = {TW, KxTma<N>::NY, 3};
-      const int ctas = xl ? tma_lin_ctas : tma_ctas;
-      if (c.sched.x_bulk && ctas > 0 && tma_encode(&map, us, 3, dims, strides, box)) {
+      // (the scaling of a band-fused stage always runs in the one-tile kernel, which has no
+      // register cap: per 256^3 launch 116 against 127 us, 512^3 1140 against 1360 us)
+      if (!xl && c.sched.x_bulk && tma_ctas > 0 && tma_encode(&map, us, 3, dims, strides, box)) {
         const int ntiles = (int)(mc / TW);
-        const int gx = std::max(1, std::min(ntiles, ctas / c.batch));
-        if constexpr (N >= kBandMin3d)
-          if (xl) {
-            L3ES_LAUNCH(c, KK_X_INV, bytes, s,
-                        pdl_launch(kx_inv_tma<N, true, true, true>, dim3(gx, c.batch), TX, KxTma<N>::SMEM, s, map,
-                                   c.W, c.fs, c.tw, ntiles, c.err, c.Wx, *xl));
-            return;
-          }
+        const int gx = std::max(1, std::min(ntiles, tma_ctas / c.batch));
         L3ES_LAUNCH(c, KK_X_INV, bytes, s,
                     pdl_launch(kx_inv_tma<N, true, true>, dim3(gx, c.batch), TX, KxTma<N>::SMEM, s, map, c.W, c.fs,
-                               c.tw, ntiles, c.err, c.Wx, XLin{}));
+                               c.tw, ntiles, c.err, c.Wx));
         return;
       }
     }
@@ -250,7 +242,7 @@ struct DnsOps {
       const BandRk br{S, c.C, c.cs, prm, c.band, c.nu_b, c.err};
       const double bb = Adu * rows + Ap * (rk == 0 ? 3.0 : rk == 1 ? 4.0 : rk == 2 ? 5.0 : 3.0);
       {
-        const bool bulk = c.sched.band_bulk < 0 ? N >= 256 : c.sched.band_bulk != 0;
+        const bool bulk = c.sched.band_bulk < 0 ? N == 256 : c.sched.band_bulk != 0;
         CUtensorMap map;
         const unsigned long long dims[4] = {(unsigned long long)c.kt, N, N, 3ull * c.batch};
         const unsigned long long strides[3] = {8ull * c.kt, 8ull * N * c.kt, 8ull * c.ds};
@@ -271,10 +263,11 @@ struct DnsOps {
     }
     // (block 0 of each trajectory also computes the constant-power coefficient of us)
     bool band_done = false;
-    // by default from 256^3: smaller grids have too few band tiles per persistent CTA to
-    // pipeline (measured at 128^3: 9.5 us persistent vs 8.4 us one-shot)
+    // by default at 256^3: smaller grids have too few band tiles per persistent CTA to
+    // pipeline (measured at 128^3: 9.5 us persistent vs 8.4 us one-shot), at 512^3 a CTA
+    // fills its SM either way (a band-fused step 20.5 ms persistent, 20.1 ms one-shot)
     if constexpr (DIM == 3 && N >= 64) {
-      const bool bulk = c.sched.band_bulk < 0 ? N >= 256 : c.sched.band_bulk != 0;
+      const bool bulk = c.sched.band_bulk < 0 ? N == 256 : c.sched.band_bulk != 0;
       CUtensorMap map;
       const unsigned long long dims[4] = {(unsigned long long)c.kt, N, N, 3ull * c.batch};
       const unsigned long long strides[3] = {8ull * c.kt, 8ull * N * c.kt, 8ull * c.ds};
@@ -404,7 +397,7 @@ struct DnsOps {
         L3ES_LAUNCH(c, KK_X_INV_PLAIN, 2.0 * A, s,
                     pdl_launch(kx_inv_tma<N, false>, dim3(gx, c.batch), TX, KxTma<N>::SMEM, s, map, c.W, c.fs, c.tw,
                                ntiles,
-                                                                                        c.err, nullptr, XLin{}));
+                                                                                        c.err, nullptr));
         x_done = true;
       }
     }

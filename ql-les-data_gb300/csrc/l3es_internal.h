@@ -123,12 +123,13 @@ inline bool misaligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p)
 // Kernel variants of one plan's step (chosen by l3es_plan_autotune; the defaults are the
 // measured best at 256^3 on GB300).
 struct Schedule {
-  int x_bulk = 1;     // 3D x passes by the persistent bulk-tensor-copy kernels (else one tile per CTA);
-                      // 2D: the step's x passes in 2-column tiles (else 8)
+  int x_bulk = 1;     // 3D x inverses other than a band-fused stage's by the persistent
+                      // bulk-tensor-copy kernels (else one tile per CTA); 2D: the x passes of
+                      // the elementwise forms and the adjoint in 2-column tiles (else 8)
   int y_var = 0;      // y-pass schedule: KyCfg variant (0: radix 16 from N = 128, 1: radix 8)
   int line_pair = 1;  // line pass: 1 two-for-one (64 <= N <= 256), 2 two-for-one radix 16 and 3 the same
                       // fed by bulk copies (N = 256; 3 is its default), 0 packed
-  int band_bulk = -1; // persistent bulk-copy band pass (-1: from N = 256, the measured default)
+  int band_bulk = -1; // persistent bulk-copy band pass (-1: at N = 256, the measured default)
 };
 
 // Geometry + scratch of one plan, handed to the per-N launch wrappers.

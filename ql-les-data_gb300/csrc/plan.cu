@@ -239,6 +239,9 @@ int l3es_plan_create(const l3es_plan_desc* desc, l3es_plan** out) {
   c.kd = dealias_kd(n);
   c.kt = ((c.kd + 1 + TW - 1) / TW) * TW;
   if (n == 256) c.sched.line_pair = 3;  // the staged radix-16 line pass (measured best at 256)
+  // y pass: radix 16 at 256^3 (a step 2062 us against 2298 us with radix 8), radix 8 at
+  // 128^3 (288 against 295 us) and 512^3 (20.07 against 20.30 ms)
+  c.sched.y_var = dim == 3 && (n == 128 || n == 512);
   // the stage combination inside the x passes (in 2D forms 1 and 2 both are kx_stage)
   c.step_form = dim == 3 ? 2 : 1;
   c.nmid = dim == 3 ? n : 1;
@@ -402,7 +405,7 @@ int l3es_plan_get_schedule(const l3es_plan* plan, int32_t* sched4) {
   sched4[0] = s.x_bulk;
   sched4[1] = s.y_var;
   sched4[2] = s.line_pair;
-  sched4[3] = s.band_bulk < 0 ? (plan->ctx.n >= 256 ? 1 : 0) : s.band_bulk;
+  sched4[3] = s.band_bulk < 0 ? (plan->ctx.n == 256 ? 1 : 0) : s.band_bulk;
   return L3ES_OK;
 }
 
