@@ -55,11 +55,15 @@ struct DnsOps {
       tma_band_ctas = persistent_ctas(kx_fwd_band_tma<N>);
       tma_plain_ctas = persistent_ctas(kx_inv_tma<N, false>);
     }
-    if constexpr (N >= kBandMin3d) {
+    if constexpr (N > kStageMax3d) {
       tma_band_fused_ctas = persistent_ctas(kx_fwd_band_tma<N, true>);
     }
     if constexpr (N >= 16) stage_attrs<2>();
-    if constexpr (N >= 16 && N <= kStageMax3d) stage_attrs<3>();
+    if constexpr (N >= 16 && N <= kStageMax3d) {
+      stage_attrs<3>();
+      cudaFuncSetAttribute(k_yz_plane<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, YzCfg<N>::SMEM);
+      cudaGetLastError();
+    }
   }
 
   // kx_stage's shape: columns per CTA and values per thread in each transform
@@ -141,7 +145,7 @@ struct DnsOps {
       }
     }
     const dim3 g((unsigned)((mc + TW - 1) / TW), c.batch);
-    if constexpr (DIM == 3 && N >= kBandMin3d)
+    if constexpr (DIM == 3 && N > kStageMax3d)
       if (xl) {
         L3ES_LAUNCH(c, KK_X_INV, bytes, s,
                     pdl_launch(kx_inv<N, 3, true, true, true>, g, TX, 0, s, us, c.cs, c.W, c.fs, c.tw, c.Wx, *xl,
@@ -209,7 +213,7 @@ struct DnsOps {
     const double rows = DIM == 3 ? (2.0 * c.kd + 1.0) / N : 1.0;  // kept y rows
     const double inv_n2d = 1.0 / (DIM == 3 ? std::pow((double)N, 6) : std::pow((double)N, 4));
     // band-fused RK step (XLin): us == S; fb = the band's share of the modes
-    const bool fused = DIM == 3 && N >= kBandMin3d && prm.band_rk && rk >= 0;
+    const bool fused = DIM == 3 && N > kStageMax3d && prm.band_rk && rk >= 0;
     const double fb = (double)c.pcs / (double)c.cs;
     XLin xl{};
     if (fused) {
@@ -235,7 +239,7 @@ struct DnsOps {
     // band x-FFT + projection into P, then the elementwise RK update
     const int nb = 2 * c.kd + 1;
     const double Ap = 8.0 * 3.0 * c.pcs * B;
-    if constexpr (DIM == 3 && N >= kBandMin3d) if (fused) {
+    if constexpr (DIM == 3 && N > kStageMax3d) if (fused) {
       // the stage combination on the band: rk 0 reads S and writes P (= u0) and S; rk 1
       // reads S, P and writes acc, S; rk 2 reads S, P, acc and writes acc, S; rk 3 reads
       // S, acc and writes S
@@ -344,19 +348,33 @@ struct DnsOps {
                            c.Tb, c.C, st, c.W, c.Wx, c.fs, c.tw));
   }
 
+  // W -> DU between two kx_stage launches: in 3D one kernel per x plane
+  template <int DIM>
+  static void between(const Ctx& c, cudaStream_t s) {
+    if constexpr (DIM == 3 && N >= 16 && N <= kStageMax3d) {
+      const double A = 8.0 * 3.0 * c.cs * c.batch, Adu = 8.0 * 3.0 * c.ds * c.batch;
+      const float scale = (float)(1.0 / ((double)N * N * N));
+      L3ES_LAUNCH(c, KK_YZ_PLANE, 5.0 / 3.0 * A + Adu * (2.0 * c.kd + 1.0) / N, s,
+                  pdl_launch(k_yz_plane<N>, dim3(N, c.batch), YzCfg<N>::THREADS, YzCfg<N>::SMEM, s, c.W, c.Wx, c.fs,
+                             c.DU, c.ds, c.kt, c.kd, 0.5f * scale * scale, c.tw, c.tw + line2_ct_offset<N>()));
+    } else {
+      nonlinear<DIM>(c, s);
+    }
+  }
+
   // One RK4 step in place on S by kx_stage (stage_kernels.cuh). first: the x inverse of S
   // is not in W yet; last: nothing follows that needs the new state's.
   template <int DIM>
   static void step_dim(const Ctx& c, float2* S, const EpiParams* prm, bool first, bool last, cudaStream_t s) {
     if constexpr (N >= 16 && (DIM == 2 || N <= kStageMax3d)) {
       if (first) x_stage<DIM, -1, true>(c, S, prm[0], s);
-      nonlinear<DIM>(c, s);
+      between<DIM>(c, s);
       x_stage<DIM, 0, true>(c, S, prm[0], s);
-      nonlinear<DIM>(c, s);
+      between<DIM>(c, s);
       x_stage<DIM, 1, true>(c, S, prm[1], s);
-      nonlinear<DIM>(c, s);
+      between<DIM>(c, s);
       x_stage<DIM, 2, true>(c, S, prm[2], s);
-      nonlinear<DIM>(c, s);
+      between<DIM>(c, s);
       if (last)
         x_stage<DIM, 3, false>(c, S, prm[3], s);
       else

@@ -33,7 +33,7 @@ const char* kernel_kind_name(int k) {
       "kx_inv_curl", "ky_pass_inv", "line_cross", "ky_pass_fwd", "kx_fwd_band",
       "force_ekin", "kx_inv", "line_c2r", "line_r2c", "kx_fwd", "reduce",
       "filter", "nufft_prep", "nufft_fft", "nufft_gather", "particle_sort", "rk_update",
-      "kx_inv_adjproj", "line_cross_adj", "adj_epilogue", "kx_stage"};
+      "kx_inv_adjproj", "line_cross_adj", "adj_epilogue", "kx_stage", "yz_plane"};
   return (k >= 0 && k < KK_COUNT) ? names[k] : "";
 }
 
@@ -515,7 +515,7 @@ static void rk4_step(l3es_plan* plan, float2* S, bool first, bool last, cudaStre
   // is one launch of four per stage, form 1 as well); the band has to lie inside the half
   // axis (kt <= N/2 + 1, i.e. N >= 16)
   const bool band = lin_ok && c.step_form >= (c.dim == 3 ? 2 : 1) && c.kt <= c.h;
-  const bool one_visit = band && step_by_kx_stage(c.dim, c.n, c.batch);
+  const bool one_visit = band && step_by_kx_stage(c.dim, c.n);
   EpiParams prm[4];
   for (int rk = 0; rk < 4; ++rk) {
     EpiParams& q = prm[rk];

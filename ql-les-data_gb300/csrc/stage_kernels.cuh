@@ -5,8 +5,8 @@
 // nonlinear term, the dealias mask, the Leray projection, the RK4 stage combination and
 // the next stage's inverse x FFT of u and curl u all act on the same column of modes, so
 // kx_stage does them in one visit: the new stage field goes from the combination into
-// the inverse transform without a trip through memory, and a stage is two launches in 2D
-// (kx_stage, line pass) and four in 3D (kx_stage, y inverse, line pass, y forward).
+// the inverse transform without a trip through memory, and a stage is two launches
+// (kx_stage and in 2D the line pass, in 3D k_yz_plane).
 //
 // The band B = {|kx| <= kd, |kmid| <= kd (3D), khalf < kt} holds every nonlinear and
 // forcing term. Outside it du = -(nu k^2 + drag) u exactly, so a stage field there is a
@@ -21,19 +21,18 @@
 
 namespace l3es {
 
-// Where the explicit step takes kx_stage: every 2D grid, 3D grids below 64^3, and 64^3 up
-// to a batch of 4. There the passes are latency: few CTAs, each a chain of dependent
-// transforms, and the launches count. Measured per step against the separate passes:
-// 2D 256^2 98.3 -> 69.7 us, 128^2 x 8 98.4 -> 70.6 us, 512^2 122.9 -> 97.7 us, 3D 32^3
-// 120.9 -> 90.5 us, 64^3 132.1 -> 107.1 us, 64^3 x 3 172 -> 157 us. Once the chip is full
-// the three groups' barriers and the thread count (one or two CTAs per SM) cost more than
-// the saved round trip: 64^3 x 6 263 -> 281 us, 128^3 (one stage's x passes) 32.6 -> 38 us,
-// 256^3 195 -> 267 us. Larger 3D grids keep kx_inv and the band-fused kx_fwd_band.
+// Where the explicit step takes kx_stage: every 2D grid and 3D grids up to 64^3 (there with
+// k_yz_plane between two x passes). Those are bound by latency: few CTAs, each a chain of
+// dependent transforms, and the launches count. Measured per step against the separate
+// passes (x inverse, y inverse, line, y forward, band pass, 2D also the update): 2D 256^2
+// 98.3 -> 69.7 us, 128^2 x 8 98.4 -> 70.6 us, 512^2 122.9 -> 97.7 us; 3D, dependent launches
+// on both sides, 64^3 89 -> 71 us, 64^3 x 6 222 -> 208 us, 64^3 x 12 425 -> 423 us; from
+// plain launches 32^3 121 -> 35 us, 16^3 130 -> 41 us. With kx_stage 128^3 takes 38 instead
+// of 32.6 us for one stage's x passes and 256^3 267 instead of 195 us: there the chip is full
+// and the barriers of the three groups cost more than the saved round trip. Larger 3D grids
+// keep kx_inv and the band-fused kx_fwd_band.
 constexpr int kStageMax3d = 64;  // largest 3D grid with kx_stage kernels
-constexpr int kBandMin3d = 64;   // smallest 3D grid with band-fused kernels
-inline bool step_by_kx_stage(int dim, int n, int batch) {
-  return dim == 2 || n < kBandMin3d || (n <= kStageMax3d && batch <= 4);
-}
+inline bool step_by_kx_stage(int dim, int n) { return dim == 2 || n <= kStageMax3d; }
 
 // Parameters of one stage.
 struct XStage {
@@ -220,6 +219,181 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
       float2* dst = w + ((long long)batch * 6 + 3 + g) * fs;
 #pragma unroll
       for (int e = 0; e < E; ++e) dst[(long long)(t + T * e) * MC + m] = v[e];
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------
+// Everything between two x passes of a small 3D grid in one kernel, one x plane per CTA:
+// y inverse of the six fields (u, curl u; curl_x formed here, as in ky_inv_rhs), the
+// half-axis lines with u x curl u (two real lines per complex FFT, as in line_cross2) and
+// the y forward of the three products, kept rows only, to du. At 64^3 the plane's six
+// fields are 123 KB of shared memory, so the three passes meet there instead of in global
+// memory, in one launch instead of three. Warps work alone inside a phase: a warp takes 32
+// / T neighbouring columns (y transforms) or 32 / T lines, T = N / 8 lanes each.
+// ct8: compact twiddle table of the N-point FFT (line2_ct_offset).
+// ------------------------------------------------------------------------------
+template <int N>
+struct YzCfg {
+  static constexpr int T = N / 8;                 // lanes per transform
+  static constexpr int XC = 32 / T;               // columns (lines) per warp
+  static constexpr int H = N / 2 + 1;
+  static constexpr int WARPS = N == 64 ? 16 : N == 32 ? 8 : 6;
+  static constexpr int THREADS = 32 * WARPS;
+  // row length of a field: the lines of a half warp's loads fall into different banks
+  static constexpr int LD = N == 64 ? 40 : N == 32 ? 20 : 12;
+  static constexpr int FIELD = N * LD;
+  static constexpr int XS1 = XC * xpad_len<1>(N), XSC = XC * xpad_len<XC>(N);
+  static constexpr int XS = XS1 > XSC ? XS1 : XSC;  // exchange slots per warp
+  static constexpr int SMEM = (6 * FIELD + WARPS * XS) * (int)sizeof(float2);
+};
+
+// Z = X_ext + i Y_ext (c2r_pair_load) from two half-spectrum rows in shared memory
+template <int N>
+__device__ __forceinline__ void c2r_pair_row(const float2* X, const float2* Y, int t, float2 (&z)[8]) {
+  constexpr int T = N / 8;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int n = t + T * e;
+    const bool lo = e < 4;
+    float2 x = X[lo ? n : N - n], y = Y[lo ? n : N - n];
+    if ((e == 0 || e == 4) && t == 0) {  // n = 0 and n = N/2: real parts only
+      x.y = 0.f;
+      y.y = 0.f;
+    }
+    z[e] = lo ? make_float2(x.x - y.y, x.y + y.x) : make_float2(x.x + y.y, y.x - x.y);
+  }
+}
+
+template <int N>
+__global__ void __launch_bounds__(YzCfg<N>::THREADS)
+k_yz_plane(const float2* __restrict__ w, const float2* __restrict__ wx, long long fs, float2* __restrict__ du,
+           long long ds, int kt, int kd, float s2, const float2* __restrict__ tw, const float2* __restrict__ ct8) {
+  pdl_begin();
+  using C = YzCfg<N>;
+  constexpr int T = C::T, XC = C::XC, H = C::H, LD = C::LD;
+  extern __shared__ __align__(16) float2 s_yz[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float2* xs = s_yz + 6 * C::FIELD + warp * C::XS;
+  const long long plane = (long long)blockIdx.x * N * H;
+  // y inverse: warp jobs (column tile, field), the field varying fastest
+  {
+    const float2* wb = w + (long long)blockIdx.y * 6 * fs + plane;
+    const float2* xb = wx + (long long)blockIdx.y * 2 * fs + plane;
+    const int p = lane % XC, t = lane / XC;
+    constexpr int TILES = (H + XC - 1) / XC;
+    for (int j = warp; j < 6 * TILES; j += C::WARPS) {
+      const int f = j % 6, col = j / 6 * XC + p;
+      const bool ok = col < H;
+      float2 v[8];
+      if (f == 3) {
+        const float kz = (float)col;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int o = (t + T * e) * H + col;
+          const float2 wy = ok ? __ldg(xb + o) : make_float2(0.f, 0.f);
+          const float2 wz = ok ? __ldg(xb + fs + o) : make_float2(0.f, 0.f);
+          const float ky = (float)kfull(t + T * e, N);
+          v[e] = mul_i<kInv>(make_float2(ky * wz.x - kz * wy.x, ky * wz.y - kz * wy.y));
+        }
+      } else {
+        const float2* src = f == 1 || f == 2 ? xb + (f - 1) * fs : wb + f * fs;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = ok ? __ldg(src + (t + T * e) * H + col) : make_float2(0.f, 0.f);
+      }
+      block_fft<N, 8, kInv, XC, kSyncWarp>(v, xs + p, t, tw, 1);
+      if (ok) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s_yz[f * C::FIELD + (t + T * e) * LD + col] = v[e];
+      }
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  // lines: slot y of T lanes; the z products of lines y and y + N/2 share one transform
+  {
+    const int y = threadIdx.x / T, t = threadIdx.x % T;
+    float2* xl = xs + lane / T * xpad_len<1>(N);
+    float2* row = s_yz + (y < N ? y : 0) * LD;
+    float pz[8];
+    auto put = [&](float2* dst, const float2 (&X)[4]) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int k = t + T * e;
+        if (k < kt) dst[k] = k <= kd ? X[e] : make_float2(0.f, 0.f);
+      }
+    };
+    if (y < N) {  // whole warps
+      float2 h1[8], h2[8], z[8];
+      c2r_pair_row<N>(row, row + C::FIELD, t, z);  // u_x + i u_y
+      warp_fft<N, 8, kInv>(z, xl, t, ct8);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) h1[e] = z[e];
+      __syncwarp();
+      c2r_pair_row<N>(row + 2 * C::FIELD, row + 3 * C::FIELD, t, z);  // u_z + i curl_x
+      warp_fft<N, 8, kInv>(z, xl, t, ct8);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) h2[e] = z[e];
+      __syncwarp();
+      c2r_pair_row<N>(row + 4 * C::FIELD, row + 5 * C::FIELD, t, z);  // curl_y + i curl_z
+      warp_fft<N, 8, kInv>(z, xl, t, ct8);
+      __syncwarp();
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float ux = h1[e].x, uy = h1[e].y, uz = h2[e].x, wx_ = h2[e].y, wy = z[e].x, wz = z[e].y;
+        pz[e] = fmaf(ux, wy, -uy * wx_);
+        z[e] = make_float2(fmaf(uy, wz, -uz * wy), fmaf(uz, wx_, -ux * wz));
+      }
+      warp_fft<N, 8, kFwd>(z, xl, t, ct8);
+      float2 X[4], Y[4];
+      r2c_pair_unpack<N>(z, t, s2, X, Y);
+      // this line's rows are read: they take its products
+      put(row, X);
+      put(row + C::FIELD, Y);
+      if (y >= N / 2) {
+        float* zr = reinterpret_cast<float*>(row + 3 * C::FIELD);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) zr[t + T * e] = pz[e];
+      }
+    }
+    __syncthreads();
+    if (y < N / 2 || (N / 2 * T < 32 && y < N)) {  // whole warps
+      const bool lower = y < N / 2;
+      const float* zr = reinterpret_cast<const float*>(s_yz + 3 * C::FIELD + (lower ? y + N / 2 : y) * LD);
+      float2 z[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) z[e] = make_float2(pz[e], zr[t + T * e]);
+      warp_fft<N, 8, kFwd>(z, xl, t, ct8);
+      float2 X[4], Y[4];
+      r2c_pair_unpack<N>(z, t, s2, X, Y);
+      if (lower) {
+        put(row + 2 * C::FIELD, X);
+        put(row + 2 * C::FIELD + N / 2 * LD, Y);
+      }
+    }
+  }
+  __syncthreads();
+  // y forward of the products' kept columns, rows |ky| <= kd to du
+  {
+    const int p = lane % XC, t = lane / XC;
+    const int tiles = (kt + XC - 1) / XC;
+    float2* db = du + (long long)blockIdx.y * 3 * ds + (long long)blockIdx.x * N * kt;
+    for (int j = warp; j < 3 * tiles; j += C::WARPS) {
+      const int c = j % 3, col = j / 3 * XC + p;
+      const bool ok = col < kt;
+      float2 v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        v[e] = ok ? s_yz[c * C::FIELD + (t + T * e) * LD + col] : make_float2(0.f, 0.f);
+      block_fft<N, 8, kFwd, XC, kSyncWarp>(v, xs + p, t, tw, 1);
+      if (ok) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int ky = t + T * e;
+          if ((unsigned)(kfull(ky, N) + kd) <= 2u * (unsigned)kd) db[c * ds + (long long)ky * kt + col] = v[e];
+        }
+      }
+      __syncwarp();
     }
   }
 }
