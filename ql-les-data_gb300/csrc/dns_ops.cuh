@@ -357,6 +357,13 @@ struct DnsOps {
       L3ES_LAUNCH(c, KK_YZ_PLANE, 5.0 / 3.0 * A + Adu * (2.0 * c.kd + 1.0) / N, s,
                   pdl_launch(k_yz_plane<N>, dim3(N, c.batch), YzCfg<N>::THREADS, YzCfg<N>::SMEM, s, c.W, c.Wx, c.fs,
                              c.DU, c.ds, c.kt, c.kd, 0.5f * scale * scale, c.tw, c.tw + line2_ct_offset<N>()));
+    } else if constexpr (DIM == 2 && N >= 16 && N <= 128) {
+      const double A = 8.0 * 3.0 * c.cs * c.batch, Adu = 8.0 * 3.0 * c.ds * c.batch;
+      const float scale = (float)(1.0 / ((double)N * N));
+      constexpr int LPC = 128 / (N / 8);
+      L3ES_LAUNCH(c, KK_LINE_CROSS, 2.0 * A + Adu, s,
+                  pdl_launch(line_cross_slots<N>, dim3((N + LPC - 1) / LPC, c.batch), 128, 0, s, c.W, c.fs, c.DU, c.ds,
+                             c.kt, c.kd, 0.5f * scale * scale, c.tw + line2_ct_offset<N>(), N));
     } else {
       nonlinear<DIM>(c, s);
     }

@@ -94,9 +94,22 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
   const long long so = ((long long)batch * 3 + g) * st.cs + m;  // + row * MC
   const float nu = st.nu_b[batch];
   float2 v[E];
+  // operands of the combination, in flight while the nonlinear term is transformed (a
+  // CTA's chain of loads and transforms is what a small grid waits for; registers are not)
+  float2 u0[RK >= 0 ? E : 1], sv[RK >= 1 ? E : 1], ac[RK >= 2 ? E : 1];
   if (RK >= 0) {
     const bool tile_band = __syncthreads_or(colband);
     if (!INV && !tile_band) return;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int row = t + T * e;
+      const bool band = colband && (unsigned)(kfull(row, N) + kd) <= ukd;
+      const long long o = so + (long long)row * MC;
+      const float2 z = make_float2(0.f, 0.f);
+      u0[RK >= 0 ? e : 0] = (band ? RK < 3 : INV && ok) ? S[o] : z;
+      if (RK >= 1) sv[RK >= 1 ? e : 0] = band ? T_[o] : z;
+      if (RK >= 2) ac[RK >= 2 ? e : 0] = band ? C[o] : z;
+    }
     if (tile_band) {
       // nonlinear term: x forward, dealias, Leray projection of this component
       const float2* db = du + ((long long)batch * 3 + g) * dcs + (long long)mid * kt + kh;
@@ -129,8 +142,7 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
       if (INV) __syncthreads();  // the products are read; su takes the new stage field
     }
   }
-  // stage combination on the band, closed form elsewhere: v becomes this component's
-  // field. Operands of four modes are loaded before the first of them is stored.
+  // stage combination on the band, closed form elsewhere: v becomes this component's field
   if constexpr (RK < 0) {
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = ok ? S[so + (long long)(t + T * e) * MC] : make_float2(0.f, 0.f);
@@ -140,50 +152,36 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
     prm.nu = nu;
     const float fscale = prm.band_kf2 > 0 ? (float)st.band_scale[batch] : 0.f;
     bool bad = false;
-    constexpr int CH = E < 4 ? E : 4;
 #pragma unroll
-    for (int e0 = 0; e0 < E; e0 += CH) {
-      float2 u0[CH], sv[CH], ac[CH];
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int row = t + T * (e0 + i);
-        const bool band = colband && (unsigned)(kfull(row, N) + kd) <= ukd;
-        const long long o = so + (long long)row * MC;
-        const float2 z = make_float2(0.f, 0.f);
-        u0[i] = (band ? RK < 3 : INV && ok) ? S[o] : z;
-        sv[i] = RK > 0 && band ? T_[o] : z;
-        ac[i] = RK > 1 && band ? C[o] : z;
-      }
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int e = e0 + i, row = t + T * e;
-        const int kx = kfull(row, N);
-        const long long o = so + (long long)row * MC;
-        const int ik2 = kx * kx + km * km + kh * kh;
-        float2 nv;
-        if (colband && (unsigned)(kx + kd) <= ukd) {
-          const float2 ra = rk_core_r<N, DIM, false>(row, mid, kh, ik2, g, v[e], RK == 0 ? u0[i] : sv[i], ac[i], u0[i],
-                                                     prm, fscale, nv);
-          if (RK == 1 || RK == 2) C[o] = ra;
-          if (RK == 3)
-            S[o] = nv;
-          else
-            T_[o] = nv;
-          if (RK == 3) bad |= !isfinite(nv.x + nv.y);
-          v[e] = nv;
-        } else if (RK == 3) {
-          v[e] = u0[i];  // the new state, written by stage 2
-        } else {
-          const float z = (nu * (float)ik2 + prm.drag) * prm.dt;
-          const float f = lin_stage_factor(RK, z);
-          if (RK == 2 && ok) {
-            const float gn = lin_stage_factor(3, z);
-            nv = make_float2(gn * u0[i].x, gn * u0[i].y);
-            S[o] = nv;
-            bad |= !isfinite(nv.x + nv.y);
-          }
-          v[e] = make_float2(f * u0[i].x, f * u0[i].y);
+    for (int e = 0; e < E; ++e) {
+      const int row = t + T * e;
+      const int kx = kfull(row, N);
+      const long long o = so + (long long)row * MC;
+      const int ik2 = kx * kx + km * km + kh * kh;
+      const float2 z0 = make_float2(0.f, 0.f);
+      float2 nv;
+      if (colband && (unsigned)(kx + kd) <= ukd) {
+        const float2 ra = rk_core_r<N, DIM, false>(row, mid, kh, ik2, g, v[e], RK == 0 ? u0[e] : sv[RK >= 1 ? e : 0],
+                                                   RK >= 2 ? ac[RK >= 2 ? e : 0] : z0, u0[e], prm, fscale, nv);
+        if (RK == 1 || RK == 2) C[o] = ra;
+        if (RK == 3)
+          S[o] = nv;
+        else
+          T_[o] = nv;
+        if (RK == 3) bad |= !isfinite(nv.x + nv.y);
+        v[e] = nv;
+      } else if (RK == 3) {
+        v[e] = u0[e];  // the new state, written by stage 2
+      } else {
+        const float z = (nu * (float)ik2 + prm.drag) * prm.dt;
+        const float f = lin_stage_factor(RK, z);
+        if (RK == 2 && ok) {
+          const float gn = lin_stage_factor(3, z);
+          nv = make_float2(gn * u0[e].x, gn * u0[e].y);
+          S[o] = nv;
+          bad |= !isfinite(nv.x + nv.y);
         }
+        v[e] = make_float2(f * u0[e].x, f * u0[e].y);
       }
     }
     if (RK >= 2 && bad) atomicOr(st.err, kErrNonFinite);
@@ -220,6 +218,61 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
 #pragma unroll
       for (int e = 0; e < E; ++e) dst[(long long)(t + T * e) * MC + m] = v[e];
     }
+  }
+}
+
+// ------------------------------------------------------------------------------
+// Half-axis line pass of 2D grids up to 128^2: one line per slot of T = N / 8 lanes, 32 / T
+// lines per warp, and the z products of two neighbouring slots in one transform that both
+// run (a slot doing two lines one after the other, as line_cross2 does, has a chain of 9
+// transforms instead of 5, on half as many warps: 8.1 us for 8 fields of 128^2). lines is
+// even.
+// ------------------------------------------------------------------------------
+template <int N>
+__global__ void __launch_bounds__(128)
+line_cross_slots(const float2* __restrict__ w, long long fs, float2* __restrict__ du, long long ds, int kt, int kd,
+                 float s2, const float2* __restrict__ ct8, int lines) {
+  pdl_begin();
+  static_assert(N >= 16 && N <= 128, "two lines per warp");
+  constexpr int T = N / 8, H = N / 2 + 1;
+  __shared__ float2 s_x[128 / T * xpad_len<1>(N)];
+  const int slot = threadIdx.x / T, t = threadIdx.x % T;
+  float2* xs = s_x + slot * xpad_len<1>(N);
+  const int line_raw = blockIdx.x * (128 / T) + slot;
+  const bool valid = line_raw < lines;
+  const int line = valid ? line_raw : lines - 2 + (slot & 1);
+  const float2* src = w + (long long)blockIdx.y * 6 * fs + (long long)line * H;
+  float2 h1[8], h2[8], z[8];
+  c2r_pair_load<N>(src, src + fs, t, h1);               // u_x + i u_y
+  c2r_pair_load<N>(src + 2 * fs, src + 3 * fs, t, h2);  // u_z + i curl_x
+  c2r_pair_load<N>(src + 4 * fs, src + 5 * fs, t, z);   // curl_y + i curl_z
+  warp_fft<N, 8, kInv>(h1, xs, t, ct8);
+  __syncwarp();
+  warp_fft<N, 8, kInv>(h2, xs, t, ct8);
+  __syncwarp();
+  warp_fft<N, 8, kInv>(z, xs, t, ct8);
+  __syncwarp();
+  float2 y[8];
+  const bool odd = slot & 1;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float ux = h1[e].x, uy = h1[e].y, uz = h2[e].x, wx = h2[e].y, wy = z[e].x, wz = z[e].y;
+    const float pz = fmaf(ux, wy, -uy * wx);
+    const float other = __shfl_xor_sync(0xffffffffu, pz, T);
+    y[e] = odd ? make_float2(other, pz) : make_float2(pz, other);
+    z[e] = make_float2(fmaf(uy, wz, -uz * wy), fmaf(uz, wx, -ux * wz));
+  }
+  warp_fft<N, 8, kFwd>(z, xs, t, ct8);
+  __syncwarp();
+  warp_fft<N, 8, kFwd>(y, xs, t, ct8);
+  float2 X[4], Y[4], A[4], B[4];
+  r2c_pair_unpack<N>(z, t, s2, X, Y);
+  r2c_pair_unpack<N>(y, t, s2, A, B);
+  if (valid) {
+    float2* dst = du + (long long)blockIdx.y * 3 * ds + (long long)line * kt;
+    store_du_line<N>(dst, X, t, kt, kd);
+    store_du_line<N>(dst + ds, Y, t, kt, kd);
+    store_du_line<N>(dst + 2 * ds, odd ? B : A, t, kt, kd);
   }
 }
 
