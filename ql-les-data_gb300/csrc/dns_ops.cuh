@@ -59,6 +59,10 @@ struct DnsOps {
       tma_band_fused_ctas = persistent_ctas(kx_fwd_band_tma<N, true>);
     }
     if constexpr (N >= 16) stage_attrs<2>();
+    if constexpr (N >= 16 && N <= kStep2dMax) {
+      cudaFuncSetAttribute(k_step2d<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Step2dCfg<N>::SMEM);
+      cudaGetLastError();
+    }
     if constexpr (N >= 16 && N <= kStageMax3d) {
       stage_attrs<3>();
       cudaFuncSetAttribute(k_yz_plane<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, YzCfg<N>::SMEM);
@@ -389,6 +393,28 @@ struct DnsOps {
     }
   }
 
+  // nsteps RK4 steps of a 2D grid in one launch (k_step2d)
+  static void steps2d(const Ctx& c, float2* S, const EpiParams* prm, int nsteps, cudaStream_t s) {
+    if constexpr (N >= 16 && N <= kStep2dMax) {
+      Step2d a{};
+      a.cs = c.cs;
+      a.nsteps = nsteps;
+      a.prm = prm[0];
+      for (int rk = 0; rk < 4; ++rk) {
+        a.a_dt[rk] = prm[rk].a_dt;
+        a.b_dt[rk] = prm[rk].b_dt;
+      }
+      a.inv_n2d = 1.0 / std::pow((double)N, 4);
+      a.eps_inj = c.eps_inj;
+      a.nu_b = c.nu_b;
+      a.err = c.err;
+      const float scale = (float)(1.0 / ((double)N * N));
+      L3ES_LAUNCH(c, KK_X_STAGE, 2.0 * 8.0 * 3.0 * c.cs * c.batch, s,
+                  pdl_launch(k_step2d<N>, c.batch, YzCfg<N>::THREADS, Step2dCfg<N>::SMEM, s, S, a, 0.5f * scale * scale,
+                             c.tw, c.tw + line2_ct_offset<N>()));
+    }
+  }
+
   static void step(const Ctx& c, float2* S, const EpiParams* prm, bool first, bool last, cudaStream_t s) {
     if (c.dim == 3)
       step_dim<3>(c, S, prm, first, last, s);
@@ -516,6 +542,7 @@ DnsTable make_dns_table() {
   DnsTable t;
   t.stage = &DnsOps<N>::stage;
   t.step = &DnsOps<N>::step;
+  t.steps2d = &DnsOps<N>::steps2d;
   t.irfftn = &DnsOps<N>::irfftn;
   t.rfftn = &DnsOps<N>::rfftn;
   t.vjp = &DnsOps<N>::vjp;

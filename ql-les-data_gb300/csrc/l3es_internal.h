@@ -179,6 +179,8 @@ struct DnsTable {
   // one explicit RK4 step in place on S by kx_stage; prm: the four stages. first / last:
   // whether the step opens with an x inverse of S / ends without one of the new state
   void (*step)(const Ctx&, float2* S, const EpiParams* prm, bool first, bool last, cudaStream_t s);
+  // nsteps explicit RK4 steps of a small 2D grid in one launch
+  void (*steps2d)(const Ctx&, float2* S, const EpiParams* prm, int nsteps, cudaStream_t s);
   void (*irfftn)(const Ctx&, const float2* uh, float* u, cudaStream_t s);
   void (*rfftn)(const Ctx&, const float* u, float2* uh, cudaStream_t s);
   // vector-Jacobian product of the RHS at a.us with cotangent a.gscale * a.g, folded

@@ -497,11 +497,11 @@ static void tune_cache_write(const char* path, const std::string& key, const int
   std::fclose(f);
 }
 
-// One RK4 step of the state S in the plan's step form (spectral_solver.py:65-80; the
-// forcing rescale of ekin_tot follows each step in run_steps). first / last: whether the
-// x inverse of S has to be made, and whether the one of the new state is left out; the
-// forms with an elementwise update do neither.
-static void rk4_step(l3es_plan* plan, float2* S, bool first, bool last, cudaStream_t s) {
+// RK4 steps of the state S in the plan's step form (spectral_solver.py:65-80; the forcing
+// rescale of ekin_tot follows each step in run_steps), at most `most` of them; returns how
+// many it made. first / last: whether the x inverse of S has to be made, and whether the
+// one of the new state is left out (kx_stage; the other forms do neither).
+static int rk4_step(l3es_plan* plan, float2* S, int most, bool first, bool last, cudaStream_t s) {
   const Ctx& c = plan->ctx;
   const l3es_plan_desc& d = plan->desc;
   static const double a_rk4[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
@@ -532,14 +532,19 @@ static void rk4_step(l3es_plan* plan, float2* S, bool first, bool last, cudaStre
     q.lin = lin_ok;
     q.band_rk = band;
   }
+  if (one_visit && c.dim == 2 && c.n <= kStep2dMax) {  // (kd, kt of these N are Step2dCfg's)
+    plan->tab.steps2d(c, S, prm, most, s);
+    return most;
+  }
   if (one_visit) {
     plan->tab.step(c, S, prm, first, last, s);
-    return;
+    return 1;
   }
   // the band-fused stages (XLin, BandRk) work in place, the accumulator in C in the band's
   // compact layout; the elementwise update keeps its stage field in T
   for (int rk = 0; rk < 4; ++rk)
     plan->tab.stage(c, band || rk == 0 ? S : c.Tb, S, band ? S : c.Tb, rk, prm[rk], s);
+  return 1;
 }
 
 // mean milliseconds of one RK4 step in the plan's step form with its current schedule,
@@ -547,10 +552,10 @@ static void rk4_step(l3es_plan* plan, float2* S, bool first, bool last, cudaStre
 // stage field with the state; zeros stay finite through every term)
 static float time_step(l3es_plan* p, cudaStream_t s, cudaEvent_t e0, cudaEvent_t e1) {
   const Ctx& c = p->ctx;
-  rk4_step(p, c.Tb, true, true, s);
+  rk4_step(p, c.Tb, 1, true, true, s);
   const int reps = c.cs * c.batch > (1 << 20) ? 2 : 5;
   cudaEventRecord(e0, s);
-  for (int i = 0; i < reps; ++i) rk4_step(p, c.Tb, true, true, s);
+  for (int i = 0; i < reps; ++i) rk4_step(p, c.Tb, 1, true, true, s);
   cudaEventRecord(e1, s);
   cudaEventSynchronize(e1);
   float ms = 0.f;
@@ -643,9 +648,16 @@ static int run_steps(l3es_plan* plan, void* u_hat, float* u_out, int32_t nsteps,
   const double inv_n2d = 1.0 / std::pow((double)c.n, 2 * c.dim);
   const double eps64 = 2.220446049250313e-16;  // jnp.finfo(float).eps, spectral_solver.py:23
   for (int st = 0; st < nsteps; ++st) {
-    // the ekin_tot rescale changes the new state, so its x inverse cannot be part of the step
+    // the ekin_tot rescale changes the new state: its x inverse cannot be part of the step,
+    // and the steps are made one by one
     const bool apart = d.forcing == L3ES_FORCING_EKIN_TOT;
-    rk4_step(plan, S, st == 0 || apart, st == nsteps - 1 || apart, s);
+    const int made = rk4_step(plan, S, apart ? 1 : nsteps - st, st == 0 || apart, st == nsteps - 1 || apart, s);
+    if (!apart && made > 1) {  // every step's e_inj is 0
+      if (e_inj_dev)
+        L3ES_TRY_CUDA(cudaMemsetAsync(e_inj_dev + (long long)st * c.batch, 0, sizeof(double) * c.batch * (made - 1), s),
+                      "l3es_step memset");
+      st += made - 1;
+    }
     double* einj = e_inj_dev ? e_inj_dev + (long long)st * c.batch : c.einj;
     double* ke_final = (ke_dev && st == nsteps - 1) ? ke_dev : nullptr;
     // energy partials of the new state by the row-wise float-float pass (a separate

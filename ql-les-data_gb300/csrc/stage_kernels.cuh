@@ -301,6 +301,11 @@ struct YzCfg {
   static constexpr int SMEM = (6 * FIELD + WARPS * XS) * (int)sizeof(float2);
 };
 
+template <int D>
+struct Dir {
+  static constexpr int value = D;
+};
+
 // Z = X_ext + i Y_ext (c2r_pair_load) from two half-spectrum rows in shared memory
 template <int N>
 __device__ __forceinline__ void c2r_pair_row(const float2* X, const float2* Y, int t, float2 (&z)[8]) {
@@ -315,6 +320,77 @@ __device__ __forceinline__ void c2r_pair_row(const float2* X, const float2* Y, i
       y.y = 0.f;
     }
     z[e] = lo ? make_float2(x.x - y.y, x.y + y.x) : make_float2(x.x + y.y, y.x - x.y);
+  }
+}
+
+// Half-axis lines of a plane in shared memory (six fields, rows of LD): u x curl u of every
+// row into the first kt columns of fields 0..2. Slot y of T lanes takes row y; the z
+// products of rows y and y + N/2 share one transform. All threads; xs: the warp's exchange
+// buffer.
+template <int N>
+__device__ __forceinline__ void plane_lines(float2* s_yz, float2* xs, int kt, int kd, float s2,
+                                            const float2* __restrict__ ct8) {
+  using C = YzCfg<N>;
+  constexpr int T = C::T, LD = C::LD;
+  const int lane = threadIdx.x & 31;
+  const int y = threadIdx.x / T, t = threadIdx.x % T;
+  float2* xl = xs + lane / T * xpad_len<1>(N);
+  float2* row = s_yz + (y < N ? y : 0) * LD;
+  float pz[8];
+  auto put = [&](float2* dst, const float2 (&X)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int k = t + T * e;
+      if (k < kt) dst[k] = k <= kd ? X[e] : make_float2(0.f, 0.f);
+    }
+  };
+  if (y < N) {  // whole warps
+    float2 h1[8], h2[8], z[8];
+    c2r_pair_row<N>(row, row + C::FIELD, t, z);  // u_x + i u_y
+    warp_fft<N, 8, kInv>(z, xl, t, ct8);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) h1[e] = z[e];
+    __syncwarp();
+    c2r_pair_row<N>(row + 2 * C::FIELD, row + 3 * C::FIELD, t, z);  // u_z + i curl_x
+    warp_fft<N, 8, kInv>(z, xl, t, ct8);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) h2[e] = z[e];
+    __syncwarp();
+    c2r_pair_row<N>(row + 4 * C::FIELD, row + 5 * C::FIELD, t, z);  // curl_y + i curl_z
+    warp_fft<N, 8, kInv>(z, xl, t, ct8);
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float ux = h1[e].x, uy = h1[e].y, uz = h2[e].x, wx_ = h2[e].y, wy = z[e].x, wz = z[e].y;
+      pz[e] = fmaf(ux, wy, -uy * wx_);
+      z[e] = make_float2(fmaf(uy, wz, -uz * wy), fmaf(uz, wx_, -ux * wz));
+    }
+    warp_fft<N, 8, kFwd>(z, xl, t, ct8);
+    float2 X[4], Y[4];
+    r2c_pair_unpack<N>(z, t, s2, X, Y);
+    // this line's rows are read: they take its products
+    put(row, X);
+    put(row + C::FIELD, Y);
+    if (y >= N / 2) {
+      float* zr = reinterpret_cast<float*>(row + 3 * C::FIELD);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) zr[t + T * e] = pz[e];
+    }
+  }
+  __syncthreads();
+  if (y < N / 2 || (N / 2 * T < 32 && y < N)) {  // whole warps
+    const bool lower = y < N / 2;
+    const float* zr = reinterpret_cast<const float*>(s_yz + 3 * C::FIELD + (lower ? y + N / 2 : y) * LD);
+    float2 z[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) z[e] = make_float2(pz[e], zr[t + T * e]);
+    warp_fft<N, 8, kFwd>(z, xl, t, ct8);
+    float2 X[4], Y[4];
+    r2c_pair_unpack<N>(z, t, s2, X, Y);
+    if (lower) {
+      put(row + 2 * C::FIELD, X);
+      put(row + 2 * C::FIELD + N / 2 * LD, Y);
+    }
   }
 }
 
@@ -363,68 +439,7 @@ k_yz_plane(const float2* __restrict__ w, const float2* __restrict__ wx, long lon
     }
   }
   __syncthreads();
-  // lines: slot y of T lanes; the z products of lines y and y + N/2 share one transform
-  {
-    const int y = threadIdx.x / T, t = threadIdx.x % T;
-    float2* xl = xs + lane / T * xpad_len<1>(N);
-    float2* row = s_yz + (y < N ? y : 0) * LD;
-    float pz[8];
-    auto put = [&](float2* dst, const float2 (&X)[4]) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int k = t + T * e;
-        if (k < kt) dst[k] = k <= kd ? X[e] : make_float2(0.f, 0.f);
-      }
-    };
-    if (y < N) {  // whole warps
-      float2 h1[8], h2[8], z[8];
-      c2r_pair_row<N>(row, row + C::FIELD, t, z);  // u_x + i u_y
-      warp_fft<N, 8, kInv>(z, xl, t, ct8);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) h1[e] = z[e];
-      __syncwarp();
-      c2r_pair_row<N>(row + 2 * C::FIELD, row + 3 * C::FIELD, t, z);  // u_z + i curl_x
-      warp_fft<N, 8, kInv>(z, xl, t, ct8);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) h2[e] = z[e];
-      __syncwarp();
-      c2r_pair_row<N>(row + 4 * C::FIELD, row + 5 * C::FIELD, t, z);  // curl_y + i curl_z
-      warp_fft<N, 8, kInv>(z, xl, t, ct8);
-      __syncwarp();
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float ux = h1[e].x, uy = h1[e].y, uz = h2[e].x, wx_ = h2[e].y, wy = z[e].x, wz = z[e].y;
-        pz[e] = fmaf(ux, wy, -uy * wx_);
-        z[e] = make_float2(fmaf(uy, wz, -uz * wy), fmaf(uz, wx_, -ux * wz));
-      }
-      warp_fft<N, 8, kFwd>(z, xl, t, ct8);
-      float2 X[4], Y[4];
-      r2c_pair_unpack<N>(z, t, s2, X, Y);
-      // this line's rows are read: they take its products
-      put(row, X);
-      put(row + C::FIELD, Y);
-      if (y >= N / 2) {
-        float* zr = reinterpret_cast<float*>(row + 3 * C::FIELD);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) zr[t + T * e] = pz[e];
-      }
-    }
-    __syncthreads();
-    if (y < N / 2 || (N / 2 * T < 32 && y < N)) {  // whole warps
-      const bool lower = y < N / 2;
-      const float* zr = reinterpret_cast<const float*>(s_yz + 3 * C::FIELD + (lower ? y + N / 2 : y) * LD);
-      float2 z[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) z[e] = make_float2(pz[e], zr[t + T * e]);
-      warp_fft<N, 8, kFwd>(z, xl, t, ct8);
-      float2 X[4], Y[4];
-      r2c_pair_unpack<N>(z, t, s2, X, Y);
-      if (lower) {
-        put(row + 2 * C::FIELD, X);
-        put(row + 2 * C::FIELD + N / 2 * LD, Y);
-      }
-    }
-  }
+  plane_lines<N>(s_yz, xs, kt, kd, s2, ct8);
   __syncthreads();
   // y forward of the products' kept columns, rows |ky| <= kd to du
   {
@@ -449,6 +464,193 @@ k_yz_plane(const float2* __restrict__ w, const float2* __restrict__ wx, long lon
       __syncwarp();
     }
   }
+}
+
+// ------------------------------------------------------------------------------
+// Whole RK4 steps of a 2D grid up to 32^2, one CTA per trajectory: the six fields of a
+// stage (31 KB at 32^2), its field and the accumulator on the band fit shared memory, and a
+// thread keeps the step's initial state of its modes in registers, so nsteps steps are one
+// launch that reads and writes the state once. A stage is the transforms and the combination
+// of kx_stage and the lines of k_yz_plane (the plane's rows are x here, its columns the half
+// axis), four block barriers in place of two launches. Ten steps at 32^2 x 9 took 266 us by
+// kx_stage and 82 us a single step from the start of plain launches; here 152 and 18 us. At
+// 64^2 one SM's issue rate is the bound (46 us a step; kx_stage over 17 SMs 33 us).
+// ------------------------------------------------------------------------------
+constexpr int kStep2dMax = 32;
+
+template <int N>
+struct Step2dCfg {
+  using Y = YzCfg<N>;
+  static constexpr int MODES = N * Y::H;
+  static constexpr int PER = (MODES + Y::THREADS - 1) / Y::THREADS;  // modes per thread
+  // the stage field and the accumulator live on the band only: [component][kx + KD][kh < KT]
+  static constexpr int KD = (N + 1) / 3, KT = (KD + 8) / 8 * 8;  // the plan's kd, kt at N = 16, 32
+  static constexpr int BAND = (2 * KD + 1) * KT;
+  static constexpr int SMEM = Y::SMEM + 2 * 3 * BAND * (int)sizeof(float2);
+};
+
+struct Step2d {
+  long long cs;
+  int nsteps;
+  float a_dt[4], b_dt[4];
+  EpiParams prm;  // what the stages share
+  double inv_n2d, eps_inj;
+  const float* nu_b;
+  int* err;
+};
+
+template <int N>
+__global__ void __launch_bounds__(YzCfg<N>::THREADS)
+k_step2d(float2* __restrict__ S, const __grid_constant__ Step2d a, float s2, const float2* __restrict__ tw,
+         const float2* __restrict__ ct8) {
+  pdl_begin();
+  using C = YzCfg<N>;
+  using K = Step2dCfg<N>;
+  constexpr int T = C::T, XC = C::XC, H = C::H, LD = C::LD, PER = K::PER;
+  extern __shared__ __align__(16) float2 s_step[];
+  __shared__ double red[32];
+  __shared__ double s_scale;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float2* xs = s_step + 6 * C::FIELD + warp * C::XS;
+  float2* us = s_step + 6 * C::FIELD + C::WARPS * C::XS;  // stage field and, behind it, accumulator
+  float2* acc = us + 3 * K::BAND;
+  float2* Sb = S + (long long)blockIdx.x * 3 * a.cs;
+  constexpr int kd = K::KD, kt = K::KT;
+  constexpr unsigned ukd = 2u * (unsigned)kd;
+  EpiParams prm = a.prm;
+  prm.nu = a.nu_b[blockIdx.x];
+  // this thread's modes threadIdx.x + i THREADS
+  auto row_of = [&](int i) { return (int)(threadIdx.x + i * C::THREADS) / H; };
+  auto col_of = [&](int i) { return (int)(threadIdx.x + i * C::THREADS) % H; };
+  auto has = [&](int i) { return (int)(threadIdx.x + i * C::THREADS) < K::MODES; };
+  float2 u0[PER][3];
+  // the stage field of mode i: kept on the band, and with its curl put on the plane
+  auto open = [&](int i, const float2 (&v)[3]) {
+    const int row = row_of(i), kh = col_of(i), kxb = kfull(row, N) + kd;
+    if (kh < kt && (unsigned)kxb <= ukd) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) us[c * K::BAND + kxb * kt + kh] = v[c];
+    }
+    float2* f = s_step + row * LD + kh;
+    float k0, k1, k2;
+    kvec<2>(kfull(row, N), 0, kh, k0, k1, k2);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) f[c * C::FIELD] = v[c];
+    f[3 * C::FIELD] = mul_i<kInv>(make_float2(k1 * v[2].x - k2 * v[1].x, k1 * v[2].y - k2 * v[1].y));
+    f[4 * C::FIELD] = mul_i<kInv>(make_float2(k2 * v[0].x - k0 * v[2].x, k2 * v[0].y - k0 * v[2].y));
+    f[5 * C::FIELD] = mul_i<kInv>(make_float2(k0 * v[1].x - k1 * v[0].x, k0 * v[1].y - k1 * v[0].y));
+  };
+  // x transforms of the first cols columns of nf fields, in place, 32 / T columns per warp
+  const int p = lane % XC, t = lane / XC;
+  auto x_pass = [&](auto dir, int nf, int cols) {
+    constexpr int D = decltype(dir)::value;
+    const int jobs = nf * ((cols + XC - 1) / XC);
+    for (int j = warp; j < jobs; j += C::WARPS) {
+      const int f = j % nf, col = j / nf * XC + p;
+      const bool ok = col < cols;
+      float2* q = s_step + f * C::FIELD + t * LD + (ok ? col : 0);
+      float2 v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = ok ? q[T * e * LD] : make_float2(0.f, 0.f);
+      block_fft<N, 8, D, XC, kSyncWarp>(v, xs + p, t, tw, 1);
+      if (ok) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) q[T * e * LD] = v[e];
+      }
+      __syncwarp();
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      u0[i][c] = has(i) ? Sb[c * a.cs + threadIdx.x + i * C::THREADS] : make_float2(0.f, 0.f);
+    if (has(i)) open(i, u0[i]);
+  }
+  bool bad = false;
+#pragma unroll 1
+  for (int q = 0; q < 4 * a.nsteps; ++q) {
+    const int rk = q & 3;
+    __syncthreads();
+    x_pass(Dir<kInv>{}, 6, H);
+    __syncthreads();
+    plane_lines<N>(s_step, xs, kt, kd, s2, ct8);
+    __syncthreads();
+    x_pass(Dir<kFwd>{}, 3, kt);
+    float fscale = 0.f;
+    if (prm.band_kf2 > 0) {  // constant-power coefficient of the stage field
+      double lo = 0.0;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int kx = kfull(row_of(i), N), kh = col_of(i), ik2 = kx * kx + kh * kh;
+        if (!has(i) || ik2 == 0 || ik2 > prm.band_kf2) continue;  // kf <= N/4 < kd
+        const int wg = kh == 0 || kh == N / 2 ? 1 : 2;
+        for (int c = 0; c < 3; ++c) {
+          const float2 v = us[c * K::BAND + (kx + kd) * kt + kh];
+          lo += wg * ((double)v.x * v.x + (double)v.y * v.y);
+        }
+      }
+      for (int o = 16; o > 0; o >>= 1) lo += __shfl_xor_sync(0xffffffffu, lo, o);
+      if (lane == 0) red[warp] = lo;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double sum = 0.0;
+        for (int i = 0; i < C::WARPS; ++i) sum += red[i];
+        s_scale = a.eps_inj / (2.0 * (0.5 * sum * a.inv_n2d) + 1e-30);
+      }
+    }
+    __syncthreads();
+    if (prm.band_kf2 > 0) fscale = (float)s_scale;
+    prm.rk = rk;
+    prm.a_dt = a.a_dt[rk];
+    prm.b_dt = a.b_dt[rk];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      if (!has(i)) continue;
+      const int row = row_of(i), kh = col_of(i), kx = kfull(row, N);
+      const int ik2 = kx * kx + kh * kh;
+      float2 nv[3];
+      if (kh < kt && (unsigned)(kx + kd) <= ukd) {
+        const float2* f = s_step + row * LD + kh;
+        const bool keep = kh <= kd;
+        float2 d[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) d[c] = keep ? f[c * C::FIELD] : make_float2(0.f, 0.f);
+        const float k0 = (float)kx, k1 = (float)kh;
+        const float inv = 1.0f / (ik2 == 0 ? 1.0f : (float)ik2);
+        const float pr = (d[0].x * k0 + d[1].x * k1) * inv, pi_ = (d[0].y * k0 + d[1].y * k1) * inv;
+        d[0] = make_float2(d[0].x - pr * k0, d[0].y - pi_ * k0);
+        d[1] = make_float2(d[1].x - pr * k1, d[1].y - pi_ * k1);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int o = c * K::BAND + (kx + kd) * kt + kh;
+          const float2 ra = rk_core_r<N, 2, false>(row, 0, kh, ik2, c, d[c], us[o], rk >= 2 ? acc[o] : d[c], u0[i][c], prm,
+                                                   fscale, nv[c]);
+          if (rk == 1 || rk == 2) acc[o] = ra;
+        }
+      } else {
+        const float z = (prm.nu * (float)ik2 + prm.drag) * prm.dt;
+        const float f = lin_stage_factor(rk, z);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) nv[c] = make_float2(f * u0[i][c].x, f * u0[i][c].y);
+      }
+      if (rk == 3) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          u0[i][c] = nv[c];
+          bad |= !isfinite(nv[c].x + nv[c].y);
+        }
+      }
+      open(i, nv);
+    }
+  }
+  if (bad) atomicOr(a.err, kErrNonFinite);
+#pragma unroll
+  for (int i = 0; i < PER; ++i)
+    if (has(i)) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) Sb[c * a.cs + threadIdx.x + i * C::THREADS] = u0[i][c];
+    }
 }
 
 // Constant-power coefficient of a stage field (one CTA per trajectory): the low modes of
