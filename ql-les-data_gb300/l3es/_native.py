@@ -144,10 +144,13 @@ def _check(rc: int, what: str) -> None:
 
 
 def _stream(stream=None) -> int:
+    if stream is not None:
+        return stream.cuda_stream
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    # the current stream's handle without the Stream object around it, which took longer to
+    # make than a small grid's kernels to launch
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _ptr(t) -> int:

@@ -130,7 +130,7 @@ class StepFn:
         p = self.plan
         uh = _as_spec(u_hat, self.N, self.dim).clone()
         u_new = torch.empty(p.phys_shape, dtype=torch.float32, device="cuda")
-        e_inj = torch.zeros(1, dtype=torch.float64, device="cuda")
+        e_inj = torch.empty(1, dtype=torch.float64, device="cuda")  # the step writes it
         p.step(uh, 1, u_out=u_new, e_inj=e_inj)
         return u_new, uh, e_inj[0]
 
