@@ -10,8 +10,8 @@
 // One evaluation:
 //   kx_inv (curl)      u, w lines (the forward kernel)
 //   kx_inv_adjproj     m lines: dealias mask, Leray projection and 1/wt in the prologue
-//                      (block 0 also reduces the constant-power band terms)
-//   ky_pass inverse    (3D) on the 9 fields
+//                      (block 0 also reduces the constant-power band terms), band columns only
+//   ky_inv_rhs, ky_inv_band  (3D) on the 9 fields
 //   line_cross_adj     c2r of m (parked), u and w; r2c of m x u and m x w, all modes
 //   ky_pass forward    (3D) on the 6 products
 //   kx_fwd_plain       x-axis forward FFT of the 6 products
@@ -68,33 +68,34 @@ __device__ __forceinline__ void band_adj_terms(const float2* __restrict__ us, co
 }
 
 // ------------------------------------------------------------------------------
-// x-axis inverse pass of m = D P (gscale g) / wt (3 fields), columns like kx_inv.
-// D: the cube band |kx|, |kmid|, khalf <= kd; P: Leray projection (k = 0 untouched).
-// With band_kf > 0, block (0, b) also writes the band terms of trajectory b.
+// x-axis inverse pass of m = D P (gscale g) / wt (3 fields). D: the cube band |kx|, |kmid|,
+// khalf <= kd; P: Leray projection (k = 0 untouched). m vanishes outside the band, so only
+// its columns are transformed and stored, in the layout of the nonlinear term: [x][mid][kt],
+// rows |kmid| <= kd. CTA = (half-axis tile inside kt, middle row inside the band,
+// trajectory). With band_kf > 0, block (0, 0, b) also writes the band terms of trajectory b.
+// (All columns, most of them zeros, took 12.7 us at 128^3, and as much again in the y pass.)
 // ------------------------------------------------------------------------------
 template <int N, int DIM>
 __global__ void __launch_bounds__(TW * Fft<N>::T)
-kx_inv_adjproj(const float2* __restrict__ g, long long cs, float gscale, int kd, float2* __restrict__ w,
-               long long fs, const float2* __restrict__ tw, const float2* __restrict__ us, int band_kf,
+kx_inv_adjproj(const float2* __restrict__ g, long long cs, float gscale, int kd, int kt, float2* __restrict__ w,
+               long long ds, const float2* __restrict__ tw, const float2* __restrict__ us, int band_kf,
                double inv_n2d, double eps_inj, double* __restrict__ band_out) {
   pdl_begin();
   constexpr int E = Fft<N>::E, T = Fft<N>::T, H = N / 2 + 1;
   constexpr int NMID = DIM == 3 ? N : 1;
-  constexpr int MC = NMID * H;
   __shared__ float2 sm[xpad_len<TW>(N) * TW];
   const int p = threadIdx.x % TW, t = threadIdx.x / TW;
-  const int m = blockIdx.x * TW + p;
-  const bool ok = m < MC;
-  const long long bg = (long long)blockIdx.y * 3 * cs, bw = (long long)blockIdx.y * 3 * fs;
-  if (band_kf > 0 && blockIdx.x == 0)
-    band_adj_terms<DIM>(us + bg, g + bg, cs, gscale, N, band_kf, inv_n2d, eps_inj, band_out + 2 * blockIdx.y);
-  const int kh = m % H;
-  const int km = DIM == 3 ? kfull(m / H, N) : 0;
+  const int kh = blockIdx.x * TW + p;
+  const int km = DIM == 3 ? (int)blockIdx.y - kd : 0;
+  const int mid = km < 0 ? km + N : km;
+  const long long bg = (long long)blockIdx.z * 3 * cs;
+  if (band_kf > 0 && blockIdx.x == 0 && blockIdx.y == 0)
+    band_adj_terms<DIM>(us + bg, g + bg, cs, gscale, N, band_kf, inv_n2d, eps_inj, band_out + 2 * blockIdx.z);
   const float inv_wt = (kh == 0 || kh == N / 2) ? gscale : 0.5f * gscale;
   // band membership as unsigned offsets: -kd <= k <= kd  <=>  (unsigned)(k + kd) <= 2 kd
   // (the signed two-sided form was observed to keep out-of-band rows on the GPU)
   const unsigned span = 2u * (unsigned)kd;
-  const bool col_keep = ok && (unsigned)(km + kd) <= span && (unsigned)kh <= (unsigned)kd;
+  const bool col_keep = (unsigned)kh <= (unsigned)kd;
   float2 a[3][E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
@@ -102,7 +103,7 @@ kx_inv_adjproj(const float2* __restrict__ g, long long cs, float gscale, int kd,
     const bool keep = col_keep && (unsigned)(kx + kd) <= span;
     float2 v0 = make_float2(0.f, 0.f), v1 = v0, v2 = v0;
     if (keep) {
-      const long long o = bg + (long long)(t + T * e) * MC + m;
+      const long long o = bg + ((long long)(t + T * e) * NMID + mid) * H + kh;
       v0 = g[o];
       v1 = g[o + cs];
       v2 = g[o + 2 * cs];
@@ -117,14 +118,39 @@ kx_inv_adjproj(const float2* __restrict__ g, long long cs, float gscale, int kd,
     a[1][e] = make_float2(inv_wt * (v1.x - pr * k1), inv_wt * (v1.y - pi_ * k1));
     a[2][e] = make_float2(inv_wt * (v2.x - pr * k2), inv_wt * (v2.y - pi_ * k2));
   }
+  float2* wb = w + (long long)blockIdx.z * 3 * ds + (long long)mid * kt + kh;
 #pragma unroll
   for (int f = 0; f < 3; ++f) {
     block_fft<N, E, kInv, TW>(a[f], sm + p, t, tw, 1);
-    if (ok) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) w[bw + f * fs + (long long)(t + T * e) * MC + m] = a[f][e];
-    }
+    for (int e = 0; e < E; ++e) wb[f * ds + (long long)(t + T * e) * NMID * kt] = a[f][e];
     __syncthreads();
+  }
+}
+
+// y-axis inverse pass of m (3D), in place: columns kh < kt of field blockIdx.z, x plane
+// blockIdx.y; rows |ky| > kd are zeros that are not stored yet.
+template <int N, int V>
+__global__ void __launch_bounds__(KyCfg<N, V>::THREADS)
+ky_inv_band(float2* __restrict__ w, long long ds, int kt, int kd, const float2* __restrict__ tw) {
+  pdl_begin();
+  using C = KyCfg<N, V>;
+  constexpr int E = C::E, T = C::T, TWY = C::TWY;
+  __shared__ float2 sm[xpad_len<TWY>(N) * TWY];
+  const int p = threadIdx.x % TWY, t = threadIdx.x / TWY;
+  const int col = blockIdx.x * TWY + p;
+  const bool ok = col < kt;
+  float2* base = w + blockIdx.z * ds + (long long)blockIdx.y * N * kt + col;
+  float2 v[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const bool in = ok && (unsigned)(kfull(t + T * e, N) + kd) <= 2u * (unsigned)kd;
+    v[e] = in ? base[(long long)(t + T * e) * kt] : make_float2(0.f, 0.f);
+  }
+  block_fft<N, E, kInv, TWY>(v, sm + p, t, tw, 1);
+  if (ok) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) base[(long long)(t + T * e) * kt] = v[e];
   }
 }
 
@@ -133,11 +159,12 @@ kx_inv_adjproj(const float2* __restrict__ g, long long cs, float gscale, int kd,
 // same thread writes and reads), then of the 3 u lines and the 3 w lines; C = m x u
 // and A = m x w accumulate in registers and are r2c'd (every half-axis mode) when
 // their triple is complete: out fields 0..2 = C, 3..5 = A.
-// wm: [batch][3][fs] (m), wuw: [batch][6][fs] (u, w), out: [batch][6][cs].
+// wm: [batch][3][ds] (m, modes k < kt of a line), wuw: [batch][6][fs] (u, w), out:
+// [batch][6][cs].
 // ------------------------------------------------------------------------------
 template <int N>
 __global__ void __launch_bounds__(LineCfg<N>::THREADS, 3)
-line_cross_adj(const float2* __restrict__ wm, const float2* __restrict__ wuw, long long fs,
+line_cross_adj(const float2* __restrict__ wm, long long ds, int kt, const float2* __restrict__ wuw, long long fs,
                float2* __restrict__ out, long long cs, float scale, const float2* __restrict__ twN, int nlines) {
   pdl_begin();
   using C = LineCfg<N>;
@@ -149,14 +176,17 @@ line_cross_adj(const float2* __restrict__ wm, const float2* __restrict__ wuw, lo
   const long long line_raw = (long long)blockIdx.x * LPC + q;
   const bool valid = line_raw < nlines;
   const long long line = valid ? line_raw : nlines - 1;  // idle lines mirror a valid one
-  const float2* srcm = wm + (long long)batch * 3 * fs + line * H;
+  const float2* srcm = wm + (long long)batch * 3 * ds + line * kt;
   const float2* srcy = wuw + (long long)batch * 6 * fs + line * H;
   float2* xs = s_x + q * C::XS;
   float2* sm_ = s_m + q * C::PS;
 #pragma unroll
   for (int f = 0; f < 3; ++f) {
     float2 v[E];
-    c2r_load_pack<M, E>(srcm + f * fs, t, v, twN, scale);
+    float2 xk[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) xk[e] = t + T * e < kt ? __ldg(srcm + f * ds + t + T * e) : make_float2(0.f, 0.f);
+    c2r_pack<M, E>(xk, M < kt ? __ldg(srcm + f * ds + M) : make_float2(0.f, 0.f), t, v, twN, scale);
     warp_fft<M, E, kInv>(v, xs, t, twN + N);
 #pragma unroll
     for (int e = 0; e < E; ++e) sm_[f * M + t + T * e] = v[e];  // physical values at 2n, 2n+1

@@ -505,17 +505,25 @@ struct DnsOps {
     // the lines the stage recomputation left (a.wlines)
     const float2* wuw = a.wlines ? a.wlines : c.W;
     if (!a.wlines) x_inverse<DIM>(c, a.us, (DIM == 3 ? 8.0 : 9.0) / 3.0 * A, s);
-    L3ES_LAUNCH(c, KK_ADJ_X_INV, 2.0 * A, s,
-                pdl_launch(kx_inv_adjproj<N, DIM>, dim3(xb, c.batch), TX, 0, s, a.g, c.cs, a.gscale, c.kd, Wm, c.fs,
-                           c.tw, a.us, a.band_kf2 > 0 ? c.kf : 0, inv_n2d,
-                    c.eps_inj, const_cast<double*>(a.band_adj)));
+    const double Adu = 8.0 * 3.0 * c.ds * c.batch, rows = DIM == 3 ? (2.0 * c.kd + 1.0) / N : 1.0;
+    const int nb = DIM == 3 ? 2 * c.kd + 1 : 1;
+    L3ES_LAUNCH(c, KK_ADJ_X_INV, 8.0 * 3.0 * c.pcs * c.batch + Adu * rows, s,
+                pdl_launch(kx_inv_adjproj<N, DIM>, dim3(c.kt / TW, nb, c.batch), TX, 0, s, a.g, c.cs, a.gscale, c.kd,
+                           c.kt, Wm, c.ds, c.tw, a.us, a.band_kf2 > 0 ? c.kf : 0, inv_n2d, c.eps_inj,
+                           const_cast<double*>(a.band_adj)));
     if (DIM == 3) {
       if (!a.wlines) y_inv_rhs(c, 11.0 / 3.0 * A, s);
-      y_pass<kInv>(c, KK_Y_INV, 2.0 * A, Wm, c.fs, H, N / 2, 3 * c.batch, s);
+      const dim3 g(ky_tiles(c.kt), N, 3 * c.batch);
+      if (c.sched.y_var == 1)
+        L3ES_LAUNCH(c, KK_Y_INV, Adu * (1.0 + rows), s,
+                    pdl_launch(ky_inv_band<N, 1>, g, KyCfg<N, 1>::THREADS, 0, s, Wm, c.ds, c.kt, c.kd, c.tw));
+      else
+        L3ES_LAUNCH(c, KK_Y_INV, Adu * (1.0 + rows), s,
+                    pdl_launch(ky_inv_band<N, 0>, g, KY::THREADS, 0, s, Wm, c.ds, c.kt, c.kd, c.tw));
     }
-    L3ES_LAUNCH(c, KK_ADJ_LINE, 5.0 * A, s,
-                pdl_launch(line_cross_adj<N>, dim3(line_blocks(lines), c.batch), L::THREADS, 0, s, Wm, wuw, c.fs, Y6,
-                           c.cs, scale, c.tw, (int)lines));
+    L3ES_LAUNCH(c, KK_ADJ_LINE, 4.0 * A + Adu, s,
+                pdl_launch(line_cross_adj<N>, dim3(line_blocks(lines), c.batch), L::THREADS, 0, s, Wm, c.ds, c.kt, wuw,
+                           c.fs, Y6, c.cs, scale, c.tw, (int)lines));
     if (DIM == 3) y_pass<kFwd>(c, KK_Y_FWD, 4.0 * A, Y6, c.cs, H, N / 2, 6 * c.batch, s);
     // Y6 (6 fields per trajectory) -> W, as 2 * batch groups of 3 fields
     L3ES_LAUNCH(c, KK_X_FWD_PLAIN, 4.0 * A, s,
