@@ -28,34 +28,49 @@ __device__ __forceinline__ double ff_sum(const float (&e)[M]) {
   return s;
 }
 
-// per block: max |u_c| for c = 0..2 and sum_c u_c^2, over ps values per component; four
-// points per thread in flight, summed in float-float before one FP64 addition (an FP64
-// addition per point and one point in flight took 68 us on a 256^3 field)
+// Eight floats from p + i on (VEC: two 16-byte loads), zeros from n on.
+template <bool VEC>
+__device__ __forceinline__ void load8(const float* __restrict__ p, unsigned i, unsigned n, float (&v)[8]) {
+  if (VEC && i + 8 <= n) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p + i)), b = __ldg(reinterpret_cast<const float4*>(p + i) + 1);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = i + q < n ? __ldg(p + i + q) : 0.f;
+  }
+}
+
+// per block: max |u_c| for c = 0..2 and sum_c u_c^2, over ps values per component; eight
+// neighbouring points per thread and turn, the sum in float-float (where that is not finite,
+// again in FP64). VEC: u is 16-byte aligned and ps a multiple of 4. With one point in flight
+// and an FP64 addition per point a 256^3 field took 68 us.
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 k_field_stats(const float* __restrict__ u, long long ps, int nblk, double* __restrict__ partial) {
   pdl_begin();
   const int batch = blockIdx.y;
   const float* ub = u + (long long)batch * 3 * ps;
   float mx[3] = {0.f, 0.f, 0.f};
-  double s = 0.0;
-  const long long step = (long long)nblk * blockDim.x;
-  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < ps; i0 += 4 * step) {
-    float v[4][3];
+  Ff acc{0.f, 0.f};
+  const unsigned n = (unsigned)ps, step = 8u * (unsigned)nblk * blockDim.x;  // ps <= 512^3
+  const unsigned first = 8u * (blockIdx.x * blockDim.x + threadIdx.x);
+  auto energy = [](float x, float y, float z) { return fmaf(z, z, fmaf(y, y, x * x)); };
+  for (unsigned i = first; i < n; i += step) {
+    float v[3][8];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int c = 0; c < 3; ++c) load8<VEC>(ub + c * ps, i, n, v[c]);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) v[q][c] = i0 + q * step < ps ? __ldg(ub + c * ps + i0 + q * step) : 0.f;
-    float e[4];
+    for (int q = 0; q < 8; ++q) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      e[q] = 0.f;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        mx[c] = fmaxf(mx[c], fabsf(v[q][c]));
-        e[q] = fmaf(v[q][c], v[q][c], e[q]);
-      }
+      for (int c = 0; c < 3; ++c) mx[c] = fmaxf(mx[c], fabsf(v[c][q]));
+      acc = ff_add(acc, energy(v[0][q], v[1][q], v[2][q]));
     }
-    s += ff_sum(e);
+  }
+  double s = (double)acc.hi + (double)acc.lo;
+  if (!isfinite(acc.hi)) {
+    s = 0.0;
+    for (unsigned i = first; i < n; i += step)
+      for (unsigned j = i; j < i + 8 && j < n; ++j) s += (double)energy(ub[j], ub[ps + j], ub[2 * ps + j]);
   }
   __shared__ float smx[3][32];
   __shared__ double ss[32];
@@ -135,33 +150,35 @@ __device__ __forceinline__ void curl_of(const float2* v, int n, int kxi, int mid
   im[2] = k0 * b.y - k1 * a.y;
 }
 
-// One mode per thread and turn over the flat half spectrum (a warp per 129-mode row left
-// every fifth turn to one lane), two modes in flight.
-template <int DIM>
+// Four neighbouring modes per thread and turn over the flat half spectrum (a warp per
+// 129-mode row left every fifth turn to one lane). VEC: uh is 16-byte aligned (cs is even).
+template <int DIM, bool VEC>
 __global__ void __launch_bounds__(256)
 k_diss_partial(const float2* __restrict__ uh, long long cs, int n, int nblk, double* __restrict__ partial) {
   pdl_begin();
   const int batch = blockIdx.y;
   const float2* ub = uh + (long long)batch * 3 * cs;
   const unsigned h = (unsigned)(n / 2 + 1), nmid = DIM == 3 ? (unsigned)n : 1u, ucs = (unsigned)cs;  // cs < 2^31
-  const unsigned step = (unsigned)nblk * blockDim.x;
+  const unsigned step = 4u * (unsigned)nblk * blockDim.x;
   Ff s{0.f, 0.f};
-  for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < ucs; i0 += 2 * step) {
-    float2 v[2][3];
+  for (unsigned i0 = 4u * (blockIdx.x * blockDim.x + threadIdx.x); i0 < ucs; i0 += step) {
+    float v[3][8];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const unsigned i = i0 + q * step;
+    for (int c = 0; c < 3; ++c) load8<VEC>(reinterpret_cast<const float*>(ub + c * cs), 2u * i0, 2u * ucs, v[c]);
+    unsigned row = i0 / h;
+    int kh = (int)(i0 - row * h);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) v[q][c] = i < ucs ? __ldg(ub + c * cs + i) : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const unsigned i = i0 + q * step;
-      if (i >= ucs) continue;
-      const unsigned row = i / h;
-      const int kh = (int)(i - row * h), mid = (int)(row % nmid), kxi = (int)(row / nmid);
+    for (int q = 0; q < 4; ++q, ++kh) {
+      if (i0 + q >= ucs) break;
+      if (kh == (int)h) {
+        kh = 0;
+        ++row;
+      }
+      const int mid = (int)(row % nmid), kxi = (int)(row / nmid);
+      const float2 a[3] = {make_float2(v[0][2 * q], v[0][2 * q + 1]), make_float2(v[1][2 * q], v[1][2 * q + 1]),
+                           make_float2(v[2][2 * q], v[2][2 * q + 1])};
       float re[3], im[3];
-      curl_of<DIM>(v[q], n, kxi, mid, kh, re, im);
+      curl_of<DIM>(a, n, kxi, mid, kh, re, im);
       float e = 0.f;
       if (kh == 0 || kh == n / 2) {
         const int mx = (n - kxi) % n, mm = DIM == 3 ? (n - mid) % n : 0;
@@ -298,9 +315,11 @@ int l3es_field_stats(l3es_plan* plan, const float* u, double* out_dev, void* str
   if (!plan || !u || !out_dev) return fail(L3ES_EINVAL, "l3es_field_stats: null argument");
   const Ctx& c = plan_ctx(plan);
   cudaStream_t s = (cudaStream_t)stream;
-  const int nblk = (int)std::min<long long>(608, (c.ps + 255) / 256);
+  const int nblk = (int)std::min<long long>(608, (c.ps + 2047) / 2048);
+  const bool vec = !misaligned16(u) && c.ps % 4 == 0;
   L3ES_LAUNCH(c, KK_REDUCE, 4.0 * 3.0 * c.ps * c.batch, s,
-              pdl_launch(k_field_stats, dim3(nblk, c.batch), 256, 0, s, u, c.ps, nblk, c.partial));
+              pdl_launch(vec ? k_field_stats<true> : k_field_stats<false>, dim3(nblk, c.batch), 256, 0, s, u, c.ps, nblk,
+                         c.partial));
   L3ES_LAUNCH(c, KK_REDUCE, 0.0, s,
               pdl_launch(k_field_stats_final, c.batch, 256, 0, s, c.partial, nblk, 1.0 / (double)c.ps, out_dev));
   return cuda_check(cudaGetLastError(), "l3es_field_stats launch");
@@ -310,16 +329,13 @@ int l3es_dissipation(l3es_plan* plan, const void* u_hat, double nu, double* out_
   if (!plan || !u_hat || !out_dev) return fail(L3ES_EINVAL, "l3es_dissipation: null argument");
   const Ctx& c = plan_ctx(plan);
   cudaStream_t s = (cudaStream_t)stream;
-  const int nblk = (int)std::min<long long>(608, (c.cs + 511) / 512);
+  const int nblk = (int)std::min<long long>(608, (c.cs + 1023) / 1024);
   const double scale = nu / std::pow((double)c.n, 2 * c.dim);
-  if (c.dim == 3)
-    L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
-                pdl_launch(k_diss_partial<3>, dim3(nblk, c.batch), 256, 0, s, (const float2*)u_hat, c.cs, c.n, nblk,
-                                                                     c.partial));
-  else
-    L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
-                pdl_launch(k_diss_partial<2>, dim3(nblk, c.batch), 256, 0, s, (const float2*)u_hat, c.cs, c.n, nblk,
-                                                                     c.partial));
+  const bool vec = !misaligned16(u_hat);
+  auto kernel = c.dim == 3 ? (vec ? k_diss_partial<3, true> : k_diss_partial<3, false>)
+                           : (vec ? k_diss_partial<2, true> : k_diss_partial<2, false>);
+  L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
+              pdl_launch(kernel, dim3(nblk, c.batch), 256, 0, s, (const float2*)u_hat, c.cs, c.n, nblk, c.partial));
   L3ES_LAUNCH(c, KK_REDUCE, 0.0, s, pdl_launch(k_diag_sum, c.batch, 256, 0, s, c.partial, nblk, scale, out_dev));
   return cuda_check(cudaGetLastError(), "l3es_dissipation launch");
 }

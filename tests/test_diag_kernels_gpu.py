@@ -68,3 +68,23 @@ def test_field_stats_and_spectrum_of_bad_values(bad):
     p.energy_spectrum(torch.from_numpy(uh[0]).cuda(), ek)
     same = np.isnan if np.isnan(bad) else np.isposinf
     assert same(st.cpu().numpy()[3]) and same(ek.cpu().numpy()[int(np.sqrt(14) + 0.5)])
+
+
+def test_dissipation_and_stats_of_misaligned_arrays():
+    """The C entry points take spectra and fields at any element's address; the kernels load
+    16 bytes at a time where the address allows it."""
+    n = 32
+    u, uh = _spec(3, n, 1, 4)
+    p = _native.Plan(dim=3, n=n, nu=1e-2, dt=1e-3)
+    lib, s = p._lib, torch.cuda.current_stream().cuda_stream
+    got = []
+    for shift in (0, 1):
+        hb = torch.zeros(uh.size + 2, dtype=torch.complex64, device="cuda")
+        hb[shift:shift + uh.size] = torch.from_numpy(uh.ravel()).cuda()
+        fb = torch.zeros(u.size + 4, dtype=torch.float32, device="cuda")
+        fb[shift:shift + u.size] = torch.from_numpy(u.ravel()).cuda()
+        out = torch.empty(5, dtype=torch.float64, device="cuda")
+        assert lib.l3es_dissipation(p._h, hb.data_ptr() + 8 * shift, 1e-2, out.data_ptr(), s) == 0
+        assert lib.l3es_field_stats(p._h, fb.data_ptr() + 4 * shift, out.data_ptr() + 8, s) == 0
+        got.append(out.cpu().numpy())
+    assert np.array_equal(got[0], got[1])
