@@ -201,30 +201,36 @@ k_diss_partial(const float2* __restrict__ uh, long long cs, int n, int nblk, dou
   block_sum_store_ff(s, partial, batch * nblk + blockIdx.x);
 }
 
-// Energy spectrum over shells int(|k| + 0.5) < n: per-block shared-memory histograms of
+constexpr int kSpecThreads = 128;
+
+// Energy spectrum over shells int(|k| + 0.5) < n: per-warp shared-memory histograms of
 // the mode count and of weight * |u_hat|^2, merged with FP64 atomics into
 // acc[batch][2][n]. The shell depends on the magnitudes of the wavenumbers only, so a warp
 // takes all rows (+-a, +-b) and (+-b, +-a) of one pair a >= b (2D: +-a) at once, sums a
 // mode's energies over them in float-float (up to 8 rows, 24 loads in flight per lane) and
 // makes one shared FP64 addition for the lot: those atomics are a compare-and-swap loop,
-// and two per mode took 289 us on a 256^3 spectrum. shell int(|k| + 0.5): |k|^2 is an
+// and two per mode into one histogram per block took 289 us on a 256^3 spectrum (76 us with
+// one addition per 8 modes, 57 us with a histogram per warp). shell int(|k| + 0.5): |k|^2 is an
 // integer below 3 (n/2)^2, whose square root is never within 1/(8|k|) of a half integer,
 // far more than the FP32 rounding.
 template <int DIM>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kSpecThreads)
 k_spectrum(const float2* __restrict__ uh, long long cs, int n, int nblk, double scale, double* __restrict__ acc) {
   pdl_begin();
-  extern __shared__ double hist[];  // [n] energies, then [n] counts (32-bit)
-  unsigned* cnt = reinterpret_cast<unsigned*>(hist + n);
+  extern __shared__ double s_hist[];  // [warp][n] energies, then [warp][n] counts (32-bit)
   const int batch = blockIdx.y;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    hist[i] = 0.0;
-    cnt[i] = 0u;
+  const int wpb = blockDim.x >> 5;
+  unsigned* s_cnt = reinterpret_cast<unsigned*>(s_hist + wpb * n);
+  for (int i = threadIdx.x; i < wpb * n; i += blockDim.x) {
+    s_hist[i] = 0.0;
+    s_cnt[i] = 0u;
   }
   __syncthreads();
+  double* hist = s_hist + (threadIdx.x >> 5) * n;
+  unsigned* cnt = s_cnt + (threadIdx.x >> 5) * n;
   const float2* ub = uh + (long long)batch * 3 * cs;
   const int h = n / 2 + 1, m = n / 2;
-  const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int tasks = DIM == 3 ? (m + 1) * (m + 2) / 2 : m + 1;
   for (int t = blockIdx.x * wpb + (threadIdx.x >> 5); t < tasks; t += nblk * wpb) {
     int a = t, b = 0;
@@ -270,11 +276,18 @@ k_spectrum(const float2* __restrict__ uh, long long cs, int n, int nblk, double 
   }
   __syncthreads();
   double* ab = acc + (long long)batch * 2 * n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
-    if (cnt[i]) {
-      atomicAdd(&ab[i], (double)cnt[i]);
-      atomicAdd(&ab[n + i], hist[i]);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    unsigned k = 0;
+    double e = 0.0;
+    for (int w = 0; w < wpb; ++w) {
+      k += s_cnt[w * n + i];
+      e += s_hist[w * n + i];
     }
+    if (k) {
+      atomicAdd(&ab[i], (double)k);
+      atomicAdd(&ab[n + i], e);
+    }
+  }
 }
 
 // sum of n partials per trajectory times scale
@@ -318,7 +331,8 @@ int l3es_field_stats(l3es_plan* plan, const float* u, double* out_dev, void* str
   const int nblk = (int)std::min<long long>(608, (c.ps + 2047) / 2048);
   const bool vec = !misaligned16(u) && c.ps % 4 == 0;
   L3ES_LAUNCH(c, KK_REDUCE, 4.0 * 3.0 * c.ps * c.batch, s,
-              pdl_launch(vec ? k_field_stats<true> : k_field_stats<false>, dim3(nblk, c.batch), 256, 0, s, u, c.ps, nblk,
+              pdl_launch(vec ? k_field_stats<true> : k_field_stats<false>, dim3(nblk, c.batch), 256, 0, s, u, c.ps,
+                         nblk,
                          c.partial));
   L3ES_LAUNCH(c, KK_REDUCE, 0.0, s,
               pdl_launch(k_field_stats_final, c.batch, 256, 0, s, c.partial, nblk, 1.0 / (double)c.ps, out_dev));
@@ -347,19 +361,22 @@ int l3es_energy_spectrum(l3es_plan* plan, const void* u_hat, double mul_fac, dou
   const int n = c.n;
   int rc = cuda_check(cudaMemsetAsync(c.partial, 0, sizeof(double) * 2 * n * c.batch, s), "l3es_energy_spectrum");
   if (rc != L3ES_OK) return rc;
-  // one warp per pair of wavenumber magnitudes, two blocks per SM
+  // one warp per pair of wavenumber magnitudes; few of them per warp, so that the last ones
+  // do not run alone (256^3, 8385 pairs: 608 blocks of 4 warps 63 us, 1216 57 us)
   const long long tasks = c.dim == 3 ? (long long)c.h * (c.h + 1) / 2 : c.h;
-  const int nblk = (int)std::min<long long>(304, (tasks + 7) / 8);
+  const int nblk = (int)std::min<long long>(1216, (tasks + kSpecThreads / 32 - 1) / (kSpecThreads / 32));
   // |u_hat / n^dim|^2 * mul_fac (utils.py:82-86)
   const double scale = mul_fac / std::pow((double)n, 2 * c.dim);
-  const size_t smem = (sizeof(double) + sizeof(unsigned)) * n;
+  const size_t smem = (sizeof(double) + sizeof(unsigned)) * n * (kSpecThreads / 32);
   if (c.dim == 3)
     L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
-                pdl_launch(k_spectrum<3>, dim3(nblk, c.batch), 256, smem, s, (const float2*)u_hat, c.cs, n, nblk, scale,
+                pdl_launch(k_spectrum<3>, dim3(nblk, c.batch), kSpecThreads, smem, s, (const float2*)u_hat, c.cs, n,
+                           nblk, scale,
                                                                     c.partial));
   else
     L3ES_LAUNCH(c, KK_REDUCE, 8.0 * 3.0 * c.cs * c.batch, s,
-                pdl_launch(k_spectrum<2>, dim3(nblk, c.batch), 256, smem, s, (const float2*)u_hat, c.cs, n, nblk, scale,
+                pdl_launch(k_spectrum<2>, dim3(nblk, c.batch), kSpecThreads, smem, s, (const float2*)u_hat, c.cs, n,
+                           nblk, scale,
                                                                     c.partial));
   L3ES_LAUNCH(c, KK_REDUCE, 0.0, s,
               pdl_launch(k_spectrum_final, dim3((n + 127) / 128, c.batch), 128, 0, s, c.partial, n,
