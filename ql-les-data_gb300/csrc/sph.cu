@@ -180,41 +180,134 @@ k_sph_order(const int* __restrict__ perm0, const int* __restrict__ cell, const i
   }
 }
 
-// Visits every candidate neighbour of the particle at slot i (cell-local position xi in
-// cell ci): f(slot j, dx, dy, dz, r^2) for pairs with r^2 < cut2, the particle itself
-// included (r = 0). Cells of the 3^dim stencil are wrapped; the displacement r_i - r_j
-// is formed from cell-local coordinates and the stencil offset.
-template <int DIM, class F>
-__device__ __forceinline__ void for_neighbours(const float4 xi, const int3 ci, const SphGeom& g,
+// Visits every neighbour of a particle (cell-local position xi in cell ci) by its kSphLanes
+// lanes: f(slot j, dx, dy, dz, r^2) for pairs with r^2 < cut2, the particle itself included
+// (r = 0). Cells of the 3^dim stencil are wrapped; the displacement r_i - r_j is formed
+// from cell-local coordinates and the stencil offset. Lane q takes candidates q, q + 8, ...
+// of every cell, cells in a fixed order, so a lane's sum runs in a fixed order.
+// One candidate in eight is a neighbour. A lane first lists its neighbours (slot and cell of
+// the stencil, in its own column of shared memory) and runs f over the list afterwards, in
+// the same order: with f inside the candidate loop nearly every turn of a warp ran it for
+// the few lanes that had a neighbour. The cells' slot ranges are fetched once by the lanes
+// together, and a cell's first five candidates per lane are in flight at once. A list that
+// could overflow (14 neighbours per lane on average) is worked off before the next cell.
+// A relaxation call of 32^3 particles: 237 us with f in the candidate loop (density 78,
+// acceleration 152 us), 199 us; 17^3 118 -> 91 us; 2D 71^2 43 us.
+constexpr int kSphList = 32;
+constexpr int kSphTurns = 5;  // candidates per lane in flight: a cell of a lattice holds about 33
+struct SphLists {
+  int slot[kSphList][kSphThreads];
+  unsigned char cell[kSphList][kSphThreads];
+};
+
+// displacement of xi from xj, a particle of the cell at offset (ox, oy, oz), and its square
+template <int DIM>
+__device__ __forceinline__ float4 pair_displacement(const float4 xi, int ox, int oy, int oz, const float4 xj,
+                                                    const SphGeom& g) {
+  const float px = xi.x - (float)ox * g.cs, py = xi.y - (float)oy * g.cs, pz = xi.z - (float)oz * g.cs;
+  const float dx = px - xj.x, dy = py - xj.y, dz = DIM == 3 ? pz - xj.z : 0.f;
+  return make_float4(dx, dy, dz, dx * dx + dy * dy + dz * dz);
+}
+
+// One cell (nc == 1): every particle is a candidate, at the minimum image.
+template <int DIM, class P, class F>
+__device__ __forceinline__ void for_all_pairs(bool live, const float4 xi, const SphGeom& g, const int* __restrict__ start,
+                                              const float4* __restrict__ xs, int lane, P&& fetch, F&& f) {
+  const int e = live ? start[1] : 0;
+  for (int jj = start[0] + lane; jj < e; jj += kSphLanes) {
+    const float4 xj = xs[jj];
+    float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = DIM == 3 ? xi.z - xj.z : 0.f;
+    dx -= g.Lf * rintf(dx / g.Lf);
+    dy -= g.Lf * rintf(dy / g.Lf);
+    if (DIM == 3) dz -= g.Lf * rintf(dz / g.Lf);
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    if (r2 < g.cut2) f(jj, dx, dy, dz, r2, fetch(jj));
+  }
+}
+
+// stencil cell k (x offset varying fastest)
+template <int DIM>
+__device__ __forceinline__ void stencil_offset(int k, int& ox, int& oy, int& oz) {
+  ox = k % 3 - 1;
+  oy = k / 3 % 3 - 1;
+  oz = DIM == 3 ? k / 9 - 1 : 0;
+}
+
+// (nc >= 3) fetch(j): what f wants of slot j beside its displacement
+template <int DIM, class P, class F>
+__device__ __forceinline__ void for_neighbours(bool live, const float4 xi, const int3 ci, const SphGeom& g,
                                                const int* __restrict__ start, const float4* __restrict__ xs, int lane,
-                                               F&& f) {
-  const int R = g.nc >= 3 ? 1 : 0;
-  const int nc = g.nc;
-  for (int oz = (DIM == 3 ? -R : 0); oz <= (DIM == 3 ? R : 0); ++oz) {
-    int cz = ci.z + oz;
-    cz = cz < 0 ? cz + nc : (cz >= nc ? cz - nc : cz);
-    for (int oy = -R; oy <= R; ++oy) {
-      int cy = ci.y + oy;
-      cy = cy < 0 ? cy + nc : (cy >= nc ? cy - nc : cy);
-      for (int ox = -R; ox <= R; ++ox) {
-        int cx = ci.x + ox;
-        cx = cx < 0 ? cx + nc : (cx >= nc ? cx - nc : cx);
-        const int c = DIM == 3 ? (cx * nc + cy) * nc + cz : cx * nc + cy;
-        const float px = xi.x - (float)ox * g.cs, py = xi.y - (float)oy * g.cs, pz = xi.z - (float)oz * g.cs;
-        const int b = start[c], e = start[c + 1];
-        for (int jj = b + lane; jj < e; jj += kSphLanes) {
-          const float4 xj = xs[jj];
-          float dx = px - xj.x, dy = py - xj.y, dz = DIM == 3 ? pz - xj.z : 0.f;
-          if (R == 0) {  // one cell: minimum image
-            dx -= g.Lf * rintf(dx / g.Lf);
-            dy -= g.Lf * rintf(dy / g.Lf);
-            if (DIM == 3) dz -= g.Lf * rintf(dz / g.Lf);
-          }
-          const float r2 = dx * dx + dy * dy + dz * dz;
-          if (r2 < g.cut2) f(jj, dx, dy, dz, r2);
+                                               SphLists& lists, P&& fetch, F&& f) {
+  const int nc = g.nc, tid = threadIdx.x, base = (tid & 31) - lane;
+  constexpr int cells = DIM == 3 ? 27 : 9;
+  constexpr int S = DIM == 3 ? 4 : 2;  // cells whose range a lane fetches: lane, lane + 8, ...
+  int rb[S], re[S];
+  auto wrap = [nc](int c) { return c < 0 ? c + nc : (c >= nc ? c - nc : c); };
+#pragma unroll
+  for (int q = 0; q < S; ++q) {
+    const int k = lane + q * kSphLanes;
+    rb[q] = re[q] = 0;
+    if (live && k < cells) {
+      int ox, oy, oz;
+      stencil_offset<DIM>(k, ox, oy, oz);
+      const int cx = wrap(ci.x + ox), cy = wrap(ci.y + oy);
+      const int c = DIM == 3 ? (cx * nc + cy) * nc + wrap(ci.z + oz) : cx * nc + cy;
+      rb[q] = start[c];
+      re[q] = start[c + 1];
+    }
+  }
+  int cnt = 0;
+#pragma unroll 1
+  for (int k = 0; k <= cells; ++k) {  // the turn after the last cell works the rest off
+    int b = rb[0], e = re[0];
+#pragma unroll
+    for (int q = 1; q < S; ++q)
+      if (k / kSphLanes == q) {
+        b = rb[q];
+        e = re[q];
+      }
+    b = __shfl_sync(0xffffffffu, b, base + k % kSphLanes);
+    e = __shfl_sync(0xffffffffu, e, base + k % kSphLanes);
+    if (k == cells) e = b;
+    int ox, oy, oz;
+    stencil_offset<DIM>(k, ox, oy, oz);
+    const unsigned char code = (unsigned char)((ox + 1) | (oy + 1) << 2 | (oz + 1) << 4);
+    do {
+      if (k == cells || cnt > kSphList - kSphTurns) {
+        int jc = cnt > 0 ? lists.slot[0][tid] : 0, oc = cnt > 0 ? lists.cell[0][tid] : 0;
+        float4 xc = xs[jc];
+        auto pc = fetch(jc);
+#pragma unroll 1
+        for (int i = 0; i < cnt; ++i) {  // the next neighbour's operands while this one's pair is formed
+          const int jn = i + 1 < cnt ? lists.slot[i + 1][tid] : 0, on = i + 1 < cnt ? lists.cell[i + 1][tid] : 0;
+          const float4 xn = i + 1 < cnt ? xs[jn] : make_float4(0.f, 0.f, 0.f, 0.f);
+          const auto pn = fetch(jn);
+          const float4 d = pair_displacement<DIM>(xi, (oc & 3) - 1, (oc >> 2 & 3) - 1, (oc >> 4) - 1, xc, g);
+          f(jc, d.x, d.y, d.z, d.w, pc);
+          jc = jn;
+          oc = on;
+          xc = xn;
+          pc = pn;
+        }
+        cnt = 0;
+      }
+      float4 xj[kSphTurns];
+#pragma unroll
+      for (int i = 0; i < kSphTurns; ++i) {
+        const int jj = b + lane + i * kSphLanes;
+        xj[i] = jj < e ? xs[jj] : make_float4(1e30f, 0.f, 0.f, 0.f);  // far from everything
+      }
+#pragma unroll
+      for (int i = 0; i < kSphTurns; ++i) {
+        const int jj = b + lane + i * kSphLanes;
+        if (jj < e && pair_displacement<DIM>(xi, ox, oy, oz, xj[i], g).w < g.cut2) {
+          lists.slot[cnt][tid] = jj;
+          lists.cell[cnt][tid] = code;
+          ++cnt;
         }
       }
-    }
+      b += kSphTurns * kSphLanes;
+    } while (b < e);
   }
 }
 
@@ -240,7 +333,7 @@ __device__ __forceinline__ int3 slot_cell(long long i, const int* __restrict__ p
 // rho[slot] = m sigma sum_j w(r_ij / h); rp[slot] = (rho, p = p_ref (rho - 1),
 // 1 / rho^2) in FP32 for the acceleration pass (the quotient once per particle: it was one
 // of three divisions per pair there); rho_out[input index] when requested
-template <int DIM>
+template <int DIM, bool ONE>
 __global__ void __launch_bounds__(kSphThreads)
 k_sph_density(const float4* __restrict__ xs, const int* __restrict__ start, const int* __restrict__ perm,
               const double* __restrict__ xw, long long np, SphGeom g, double m_sigma, double p_ref,
@@ -251,13 +344,16 @@ k_sph_density(const float4* __restrict__ xs, const int* __restrict__ start, cons
   const int lane = (int)(gt % kSphLanes);
   const bool live = i < np;  // every lane stays for the shuffles
   Ff part{0.f, 0.f};
-  if (live) {
-    const float4 xi = xs[i];
-    const int3 ci = slot_cell<DIM>(i, perm, xw, g);
-    const float inv_h = g.inv_h;
-    for_neighbours<DIM>(xi, ci, g, start, xs, lane, [&](int, float, float, float, float r2) {
-      part = ff_add(part, quintic_w(sqrtf(r2) * inv_h));
-    });
+  const long long is = live ? i : 0;
+  const float4 xi = xs[is];
+  const float inv_h = g.inv_h;
+  auto none = [](int) { return 0; };
+  auto pair = [&](int, float, float, float, float r2, int) { part = ff_add(part, quintic_w(sqrtf(r2) * inv_h)); };
+  if constexpr (ONE) {
+    for_all_pairs<DIM>(live, xi, g, start, xs, lane, none, pair);
+  } else {
+    __shared__ SphLists lists;
+    for_neighbours<DIM>(live, xi, slot_cell<DIM>(is, perm, xw, g), g, start, xs, lane, lists, none, pair);
   }
   const double acc = lanes_sum((double)part.hi + (double)part.lo);
   if (!live || lane != 0) return;
@@ -292,7 +388,7 @@ struct SphAccelArgs {
 //   grad = dW/dr * r_ij / (r + eps)
 //   acc_p = -pref p_ij grad, acc_tvf = -pref p_ref grad, acc_visc = pref u_ij dW/dr / (r + eps)
 // Relaxation acceleration = acc_p + acc_tvf / 2.
-template <int DIM, int MODE>
+template <int DIM, int MODE, bool ONE>
 __global__ void __launch_bounds__(kSphThreads) k_sph_accel(SphAccelArgs a, SphGeom g) {
   pdl_begin();
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -301,12 +397,11 @@ __global__ void __launch_bounds__(kSphThreads) k_sph_accel(SphAccelArgs a, SphGe
   const bool live = i < a.np;  // every lane stays for the shuffles
   const long long is = live ? i : 0;
   const float4 xi = a.xs[is];
-  const int3 ci = slot_cell<DIM>(is, a.perm, a.xw, g);
   const float4 rpi = a.rp[is];
   const float4 ui = MODE == kSphForces ? a.us[is] : make_float4(0.f, 0.f, 0.f, 0.f);
   Ff fp[3] = {}, ft[3] = {}, fv[3] = {};
-  if (live) for_neighbours<DIM>(xi, ci, g, a.start, a.xs, lane, [&](int jj, float dx, float dy, float dz, float r2) {
-    const float4 rpj = a.rp[jj];
+  auto fetch = [&](int jj) { return a.rp[jj]; };
+  auto pair = [&](int jj, float dx, float dy, float dz, float r2, const float4 rpj) {
     const float r = sqrtf(r2);
     const float dw = a.grad_scale * quintic_dw(r * g.inv_h);
     const float pref = a.mass * (rpi.z + rpj.z);
@@ -325,7 +420,13 @@ __global__ void __launch_bounds__(kSphThreads) k_sph_accel(SphAccelArgs a, SphGe
       const float cp = -pref * (pij + 0.5f * a.p_ref) * s;
       fp[0] = ff_add(fp[0], cp * dx); fp[1] = ff_add(fp[1], cp * dy); fp[2] = ff_add(fp[2], cp * dz);
     }
-  });
+  };
+  if constexpr (ONE) {
+    for_all_pairs<DIM>(live, xi, g, a.start, a.xs, lane, fetch, pair);
+  } else {
+    __shared__ SphLists lists;
+    for_neighbours<DIM>(live, xi, slot_cell<DIM>(is, a.perm, a.xw, g), g, a.start, a.xs, lane, lists, fetch, pair);
+  }
   double ap[3], at[3] = {0.0, 0.0, 0.0}, av[3] = {0.0, 0.0, 0.0};
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -425,24 +526,20 @@ static int sph_build(l3es_sph_plan* p, const double* r, const double* u_pred, do
 
 static void sph_density(l3es_sph_plan* p, long long np, double p_ref, double* rho_out, cudaStream_t s) {
   const unsigned pb = (unsigned)((np * kSphLanes + kSphThreads - 1) / kSphThreads);
-  const double m_sigma = p->mass * p->sigma;
-  if (p->dim == 3)
-    pdl_launch(k_sph_density<3>, pb, kSphThreads, 0, s, p->xs, p->start, p->perm, p->xw, np, p->g, m_sigma, p_ref,
-               p->rp,
-                                                 rho_out);
-  else
-    pdl_launch(k_sph_density<2>, pb, kSphThreads, 0, s, p->xs, p->start, p->perm, p->xw, np, p->g, m_sigma, p_ref,
-               p->rp,
-                                                 rho_out);
+  const bool one = p->g.nc < 3;
+  auto kernel = p->dim == 3 ? (one ? k_sph_density<3, true> : k_sph_density<3, false>)
+                            : (one ? k_sph_density<2, true> : k_sph_density<2, false>);
+  pdl_launch(kernel, pb, kSphThreads, 0, s, p->xs, p->start, p->perm, p->xw, np, p->g, p->mass * p->sigma, p_ref, p->rp,
+             rho_out);
 }
 
 template <int MODE>
 static void sph_accel(l3es_sph_plan* p, SphAccelArgs& a, cudaStream_t s) {
   const unsigned pb = (unsigned)((a.np * kSphLanes + kSphThreads - 1) / kSphThreads);
-  if (p->dim == 3)
-    pdl_launch(k_sph_accel<3, MODE>, pb, kSphThreads, 0, s, a, p->g);
-  else
-    pdl_launch(k_sph_accel<2, MODE>, pb, kSphThreads, 0, s, a, p->g);
+  const bool one = p->g.nc < 3;
+  auto kernel = p->dim == 3 ? (one ? k_sph_accel<3, MODE, true> : k_sph_accel<3, MODE, false>)
+                            : (one ? k_sph_accel<2, MODE, true> : k_sph_accel<2, MODE, false>);
+  pdl_launch(kernel, pb, kSphThreads, 0, s, a, p->g);
 }
 
 static SphAccelArgs sph_args(l3es_sph_plan* p, long long np, double u_ref) {
