@@ -81,51 +81,57 @@ k_crop(const float2* __restrict__ uh, long long cs, int N, float2* __restrict__ 
 // those over ky, an FP64 sum over kx; phase tables in shared memory (exp(i k x) per
 // particle and axis by an FP64 recurrence, stored FP32).
 //
-// A block takes 32 particles. Each half warp owns a slice of the kx range and holds two
-// particles per lane, so one mode (a broadcast 16-byte read of its staged copy
-// (x, x, y, y)) feeds 4 paired FP32 FMAs per lane, and RB rows times DIM components share
-// a particle's phase read; the half warps' FP64 partial sums are added in kx order. The
-// FP32 sums run in the order of the plain loops, whatever the split, so a particle's
+// A block takes 8 P particles. Each part of a warp (8 lanes) owns a slice of the kx range
+// and holds P particles per lane. Two rows are staged side by side as (x0, x1, y0, y1), so
+// one broadcast 16-byte read feeds 4 P paired FP32 FMAs per lane; the read returns 512 bytes
+// to a warp, 4 cycles of the SM's shared memory, which is why a lane holds several particles
+// and the modes are not stored doubled. The parts' FP64 partial sums are added in kx order.
+// The FP32 sums run in the order of the plain loops, whatever the split, so a particle's
 // velocity does not depend on it beyond FP64 rounding. Bound by FP32 FMAs (4 per mode,
-// component and particle). With one thread per particle, one component after the other
-// and the mode index arithmetic in the inner loop, 10007 particles on 32^3 modes took
-// 14.2 ms (79 blocks of 4 warps); now 0.31 ms, a third of the FP32 FMA rate, 32768
-// particles 0.67 ms, half of it.
+// component and particle). With one thread per particle, one component after the other and
+// the mode index arithmetic in the inner loop, 10007 particles on 32^3 modes took 14.2 ms
+// (79 blocks of 4 warps); with 2 particles per lane, parts of 16 lanes and each mode stored
+// as (x, x, y, y), 306 us; now 244 (32768 particles: 529 us, 77 % of the FMA rate).
 // ------------------------------------------------------------------------------
-constexpr int kDftTile = 32;                                 // particles per block
-inline int dft_threads(int c) { return c >= 16 ? 256 : c > 2 ? 16 * c : 32; }
-inline int dft_rows(int c) { return c <= 32 ? 2 : 1; }       // RB: staged rows per half warp
-// shared memory of k_dft_interp: phase tables, then the warps' staged rows (which the
-// FP64 partial sums reuse: 16 bytes a mode and two halves of RB c DIM modes per warp
-// hold 2 x 32 x DIM doubles as long as RB c >= 32)
-inline size_t dft_smem(int dim, int c) {
-  const size_t table = sizeof(float2) * dim * c * kDftTile;
-  const size_t rows = (size_t)(dft_threads(c) / 32) * 2 * dft_rows(c) * c * dim * sizeof(float4);
-  const size_t sums = (size_t)(dft_threads(c) / 16) * kDftTile * dim * sizeof(double);
-  return table + (rows > sums ? rows : sums);
-}
+template <int DIM, int P>
+struct DftCfg {
+  static constexpr int LN = 8;          // lanes per part
+  static constexpr int TILE = P * LN;   // particles per block
+  // 3D: a kx per part up to c = 32, four at c = 64 (two blocks per SM); 2D: row pairs of kx
+  static int threads(int c) {
+    const int t = DIM == 3 ? (c <= 32 ? c * LN : 128) : (c / 2) * LN;
+    return t >= 256 ? 256 : t > 32 ? t : 32;
+  }
+  // row pairs staged per part, [kz][component], and one to spread the parts over the banks
+  static __host__ __device__ int stage(int c) { return c * DIM + 1; }
+  // shared memory: phase tables, FP64 partial sums, staged rows
+  static size_t smem(int c) {
+    const size_t parts = threads(c) / LN;
+    return sizeof(float2) * DIM * c * TILE + parts * (TILE * DIM * sizeof(double) + stage(c) * sizeof(float4));
+  }
+};
 
 // (a.x, a.y) <- (a.x + s.x b.x, a.y + s.y b.y) in one paired FP32 FMA
 __device__ __forceinline__ float2 fma2(float2 s, float2 b, float2 a) { return __ffma2_rn(s, b, a); }
 
-// Two blocks per SM up to c = 32 (128 registers: 306 against 334 us at 160 registers and
-// one block, 10007 particles on 32^3 modes); at c = 64 shared memory holds one block.
-template <int DIM, int RB>
-__global__ void __launch_bounds__(256, RB == 2 ? 2 : 1)
+template <int DIM, int P>
+__global__ void __launch_bounds__(256, 2)
 k_dft_interp(const float2* __restrict__ hh, long long hcs, int c, const double* __restrict__ r, long long np,
              double* __restrict__ u_r, double dt, double* __restrict__ r_out) {
   pdl_begin();
+  using K = DftCfg<DIM, P>;
+  constexpr int LN = K::LN, kDftTile = K::TILE, PARTS = 32 / LN;  // parts of a warp
   extern __shared__ __align__(16) unsigned char s_dft[];
-  float2* ph = reinterpret_cast<float2*>(s_dft);  // [DIM][c][kDftTile]
-  float4* rows = reinterpret_cast<float4*>(s_dft + sizeof(float2) * DIM * c * kDftTile);
-  double* sums = reinterpret_cast<double*>(rows);  // [half warp][kDftTile][DIM], after the transform
-  const int tid = threadIdx.x, lane = tid & 31, hl = lane & 15, half = lane >> 4;
-  const int hw = tid >> 4, nhw = blockDim.x >> 4;
+  const int tid = threadIdx.x, lane = tid & 31, hl = lane % LN;
+  const int hw = tid / LN, nhw = blockDim.x / LN;
   const int msk = c - 1, hc = c / 2 + 1, lc = 31 - __clz(c);  // c is a power of two
-  const int stage = RB * c * DIM;                    // modes staged per half warp: [row][kz][comp]
-  float4* my = rows + (long long)(tid >> 5) * 2 * stage + half * stage;
-  float4* warp_rows = rows + (long long)(tid >> 5) * 2 * stage;
-  const int per = (c + nhw - 1) / nhw;               // kx slice of a half warp
+  const int stage = K::stage(c);
+  float2* ph = reinterpret_cast<float2*>(s_dft);              // [DIM][c][kDftTile]
+  double* sums = reinterpret_cast<double*>(ph + DIM * c * kDftTile);  // [part][DIM][kDftTile]
+  float4* rows = reinterpret_cast<float4*>(sums + nhw * DIM * kDftTile);
+  const float4* my = rows + hw * stage;
+  double* mine = sums + hw * DIM * kDftTile + hl;  // this lane's particles: hl + LN q
+  const int per = (c + nhw - 1) / nhw;               // kx slice of a part
   const long long tiles = (np + kDftTile - 1) / kDftTile;
   for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const long long j0 = tile * kDftTile;
@@ -146,132 +152,104 @@ k_dft_interp(const float2* __restrict__ hh, long long hcs, int c, const double* 
       }
     }
     __syncthreads();
-    const float2* pz = ph + (DIM - 1) * c * kDftTile + hl;  // this lane's particles: hl, hl + 16
+    const float2* pz = ph + (DIM - 1) * c * kDftTile + hl;
     const float2* py = ph + c * kDftTile + hl;              // (3D)
-    double tot[2][DIM];
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) tot[q][d] = 0.0;
-    // 3D: rows are ky at one kx; 2D: rows are kx
-    const int blocks = DIM == 3 ? per * (c / RB) : (per + RB - 1) / RB;
-    float2 sx[2][DIM];
-    const int yb = DIM == 3 ? c / RB : 1;                   // 3D: row blocks per kx
-    // Row block b of both half warps: modes (kx, ky, kz), kz = -c/2 .. c/2-1 (Hermitian
-    // below 0), one (row, kz) per lane and turn. It is loaded into registers while the
-    // block before it is summed (up to 64 modes per half warp, else at once).
-    constexpr int TURNS = 2;  // RB c <= 64
-    float2 nx[TURNS][2][DIM];
-    auto fetch = [&](int b) {
-      const int xo = DIM == 3 ? b / yb : b * RB, yo = DIM == 3 ? (b - b / yb * yb) * RB : 0;
-#pragma unroll
-      for (int n = 0; n < TURNS; ++n) {
-        const int i = lane + 32 * n;
+    for (int i = 0; i < P * DIM; ++i) mine[LN * i] = 0.0;
+    // row pairs: 3D two ky of one kx; 2D two kx
+    const int yb = DIM == 3 ? c / 2 : 1;                    // 3D: row pairs per kx
+    const int blocks = DIM == 3 ? per * yb : (per + 1) / 2;
+    float2 sx[P][DIM];
+    for (int b = 0; b < blocks; ++b) {
+      const int xo = DIM == 3 ? b / yb : 2 * b, y0 = DIM == 3 ? (b - xo * yb) * 2 : 0;
+      const int kxi = hw * per + xo;  // table index of the (first) kx
+      // Stage the pair's modes (kx, ky, kz), kz = -c/2 .. c/2-1 (Hermitian below 0), one
+      // (row, kz) per lane and turn; the other warps cover the loads.
+      __syncwarp();
+      for (int i = lane; i < 2 * c; i += 32) {
         const int row = i >> lc, kz = (i & msk) - c / 2, sg = kz >= 0 ? 1 : -1;
+        float2 v[PARTS][DIM];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int xb = ((tid >> 5) * 2 + h) * per + xo + (DIM == 3 ? 0 : row);
-          const int kx = xb - c / 2, ky = DIM == 3 ? yo + row - c / 2 : 0;
-          const bool in = i < RB * c && xb < c;
+        for (int h = 0; h < PARTS; ++h) {
+          const int xb = ((tid >> 5) * PARTS + h) * per + xo + (DIM == 3 ? 0 : row);
+          const int kx = xb - c / 2, ky = DIM == 3 ? y0 + row - c / 2 : 0;
           const long long o = DIM == 3 ? ((long long)((sg * kx) & msk) * c + ((sg * ky) & msk)) * hc + sg * kz
                                        : (long long)((sg * kx) & msk) * hc + sg * kz;
 #pragma unroll
+          for (int d = 0; d < DIM; ++d) v[h][d] = xb < c ? __ldg(hh + d * hcs + o) : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int h = 0; h < PARTS; ++h)
+#pragma unroll
           for (int d = 0; d < DIM; ++d) {
-            nx[n][h][d] = in ? __ldg(hh + d * hcs + o) : make_float2(0.f, 0.f);
-            if (kz < 0) nx[n][h][d].y = -nx[n][h][d].y;
+            float* w = reinterpret_cast<float*>(rows + ((tid >> 5) * PARTS + h) * stage + (i & msk) * DIM + d);
+            w[row] = v[h][d].x;
+            w[2 + row] = kz < 0 ? -v[h][d].y : v[h][d].y;
           }
-        }
-      }
-    };
-    fetch(0);
-    for (int b = 0; b < blocks; ++b) {
-      const int kxi = hw * per + (DIM == 3 ? b / yb : b * RB);  // table index of the (first) kx
-      const int y0 = DIM == 3 ? (b - b / yb * yb) * RB : 0;
-      __syncwarp();
-#pragma unroll
-      for (int n = 0; n < TURNS; ++n) {
-        const int i = lane + 32 * n;
-        if (i < RB * c) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) {
-              const float2 v = nx[n][h][d];
-              warp_rows[h * stage + i * DIM + d] = make_float4(v.x, v.x, v.y, v.y);
-            }
-        }
       }
       __syncwarp();
-      if (b + 1 < blocks) fetch(b + 1);
       if (DIM == 3 && y0 == 0) {
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
+        for (int q = 0; q < P; ++q)
 #pragma unroll
           for (int d = 0; d < DIM; ++d) sx[q][d] = make_float2(0.f, 0.f);
       }
-      float2 sy[RB][2][DIM];
+      float2 re[P][DIM], im[P][DIM];  // (row 0, row 1)
 #pragma unroll
-      for (int w = 0; w < RB; ++w)
+      for (int q = 0; q < P; ++q)
 #pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) sy[w][q][d] = make_float2(0.f, 0.f);
-#pragma unroll 4
+        for (int d = 0; d < DIM; ++d) re[q][d] = im[q][d] = make_float2(0.f, 0.f);
+#pragma unroll 2
       for (int kz = 0; kz < c; ++kz) {
-        const float2 e0 = pz[kz * kDftTile], e1 = pz[kz * kDftTile + 16];
-        const float2 i0 = make_float2(-e0.y, e0.x), i1 = make_float2(-e1.y, e1.x);
+        float4 v[DIM];
 #pragma unroll
-        for (int w = 0; w < RB; ++w)
+        for (int d = 0; d < DIM; ++d) v[d] = my[kz * DIM + d];
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+          const float2 e = pz[kz * kDftTile + LN * q];
+          const float2 ex = make_float2(e.x, e.x), ey = make_float2(e.y, e.y), en = make_float2(-e.y, -e.y);
 #pragma unroll
           for (int d = 0; d < DIM; ++d) {
-            const float4 v = my[(w * c + kz) * DIM + d];
-            const float2 vx = make_float2(v.x, v.y), vy = make_float2(v.z, v.w);
-            sy[w][0][d] = fma2(vy, i0, fma2(vx, e0, sy[w][0][d]));
-            sy[w][1][d] = fma2(vy, i1, fma2(vx, e1, sy[w][1][d]));
-          }
-      }
-#pragma unroll
-      for (int w = 0; w < RB; ++w) {
-        const int xi = DIM == 3 ? kxi : kxi + w;
-        if (DIM == 2 && (xi >= (hw + 1) * per || xi >= c)) continue;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          if (DIM == 3) {
-            const float2 ey = py[(y0 + w) * kDftTile + 16 * q];
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) {
-              const float2 t = sy[w][q][d];
-              sx[q][d] = make_float2(fmaf(-t.y, ey.y, fmaf(t.x, ey.x, sx[q][d].x)),
-                                     fmaf(t.y, ey.x, fmaf(t.x, ey.y, sx[q][d].y)));
-            }
-          } else {
-            const float2 ex = ph[xi * kDftTile + hl + 16 * q];
-#pragma unroll
-            for (int d = 0; d < DIM; ++d)
-              tot[q][d] += (double)sy[w][q][d].x * ex.x - (double)sy[w][q][d].y * ex.y;
+            const float2 x = make_float2(v[d].x, v[d].y), y = make_float2(v[d].z, v[d].w);
+            re[q][d] = fma2(y, en, fma2(x, ex, re[q][d]));
+            im[q][d] = fma2(y, ex, fma2(x, ey, im[q][d]));
           }
         }
       }
-      if (DIM == 3 && y0 + RB == c && kxi < c) {
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const float2 ex = ph[kxi * kDftTile + hl + 16 * q];
+      for (int w = 0; w < 2; ++w) {
+        const int xi = kxi + w;
+        if (DIM == 2 && (xi >= (hw + 1) * per || xi >= c)) continue;
 #pragma unroll
-          for (int d = 0; d < DIM; ++d) tot[q][d] += (double)sx[q][d].x * ex.x - (double)sx[q][d].y * ex.y;
+        for (int q = 0; q < P; ++q) {
+          const float2 e = DIM == 3 ? py[(y0 + w) * kDftTile + LN * q] : ph[xi * kDftTile + hl + LN * q];
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) {
+            const float tx = w ? re[q][d].y : re[q][d].x, ty = w ? im[q][d].y : im[q][d].x;
+            if (DIM == 3)
+              sx[q][d] = make_float2(fmaf(-ty, e.y, fmaf(tx, e.x, sx[q][d].x)),
+                                     fmaf(ty, e.x, fmaf(tx, e.y, sx[q][d].y)));
+            else
+              mine[d * kDftTile + LN * q] += (double)tx * e.x - (double)ty * e.y;
+          }
+        }
+      }
+      if (DIM == 3 && y0 + 2 == c && kxi < c) {
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+          const float2 ex = ph[kxi * kDftTile + hl + LN * q];
+#pragma unroll
+          for (int d = 0; d < DIM; ++d)
+            mine[d * kDftTile + LN * q] += (double)sx[q][d].x * ex.x - (double)sx[q][d].y * ex.y;
         }
       }
     }
-    __syncthreads();  // the staged rows are read
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) sums[(hw * kDftTile + hl + 16 * q) * DIM + d] = tot[q][d];
     __syncthreads();
     for (int i = tid; i < kDftTile * DIM; i += blockDim.x) {
       const long long j = j0 + i / DIM;
       if (j >= np) continue;
       double t = 0.0;
-      for (int h = 0; h < nhw; ++h) t += sums[h * kDftTile * DIM + i];
+      for (int h = 0; h < nhw; ++h) t += sums[(h * DIM + i % DIM) * kDftTile + i / DIM];
       const double ur = t / (DIM == 3 ? (double)c * c * c : (double)c * c);
       u_r[j * DIM + i % DIM] = ur;
       if (r_out) {
@@ -286,24 +264,28 @@ k_dft_interp(const float2* __restrict__ hh, long long hcs, int c, const double* 
   }
 }
 
-// Launches k_dft_interp<dim> over np particles. Grids that a one-thread-per-particle block
-// of 128 could not serve (phase tables above 227 KB: c = 128, or c = 64 with more axes than
-// fit) are refused by the caller's check of dft_supported.
+// Grids that a one-thread-per-particle block of 128 could not serve (phase tables above
+// 227 KB) stay refused by the callers.
 inline bool dft_supported(int dim, int c) { return sizeof(float2) * dim * c * 128 <= 227 * 1024; }
 
+// Launches k_dft_interp over np particles: two per lane while one round of two blocks per
+// SM takes them all (32^3 modes: 300 particles 74 against 103 us with four), four above, where
+// the shared memory reads bound (9000: 205 two per lane, 177 four; 32768: 653, 529).
 inline cudaError_t dft_launch(int dim, const float2* hh, long long hcs, int c, const double* r, long long np,
                               double* u_r, double dt, double* r_out, cudaStream_t s) {
-  const long long tiles = (np + kDftTile - 1) / kDftTile;
-  const unsigned grid = (unsigned)(tiles < (1LL << 30) ? tiles : (1LL << 30));
-  const size_t smem = dft_smem(dim, c);
-  auto go = [&](auto kernel) {
+  auto go = [&](auto cfg, auto kernel) {
+    using K = decltype(cfg);
+    const long long tiles = (np + K::TILE - 1) / K::TILE;
+    const unsigned grid = (unsigned)(tiles < (1LL << 30) ? tiles : (1LL << 30));
+    const size_t smem = K::smem(c);
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    pdl_launch(kernel, grid, dft_threads(c), smem, s, hh, hcs, c, r, np, u_r, dt, r_out);
+    pdl_launch(kernel, grid, K::threads(c), smem, s, hh, hcs, c, r, np, u_r, dt, r_out);
     return cudaGetLastError();
   };
-  if (dim == 3) return dft_rows(c) == 2 ? go(k_dft_interp<3, 2>) : go(k_dft_interp<3, 1>);
-  return dft_rows(c) == 2 ? go(k_dft_interp<2, 2>) : go(k_dft_interp<2, 1>);
+  const bool small = np <= 2 * 152 * DftCfg<3, 2>::TILE;
+  if (dim == 3) return small ? go(DftCfg<3, 2>{}, k_dft_interp<3, 2>) : go(DftCfg<3, 4>{}, k_dft_interp<3, 4>);
+  return small ? go(DftCfg<2, 2>{}, k_dft_interp<2, 2>) : go(DftCfg<2, 4>{}, k_dft_interp<2, 4>);
 }
 
 }  // namespace l3es

@@ -1,6 +1,6 @@
 """The exact spectral interpolation kernel at the edges of its split: particle counts around
-a block's 32 particles and a lane's pair, kx ranges smaller and larger than the half warps
-of a block, one and two staged rows. Against the FP64 sum over the same modes."""
+a block's 16 or 32 particles and the change from one to the other, kx ranges smaller and
+larger than the parts of a block. Against the FP64 sum over the same modes."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,8 @@ from l3es import _native  # noqa: E402
 
 
 @pytest.mark.parametrize("dim,c,np_", [(3, 8, 1), (3, 8, 33), (3, 16, 17), (3, 32, 95), (3, 64, 31), (2, 8, 16),
-                                       (2, 16, 32), (2, 32, 257), (2, 64, 63)])
+                                       (2, 16, 32), (2, 32, 257), (2, 64, 63), (3, 8, 4864), (3, 8, 4865), (3, 16, 4897),
+                                       (2, 8, 4881)])
 def test_dft_interpolation_matches_the_sum(dim, c, np_):
     rng = np.random.default_rng(c + np_)
     u = rng.standard_normal((3,) + (c,) * dim).astype(np.float32)
