@@ -195,7 +195,9 @@ __device__ __forceinline__ void kx_inv_fields(float2 (&a)[3][Fft<N>::E], int t, 
         v[e] = mul_i<kInv>(cr);  // times 1j
       }
     }
-    block_fft<N, E, kInv, XW>(v, sm, t, tw, 1);
+    // single adds from 256: paired, the 512^3 pass took 1235 us instead of 1222, the 256^3
+    // pass 116 and 115; two 128^3 steps 338 us instead of 330 without them
+    block_fft<N, E, kInv, XW, kSyncCta, false, N <= 128>(v, sm, t, tw, 1);
     if (ok) {
       float2* dst = (SKIPWX && (f == 1 || f == 2)) ? wx + wxofs + (f - 1) * fs : w + wofs + f * fs;
 #pragma unroll
@@ -383,7 +385,9 @@ ky_inv_rhs(float2* __restrict__ w, const float2* __restrict__ wx, long long fs, 
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = ok ? src[(long long)(t + T * e) * H] : make_float2(0.f, 0.f);
   }
-  block_fft<N, E, kInv, TWY>(v, sm + p, t, tw, 1);
+  // single adds at 512: paired, the registers pass the limit of three CTAs per SM (1416 us
+  // instead of 1291; held to that limit 1314)
+  block_fft<N, E, kInv, TWY, kSyncCta, false, kPaired<E> && N <= 256>(v, sm + p, t, tw, 1);
   if (ok) {
     const int f = job == 0 ? 0 : job < 3 ? job + 3 : job == 3 ? 3 : job - 3;
     float2* dst = wb + f * fs;
@@ -867,8 +871,11 @@ __device__ __forceinline__ void c2r_pair_smem16(const float2* X, const float2* Y
 // (bounded) for its copies in flight and returns. Measured and kept out: two line pairs
 // per warp with the copies running on across them (131.0 us: spills), Blackwell's paired
 // FP32 adds in the FFT butterflies (130.9 us: register pairs, spills).
-template <int N, bool STAGED>
-__global__ void __launch_bounds__(Line3Cfg<N>::THREADS, 3)
+//
+// FEW (STAGED only): a launch of at most one CTA per SM, where latency counts and not
+// occupancy: paired adds with the registers they need (212; ten 256^2 steps 492 -> 481 us).
+template <int N, bool STAGED, bool FEW = false>
+__global__ void __launch_bounds__(Line3Cfg<N>::THREADS, FEW ? 1 : 3)
 line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du, long long ds, int kt, int kd,
             float s2, const float2* __restrict__ ct8, const float2* __restrict__ ct16, int nlines, int* err) {
   pdl_begin();
@@ -930,7 +937,7 @@ line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du,
       bulk_load(stg0, rows + 4 * fs, kPairBytes / 2, &bar[0]);
       bulk_load(stg0 + C::ROW2, rows + 5 * fs, kPairBytes / 2, &bar[0]);
     }
-    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true, FEW>(z, xs, t, ct16, 0);
 #pragma unroll
     for (int e = 0; e < E; ++e) h1[e] = z[e];
     __syncwarp();
@@ -939,7 +946,7 @@ line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du,
       return;
     }
     c2r_pair_smem16<N>(stg1 + rsel, stg1 + C::ROW2 + rsel, t, z);  // u_z + i curl_x
-    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true, FEW>(z, xs, t, ct16, 0);
 #pragma unroll
     for (int e = 0; e < E; ++e) h2[e] = z[e];
     __syncwarp();
@@ -948,7 +955,7 @@ line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du,
       return;
     }
     c2r_pair_smem16<N>(stg0 + rsel, stg0 + C::ROW2 + rsel, t, z);  // curl_y + i curl_z
-    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true, FEW>(z, xs, t, ct16, 0);
     __syncwarp();
   } else {
     __shared__ float2 s_xs[C::LPC * C::XS];
@@ -956,17 +963,17 @@ line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du,
     float2* xs = s_x + (2 * warp + half) * C::XS;
     const float2* src = wb + line * H;
     c2r_pair_load16<N>(src, src + fs, t, z);  // u_x + i u_y
-    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true, FEW>(z, xs, t, ct16, 0);
 #pragma unroll
     for (int e = 0; e < E; ++e) h1[e] = z[e];
     __syncwarp();
     c2r_pair_load16<N>(src + 2 * fs, src + 3 * fs, t, z);  // u_z + i curl_x
-    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true, FEW>(z, xs, t, ct16, 0);
 #pragma unroll
     for (int e = 0; e < E; ++e) h2[e] = z[e];
     __syncwarp();
     c2r_pair_load16<N>(src + 4 * fs, src + 5 * fs, t, z);  // curl_y + i curl_z
-    block_fft<N, E, kInv, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
+    block_fft<N, E, kInv, 1, kSyncWarp, true, FEW>(z, xs, t, ct16, 0);
     __syncwarp();
   }
   float2* xs = s_x + (2 * warp + half) * C::XS;
@@ -978,7 +985,7 @@ line_cross3(const float2* __restrict__ w, long long fs, float2* __restrict__ du,
     pz[e] = fmaf(ux, wy, -uy * wx);
     z[e] = make_float2(fmaf(uy, wz, -uz * wy), fmaf(uz, wx, -ux * wz));
   }
-  block_fft<N, E, kFwd, 1, kSyncWarp, true>(z, xs, t, ct16, 0);
+  block_fft<N, E, kFwd, 1, kSyncWarp, true, FEW>(z, xs, t, ct16, 0);
   {
     float2 X[NE], Y[NE];
     r2c_pair_unpack16<N, NE>(z, t, s2, X, Y);
@@ -1344,7 +1351,8 @@ struct BandRk {
 // ------------------------------------------------------------------------------
 // One tile of kx_fwd_band: d[c][e] = DU component c at x row t + T e of column kh of
 // middle row kmb (band index); x forward FFT, dealias mask, Leray projection into P.
-template <int N, int DIM, bool FUSED = false, int XW = TW>
+// PK: paired adds (the bulk-load variant; with direct loads the 128^3 pass took 14.0 us, not 13.5).
+template <int N, int DIM, bool FUSED = false, int XW = TW, bool PK = false>
 __device__ __forceinline__ void kx_fwd_band_tile(float2 (&d)[3][Fft<N>::E], int t, int kh, int kmb, int kd, int kt,
                                                  float2* sm, float2* __restrict__ P, long long pcs, long long bp,
                                                  const float2* __restrict__ tw, const BandRk* br = nullptr,
@@ -1356,7 +1364,7 @@ __device__ __forceinline__ void kx_fwd_band_tile(float2 (&d)[3][Fft<N>::E], int 
   const int mid = km < 0 ? km + N : km;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    block_fft<N, E, kFwd, XW>(d[c], sm, t, tw, 1);
+    block_fft<N, E, kFwd, XW, kSyncCta, false, PK>(d[c], sm, t, tw, 1);
     __syncthreads();
   }
   // (kt can exceed the half axis only at N = 8: those columns hold no mode of S)
@@ -1531,7 +1539,7 @@ kx_fwd_band_tma(const __grid_constant__ CUtensorMap dmap, int kt, int kd, float2
       fence_proxy_async_smem();
       issue(next);
     }
-    kx_fwd_band_tile<N, 3, FUSED>(d, t, (tile % ntx) * TW + p, tile / ntx, kd, kt, sm + p, P, pcs,
+    kx_fwd_band_tile<N, 3, FUSED, TW, true>(d, t, (tile % ntx) * TW + p, tile / ntx, kd, kt, sm + p, P, pcs,
                                   (long long)batch * 3 * pcs, tw, &br, batch);
   }
 }

@@ -47,6 +47,8 @@ struct DnsOps {
   static void init_attrs() {
     if constexpr (N == 256) {
       lc3_staged_ok = cudaFuncSetAttribute(line_cross3<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           Line3Cfg<N>::SMEM_STAGED) == cudaSuccess &&
+                      cudaFuncSetAttribute(line_cross3<N, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            Line3Cfg<N>::SMEM_STAGED) == cudaSuccess;
       cudaGetLastError();
     }
@@ -180,9 +182,10 @@ struct DnsOps {
           const long long tiles = (lines + L3::LPC - 1) / L3::LPC;
           if (c.sched.line_pair == 3 && lc3_staged_ok && lines % L3::LPC == 0)
             L3ES_LAUNCH(c, KK_LINE_CROSS, 2.0 * A + Adu, s,
-                        pdl_launch(line_cross3<N, true>, dim3((unsigned)tiles, c.batch), L3::THREADS, L3::SMEM_STAGED,
-                                   s, c.W, c.fs, c.DU, c.ds, c.kt, c.kd, s2, c.tw + line2_ct_offset<N>(),
-                            c.tw + line3_ct16_offset<N>(), (int)lines, c.err));
+                        pdl_launch(tiles * c.batch <= 152 ? line_cross3<N, true, true> : line_cross3<N, true>,
+                                   dim3((unsigned)tiles, c.batch), L3::THREADS, L3::SMEM_STAGED, s, c.W, c.fs, c.DU,
+                                   c.ds, c.kt, c.kd, s2, c.tw + line2_ct_offset<N>(),
+                                   c.tw + line3_ct16_offset<N>(), (int)lines, c.err));
           else
             L3ES_LAUNCH(c, KK_LINE_CROSS, 2.0 * A + Adu, s,
                         pdl_launch(line_cross3<N, false>, dim3((unsigned)tiles, c.batch), L3::THREADS, 0, s, c.W,

@@ -46,38 +46,55 @@ __device__ __forceinline__ float c16(int k) {
   return k == 0 ? 1.0f : k == 1 ? 0.92387953251128674f : k == 2 ? 0.70710678118654752f : 0.38268343236508978f;
 }
 
+// a + b, a - b as one paired FP32 instruction (PK; the same roundings) or two
+template <bool PK>
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  if constexpr (PK) return __fadd2_rn(a, b);
+  return cadd(a, b);
+}
+template <bool PK>
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  if constexpr (PK) return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
+  return csub(a, b);
+}
+// a + DIR i b
+template <int DIR>
+__device__ __forceinline__ float2 cadd_i(float2 a, float2 b) {
+  return DIR < 0 ? make_float2(a.x + b.y, a.y - b.x) : make_float2(a.x - b.y, a.y + b.x);
+}
+
 // In-register DFT of size R (2, 4, 8, 16), natural order in and out.
-template <int R, int DIR>
+template <int R, int DIR, bool PK>
 struct Dft;
 
-template <int DIR>
-struct Dft<1, DIR> {
+template <int DIR, bool PK>
+struct Dft<1, DIR, PK> {
   static __device__ __forceinline__ void run(float2*) {}
 };
 
-template <int DIR>
-struct Dft<2, DIR> {
+template <int DIR, bool PK>
+struct Dft<2, DIR, PK> {
   static __device__ __forceinline__ void run(float2* v) {
     float2 a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
+    v[0] = add2<PK>(a, b);
+    v[1] = sub2<PK>(a, b);
   }
 };
 
-template <int DIR>
-struct Dft<4, DIR> {
+template <int DIR, bool PK>
+struct Dft<4, DIR, PK> {
   static __device__ __forceinline__ void run(float2* v) {
-    float2 s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-    float2 s13 = cadd(v[1], v[3]), d13 = mul_i<DIR>(csub(v[1], v[3]));
-    v[0] = cadd(s02, s13);
-    v[2] = csub(s02, s13);
-    v[1] = cadd(d02, d13);
-    v[3] = csub(d02, d13);
+    float2 s02 = add2<PK>(v[0], v[2]), d02 = sub2<PK>(v[0], v[2]);
+    float2 s13 = add2<PK>(v[1], v[3]), d13 = sub2<PK>(v[1], v[3]);
+    v[0] = add2<PK>(s02, s13);
+    v[2] = sub2<PK>(s02, s13);
+    v[1] = cadd_i<DIR>(d02, d13);
+    v[3] = cadd_i<-DIR>(d02, d13);
   }
 };
 
 // radix-2 decimation in time on top of two half-size DFTs
-template <int R, int DIR>
+template <int R, int DIR, bool PK>
 struct DftSplit {
   static __device__ __forceinline__ void run(float2* v) {
     float2 e[R / 2], o[R / 2];
@@ -86,17 +103,20 @@ struct DftSplit {
       e[i] = v[2 * i];
       o[i] = v[2 * i + 1];
     }
-    Dft<R / 2, DIR>::run(e);
-    Dft<R / 2, DIR>::run(o);
+    Dft<R / 2, DIR, PK>::run(e);
+    Dft<R / 2, DIR, PK>::run(o);
 #pragma unroll
     for (int k = 0; k < R / 2; ++k) {
       float2 t;
       // W_R^k = exp(DIR * 2 pi i k / R) expressed in sixteenths of a turn
       const int q = k * (16 / R);  // 0..7
+      if (q == 4) {
+        v[k] = cadd_i<DIR>(e[k], o[k]);
+        v[k + R / 2] = cadd_i<-DIR>(e[k], o[k]);
+        continue;
+      }
       if (q == 0) {
         t = o[k];
-      } else if (q == 4) {
-        t = mul_i<DIR>(o[k]);
       } else {
         // angle 2 pi q / 16 in (0, pi): cos = c16(q) (q<4) or -c16(8-q) ...
         float cr, si;
@@ -110,19 +130,19 @@ struct DftSplit {
         const float2 w = make_float2(cr, DIR * si);
         t = cmul(o[k], w);
       }
-      v[k] = cadd(e[k], t);
-      v[k + R / 2] = csub(e[k], t);
+      v[k] = add2<PK>(e[k], t);
+      v[k + R / 2] = sub2<PK>(e[k], t);
     }
   }
 };
 
-template <int DIR>
-struct Dft<8, DIR> {
-  static __device__ __forceinline__ void run(float2* v) { DftSplit<8, DIR>::run(v); }
+template <int DIR, bool PK>
+struct Dft<8, DIR, PK> {
+  static __device__ __forceinline__ void run(float2* v) { DftSplit<8, DIR, PK>::run(v); }
 };
-template <int DIR>
-struct Dft<16, DIR> {
-  static __device__ __forceinline__ void run(float2* v) { DftSplit<16, DIR>::run(v); }
+template <int DIR, bool PK>
+struct Dft<16, DIR, PK> {
+  static __device__ __forceinline__ void run(float2* v) { DftSplit<16, DIR, PK>::run(v); }
 };
 
 // Compile-time stage schedule: radix E until the remainder is smaller than E.
@@ -155,6 +175,13 @@ __device__ __forceinline__ int xpad(int n) {
 template <int SS>
 __host__ __device__ constexpr int xpad_len(int n) { return SS == 1 ? n + 8 : n + n / 8; }
 
+// Whether a thread's butterflies add in pairs (the default of an FFT below): half the
+// issue slots of those adds. 512^3 line pass 1320 -> 1259 us, y forward pass 433 -> 405, 256^3
+// band pass 86 -> 83, ten 256^2 steps 505 -> 492; with 16 values per thread the register pairs spill
+// (256^3 line pass 125 -> 131). Passes that wait on memory and lose to it ask for single adds.
+template <int E>
+constexpr bool kPaired = E <= 8;
+
 // Scope of an FFT's exchange barriers: the whole CTA, one warp, or one group of
 // consecutive threads of a CTA that runs several FFTs side by side (group g of G threads
 // waits on named barrier 1 + g; G is a multiple of 32).
@@ -180,7 +207,8 @@ __device__ __forceinline__ void fft_sync() {
 // sm: exchange buffer, element n at sm[xpad<SS>(n) * SS]. SYNC: the scope of the
 // exchange barriers (kSync*; a group holds the SS T threads of SS interleaved FFTs).
 // CT: tw is the compact table at this stage's offset (tws unused).
-template <int N, int E, int R, int NS, int DIR, int SS, int SYNC, bool FIRST, bool LAST, bool CT = false>
+template <int N, int E, int R, int NS, int DIR, int SS, int SYNC, bool FIRST, bool LAST, bool CT = false,
+          bool PK = kPaired<E>>
 __device__ __forceinline__ void stockham_stage(float2 (&v)[E], float2* sm, int t,
                                                const float2* __restrict__ tw, int tws) {
   constexpr int T = N / E;
@@ -204,7 +232,7 @@ __device__ __forceinline__ void stockham_stage(float2 (&v)[E], float2* sm, int t
       for (int r = 1; r < R; ++r)
         x[b][r] = cmul(x[b][r], twid<DIR>(tw, CT ? (r - 1) * NS + jm : r * jm * (N / (NS * R)) * tws));
     }
-    Dft<R, DIR>::run(x[b]);
+    Dft<R, DIR, PK>::run(x[b]);
     if (LAST) {
 #pragma unroll
       for (int r = 0; r < R; ++r) v[b + r * BPT] = x[b][r];
@@ -217,20 +245,20 @@ __device__ __forceinline__ void stockham_stage(float2 (&v)[E], float2* sm, int t
   if (!LAST) fft_sync<SYNC, SS * (N / E)>();
 }
 
-template <int N, int E, int DIR, int SS, int SYNC, bool CT, int S, bool DONE = (S >= Sched<N, E>::kStages)>
+template <int N, int E, int DIR, int SS, int SYNC, bool CT, bool PK, int S, bool DONE = (S >= Sched<N, E>::kStages)>
 struct Stages;
-template <int N, int E, int DIR, int SS, int SYNC, bool CT, int S>
-struct Stages<N, E, DIR, SS, SYNC, CT, S, false> {
+template <int N, int E, int DIR, int SS, int SYNC, bool CT, bool PK, int S>
+struct Stages<N, E, DIR, SS, SYNC, CT, PK, S, false> {
   using Sc = Sched<N, E>;
   static __device__ __forceinline__ void run(float2 (&v)[E], float2* sm, int t,
                                              const float2* __restrict__ tw, int tws) {
-    stockham_stage<N, E, Sc::radix(S), Sc::ns(S), DIR, SS, SYNC, S == 0, S == Sc::kStages - 1, CT>(
+    stockham_stage<N, E, Sc::radix(S), Sc::ns(S), DIR, SS, SYNC, S == 0, S == Sc::kStages - 1, CT, PK>(
         v, sm, t, CT ? tw + Sc::ctoff(S) : tw, tws);
-    Stages<N, E, DIR, SS, SYNC, CT, S + 1>::run(v, sm, t, tw, tws);
+    Stages<N, E, DIR, SS, SYNC, CT, PK, S + 1>::run(v, sm, t, tw, tws);
   }
 };
-template <int N, int E, int DIR, int SS, int SYNC, bool CT, int S>
-struct Stages<N, E, DIR, SS, SYNC, CT, S, true> {
+template <int N, int E, int DIR, int SS, int SYNC, bool CT, bool PK, int S>
+struct Stages<N, E, DIR, SS, SYNC, CT, PK, S, true> {
   static __device__ __forceinline__ void run(float2 (&)[E], float2*, int, const float2* __restrict__, int) {}
 };
 
@@ -239,10 +267,10 @@ struct Stages<N, E, DIR, SS, SYNC, CT, S, true> {
 // element t + T*e on entry and on exit. tws: stride into the twiddle table (table
 // length / N); with CT, tw is the compact table of the N-point FFT instead. The exchange buffer is free on return only after the caller's next
 // barrier of the same scope.
-template <int N, int E, int DIR, int SS, int SYNC = kSyncCta, bool CT = false>
+template <int N, int E, int DIR, int SS, int SYNC = kSyncCta, bool CT = false, bool PK = kPaired<E>>
 __device__ __forceinline__ void block_fft(float2 (&v)[E], float2* sm, int t,
                                           const float2* __restrict__ tw, int tws) {
-  Stages<N, E, DIR, SS, SYNC, CT, 0>::run(v, sm, t, tw, tws);
+  Stages<N, E, DIR, SS, SYNC, CT, PK, 0>::run(v, sm, t, tw, tws);
 }
 
 // N-point FFT whose T = N/E threads sit in one warp (per-line buffers, SS = 1). For
@@ -271,7 +299,7 @@ __device__ __forceinline__ void warp_fft(float2 (&v)[E], float2* sm, int t, cons
       const int jm = t % E;
 #pragma unroll
       for (int r = 1; r < E; ++r) x[r] = cmul(x[r], twid<DIR>(ct, Sc::ctoff(1) + (r - 1) * E + jm));
-      Dft<E, DIR>::run(x);
+      Dft<E, DIR, kPaired<E>>::run(x);
 #pragma unroll
       for (int r = 0; r < E; ++r) v[r] = x[r];
     }
@@ -290,8 +318,8 @@ __device__ __forceinline__ void warp_fft(float2 (&v)[E], float2* sm, int t, cons
         float2 c = hi ? v[2 * b + 1] : got;
         const int j = t + T * b;
         c = cmul(c, twid<DIR>(ct, Sc::ctoff(2) + j));
-        y[b] = cadd(a, c);
-        y[b + E / 2] = csub(a, c);
+        y[b] = add2<kPaired<E>>(a, c);
+        y[b + E / 2] = sub2<kPaired<E>>(a, c);
       }
 #pragma unroll
       for (int e = 0; e < E; ++e) v[e] = y[e];
