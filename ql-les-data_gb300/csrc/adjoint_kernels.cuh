@@ -16,6 +16,7 @@
 //   ky_pass forward    (3D) on the 6 products
 //   kx_fwd_plain       x-axis forward FFT of the 6 products
 //   k_adj_epi          elementwise vjp assembly and the RK4 reverse recursion
+//   (kx_fwd_adj        both in one pass, 3D from 64^3)
 #pragma once
 
 #include "dns_kernels.cuh"
@@ -247,7 +248,7 @@ line_cross_adj(const float2* __restrict__ wm, long long ds, int kt, const float2
   }
 }
 
-// Epilogue operands of k_adj_epi. The stage's cotangent is gscale * g; the step's
+// Epilogue operands of k_adj_epi and kx_fwd_adj. The stage's cotangent is gscale * g; the step's
 // accumulated cotangent becomes lam_out = lam_in + vjp (lam_in = lam1 when null, and
 // lam1 = 0 when null) and the next stage's cotangent g_out = a_next lam1 + b_next vjp
 // (skipped when null). g_out may alias g and lam_out may alias lam_in or lam1 (each
@@ -358,6 +359,103 @@ k_adj_epi(const float2* __restrict__ y, long long cs, AdjEpi a, const float* __r
   for (int c = 0; c < 3; ++c) {
     reinterpret_cast<float4*>(a.lam_out + bo + c * cs)[q] = lo[c];
     if (a.g_out) reinterpret_cast<float4*>(a.g_out + bo + c * cs)[q] = go[c];
+  }
+}
+
+// ------------------------------------------------------------------------------
+// k_adj_epi's result straight from the products (y: fields 0..2 m x u, 3..5 m x w, before the
+// x transform; 3D from 64^3). A thread transforms Cp, holds k x Cp of its modes in registers
+// and adds one component of Ap, g and the cotangents at a time, so the 6 transformed fields
+// are neither written nor read back: bound by latency at 16 warps per SM (128 registers;
+// with more of either spent on loads in flight it is slower). Adjoint step against the two
+// kernels: 256^3 5327 -> 5092 us, 128^3 702 -> 695, 64^3 215 -> 206. On 2D grids and smaller 3D
+// ones six transforms in a row cost more than the launch saved (32^3 148 -> 156, 256^2
+// 138 -> 166), so those keep the two kernels.
+// ------------------------------------------------------------------------------
+constexpr int kAdjFusedMin3d = 64;
+
+template <int N>
+__global__ void __launch_bounds__(TW * Fft<N>::T, N >= 128 ? 512 / (TW * Fft<N>::T) : 1)
+kx_fwd_adj(const float2* __restrict__ y, long long cs, AdjEpi a, const float* __restrict__ nu_b,
+           const float2* __restrict__ tw) {
+  pdl_begin();
+  constexpr int E = Fft<N>::E, T = Fft<N>::T, H = N / 2 + 1;
+  constexpr int MC = N * H;
+  __shared__ float2 sm[xpad_len<TW>(N) * TW];
+  const int p = threadIdx.x % TW, t = threadIdx.x / TW;
+  const int m = blockIdx.x * TW + p;
+  const bool ok = m < MC;
+  const int batch = blockIdx.y;
+  const float2* yb = y + (long long)batch * 6 * cs + m;
+  const long long bo = (long long)batch * 3 * cs + m;
+  const float nu = nu_b[batch];
+  float fs_ = 0.f, fc = 0.f;
+  if (a.band_kf2 > 0) {
+    fs_ = (float)a.band_adj[2 * batch];
+    fc = (float)a.band_adj[2 * batch + 1];
+  }
+  const int kh = m % H, km = kfull(m / H, N);
+  const float wt = (kh == 0 || kh == N / 2) ? 1.f : 2.f;
+  float2 x[3][E];  // Cp, then k x Cp
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      x[c][e] = ok ? yb[c * cs + (long long)(t + T * e) * MC] : make_float2(0.f, 0.f);
+    block_fft<N, E, kFwd, TW>(x[c], sm + p, t, tw, 1);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    float k0, k1, k2;
+    kvec<3>(kfull(t + T * e, N), km, kh, k0, k1, k2);
+    const float2 c0 = x[0][e], c1 = x[1][e], c2 = x[2][e];
+    x[0][e] = make_float2(k1 * c2.x - k2 * c1.x, k1 * c2.y - k2 * c1.y);
+    x[1][e] = make_float2(k2 * c0.x - k0 * c2.x, k2 * c0.y - k0 * c2.y);
+    x[2][e] = make_float2(k0 * c1.x - k1 * c0.x, k0 * c1.y - k1 * c0.y);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    float2 v[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      v[e] = ok ? yb[(3 + c) * cs + (long long)(t + T * e) * MC] : make_float2(0.f, 0.f);
+    block_fft<N, E, kFwd, TW>(v, sm + p, t, tw, 1);
+    if (ok) {
+      float2 gg[4], l1s[4], lis[4];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        // lam_out and g_out may be the arrays read here: EL modes' reads go first
+        constexpr int EL = E < 4 ? E : 4;
+        if (e % EL == 0) {
+#pragma unroll
+          for (int q = 0; q < EL; ++q) {
+            const long long o = bo + c * cs + (long long)(t + T * (e + q)) * MC;
+            gg[q] = a.g[o];
+            l1s[q] = a.lam1 ? a.lam1[o] : make_float2(0.f, 0.f);
+            lis[q] = a.lam_in ? a.lam_in[o] : l1s[q];
+          }
+        }
+        const long long o = bo + c * cs + (long long)(t + T * e) * MC;
+        const int kx = kfull(t + T * e, N);
+        const int ik2 = kx * kx + km * km + kh * kh;
+        const float lin = nu * (float)ik2 + a.drag;
+        const float2 l1 = l1s[e % EL], li = lis[e % EL];
+        const float2 g = make_float2(gg[e % EL].x * a.gscale, gg[e % EL].y * a.gscale);
+        // wt (i (k x C) - A),  i (x + i y) = -y + i x
+        float2 r = make_float2(wt * (-x[c][e].y - v[e].x), wt * (x[c][e].x - v[e].y));
+        r.x -= lin * g.x;
+        r.y -= lin * g.y;
+        if (a.band_kf2 > 0 && ik2 > 0 && ik2 <= a.band_kf2) {
+          const float2 uv = a.us[o];
+          r.x += fs_ * g.x + fc * wt * uv.x;
+          r.y += fs_ * g.y + fc * wt * uv.y;
+        }
+        a.lam_out[o] = make_float2(li.x + r.x, li.y + r.y);
+        if (a.g_out) a.g_out[o] = make_float2(a.a_next * l1.x + a.b_next * r.x, a.a_next * l1.y + a.b_next * r.y);
+      }
+    }
+    __syncthreads();
   }
 }
 

@@ -196,7 +196,7 @@ __device__ __forceinline__ void kx_inv_fields(float2 (&a)[3][Fft<N>::E], int t, 
       }
     }
     // single adds from 256: paired, the 512^3 pass took 1235 us instead of 1222, the 256^3
-    // pass 116 and 115; two 128^3 steps 338 us instead of 330 without them
+    // pass 116 and 115; a 128^3 step and its physical field 338 us instead of 330 so
     block_fft<N, E, kInv, XW, kSyncCta, false, N <= 128>(v, sm, t, tw, 1);
     if (ok) {
       float2* dst = (SKIPWX && (f == 1 || f == 2)) ? wx + wxofs + (f - 1) * fs : w + wofs + f * fs;

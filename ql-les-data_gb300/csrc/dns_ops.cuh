@@ -528,12 +528,17 @@ struct DnsOps {
                 pdl_launch(line_cross_adj<N>, dim3(line_blocks(lines), c.batch), L::THREADS, 0, s, Wm, c.ds, c.kt, wuw,
                            c.fs, Y6, c.cs, scale, c.tw, (int)lines));
     if (DIM == 3) y_pass<kFwd>(c, KK_Y_FWD, 4.0 * A, Y6, c.cs, H, N / 2, 6 * c.batch, s);
+    // reads: 2 product spectra, g, lam1, lam_in; writes: lam_out, g_out
+    const double epi = (3.0 + (a.lam1 ? 1.0 : 0.0) + (a.lam_in ? 1.0 : 0.0) + 1.0 + (a.g_out ? 1.0 : 0.0)) * A;
+    if constexpr (DIM == 3 && N >= kAdjFusedMin3d) {
+      L3ES_LAUNCH(c, KK_ADJ_EPI, epi, s,
+                  pdl_launch(kx_fwd_adj<N>, dim3(xb, c.batch), TX, 0, s, Y6, c.cs, a, c.nu_b, c.tw));
+      return;
+    }
     // Y6 (6 fields per trajectory) -> W, as 2 * batch groups of 3 fields
     L3ES_LAUNCH(c, KK_X_FWD_PLAIN, 4.0 * A, s,
                 pdl_launch(kx_fwd_plain<N, DIM>, dim3(xb, 2 * c.batch), TX, 0, s, Y6, c.cs, c.W, c.fs, c.tw));
     const long long pairs = c.cs / 2;
-    // reads: 2 product spectra, g, lam1, lam_in; writes: lam_out, g_out
-    const double epi = (3.0 + (a.lam1 ? 1.0 : 0.0) + (a.lam_in ? 1.0 : 0.0) + 1.0 + (a.g_out ? 1.0 : 0.0)) * A;
     L3ES_LAUNCH(c, KK_ADJ_EPI, epi, s,
                 pdl_launch(k_adj_epi<N, DIM>, dim3((unsigned)((pairs + 255) / 256), c.batch), 256, 0, s, c.W, c.cs, a,
                                                                                                  c.nu_b));

@@ -35,7 +35,7 @@ enum KernelKind {
   KK_RK_UPDATE,     // k_rk_update (elementwise RK4 combination)
   KK_ADJ_X_INV,     // kx_inv_adjproj (projected cotangent, x inverse, band terms)
   KK_ADJ_LINE,      // line_cross_adj (both adjoint products)
-  KK_ADJ_EPI,       // k_adj_epi (vjp assembly + RK4 reverse recursion)
+  KK_ADJ_EPI,       // k_adj_epi / kx_fwd_adj (vjp assembly + RK4 reverse recursion)
   KK_X_STAGE,       // kx_stage (closes an RK stage on the x pencils, opens the next)
   KK_YZ_PLANE,      // k_yz_plane (small 3D grids: everything between two x passes)
   KK_COUNT
