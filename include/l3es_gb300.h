@@ -102,13 +102,18 @@ int64_t l3es_plan_workspace_bytes(const l3es_plan* plan);
 
 /* Kernel schedule of the plan's step (no counterpart in the reference, whose XLA
  * compiler picks its own kernels, spectral_solver.py:130-153): four choices,
- *   [0] 3D: x passes by the persistent bulk-tensor-copy kernels (else one tile per CTA);
- *       2D: the step's x passes in 2-column tiles (else 8 columns per CTA),
- *   [1] y passes with the radix-8 schedule (else radix 16 from N = 128),
+ *   [0] 3D: x inverse passes by the persistent bulk-tensor-copy kernels (else one tile per
+ *       CTA); 2D: x passes in 2-column tiles (else 8 columns per CTA). Reaches l3es_rhs,
+ *       l3es_irfftn, the adjoint and the step forms with an elementwise update,
+ *   [1] y passes with the radix-8 schedule (else radix 16 from N = 128); plans start with 1
+ *       for 128^3 and 512^3,
  *   [2] the half-axis line pass: 1 two-for-one for 64 <= N <= 256, 2 two-for-one with
  *       radix-16 line FFTs, 3 the same fed by bulk copies (2 and 3: N = 256 only),
  *       0 the packed half-length one,
- *   [3] the persistent bulk-copy band x pass (else one tile per CTA).
+ *   [3] the persistent bulk-copy band x pass (else one tile per CTA); plans start with 1 at
+ *       N = 256.
+ * The step of 2D grids and of 3D grids up to 64^3 has stage kernels of its own in the
+ * forms it starts with; of these choices only [2] reaches them (2D, N = 256).
  * Every schedule computes the same step; only speed differs. */
 int l3es_plan_get_schedule(const l3es_plan* plan, int32_t* sched4);
 int l3es_plan_set_schedule(l3es_plan* plan, const int32_t* sched4);
@@ -118,11 +123,12 @@ int l3es_plan_set_schedule(l3es_plan* plan, const int32_t* sched4);
  *   0 one elementwise update of the whole spectrum per stage,
  *   1 the same, with modes outside the dealiased rows taking the closed form of their
  *     linear decay (no nonlinear or forcing term reaches them),
- *   2 the stage combination fused into the band x pass, in place on the band, and
- *     every other mode scaled by its closed form inside the next stage's x inverse (no
+ *   2 the stage combination inside the x passes: up to 64^3 one kernel closes a stage and
+ *     opens the next; above, the band x pass combines the stages in place on the band and
+ *     every other mode is scaled by its closed form inside the next stage's x inverse (no
  *     elementwise pass).
- * Plans start with form 2 in 3D and form 1 in 2D (the 2D band pass has too few CTAs to
- * hide the fused epilogue's memory latency).
+ * Plans start with form 2 in 3D and form 1 in 2D; in 2D forms 1 and 2 are the same kernels,
+ * the stage combination inside the x passes (and nsteps steps in one launch up to 32^2).
  * Forms 1 and 2 apply when the forcing lies inside the band (constant-power kf <= kd,
  * Kolmogorov wavenumber < kt); otherwise, and for the integrating-factor scheme, the
  * step takes form 0. */

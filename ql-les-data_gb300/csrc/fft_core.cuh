@@ -265,8 +265,8 @@ struct Stages<N, E, DIR, SS, SYNC, CT, PK, S, true> {
 // N-point FFT by T = N/E threads; every thread of the CTA, warp or group (SYNC) must
 // call it, since it synchronises between stages. v[e] holds
 // element t + T*e on entry and on exit. tws: stride into the twiddle table (table
-// length / N); with CT, tw is the compact table of the N-point FFT instead. The exchange buffer is free on return only after the caller's next
-// barrier of the same scope.
+// length / N); with CT, tw is the compact table of the N-point FFT instead. The exchange
+// buffer is free on return only after the caller's next barrier of the same scope.
 template <int N, int E, int DIR, int SS, int SYNC = kSyncCta, bool CT = false, bool PK = kPaired<E>>
 __device__ __forceinline__ void block_fft(float2 (&v)[E], float2* sm, int t,
                                           const float2* __restrict__ tw, int tws) {

@@ -187,7 +187,8 @@ line_c2c_re(const float2* __restrict__ g, float* __restrict__ gre, long long nli
 
 // ------------------------------------------------------------------------------
 // Particle binning by cell (counting sort) so that consecutive threads of the spread
-// (and of the gather on grids beyond L2) work on neighbouring grid points. Bins: cubes of (n/nb)^dim fine cells.
+// (and of the gather on grids beyond L2) work on neighbouring grid points. Bins: cubes of
+// (n/nb)^dim fine cells.
 // ------------------------------------------------------------------------------
 template <int DIM>
 __device__ __forceinline__ int particle_bin(const double* __restrict__ r, long long j, int nb) {
@@ -252,7 +253,7 @@ __global__ void k_bin_scatter(const double* __restrict__ r, long long np, int nb
 }
 
 // ------------------------------------------------------------------------------
-// ES-kernel gather + Euler advection. For particle j (in binned order):
+// ES-kernel gather + Euler advection. For particle j (in input order; in bin order where nufft_binned):
 //   u_r[j] = (1 / (n^dim c^dim)) sum_l Re g(l) prod_d phi((x_d/h - l_d) / (w/2))
 //   r_out[j] = (r[j] + dt u_r[j]) mod 2 pi                 (integrator.py:21-23)
 // phi(z) = exp(beta (sqrt(1 - z^2) - 1)); w-point support per axis.

@@ -239,8 +239,8 @@ int l3es_plan_create(const l3es_plan_desc* desc, l3es_plan** out) {
   c.kd = dealias_kd(n);
   c.kt = ((c.kd + 1 + TW - 1) / TW) * TW;
   if (n == 256) c.sched.line_pair = 3;  // the staged radix-16 line pass (measured best at 256)
-  // y pass: radix 16 at 256^3 (a step 2062 us against 2298 us with radix 8), radix 8 at
-  // 128^3 (288 against 295 us) and 512^3 (20.07 against 20.30 ms)
+  // y pass: radix 16 at 256^3 (a step 2055 us against 2153 us with radix 8), radix 8 at
+  // 128^3 (283 against 292 us) and 512^3 (20.07 against 20.30 ms before the paired adds)
   c.sched.y_var = dim == 3 && (n == 128 || n == 512);
   // the stage combination inside the x passes (in 2D forms 1 and 2 both are kx_stage)
   c.step_form = dim == 3 ? 2 : 1;
@@ -442,9 +442,11 @@ int l3es_plan_set_step_form(l3es_plan* plan, int32_t form) {
 // ---------------------------------------------------------------------------------
 // Autotuner: picks the plan's kernel variants (bulk-copy or one-tile x passes, radix-16 or
 // radix-8 y passes, two-for-one or packed line pass, bulk-copy or one-tile band pass) by
-// timing the right-hand side on the plan's own scratch (coordinate descent, each knob
-// with the others at their current choice), and caches the result in a text file, one
-// line per (GPU, dim, N, batch): "<key> x_bulk y_var line_pair band_bulk".
+// timing one RK4 step in the plan's step form on its own scratch (coordinate descent, each
+// knob with the others at their current choice), and caches the result in a text file, one
+// line per (GPU, dim, N, batch, step form): "<key> x_bulk y_var line_pair band_bulk". Where
+// the step runs kernels that a knob does not reach (XStage, k_yz_plane, k_step2d) its two
+// settings time alike and either may be kept.
 // ---------------------------------------------------------------------------------
 static std::string tune_key(const l3es_plan* p) {
   cudaDeviceProp prop{};

@@ -27,7 +27,8 @@ namespace l3es {
 // passes (x inverse, y inverse, line, y forward, band pass, 2D also the update): 2D 256^2
 // 98.3 -> 69.7 us, 128^2 x 8 98.4 -> 70.6 us, 512^2 122.9 -> 97.7 us; 3D, dependent launches
 // on both sides, 64^3 89 -> 71 us, 64^3 x 6 222 -> 208 us, 64^3 x 12 425 -> 423 us; from
-// plain launches 32^3 121 -> 35 us, 16^3 130 -> 41 us. With kx_stage 128^3 takes 38 instead
+// plain launches 32^3 121 -> 35 us, 16^3 130 -> 41 us. (With dependent launches, paired adds
+// and the line passes of their size those steps now take 48, 42 and 68 us.) With kx_stage 128^3 takes 38 instead
 // of 32.6 us for one stage's x passes and 256^3 267 instead of 195 us: there the chip is full
 // and the barriers of the three groups cost more than the saved round trip. Larger 3D grids
 // keep kx_inv and the band-fused kx_fwd_band.

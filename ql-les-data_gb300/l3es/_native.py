@@ -326,7 +326,8 @@ class Plan:
     def schedule(self) -> dict:
         """The plan's kernel schedule (l3es_plan_get_schedule) as {name: 0 or 1}; line_pair
         is 2 or 3 for the radix-16 line passes (N = 256; 3 fed by bulk copies); x_bulk
-        selects the bulk-copy x passes in 3D and 2-column x-pass tiles in 2D."""
+        selects the bulk-copy x inverse passes in 3D and 2-column x-pass tiles in 2D, in
+        rhs, irfftn, the adjoint and the step forms with an elementwise update."""
         v = (ctypes.c_int32 * 4)()
         _check(self._lib.l3es_plan_get_schedule(self._h, v), "l3es_plan_get_schedule")
         return dict(zip(self.SCHEDULE_KEYS, list(v)))
@@ -343,8 +344,9 @@ class Plan:
     def step_form(self) -> int:
         """Form of the explicit RK4 step (l3es_plan_get_step_form): 0 one elementwise
         update of the whole spectrum per stage, 1 the closed form of the linear decay
-        outside the dealiased rows, 2 the stage combination fused into the band pass
-        (plans start at 2 in 3D, 1 in 2D). All forms compute the reference's RK4 step."""
+        outside the dealiased rows, 2 the stage combination inside the x passes (plans
+        start at 2 in 3D and at 1 in 2D, where 1 is the same as 2). All forms compute the
+        reference's RK4 step."""
         v = ctypes.c_int32()
         _check(self._lib.l3es_plan_get_step_form(self._h, ctypes.byref(v)), "l3es_plan_get_step_form")
         return int(v.value)
