@@ -848,9 +848,8 @@ def run_ours(args):
     stats = plan.kernel_stats()
     plan.timing(False)
     plan.check()  # no kernel gave up a bounded wait during the timed or instrumented steps
-    # launches of the particle layer per step (crop, prep, 3 grid passes, memset-free
-    # binning: count + scan + scatter, gather)
-    part_launches = 8 * args.steps if WITH_PARTICLES else 0
+    # launches of the particle layer per step (crop, 3 grid passes, gather)
+    part_launches = 5 * args.steps if WITH_PARTICLES else 0
     launches = sum(v[0] for v in stats.values()) + part_launches
     top = max(stats.items(), key=lambda kv: kv[1][1])
     name, (nl, tms, tb) = top
