@@ -334,7 +334,9 @@ int l3es_interp_coarse_mse(l3es_interp_plan* plan, const void* u_hat_fine, const
  * of smoothing length dx and cutoff 3 dx, pressure p = p_ref (rho - 1) with
  * p_ref = (10 u_ref)^2. Positions, velocities and outputs are float64 (np, dim) device
  * arrays; np <= np_max. Positions are wrapped into the box before use. Outputs depend
- * only on the inputs (fixed neighbour order), not on the launch. */
+ * only on the inputs (fixed neighbour order), not on the launch. Beside its per-particle
+ * arrays a plan holds neighbour lists of 1056 (3D) or 416 (2D) bytes per particle, if they
+ * stay within 1 GiB and can be allocated; without them the calls take longer. */
 typedef struct l3es_sph_plan l3es_sph_plan;
 int l3es_sph_plan_create(int32_t dim, int32_t n, double box, int64_t np_max, l3es_sph_plan** out);
 int l3es_sph_plan_destroy(l3es_sph_plan* plan);

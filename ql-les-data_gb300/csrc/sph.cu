@@ -40,6 +40,7 @@ constexpr int kSphLanes = 8;
 
 struct SphGeom {
   double L;      // box side
+  double inv_L;
   double inv_cs; // cells per unit length (nc / L)
   double cs_d;   // cell side L / nc (cell origins; nc * cs_d == L up to FP64 rounding)
   float cs;      // cell side (stencil offsets)
@@ -50,9 +51,16 @@ struct SphGeom {
 };
 
 // position wrapped into [0, L), as the periodic shift of integrator.py:21-23 leaves it
-__device__ __forceinline__ double wrap_box(double x, double L) {
-  x = x - L * floor(x / L);
-  return x >= L ? x - L : x;
+// (floor(x / L) from x times 1 / L where that cannot differ: an FP64 division is some twenty
+// instructions at two a clock and SM here)
+__device__ __forceinline__ double floor_quotient(double x, const SphGeom& g) {
+  const double q = x * g.inv_L, f = floor(q), d = q - f;
+  if (d > 1e-9 && d < 1.0 - 1e-9 && fabs(q) < 1e6) return f;
+  return floor(x / g.L);
+}
+__device__ __forceinline__ double wrap_box(double x, const SphGeom& g) {
+  x = x - g.L * floor_quotient(x, g);
+  return x >= g.L ? x - g.L : x;
 }
 
 __device__ __forceinline__ int cell_coord(double x, const SphGeom& g) {
@@ -94,7 +102,7 @@ k_sph_bin(const double* __restrict__ r, const double* __restrict__ u, double dt,
   for (int d = 0; d < DIM; ++d) {
     double x = r[j * DIM + d];
     if (u) x += dt * u[j * DIM + d];
-    x = wrap_box(x, g.L);
+    x = wrap_box(x, g);
     xw[j * DIM + d] = x;
     ci[d] = cell_coord(x, g);
   }
@@ -192,7 +200,7 @@ k_sph_order(const int* __restrict__ perm0, const int* __restrict__ cell, const i
 // together, and a cell's first five candidates per lane are in flight at once. A list that
 // could overflow (14 neighbours per lane on average) is worked off before the next cell.
 // A relaxation call of 32^3 particles: 237 us with f in the candidate loop (density 78,
-// acceleration 152 us), 199 us; 17^3 118 -> 91 us; 2D 71^2 43 us.
+// acceleration 152 us), 199 us with lists; 17^3 118 -> 91 us.
 constexpr int kSphList = 32;
 constexpr int kSphTurns = 5;  // candidates per lane in flight: a cell of a lattice holds about 33
 struct SphLists {
@@ -211,8 +219,9 @@ __device__ __forceinline__ float4 pair_displacement(const float4 xi, int ox, int
 
 // One cell (nc == 1): every particle is a candidate, at the minimum image.
 template <int DIM, class P, class F>
-__device__ __forceinline__ void for_all_pairs(bool live, const float4 xi, const SphGeom& g, const int* __restrict__ start,
-                                              const float4* __restrict__ xs, int lane, P&& fetch, F&& f) {
+__device__ __forceinline__ void for_all_pairs(bool live, const float4 xi, const SphGeom& g,
+                                              const int* __restrict__ start, const float4* __restrict__ xs, int lane,
+                                              P&& fetch, F&& f) {
   const int e = live ? start[1] : 0;
   for (int jj = start[0] + lane; jj < e; jj += kSphLanes) {
     const float4 xj = xs[jj];
@@ -233,11 +242,12 @@ __device__ __forceinline__ void stencil_offset(int k, int& ox, int& oy, int& oz)
   oz = DIM == 3 ? k / 9 - 1 : 0;
 }
 
-// (nc >= 3) fetch(j): what f wants of slot j beside its displacement
-template <int DIM, class P, class F>
+// (nc >= 3) fetch(j): what f wants of slot j beside its displacement. keep(i, j, code):
+// called with f, the lane's i-th neighbour.
+template <int DIM, class P, class F, class K>
 __device__ __forceinline__ void for_neighbours(bool live, const float4 xi, const int3 ci, const SphGeom& g,
                                                const int* __restrict__ start, const float4* __restrict__ xs, int lane,
-                                               SphLists& lists, P&& fetch, F&& f) {
+                                               SphLists& lists, P&& fetch, F&& f, K&& keep) {
   const int nc = g.nc, tid = threadIdx.x, base = (tid & 31) - lane;
   constexpr int cells = DIM == 3 ? 27 : 9;
   constexpr int S = DIM == 3 ? 4 : 2;  // cells whose range a lane fetches: lane, lane + 8, ...
@@ -256,7 +266,7 @@ __device__ __forceinline__ void for_neighbours(bool live, const float4 xi, const
       re[q] = start[c + 1];
     }
   }
-  int cnt = 0;
+  int cnt = 0, done = 0;
 #pragma unroll 1
   for (int k = 0; k <= cells; ++k) {  // the turn after the last cell works the rest off
     int b = rb[0], e = re[0];
@@ -284,11 +294,13 @@ __device__ __forceinline__ void for_neighbours(bool live, const float4 xi, const
           const auto pn = fetch(jn);
           const float4 d = pair_displacement<DIM>(xi, (oc & 3) - 1, (oc >> 2 & 3) - 1, (oc >> 4) - 1, xc, g);
           f(jc, d.x, d.y, d.z, d.w, pc);
+          keep(done + i, jc, oc);
           jc = jn;
           oc = on;
           xc = xn;
           pc = pn;
         }
+        done += cnt;
         cnt = 0;
       }
       float4 xj[kSphTurns];
@@ -309,25 +321,116 @@ __device__ __forceinline__ void for_neighbours(bool live, const float4 xi, const
       b += kSphTurns * kSphLanes;
     } while (b < e);
   }
+  keep(done, -1, 0);
 }
 
-// sum of v over the kSphLanes lanes of a particle (fixed order), in every lane
-__device__ __forceinline__ double lanes_sum(double v) {
+// Neighbours that the density pass leaves for the acceleration pass of the same call, so
+// that the search (27 cells, eight candidates for one neighbour) runs once: entry k of
+// lane q of slot i at nb[k stride + 8 i + q] (slot | stencil cell << kSphCodeShift; a warp
+// reads 32 neighbouring words), counts at n. A lane with more than `cap` of them searches
+// again. The order is the search's, so the sums are the same to the bit. A relaxation call of
+// 32^3 particles 199 -> 175 us, 9^3 80 -> 49, 160^2 (2D) 92 -> 83.
+struct SphKept {
+  unsigned* nb;  // null: not kept
+  int* n;
+  long long stride;
+  int cap;
+};
+constexpr int kSphCodeShift = 26;
+constexpr int kSphKept3d = 32, kSphKept2d = 12;  // about 14 and 4 per lane on a lattice
+constexpr size_t kSphKeptBytes = (size_t)1 << 30;  // plans above it (10^6 particles in 3D) search twice
+
+// the pairs of one lane without lists, in the order of for_neighbours
+template <int DIM, class P, class F>
+__device__ __forceinline__ void for_neighbours_direct(const float4 xi, const int3 ci, const SphGeom& g,
+                                                   const int* __restrict__ start, const float4* __restrict__ xs,
+                                                   int lane, P&& fetch, F&& f) {
+  const int nc = g.nc;
+  auto wrap = [nc](int c) { return c < 0 ? c + nc : (c >= nc ? c - nc : c); };
+  constexpr int cells = DIM == 3 ? 27 : 9;
+  for (int k = 0; k < cells; ++k) {
+    int ox, oy, oz;
+    stencil_offset<DIM>(k, ox, oy, oz);
+    const int cx = wrap(ci.x + ox), cy = wrap(ci.y + oy);
+    const int c = DIM == 3 ? (cx * nc + cy) * nc + wrap(ci.z + oz) : cx * nc + cy;
+    for (int j = start[c] + lane; j < start[c + 1]; j += kSphLanes) {
+      const float4 d = pair_displacement<DIM>(xi, ox, oy, oz, xs[j], g);
+      if (d.w < g.cut2) f(j, d.x, d.y, d.z, d.w, fetch(j));
+    }
+  }
+}
+
+// the pairs of one lane from its kept list
+template <int DIM, class P, class F>
+__device__ __forceinline__ void for_kept(const float4 xi, const SphGeom& g, const float4* __restrict__ xs,
+                                         const unsigned* __restrict__ nb, long long stride, int n, P&& fetch, F&& f) {
+  constexpr int U = 2;  // pairs whose operands are in flight beside the two being formed
+  unsigned cc[U];
+  float4 xc[U];
+  decltype(fetch(0)) pc[U];
+  auto load = [&](int i, int q) {
+    cc[q] = i < n ? nb[i * stride] : 0u;
+    const int j = (int)(cc[q] & ((1u << kSphCodeShift) - 1));
+    xc[q] = xs[j];
+    pc[q] = fetch(j);
+  };
 #pragma unroll
-  for (int o = 1; o < kSphLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int q = 0; q < U; ++q) load(q, q);
+#pragma unroll 1
+  for (int i = 0; i < n; i += U) {
+    unsigned c0[U];
+    float4 x0[U];
+    decltype(fetch(0)) p0[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      c0[q] = cc[q];
+      x0[q] = xc[q];
+      p0[q] = pc[q];
+      load(i + U + q, q);
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const int o = (int)(c0[q] >> kSphCodeShift);
+      const float4 d = pair_displacement<DIM>(xi, (o & 3) - 1, (o >> 2 & 3) - 1, (o >> 4) - 1, x0[q], g);
+      if (i + q < n) f((int)(c0[q] & ((1u << kSphCodeShift) - 1)), d.x, d.y, d.z, d.w, p0[q]);
+    }
+  }
 }
 
-// cell coordinates of the particle at slot i, from its FP64 wrapped position
+// cell coordinates of the particle at slot i
 template <int DIM>
-__device__ __forceinline__ int3 slot_cell(long long i, const int* __restrict__ perm, const double* __restrict__ xw,
-                                          const SphGeom& g) {
-  const long long j = perm[i];
-  int3 c;
-  c.x = cell_coord(xw[j * DIM], g);
-  c.y = cell_coord(xw[j * DIM + 1], g);
-  c.z = DIM == 3 ? cell_coord(xw[j * DIM + 2], g) : 0;
-  return c;
+__device__ __forceinline__ int3 slot_cell(long long i, const int* __restrict__ perm, const int* __restrict__ cell,
+                                          int nc) {
+  const int c = cell[perm[i]], q = c / nc;
+  return DIM == 3 ? make_int3(q / nc, q % nc, c % nc) : make_int3(q, c % nc, 0);
+}
+
+// The lanes' float-float sums of F values per particle, in FP64: (particle of the block,
+// value) at sums[particle F + value]. The tree is that of a butterfly over the lanes. FP64 is
+// scarce on this GPU, so the sums meet in shared memory and whole warps add them: lanes 0-3
+// and 4-7 of a value by a thread each, instead of every lane adding every value; the
+// acceleration pass' wraps and divisions follow with a thread per particle and component (a
+// lane per particle made each warp run them three times for four live lanes). With the cells
+// read instead of formed again from FP64 positions, and floor_quotient: a relaxation call of
+// 32^3 particles 175 -> 125 us, 160^2 (2D) 83 -> 50.
+constexpr int kSphGroup = kSphThreads / kSphLanes;  // particles per block
+template <int F>
+struct SphSums {
+  float2 lane[F][kSphThreads];
+  double half[2][kSphGroup * F];
+};
+template <int F>
+__device__ __forceinline__ void block_sums(const Ff (&part)[F], SphSums<F>& m) {
+#pragma unroll
+  for (int f = 0; f < F; ++f) m.lane[f][threadIdx.x] = make_float2(part[f].hi, part[f].lo);
+  __syncthreads();
+  for (int task = threadIdx.x; task < 2 * kSphGroup * F; task += kSphThreads) {
+    const int h = task / (kSphGroup * F), v = task % (kSphGroup * F);
+    const float2* l = &m.lane[v % F][v / F * kSphLanes + 4 * h];
+    auto d = [&](int q) { return (double)l[q].x + (double)l[q].y; };
+    m.half[h][v] = (d(0) + d(1)) + (d(2) + d(3));
+  }
+  __syncthreads();
 }
 
 // rho[slot] = m sigma sum_j w(r_ij / h); rp[slot] = (rho, p = p_ref (rho - 1),
@@ -336,27 +439,38 @@ __device__ __forceinline__ int3 slot_cell(long long i, const int* __restrict__ p
 template <int DIM, bool ONE>
 __global__ void __launch_bounds__(kSphThreads)
 k_sph_density(const float4* __restrict__ xs, const int* __restrict__ start, const int* __restrict__ perm,
-              const double* __restrict__ xw, long long np, SphGeom g, double m_sigma, double p_ref,
-              float4* __restrict__ rp, double* __restrict__ rho_out) {
+              const int* __restrict__ cell, long long np, SphGeom g, double m_sigma, double p_ref,
+              float4* __restrict__ rp, double* __restrict__ rho_out, SphKept kept) {
   pdl_begin();
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long i = gt / kSphLanes;
   const int lane = (int)(gt % kSphLanes);
-  const bool live = i < np;  // every lane stays for the shuffles
-  Ff part{0.f, 0.f};
-  const long long is = live ? i : 0;
+  const bool live = gt / kSphLanes < np;  // every lane stays for the shuffles
+  Ff part[1] = {};
+  const long long is = live ? gt / kSphLanes : 0;
   const float4 xi = xs[is];
   const float inv_h = g.inv_h;
   auto none = [](int) { return 0; };
-  auto pair = [&](int, float, float, float, float r2, int) { part = ff_add(part, quintic_w(sqrtf(r2) * inv_h)); };
+  auto pair = [&](int, float, float, float, float r2, int) {
+    part[0] = ff_add(part[0], quintic_w(sqrtf(r2) * inv_h));
+  };
   if constexpr (ONE) {
     for_all_pairs<DIM>(live, xi, g, start, xs, lane, none, pair);
   } else {
     __shared__ SphLists lists;
-    for_neighbours<DIM>(live, xi, slot_cell<DIM>(is, perm, xw, g), g, start, xs, lane, lists, none, pair);
+    for_neighbours<DIM>(live, xi, slot_cell<DIM>(is, perm, cell, g.nc), g, start, xs, lane, lists, none, pair,
+                        [&](int k, int j, int code) {
+                          if (!kept.nb) return;
+                          if (j < 0)
+                            kept.n[gt] = k;
+                          else if (k < kept.cap)
+                            kept.nb[k * kept.stride + gt] = (unsigned)j | (unsigned)code << kSphCodeShift;
+                        });
   }
-  const double acc = lanes_sum((double)part.hi + (double)part.lo);
-  if (!live || lane != 0) return;
+  __shared__ SphSums<1> m;
+  block_sums<1>(part, m);
+  const long long i = (long long)blockIdx.x * kSphGroup + threadIdx.x;
+  if (threadIdx.x >= kSphGroup || i >= np) return;
+  const double acc = m.half[0][threadIdx.x] + m.half[1][threadIdx.x];
   const double rho = m_sigma * acc;
   const float rf = (float)rho;
   rp[i] = make_float4(rf, (float)(p_ref * (rho - 1.0)), 1.f / (rf * rf), 0.f);
@@ -369,6 +483,7 @@ struct SphAccelArgs {
   const float4* xs;
   const int* start;
   const int* perm;
+  const int* cell;      // per particle, input order
   const double* xw;     // wrapped (predicted) positions, input order
   const float4* rp;     // (rho, p, 1 / rho^2, -) per slot
   const float4* us;     // velocities per slot (forces only)
@@ -388,18 +503,20 @@ struct SphAccelArgs {
 //   grad = dW/dr * r_ij / (r + eps)
 //   acc_p = -pref p_ij grad, acc_tvf = -pref p_ref grad, acc_visc = pref u_ij dW/dr / (r + eps)
 // Relaxation acceleration = acc_p + acc_tvf / 2.
-template <int DIM, int MODE, bool ONE>
-__global__ void __launch_bounds__(kSphThreads) k_sph_accel(SphAccelArgs a, SphGeom g) {
+// HOW: the pairs come from a search, from the density pass's lists, or (one cell) are all.
+constexpr int kPairsSearch = 0, kPairsKept = 1, kPairsAll = 2;
+template <int DIM, int MODE, int HOW>
+__global__ void __launch_bounds__(kSphThreads) k_sph_accel(SphAccelArgs a, SphGeom g, SphKept kept) {
   pdl_begin();
   const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long i = gt / kSphLanes;
   const int lane = (int)(gt % kSphLanes);
-  const bool live = i < a.np;  // every lane stays for the shuffles
-  const long long is = live ? i : 0;
+  const bool live = gt / kSphLanes < a.np;  // every lane stays for the shuffles
+  const long long is = live ? gt / kSphLanes : 0;
   const float4 xi = a.xs[is];
   const float4 rpi = a.rp[is];
   const float4 ui = MODE == kSphForces ? a.us[is] : make_float4(0.f, 0.f, 0.f, 0.f);
-  Ff fp[3] = {}, ft[3] = {}, fv[3] = {};
+  constexpr int F = MODE == kSphForces ? 3 * DIM : DIM;  // values per particle
+  Ff sum[F] = {};  // acc_p (relaxation: acc), forces: acc_visc, acc_tvf behind it
   auto fetch = [&](int jj) { return a.rp[jj]; };
   auto pair = [&](int jj, float dx, float dy, float dz, float r2, const float4 rpj) {
     const float r = sqrtf(r2);
@@ -409,57 +526,58 @@ __global__ void __launch_bounds__(kSphThreads) k_sph_accel(SphAccelArgs a, SphGe
     const float s = dw / (r + a.eps);
     if (MODE == kSphForces) {
       const float cp = -pref * pij * s, ct = -pref * a.p_ref * s;
-      fp[0] = ff_add(fp[0], cp * dx); fp[1] = ff_add(fp[1], cp * dy); fp[2] = ff_add(fp[2], cp * dz);
-      ft[0] = ff_add(ft[0], ct * dx); ft[1] = ff_add(ft[1], ct * dy); ft[2] = ff_add(ft[2], ct * dz);
       const float4 uj = a.us[jj];
       const float cv = pref * s;
-      fv[0] = ff_add(fv[0], cv * (ui.x - uj.x));
-      fv[1] = ff_add(fv[1], cv * (ui.y - uj.y));
-      fv[2] = ff_add(fv[2], cv * (ui.z - uj.z));
+      const float e[3] = {dx, dy, dz}, w[3] = {ui.x - uj.x, ui.y - uj.y, ui.z - uj.z};
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        sum[d] = ff_add(sum[d], cp * e[d]);
+        sum[DIM + d] = ff_add(sum[DIM + d], cv * w[d]);
+        sum[2 * DIM + d] = ff_add(sum[2 * DIM + d], ct * e[d]);
+      }
     } else {
       const float cp = -pref * (pij + 0.5f * a.p_ref) * s;
-      fp[0] = ff_add(fp[0], cp * dx); fp[1] = ff_add(fp[1], cp * dy); fp[2] = ff_add(fp[2], cp * dz);
+      const float e[3] = {dx, dy, dz};
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) sum[d] = ff_add(sum[d], cp * e[d]);
     }
   };
-  if constexpr (ONE) {
+  if constexpr (HOW == kPairsAll) {
     for_all_pairs<DIM>(live, xi, g, a.start, a.xs, lane, fetch, pair);
+  } else if constexpr (HOW == kPairsKept) {
+    const int n = live ? kept.n[gt] : 0;
+    if (n <= kept.cap)
+      for_kept<DIM>(xi, g, a.xs, kept.nb + gt, kept.stride, n, fetch, pair);
+    else
+      for_neighbours_direct<DIM>(xi, slot_cell<DIM>(is, a.perm, a.cell, g.nc), g, a.start, a.xs, lane, fetch, pair);
   } else {
     __shared__ SphLists lists;
-    for_neighbours<DIM>(live, xi, slot_cell<DIM>(is, a.perm, a.xw, g), g, a.start, a.xs, lane, lists, fetch, pair);
+    for_neighbours<DIM>(live, xi, slot_cell<DIM>(is, a.perm, a.cell, g.nc), g, a.start, a.xs, lane, lists, fetch,
+                        pair, [](int, int, int) {});
   }
-  double ap[3], at[3] = {0.0, 0.0, 0.0}, av[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    ap[d] = lanes_sum((double)fp[d].hi + (double)fp[d].lo);
-    if (MODE == kSphForces) {
-      at[d] = lanes_sum((double)ft[d].hi + (double)ft[d].lo);
-      av[d] = lanes_sum((double)fv[d].hi + (double)fv[d].lo);
-    }
-  }
-  if (!live || lane != 0) return;
-  const long long j = a.perm[i];
-  if (MODE == kSphRelaxAcc) {
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) a.out0[j * DIM + d] = ap[d];
-  } else if (MODE == kSphRelaxVel) {
-    // r_temp <- shift(r_temp, kick * acc); u = displacement(r_temp, r0) / dt, with the
-    // periodic displacement mod(d + L/2, L) - L/2; optionally r_out = shift(r0, dt u)
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      const double x = wrap_box(a.xw[j * DIM + d] + a.kick * ap[d], g.L);
+  __shared__ SphSums<F> m;
+  block_sums<F>(sum, m);
+  // one thread per particle and value
+  for (int v = threadIdx.x; v < kSphGroup * F; v += kSphThreads) {
+    const long long i = (long long)blockIdx.x * kSphGroup + v / F;
+    if (i >= a.np) continue;
+    const int f = v % F, d = f % DIM;
+    const long long j = a.perm[i];
+    const double ap = m.half[0][v] + m.half[1][v];
+    if (MODE == kSphRelaxAcc) {
+      a.out0[j * DIM + d] = ap;
+    } else if (MODE == kSphRelaxVel) {
+      // r_temp <- shift(r_temp, kick * acc); u = displacement(r_temp, r0) / dt, with the
+      // periodic displacement mod(d + L/2, L) - L/2; optionally r_out = shift(r0, dt u)
+      const double x = wrap_box(a.xw[j * DIM + d] + a.kick * ap, g);
       double dd = x - a.r0[j * DIM + d] + 0.5 * g.L;
-      dd = dd - g.L * floor(dd / g.L);
+      dd = dd - g.L * floor_quotient(dd, g);
       if (dd >= g.L) dd -= g.L;
       const double uv = (dd - 0.5 * g.L) / a.dt;
       a.out0[j * DIM + d] = uv;
-      if (a.out1) a.out1[j * DIM + d] = wrap_box(a.r0[j * DIM + d] + a.dt * uv, g.L);
-    }
-  } else {
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) {
-      a.out0[j * DIM + d] = ap[d];
-      a.out1[j * DIM + d] = av[d];
-      a.out2[j * DIM + d] = at[d];
+      if (a.out1) a.out1[j * DIM + d] = wrap_box(a.r0[j * DIM + d] + a.dt * uv, g);
+    } else {
+      (f < DIM ? a.out0 : f < 2 * DIM ? a.out1 : a.out2)[j * DIM + d] = ap;
     }
   }
 }
@@ -484,6 +602,7 @@ struct l3es_sph_plan {
   float4* xs = nullptr;    // [np_max] cell-local coordinates per slot
   float4* us = nullptr;    // [np_max] velocity per slot (forces)
   float4* rp = nullptr;    // [np_max] (rho, p, 1 / rho^2, -) per slot
+  SphKept kept{};          // neighbour lists of np_max particles (null: searched twice)
   std::vector<void*> allocs;
 };
 
@@ -524,22 +643,30 @@ static int sph_build(l3es_sph_plan* p, const double* r, const double* u_pred, do
   return cuda_check(cudaGetLastError(), "l3es_sph cell list");
 }
 
-static void sph_density(l3es_sph_plan* p, long long np, double p_ref, double* rho_out, cudaStream_t s) {
+// keep: an acceleration pass over the same particles follows
+static void sph_density(l3es_sph_plan* p, long long np, double p_ref, double* rho_out, bool keep, cudaStream_t s) {
   const unsigned pb = (unsigned)((np * kSphLanes + kSphThreads - 1) / kSphThreads);
   const bool one = p->g.nc < 3;
   auto kernel = p->dim == 3 ? (one ? k_sph_density<3, true> : k_sph_density<3, false>)
                             : (one ? k_sph_density<2, true> : k_sph_density<2, false>);
-  pdl_launch(kernel, pb, kSphThreads, 0, s, p->xs, p->start, p->perm, p->xw, np, p->g, p->mass * p->sigma, p_ref, p->rp,
-             rho_out);
+  pdl_launch(kernel, pb, kSphThreads, 0, s, p->xs, p->start, p->perm, p->cell, np, p->g, p->mass * p->sigma, p_ref,
+             p->rp, rho_out, keep ? p->kept : SphKept{});
+}
+
+template <int DIM, int MODE>
+static void sph_accel_dim(l3es_sph_plan* p, SphAccelArgs& a, cudaStream_t s) {
+  const unsigned pb = (unsigned)((a.np * kSphLanes + kSphThreads - 1) / kSphThreads);
+  auto kernel = p->g.nc < 3 ? k_sph_accel<DIM, MODE, kPairsAll>
+                : p->kept.nb ? k_sph_accel<DIM, MODE, kPairsKept> : k_sph_accel<DIM, MODE, kPairsSearch>;
+  pdl_launch(kernel, pb, kSphThreads, 0, s, a, p->g, p->kept);
 }
 
 template <int MODE>
 static void sph_accel(l3es_sph_plan* p, SphAccelArgs& a, cudaStream_t s) {
-  const unsigned pb = (unsigned)((a.np * kSphLanes + kSphThreads - 1) / kSphThreads);
-  const bool one = p->g.nc < 3;
-  auto kernel = p->dim == 3 ? (one ? k_sph_accel<3, MODE, true> : k_sph_accel<3, MODE, false>)
-                            : (one ? k_sph_accel<2, MODE, true> : k_sph_accel<2, MODE, false>);
-  pdl_launch(kernel, pb, kSphThreads, 0, s, a, p->g);
+  if (p->dim == 3)
+    sph_accel_dim<3, MODE>(p, a, s);
+  else
+    sph_accel_dim<2, MODE>(p, a, s);
 }
 
 static SphAccelArgs sph_args(l3es_sph_plan* p, long long np, double u_ref) {
@@ -547,6 +674,7 @@ static SphAccelArgs sph_args(l3es_sph_plan* p, long long np, double u_ref) {
   a.xs = p->xs;
   a.start = p->start;
   a.perm = p->perm;
+  a.cell = p->cell;
   a.xw = p->xw;
   a.rp = p->rp;
   a.us = p->us;
@@ -586,6 +714,7 @@ int l3es_sph_plan_create(int32_t dim, int32_t n, double box, int64_t np_max, l3e
   int nc = n / 3;  // cell side L / nc >= cutoff 3 dx
   if (nc < 3) nc = 1;
   p->g.L = box;
+  p->g.inv_L = 1.0 / box;
   p->g.nc = nc;
   p->g.inv_cs = nc / box;
   p->g.cs_d = box / nc;
@@ -611,6 +740,19 @@ int l3es_sph_plan_create(int32_t dim, int32_t n, double box, int64_t np_max, l3e
     delete p;
     return rc;
   }
+  // neighbour lists, where they and the slot numbers fit (128 np_max words' rows: whole blocks)
+  const size_t lanes = (npm * kSphLanes + kSphThreads - 1) / kSphThreads * kSphThreads;
+  const int cap = dim == 3 ? kSphKept3d : kSphKept2d;
+  const size_t words = lanes * (cap + 1);
+  if (nc >= 3 && np_max <= (1LL << kSphCodeShift) && words * sizeof(unsigned) <= kSphKeptBytes) {
+    unsigned* nb = nullptr;
+    if (cudaMalloc((void**)&nb, words * sizeof(unsigned)) == cudaSuccess) {
+      p->allocs.push_back(nb);
+      p->kept = SphKept{nb, reinterpret_cast<int*>(nb + lanes * cap), (long long)lanes, cap};
+    } else {
+      cudaGetLastError();  // without them the calls search twice
+    }
+  }
   *out = p;
   return L3ES_OK;
 }
@@ -630,7 +772,7 @@ int l3es_sph_density(l3es_sph_plan* p, const double* r, int64_t np, double* rho,
   cudaStream_t s = (cudaStream_t)stream;
   rc = sph_build(p, r, nullptr, 0.0, nullptr, np, s);
   if (rc != L3ES_OK) return rc;
-  sph_density(p, np, 0.0, rho, s);
+  sph_density(p, np, 0.0, rho, false, s);
   return cuda_check(cudaGetLastError(), "l3es_sph_density launch");
 }
 
@@ -644,7 +786,7 @@ int l3es_sph_relax_acceleration(l3es_sph_plan* p, const double* r, int64_t np, d
   rc = sph_build(p, r, nullptr, 0.0, nullptr, np, s);
   if (rc != L3ES_OK) return rc;
   const double p_ref = 100.0 * u_ref * u_ref;
-  sph_density(p, np, p_ref, nullptr, s);
+  sph_density(p, np, p_ref, nullptr, true, s);
   SphAccelArgs a = sph_args(p, np, u_ref);
   a.out0 = acc;
   sph_accel<kSphRelaxAcc>(p, a, s);
@@ -661,7 +803,7 @@ int l3es_sph_forces(l3es_sph_plan* p, const double* r, const double* u, int64_t 
   rc = sph_build(p, r, nullptr, 0.0, u, np, s);
   if (rc != L3ES_OK) return rc;
   const double p_ref = 100.0 * u_ref * u_ref;
-  sph_density(p, np, p_ref, nullptr, s);
+  sph_density(p, np, p_ref, nullptr, true, s);
   SphAccelArgs a = sph_args(p, np, u_ref);
   a.out0 = acc_p;
   a.out1 = acc_visc;
@@ -683,7 +825,7 @@ int l3es_sph_relax_velocity(l3es_sph_plan* p, const double* r0, const double* u_
   rc = sph_build(p, r0, u_r, dt, nullptr, np, s);
   if (rc != L3ES_OK) return rc;
   const double p_ref = 100.0 * u_ref * u_ref;
-  sph_density(p, np, p_ref, nullptr, s);
+  sph_density(p, np, p_ref, nullptr, true, s);
   SphAccelArgs a = sph_args(p, np, u_ref);
   a.r0 = r0;
   a.kick = (relax_dt_factor * dt) * (relax_dt_factor * dt);
