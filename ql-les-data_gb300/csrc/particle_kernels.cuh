@@ -9,6 +9,18 @@
 
 namespace l3es {
 
+// x in [0, L) by whole periods (the periodic shift of integrator.py:21-23; Python's % never
+// returns the modulus itself). For x in [+0, L) the quotient's floor is 0 (x / L never rounds
+// up to 1) and x stays as it is; that is told from the bits, since an FP64 division is some
+// twenty instructions on a pipe of two a clock and SM.
+__device__ __forceinline__ double wrap_period(double x, double L) {
+  const unsigned long long xb = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long lb = (unsigned long long)__double_as_longlong(L);
+  if (lb < 0x7ff0000000000000ull && xb < lb) return x;  // (L positive and finite)
+  x = x - L * floor(x / L);
+  return x >= L ? x - L : x;
+}
+
 // ------------------------------------------------------------------------------
 // Coarse spectrum of spectral_filtering: Hh(f) = 0.5 (C(f) + conj C(p)), with
 // C(f) = U_fine(f) / (N/c)^dim on the crop set f in [-c/2, c/2-1]^dim and p the
@@ -250,14 +262,10 @@ k_dft_interp(const float2* __restrict__ hh, long long hcs, int c, const double* 
       if (j >= np) continue;
       double t = 0.0;
       for (int h = 0; h < nhw; ++h) t += sums[(h * DIM + i % DIM) * kDftTile + i / DIM];
-      const double ur = t / (DIM == 3 ? (double)c * c * c : (double)c * c);
+      const double ur = t * __longlong_as_double((1023LL - DIM * lc) << 52);  // / c^DIM
       u_r[j * DIM + i % DIM] = ur;
       if (r_out) {
-        const double two_pi = 2.0 * 3.14159265358979323846;
-        double x = r[j * DIM + i % DIM] + dt * ur;
-        x = x - two_pi * floor(x / two_pi);
-        if (x >= two_pi) x -= two_pi;
-        r_out[j * DIM + i % DIM] = x;
+        r_out[j * DIM + i % DIM] = wrap_period(r[j * DIM + i % DIM] + dt * ur, 2.0 * 3.14159265358979323846);
       }
     }
     __syncthreads();  // before the next tile's tables

@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "l3es_internal.h"
+#include "particle_kernels.cuh"
 
 namespace l3es {
 
@@ -40,7 +41,6 @@ constexpr int kSphLanes = 8;
 
 struct SphGeom {
   double L;      // box side
-  double inv_L;
   double inv_cs; // cells per unit length (nc / L)
   double cs_d;   // cell side L / nc (cell origins; nc * cs_d == L up to FP64 rounding)
   float cs;      // cell side (stencil offsets)
@@ -49,19 +49,6 @@ struct SphGeom {
   float inv_h;   // 1 / dx
   float cut2;    // (3 dx)^2
 };
-
-// position wrapped into [0, L), as the periodic shift of integrator.py:21-23 leaves it
-// (floor(x / L) from x times 1 / L where that cannot differ: an FP64 division is some twenty
-// instructions at two a clock and SM here)
-__device__ __forceinline__ double floor_quotient(double x, const SphGeom& g) {
-  const double q = x * g.inv_L, f = floor(q), d = q - f;
-  if (d > 1e-9 && d < 1.0 - 1e-9 && fabs(q) < 1e6) return f;
-  return floor(x / g.L);
-}
-__device__ __forceinline__ double wrap_box(double x, const SphGeom& g) {
-  x = x - g.L * floor_quotient(x, g);
-  return x >= g.L ? x - g.L : x;
-}
 
 __device__ __forceinline__ int cell_coord(double x, const SphGeom& g) {
   int c = (int)(x * g.inv_cs);
@@ -102,7 +89,7 @@ k_sph_bin(const double* __restrict__ r, const double* __restrict__ u, double dt,
   for (int d = 0; d < DIM; ++d) {
     double x = r[j * DIM + d];
     if (u) x += dt * u[j * DIM + d];
-    x = wrap_box(x, g);
+    x = wrap_period(x, g.L);
     xw[j * DIM + d] = x;
     ci[d] = cell_coord(x, g);
   }
@@ -177,7 +164,9 @@ k_sph_order(const int* __restrict__ perm0, const int* __restrict__ cell, const i
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
     const double x = xw[(long long)j * DIM + d];
-    loc[d] = (float)(x - (double)cell_coord(x, g) * g.cs_d);
+    // its cell on axis d
+    const int q = d == DIM - 1 ? c % g.nc : d == DIM - 2 ? c / g.nc % g.nc : c / (g.nc * g.nc);
+    loc[d] = (float)(x - (double)q * g.cs_d);
   }
   xs[t] = make_float4(loc[0], loc[1], loc[2], 0.f);
   if (us) {
@@ -411,8 +400,8 @@ __device__ __forceinline__ int3 slot_cell(long long i, const int* __restrict__ p
 // and 4-7 of a value by a thread each, instead of every lane adding every value; the
 // acceleration pass' wraps and divisions follow with a thread per particle and component (a
 // lane per particle made each warp run them three times for four live lanes). With the cells
-// read instead of formed again from FP64 positions, and floor_quotient: a relaxation call of
-// 32^3 particles 175 -> 125 us, 160^2 (2D) 83 -> 50.
+// read instead of formed again from FP64 positions, and the wraps' quotients made only where
+// they are not zero: a relaxation call of 32^3 particles 175 -> 118 us, 160^2 (2D) 83 -> 47.
 constexpr int kSphGroup = kSphThreads / kSphLanes;  // particles per block
 template <int F>
 struct SphSums {
@@ -569,13 +558,11 @@ __global__ void __launch_bounds__(kSphThreads) k_sph_accel(SphAccelArgs a, SphGe
     } else if (MODE == kSphRelaxVel) {
       // r_temp <- shift(r_temp, kick * acc); u = displacement(r_temp, r0) / dt, with the
       // periodic displacement mod(d + L/2, L) - L/2; optionally r_out = shift(r0, dt u)
-      const double x = wrap_box(a.xw[j * DIM + d] + a.kick * ap, g);
-      double dd = x - a.r0[j * DIM + d] + 0.5 * g.L;
-      dd = dd - g.L * floor_quotient(dd, g);
-      if (dd >= g.L) dd -= g.L;
+      const double x = wrap_period(a.xw[j * DIM + d] + a.kick * ap, g.L);
+      const double dd = wrap_period(x - a.r0[j * DIM + d] + 0.5 * g.L, g.L);
       const double uv = (dd - 0.5 * g.L) / a.dt;
       a.out0[j * DIM + d] = uv;
-      if (a.out1) a.out1[j * DIM + d] = wrap_box(a.r0[j * DIM + d] + a.dt * uv, g);
+      if (a.out1) a.out1[j * DIM + d] = wrap_period(a.r0[j * DIM + d] + a.dt * uv, g.L);
     } else {
       (f < DIM ? a.out0 : f < 2 * DIM ? a.out1 : a.out2)[j * DIM + d] = ap;
     }
@@ -714,7 +701,6 @@ int l3es_sph_plan_create(int32_t dim, int32_t n, double box, int64_t np_max, l3e
   int nc = n / 3;  // cell side L / nc >= cutoff 3 dx
   if (nc < 3) nc = 1;
   p->g.L = box;
-  p->g.inv_L = 1.0 / box;
   p->g.nc = nc;
   p->g.inv_cs = nc / box;
   p->g.cs_d = box / nc;
