@@ -275,8 +275,8 @@ struct DnsOps {
     // (block 0 of each trajectory also computes the constant-power coefficient of us)
     bool band_done = false;
     // by default at 256^3: smaller grids have too few band tiles per persistent CTA to
-    // pipeline (measured at 128^3: 9.5 us persistent vs 8.4 us one-shot), at 512^3 a CTA
-    // fills its SM either way (a band-fused step 20.5 ms persistent, 20.1 ms one-shot)
+    // pipeline (a band-fused step at 128^3: 309 us persistent, 286 us one-shot), at 512^3 a
+    // CTA fills its SM either way (20.1 ms persistent, 19.7 ms one-shot; 256^3 2053, 2069 us)
     if constexpr (DIM == 3 && N >= 64) {
       const bool bulk = c.sched.band_bulk < 0 ? N == 256 : c.sched.band_bulk != 0;
       CUtensorMap map;

@@ -240,7 +240,7 @@ int l3es_plan_create(const l3es_plan_desc* desc, l3es_plan** out) {
   c.kt = ((c.kd + 1 + TW - 1) / TW) * TW;
   if (n == 256) c.sched.line_pair = 3;  // the staged radix-16 line pass (measured best at 256)
   // y pass: radix 16 at 256^3 (a step 2055 us against 2153 us with radix 8), radix 8 at
-  // 128^3 (283 against 292 us) and 512^3 (20.07 against 20.30 ms before the paired adds)
+  // 128^3 (286 against 294 us) and 512^3 (19.67 against 19.97 ms)
   c.sched.y_var = dim == 3 && (n == 128 || n == 512);
   // the stage combination inside the x passes (in 2D forms 1 and 2 both are kx_stage)
   c.step_form = dim == 3 ? 2 : 1;
