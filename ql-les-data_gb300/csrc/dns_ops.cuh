@@ -68,6 +68,8 @@ struct DnsOps {
     if constexpr (N >= 16 && N <= kStageMax3d) {
       stage_attrs<3>();
       cudaFuncSetAttribute(k_yz_plane<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, YzCfg<N>::SMEM);
+      if constexpr (N >= 32)
+        cudaFuncSetAttribute(k_yz_half<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, YzHalfCfg<N>::SMEM);
       cudaGetLastError();
     }
   }
@@ -348,11 +350,19 @@ struct DnsOps {
                                                                   c.band));
     }
     using K = Stage<DIM>;
-    const XStage st{c.cs, c.kd, c.kt, prm, c.band, c.nu_b, c.err};
+    const XStage st{c.cs, c.kd, c.kt, prm, c.band, c.nu_b, c.err, DIM == 3 && yz_half(c)};
     const dim3 g((unsigned)((c.nmid * H + XS<DIM> - 1) / XS<DIM>), c.batch);
     L3ES_LAUNCH(c, KK_X_STAGE, b, s,
                 pdl_launch(kx_stage<N, DIM, XS<DIM>, ES<DIM>, RK, INV>, g, K::THREADS, K::SMEM, s, c.DU, c.ds, S,
                            c.Tb, c.C, st, c.W, c.Wx, c.fs, c.tw));
+  }
+
+  // Whether two CTAs share a plane between two kx_stage launches (k_yz_half): while the
+  // doubled grid still has an SM per CTA. Ten steps, one CTA per plane and two: 64^3 664 and
+  // 521 us, 32^3 347 and 332, 32^3 x 2 423 and 410; above, 64^3 x 2 823 and 916, 32^3 x 4 473
+  // and 495 (16^3 has too few rows for a warp).
+  static bool yz_half(const Ctx& c) {
+    return c.dim == 3 && N >= 32 && N <= kStageMax3d && 2LL * N * c.batch <= 152;
   }
 
   // W -> DU between two kx_stage launches: in 3D one kernel per x plane
@@ -361,6 +371,15 @@ struct DnsOps {
     if constexpr (DIM == 3 && N >= 16 && N <= kStageMax3d) {
       const double A = 8.0 * 3.0 * c.cs * c.batch, Adu = 8.0 * 3.0 * c.ds * c.batch;
       const float scale = (float)(1.0 / ((double)N * N * N));
+      if constexpr (N >= 32) {
+        if (yz_half(c)) {
+          L3ES_LAUNCH(c, KK_YZ_PLANE, 5.0 / 3.0 * A + Adu, s,
+                      pdl_launch(k_yz_half<N>, dim3(2 * N, c.batch), YzHalfCfg<N>::THREADS, YzHalfCfg<N>::SMEM, s, c.W,
+                                 c.Wx, c.fs, c.DU, c.ds, c.kt, c.kd, 0.5f * scale * scale, c.tw,
+                                 c.tw + line2_ct_offset<N>()));
+          return;
+        }
+      }
       L3ES_LAUNCH(c, KK_YZ_PLANE, 5.0 / 3.0 * A + Adu * (2.0 * c.kd + 1.0) / N, s,
                   pdl_launch(k_yz_plane<N>, dim3(N, c.batch), YzCfg<N>::THREADS, YzCfg<N>::SMEM, s, c.W, c.Wx, c.fs,
                              c.DU, c.ds, c.kt, c.kd, 0.5f * scale * scale, c.tw, c.tw + line2_ct_offset<N>()));

@@ -28,7 +28,7 @@ namespace l3es {
 // 98.3 -> 69.7 us, 128^2 x 8 98.4 -> 70.6 us, 512^2 122.9 -> 97.7 us; 3D, dependent launches
 // on both sides, 64^3 89 -> 71 us, 64^3 x 6 222 -> 208 us, 64^3 x 12 425 -> 423 us; from
 // plain launches 32^3 121 -> 35 us, 16^3 130 -> 41 us. (With dependent launches, paired adds
-// and the line passes of their size those steps now take 48, 42 and 68 us.) With kx_stage 128^3 takes 38 instead
+// and the line passes of their size those steps now take 48, 42 and 52 us.) With kx_stage 128^3 takes 38 instead
 // of 32.6 us for one stage's x passes and 256^3 267 instead of 195 us: there the chip is full
 // and the barriers of the three groups cost more than the saved round trip. Larger 3D grids
 // keep kx_inv and the band-fused kx_fwd_band.
@@ -43,6 +43,7 @@ struct XStage {
   const double* band_scale;  // [batch] constant-power coefficient of the stage's input field
   const float* nu_b;         // [batch] viscosities
   int* err;
+  int half = 0;              // 3D: du holds the halves of the y transform (k_yz_half)
 };
 
 // XW columns per CTA and one thread group per velocity component, XW T threads each
@@ -113,10 +114,17 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
     }
     if (tile_band) {
       // nonlinear term: x forward, dealias, Leray projection of this component
-      const float2* db = du + ((long long)batch * 3 + g) * dcs + (long long)mid * kt + kh;
+      const bool half = DIM == 3 && st.half;
+      const float2* db = du + ((long long)batch * 3 + g) * dcs + (long long)(half ? mid % (N / 2) : mid) * kt + kh;
 #pragma unroll
-      for (int e = 0; e < E; ++e)
-        v[e] = colband ? __ldg(db + (long long)(t + T * e) * NMID * kt) : make_float2(0.f, 0.f);
+      for (int e = 0; e < E; ++e) {
+        const float2* d = db + (long long)(t + T * e) * NMID * kt;
+        v[e] = colband ? __ldg(d) : make_float2(0.f, 0.f);
+        if (half && colband) {
+          const float2 o = __ldg(d + N / 2 * kt);
+          v[e] = mid < N / 2 ? cadd(v[e], o) : csub(v[e], o);
+        }
+      }
       block_fft<N, E, kFwd, XW, K::SYNC>(v, sx + p, t, tw, 1);
 #pragma unroll
       for (int e = 0; e < E; ++e) su[g * K::US + (t + T * e) * XW + p] = v[e];
@@ -326,17 +334,17 @@ __device__ __forceinline__ void c2r_pair_row(const float2* X, const float2* Y, i
 
 // Half-axis lines of a plane in shared memory (six fields, rows of LD): u x curl u of every
 // row into the first kt columns of fields 0..2. Slot y of T lanes takes row y; the z
-// products of rows y and y + N/2 share one transform. All threads; xs: the warp's exchange
+// products of rows y and y + ROWS/2 share one transform. All threads; xs: the warp's exchange
 // buffer.
-template <int N>
+template <int N, int ROWS = N>
 __device__ __forceinline__ void plane_lines(float2* s_yz, float2* xs, int kt, int kd, float s2,
                                             const float2* __restrict__ ct8) {
   using C = YzCfg<N>;
-  constexpr int T = C::T, LD = C::LD;
+  constexpr int T = C::T, LD = C::LD, FIELD = ROWS * LD;
   const int lane = threadIdx.x & 31;
   const int y = threadIdx.x / T, t = threadIdx.x % T;
   float2* xl = xs + lane / T * xpad_len<1>(N);
-  float2* row = s_yz + (y < N ? y : 0) * LD;
+  float2* row = s_yz + (y < ROWS ? y : 0) * LD;
   float pz[8];
   auto put = [&](float2* dst, const float2 (&X)[4]) {
 #pragma unroll
@@ -345,19 +353,19 @@ __device__ __forceinline__ void plane_lines(float2* s_yz, float2* xs, int kt, in
       if (k < kt) dst[k] = k <= kd ? X[e] : make_float2(0.f, 0.f);
     }
   };
-  if (y < N) {  // whole warps
+  if (y < ROWS) {  // whole warps
     float2 h1[8], h2[8], z[8];
-    c2r_pair_row<N>(row, row + C::FIELD, t, z);  // u_x + i u_y
+    c2r_pair_row<N>(row, row + FIELD, t, z);  // u_x + i u_y
     warp_fft<N, 8, kInv>(z, xl, t, ct8);
 #pragma unroll
     for (int e = 0; e < 8; ++e) h1[e] = z[e];
     __syncwarp();
-    c2r_pair_row<N>(row + 2 * C::FIELD, row + 3 * C::FIELD, t, z);  // u_z + i curl_x
+    c2r_pair_row<N>(row + 2 * FIELD, row + 3 * FIELD, t, z);  // u_z + i curl_x
     warp_fft<N, 8, kInv>(z, xl, t, ct8);
 #pragma unroll
     for (int e = 0; e < 8; ++e) h2[e] = z[e];
     __syncwarp();
-    c2r_pair_row<N>(row + 4 * C::FIELD, row + 5 * C::FIELD, t, z);  // curl_y + i curl_z
+    c2r_pair_row<N>(row + 4 * FIELD, row + 5 * FIELD, t, z);  // curl_y + i curl_z
     warp_fft<N, 8, kInv>(z, xl, t, ct8);
     __syncwarp();
 #pragma unroll
@@ -371,17 +379,17 @@ __device__ __forceinline__ void plane_lines(float2* s_yz, float2* xs, int kt, in
     r2c_pair_unpack<N>(z, t, s2, X, Y);
     // this line's rows are read: they take its products
     put(row, X);
-    put(row + C::FIELD, Y);
-    if (y >= N / 2) {
-      float* zr = reinterpret_cast<float*>(row + 3 * C::FIELD);
+    put(row + FIELD, Y);
+    if (y >= ROWS / 2) {
+      float* zr = reinterpret_cast<float*>(row + 3 * FIELD);
 #pragma unroll
       for (int e = 0; e < 8; ++e) zr[t + T * e] = pz[e];
     }
   }
   __syncthreads();
-  if (y < N / 2 || (N / 2 * T < 32 && y < N)) {  // whole warps
-    const bool lower = y < N / 2;
-    const float* zr = reinterpret_cast<const float*>(s_yz + 3 * C::FIELD + (lower ? y + N / 2 : y) * LD);
+  if (y < ROWS / 2 || (ROWS / 2 * T < 32 && y < ROWS)) {  // whole warps
+    const bool lower = y < ROWS / 2;
+    const float* zr = reinterpret_cast<const float*>(s_yz + 3 * FIELD + (lower ? y + ROWS / 2 : y) * LD);
     float2 z[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) z[e] = make_float2(pz[e], zr[t + T * e]);
@@ -389,8 +397,8 @@ __device__ __forceinline__ void plane_lines(float2* s_yz, float2* xs, int kt, in
     float2 X[4], Y[4];
     r2c_pair_unpack<N>(z, t, s2, X, Y);
     if (lower) {
-      put(row + 2 * C::FIELD, X);
-      put(row + 2 * C::FIELD + N / 2 * LD, Y);
+      put(row + 2 * FIELD, X);
+      put(row + 2 * FIELD + ROWS / 2 * LD, Y);
     }
   }
 }
@@ -461,6 +469,109 @@ k_yz_plane(const float2* __restrict__ w, const float2* __restrict__ wx, long lon
           const int ky = t + T * e;
           if ((unsigned)(kfull(ky, N) + kd) <= 2u * (unsigned)kd) db[c * ds + (long long)ky * kt + col] = v[e];
         }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------
+// k_yz_plane with a plane shared by two CTAs, one for the even rows y and one for the odd: the
+// inverse y transform gives a CTA its rows from one N/2-point transform of the folded columns
+// (V[k] + V[k + N/2], or their difference turned by exp(2 pi i k / N)), the lines of its rows
+// need nothing else, and the halves of the forward transform meet where kx_stage reads them:
+//   X[k] = E[k] + exp(-2 pi i k / N) O[k],  X[k + N/2] = E[k] - exp(-2 pi i k / N) O[k],
+// E and the turned O in rows k and N/2 + k of du (XStage::half). Twice the CTAs, for launches
+// that leave SMs idle. Bound by latency: the 16 loads of a column stay unbranched so that
+// they are in flight together, and a CTA has twice the warps that the lines need, for the
+// columns (ten 64^3 steps 705 us with half of them, 521 us).
+// ------------------------------------------------------------------------------
+template <int N>
+struct YzHalfCfg {
+  static constexpr int R = N / 2;                 // rows of a CTA
+  static constexpr int T = R / 8;                 // lanes per y transform
+  static constexpr int XC = 32 / T;               // columns per warp
+  static constexpr int THREADS = 2 * R * YzCfg<N>::T;  // twice a slot per row
+  static constexpr int WARPS = THREADS / 32;
+  static constexpr int FIELD = R * YzCfg<N>::LD;
+  static constexpr int XSC = XC * xpad_len<XC>(R);
+  static constexpr int XS = YzCfg<N>::XS1 > XSC ? YzCfg<N>::XS1 : XSC;
+  static constexpr int SMEM = (6 * FIELD + WARPS * XS) * (int)sizeof(float2);
+};
+
+template <int N>
+__global__ void __launch_bounds__(YzHalfCfg<N>::THREADS)
+k_yz_half(const float2* __restrict__ w, const float2* __restrict__ wx, long long fs, float2* __restrict__ du,
+          long long ds, int kt, int kd, float s2, const float2* __restrict__ tw, const float2* __restrict__ ct8) {
+  pdl_begin();
+  using C = YzHalfCfg<N>;
+  constexpr int R = C::R, T = C::T, XC = C::XC, H = YzCfg<N>::H, LD = YzCfg<N>::LD;
+  extern __shared__ __align__(16) float2 s_yz[];
+  const int odd = blockIdx.x & 1, x = blockIdx.x / 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int p = lane % XC, t = lane / XC;
+  float2* xs = s_yz + 6 * C::FIELD + warp * C::XS;
+  {
+    const long long plane = (long long)x * N * H;
+    const float2* wb = w + (long long)blockIdx.y * 6 * fs + plane;
+    const float2* xb = wx + (long long)blockIdx.y * 2 * fs + plane;
+    constexpr int TILES = (H + XC - 1) / XC;
+    for (int j = warp; j < 6 * TILES; j += C::WARPS) {
+      const int f = j % 6, col = j / 6 * XC + p;
+      const bool ok = col < H;
+      float2 v[8], b[8];
+      if (f == 3) {
+        const float kz = (float)col;
+        float2 y[16], z[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const int o = (t + T * (e & 7) + R * (e >> 3)) * H + col;
+          y[e] = ok ? __ldg(xb + o) : make_float2(0.f, 0.f);
+          z[e] = ok ? __ldg(xb + fs + o) : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const float ky = (float)kfull(t + T * (e & 7) + R * (e >> 3), N);
+          (e < 8 ? v[e & 7] : b[e & 7]) =
+              mul_i<kInv>(make_float2(ky * z[e].x - kz * y[e].x, ky * z[e].y - kz * y[e].y));
+        }
+      } else {
+        const float2* src = f == 1 || f == 2 ? xb + (f - 1) * fs : wb + f * fs;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = ok ? __ldg(src + (t + T * e) * H + col) : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) b[e] = ok ? __ldg(src + (t + T * e + R) * H + col) : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        v[e] = odd ? cmul(csub(v[e], b[e]), twid<kInv>(tw, t + T * e)) : cadd(v[e], b[e]);
+      block_fft<R, 8, kInv, XC, kSyncWarp>(v, xs + p, t, tw, 2);
+      if (ok) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s_yz[f * C::FIELD + (t + T * e) * LD + col] = v[e];
+      }
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  plane_lines<N, R>(s_yz, xs, kt, kd, s2, ct8);
+  __syncthreads();
+  // y forward of this CTA's rows, kept columns
+  {
+    float2* db = du + (long long)blockIdx.y * 3 * ds + ((long long)x * N + odd * R) * kt;
+    const int tiles = (kt + XC - 1) / XC;
+    for (int j = warp; j < 3 * tiles; j += C::WARPS) {
+      const int c = j % 3, col = j / 3 * XC + p;
+      const bool ok = col < kt;
+      float2 v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        v[e] = ok ? s_yz[c * C::FIELD + (t + T * e) * LD + col] : make_float2(0.f, 0.f);
+      block_fft<R, 8, kFwd, XC, kSyncWarp>(v, xs + p, t, tw, 2);
+      if (ok) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          db[c * ds + (long long)(t + T * e) * kt + col] = odd ? cmul(v[e], twid<kFwd>(tw, t + T * e)) : v[e];
       }
       __syncwarp();
     }

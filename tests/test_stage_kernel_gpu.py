@@ -28,7 +28,8 @@ def _initial(dim, n, seed):
     (3, 16, 1, "const_power"), (3, 32, 2, "none"), (3, 32, 1, "ekin_tot"), (3, 64, 4, "const_power"),
     (3, 64, 5, "none"), (2, 16, 3, "kolmogorov"), (2, 32, 1, "const_power"), (2, 64, 1, "ekin_tot"),
     (2, 128, 2, "kolmogorov"), (2, 512, 1, "kolmogorov"),
-    (2, 256, 1, "kolmogorov"), (2, 256, 4, "none"), (2, 256, 5, "none")])
+    (2, 256, 1, "kolmogorov"), (2, 256, 4, "none"), (2, 256, 5, "none"),
+    (3, 64, 1, "const_power"), (3, 64, 2, "none"), (3, 32, 3, "none")])
 def test_steps_match_the_oracle(dim, n, batch, forcing):
     axes = (1, 2, 3) if dim == 3 else (1, 2)
     nu, dt, drag = 5e-3, 2e-3 if dim == 3 else 1e-3, 0.1 if forcing == "kolmogorov" else 0.0
