@@ -67,9 +67,12 @@ struct DnsOps {
     }
     if constexpr (N >= 16 && N <= kStageMax3d) {
       stage_attrs<3>();
-      cudaFuncSetAttribute(k_yz_plane<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, YzCfg<N>::SMEM);
-      if constexpr (N >= 32)
-        cudaFuncSetAttribute(k_yz_half<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, YzHalfCfg<N>::SMEM);
+      if constexpr (yz_by_halves(N)) {
+        cudaFuncSetAttribute(k_yz_half<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, YzHalfCfg<N, 1>::SMEM);
+        cudaFuncSetAttribute(k_yz_half<N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, YzHalfCfg<N, 2>::SMEM);
+      } else {
+        cudaFuncSetAttribute(k_yz_plane<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, YzCfg<N>::SMEM);
+      }
       cudaGetLastError();
     }
   }
@@ -350,7 +353,7 @@ struct DnsOps {
                                                                   c.band));
     }
     using K = Stage<DIM>;
-    const XStage st{c.cs, c.kd, c.kt, prm, c.band, c.nu_b, c.err, DIM == 3 && yz_half(c)};
+    const XStage st{c.cs, c.kd, c.kt, prm, c.band, c.nu_b, c.err};
     const dim3 g((unsigned)((c.nmid * H + XS<DIM> - 1) / XS<DIM>), c.batch);
     L3ES_LAUNCH(c, KK_X_STAGE, b, s,
                 pdl_launch(kx_stage<N, DIM, XS<DIM>, ES<DIM>, RK, INV>, g, K::THREADS, K::SMEM, s, c.DU, c.ds, S,
@@ -358,12 +361,10 @@ struct DnsOps {
   }
 
   // Whether two CTAs share a plane between two kx_stage launches (k_yz_half): while the
-  // doubled grid still has an SM per CTA. Ten steps, one CTA per plane and two: 64^3 664 and
-  // 521 us, 32^3 347 and 332, 32^3 x 2 423 and 410; above, 64^3 x 2 823 and 916, 32^3 x 4 473
-  // and 495 (16^3 has too few rows for a warp).
-  static bool yz_half(const Ctx& c) {
-    return c.dim == 3 && N >= 32 && N <= kStageMax3d && 2LL * N * c.batch <= 152;
-  }
+  // doubled grid still has an SM per CTA. Ten steps with one CTA per plane and with two:
+  // 64^3 664 and 532 us, 32^3 347 and 322, 32^3 x 2 423 and 371; above that two lose, 64^3 x 2
+  // 808 and 916, 32^3 x 4 488 and 495.
+  static bool two_ctas(const Ctx& c) { return 2LL * N * c.batch <= 152; }
 
   // W -> DU between two kx_stage launches: in 3D one kernel per x plane
   template <int DIM>
@@ -371,18 +372,25 @@ struct DnsOps {
     if constexpr (DIM == 3 && N >= 16 && N <= kStageMax3d) {
       const double A = 8.0 * 3.0 * c.cs * c.batch, Adu = 8.0 * 3.0 * c.ds * c.batch;
       const float scale = (float)(1.0 / ((double)N * N * N));
-      if constexpr (N >= 32) {
-        if (yz_half(c)) {
-          L3ES_LAUNCH(c, KK_YZ_PLANE, 5.0 / 3.0 * A + Adu, s,
-                      pdl_launch(k_yz_half<N>, dim3(2 * N, c.batch), YzHalfCfg<N>::THREADS, YzHalfCfg<N>::SMEM, s, c.W,
-                                 c.Wx, c.fs, c.DU, c.ds, c.kt, c.kd, 0.5f * scale * scale, c.tw,
-                                 c.tw + line2_ct_offset<N>()));
-          return;
-        }
+      const double bytes = 5.0 / 3.0 * A + Adu * (yz_by_halves(N) ? 1.0 : (2.0 * c.kd + 1.0) / N);
+      const float2* ct = c.tw + line2_ct_offset<N>();
+      const float s2 = 0.5f * scale * scale;
+      if constexpr (yz_by_halves(N)) {
+        using Y1 = YzHalfCfg<N, 1>;
+        using Y2 = YzHalfCfg<N, 2>;
+        if (two_ctas(c))
+          L3ES_LAUNCH(c, KK_YZ_PLANE, bytes, s,
+                      pdl_launch(k_yz_half<N, 2>, dim3(2 * N, c.batch), Y2::THREADS, Y2::SMEM, s, c.W, c.Wx, c.fs,
+                                 c.DU, c.ds, c.kt, c.kd, s2, c.tw, ct));
+        else
+          L3ES_LAUNCH(c, KK_YZ_PLANE, bytes, s,
+                      pdl_launch(k_yz_half<N, 1>, dim3(N, c.batch), Y1::THREADS, Y1::SMEM, s, c.W, c.Wx, c.fs, c.DU,
+                                 c.ds, c.kt, c.kd, s2, c.tw, ct));
+      } else {
+        L3ES_LAUNCH(c, KK_YZ_PLANE, bytes, s,
+                    pdl_launch(k_yz_plane<N>, dim3(N, c.batch), YzCfg<N>::THREADS, YzCfg<N>::SMEM, s, c.W, c.Wx, c.fs,
+                               c.DU, c.ds, c.kt, c.kd, s2, c.tw, ct));
       }
-      L3ES_LAUNCH(c, KK_YZ_PLANE, 5.0 / 3.0 * A + Adu * (2.0 * c.kd + 1.0) / N, s,
-                  pdl_launch(k_yz_plane<N>, dim3(N, c.batch), YzCfg<N>::THREADS, YzCfg<N>::SMEM, s, c.W, c.Wx, c.fs,
-                             c.DU, c.ds, c.kt, c.kd, 0.5f * scale * scale, c.tw, c.tw + line2_ct_offset<N>()));
     } else if constexpr (DIM == 2 && N >= 16 && N <= 128) {
       const double A = 8.0 * 3.0 * c.cs * c.batch, Adu = 8.0 * 3.0 * c.ds * c.batch;
       const float scale = (float)(1.0 / ((double)N * N));

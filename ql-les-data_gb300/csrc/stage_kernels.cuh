@@ -6,7 +6,7 @@
 // the next stage's inverse x FFT of u and curl u all act on the same column of modes, so
 // kx_stage does them in one visit: the new stage field goes from the combination into
 // the inverse transform without a trip through memory, and a stage is two launches
-// (kx_stage and in 2D the line pass, in 3D k_yz_plane).
+// (kx_stage and in 2D the line pass, in 3D k_yz_plane or k_yz_half).
 //
 // The band B = {|kx| <= kd, |kmid| <= kd (3D), khalf < kt} holds every nonlinear and
 // forcing term. Outside it du = -(nu k^2 + drag) u exactly, so a stage field there is a
@@ -28,12 +28,16 @@ namespace l3es {
 // 98.3 -> 69.7 us, 128^2 x 8 98.4 -> 70.6 us, 512^2 122.9 -> 97.7 us; 3D, dependent launches
 // on both sides, 64^3 89 -> 71 us, 64^3 x 6 222 -> 208 us, 64^3 x 12 425 -> 423 us; from
 // plain launches 32^3 121 -> 35 us, 16^3 130 -> 41 us. (With dependent launches, paired adds
-// and the line passes of their size those steps now take 48, 42 and 52 us.) With kx_stage 128^3 takes 38 instead
+// and the line passes of their size those steps now take 47, 42 and 53 us.) With kx_stage 128^3 takes 38 instead
 // of 32.6 us for one stage's x passes and 256^3 267 instead of 195 us: there the chip is full
 // and the barriers of the three groups cost more than the saved round trip. Larger 3D grids
 // keep kx_inv and the band-fused kx_fwd_band.
 constexpr int kStageMax3d = 64;  // largest 3D grid with kx_stage kernels
 inline bool step_by_kx_stage(int dim, int n) { return dim == 2 || n <= kStageMax3d; }
+
+// 3D grids whose y transforms between two x passes go by halves (k_yz_half; 16^3 has too few
+// rows for a warp and takes k_yz_plane)
+constexpr bool yz_by_halves(int n) { return n >= 32 && n <= kStageMax3d; }
 
 // Parameters of one stage.
 struct XStage {
@@ -43,7 +47,6 @@ struct XStage {
   const double* band_scale;  // [batch] constant-power coefficient of the stage's input field
   const float* nu_b;         // [batch] viscosities
   int* err;
-  int half = 0;              // 3D: du holds the halves of the y transform (k_yz_half)
 };
 
 // XW columns per CTA and one thread group per velocity component, XW T threads each
@@ -114,7 +117,7 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
     }
     if (tile_band) {
       // nonlinear term: x forward, dealias, Leray projection of this component
-      const bool half = DIM == 3 && st.half;
+      constexpr bool half = DIM == 3 && yz_by_halves(N);  // du holds the halves of the y transform
       const float2* db = du + ((long long)batch * 3 + g) * dcs + (long long)(half ? mid % (N / 2) : mid) * kt + kh;
 #pragma unroll
       for (int e = 0; e < E; ++e) {
@@ -286,13 +289,13 @@ line_cross_slots(const float2* __restrict__ w, long long fs, float2* __restrict_
 }
 
 // ------------------------------------------------------------------------------
-// Everything between two x passes of a small 3D grid in one kernel, one x plane per CTA:
-// y inverse of the six fields (u, curl u; curl_x formed here, as in ky_inv_rhs), the
-// half-axis lines with u x curl u (two real lines per complex FFT, as in line_cross2) and
-// the y forward of the three products, kept rows only, to du. At 64^3 the plane's six
-// fields are 123 KB of shared memory, so the three passes meet there instead of in global
-// memory, in one launch instead of three. Warps work alone inside a phase: a warp takes 32
-// / T neighbouring columns (y transforms) or 32 / T lines, T = N / 8 lanes each.
+// Everything between two x passes of a small 3D grid in one kernel, one x plane per CTA (16^3;
+// 32^3 and 64^3 take k_yz_half): y inverse of the six fields (u, curl u; curl_x formed here,
+// as in ky_inv_rhs), the half-axis lines with u x curl u (two real lines per complex FFT, as
+// in line_cross2) and the y forward of the three products, kept rows only, to du. A plane's
+// six fields (123 KB at 64^3) fit shared memory, so the three passes meet there instead of in
+// global memory, in one launch instead of three. Warps work alone inside a phase: a warp
+// takes 32 / T neighbouring columns (y transforms) or 32 / T lines, T = N / 8 lanes each.
 // ct8: compact twiddle table of the N-point FFT (line2_ct_offset).
 // ------------------------------------------------------------------------------
 template <int N>
@@ -334,9 +337,9 @@ __device__ __forceinline__ void c2r_pair_row(const float2* X, const float2* Y, i
 
 // Half-axis lines of a plane in shared memory (six fields, rows of LD): u x curl u of every
 // row into the first kt columns of fields 0..2. Slot y of T lanes takes row y; the z
-// products of rows y and y + ROWS/2 share one transform. All threads; xs: the warp's exchange
+// products of rows y and y + PB/2 of a block of PB rows share one transform. All threads; xs: the warp's exchange
 // buffer.
-template <int N, int ROWS = N>
+template <int N, int ROWS = N, int PB = ROWS>
 __device__ __forceinline__ void plane_lines(float2* s_yz, float2* xs, int kt, int kd, float s2,
                                             const float2* __restrict__ ct8) {
   using C = YzCfg<N>;
@@ -380,16 +383,16 @@ __device__ __forceinline__ void plane_lines(float2* s_yz, float2* xs, int kt, in
     // this line's rows are read: they take its products
     put(row, X);
     put(row + FIELD, Y);
-    if (y >= ROWS / 2) {
+    if (y % PB >= PB / 2) {
       float* zr = reinterpret_cast<float*>(row + 3 * FIELD);
 #pragma unroll
       for (int e = 0; e < 8; ++e) zr[t + T * e] = pz[e];
     }
   }
   __syncthreads();
-  if (y < ROWS / 2 || (ROWS / 2 * T < 32 && y < ROWS)) {  // whole warps
-    const bool lower = y < ROWS / 2;
-    const float* zr = reinterpret_cast<const float*>(s_yz + 3 * FIELD + (lower ? y + ROWS / 2 : y) * LD);
+  if (y < ROWS && (y % PB < PB / 2 || PB / 2 * T < 32)) {  // whole warps
+    const bool lower = y % PB < PB / 2;
+    const float* zr = reinterpret_cast<const float*>(s_yz + 3 * FIELD + (lower ? y + PB / 2 : y) * LD);
     float2 z[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) z[e] = make_float2(pz[e], zr[t + T * e]);
@@ -398,7 +401,7 @@ __device__ __forceinline__ void plane_lines(float2* s_yz, float2* xs, int kt, in
     r2c_pair_unpack<N>(z, t, s2, X, Y);
     if (lower) {
       put(row + 2 * FIELD, X);
-      put(row + 2 * FIELD + ROWS / 2 * LD, Y);
+      put(row + 2 * FIELD + PB / 2 * LD, Y);
     }
   }
 }
@@ -481,33 +484,36 @@ k_yz_plane(const float2* __restrict__ w, const float2* __restrict__ wx, long lon
 // (V[k] + V[k + N/2], or their difference turned by exp(2 pi i k / N)), the lines of its rows
 // need nothing else, and the halves of the forward transform meet where kx_stage reads them:
 //   X[k] = E[k] + exp(-2 pi i k / N) O[k],  X[k + N/2] = E[k] - exp(-2 pi i k / N) O[k],
-// E and the turned O in rows k and N/2 + k of du (XStage::half). Twice the CTAs, for launches
-// that leave SMs idle. Bound by latency: the 16 loads of a column stay unbranched so that
+// E and the turned O in rows k and N/2 + k of du. Twice the CTAs, for launches that leave SMs
+// idle. Bound by latency: the 16 loads of a column stay unbranched so that
 // they are in flight together, and a CTA has twice the warps that the lines need, for the
-// columns (ten 64^3 steps 705 us with half of them, 521 us).
+// columns (ten 64^3 steps 705 us with half of them, 532 us; 676 us by k_yz_plane).
 // ------------------------------------------------------------------------------
-template <int N>
+template <int N, int CTAS>
 struct YzHalfCfg {
-  static constexpr int R = N / 2;                 // rows of a CTA
+  static constexpr int R = N / 2;                 // rows of a half
   static constexpr int T = R / 8;                 // lanes per y transform
   static constexpr int XC = 32 / T;               // columns per warp
-  static constexpr int THREADS = 2 * R * YzCfg<N>::T;  // twice a slot per row
+  static constexpr int ROWS = N / CTAS;
+  static constexpr int THREADS = YzCfg<N>::THREADS;  // at least a slot per row in the lines
   static constexpr int WARPS = THREADS / 32;
-  static constexpr int FIELD = R * YzCfg<N>::LD;
+  static constexpr int FIELD = ROWS * YzCfg<N>::LD;
   static constexpr int XSC = XC * xpad_len<XC>(R);
   static constexpr int XS = YzCfg<N>::XS1 > XSC ? YzCfg<N>::XS1 : XSC;
   static constexpr int SMEM = (6 * FIELD + WARPS * XS) * (int)sizeof(float2);
 };
 
-template <int N>
-__global__ void __launch_bounds__(YzHalfCfg<N>::THREADS)
+// CTAS: per plane, 2 or 1 (both halves in turn: the same arithmetic, so that a trajectory's
+// result does not depend on the batch)
+template <int N, int CTAS>
+__global__ void __launch_bounds__(YzHalfCfg<N, CTAS>::THREADS)
 k_yz_half(const float2* __restrict__ w, const float2* __restrict__ wx, long long fs, float2* __restrict__ du,
           long long ds, int kt, int kd, float s2, const float2* __restrict__ tw, const float2* __restrict__ ct8) {
   pdl_begin();
-  using C = YzHalfCfg<N>;
+  using C = YzHalfCfg<N, CTAS>;
   constexpr int R = C::R, T = C::T, XC = C::XC, H = YzCfg<N>::H, LD = YzCfg<N>::LD;
   extern __shared__ __align__(16) float2 s_yz[];
-  const int odd = blockIdx.x & 1, x = blockIdx.x / 2;
+  const int first = CTAS == 2 ? blockIdx.x & 1 : 0, x = blockIdx.x / CTAS;  // the CTA's first half
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int p = lane % XC, t = lane / XC;
   float2* xs = s_yz + 6 * C::FIELD + warp * C::XS;
@@ -543,35 +549,41 @@ k_yz_half(const float2* __restrict__ w, const float2* __restrict__ wx, long long
         for (int e = 0; e < 8; ++e) b[e] = ok ? __ldg(src + (t + T * e + R) * H + col) : make_float2(0.f, 0.f);
       }
 #pragma unroll
-      for (int e = 0; e < 8; ++e)
-        v[e] = odd ? cmul(csub(v[e], b[e]), twid<kInv>(tw, t + T * e)) : cadd(v[e], b[e]);
-      block_fft<R, 8, kInv, XC, kSyncWarp>(v, xs + p, t, tw, 2);
-      if (ok) {
+      for (int h = 0; h < 3 - CTAS; ++h) {
+        const int odd = first + h;
+        float2 z[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) s_yz[f * C::FIELD + (t + T * e) * LD + col] = v[e];
+        for (int e = 0; e < 8; ++e)
+          z[e] = odd ? cmul(csub(v[e], b[e]), twid<kInv>(tw, t + T * e)) : cadd(v[e], b[e]);
+        block_fft<R, 8, kInv, XC, kSyncWarp>(z, xs + p, t, tw, 2);
+        if (ok) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) s_yz[f * C::FIELD + (h * R + t + T * e) * LD + col] = z[e];
+        }
+        __syncwarp();
       }
-      __syncwarp();
     }
   }
   __syncthreads();
-  plane_lines<N, R>(s_yz, xs, kt, kd, s2, ct8);
+  plane_lines<N, C::ROWS, R>(s_yz, xs, kt, kd, s2, ct8);
   __syncthreads();
-  // y forward of this CTA's rows, kept columns
+  // y forward of the CTA's halves, kept columns
   {
-    float2* db = du + (long long)blockIdx.y * 3 * ds + ((long long)x * N + odd * R) * kt;
     const int tiles = (kt + XC - 1) / XC;
-    for (int j = warp; j < 3 * tiles; j += C::WARPS) {
-      const int c = j % 3, col = j / 3 * XC + p;
+    float2* db = du + (long long)blockIdx.y * 3 * ds + (long long)x * N * kt;
+    for (int j = warp; j < 3 * (3 - CTAS) * tiles; j += C::WARPS) {
+      const int c = j % 3, h = j / 3 / tiles, odd = first + h, col = j / 3 % tiles * XC + p;
       const bool ok = col < kt;
       float2 v[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e)
-        v[e] = ok ? s_yz[c * C::FIELD + (t + T * e) * LD + col] : make_float2(0.f, 0.f);
+        v[e] = ok ? s_yz[c * C::FIELD + (h * R + t + T * e) * LD + col] : make_float2(0.f, 0.f);
       block_fft<R, 8, kFwd, XC, kSyncWarp>(v, xs + p, t, tw, 2);
       if (ok) {
 #pragma unroll
         for (int e = 0; e < 8; ++e)
-          db[c * ds + (long long)(t + T * e) * kt + col] = odd ? cmul(v[e], twid<kFwd>(tw, t + T * e)) : v[e];
+          db[c * ds + (long long)(odd * R + t + T * e) * kt + col] =
+              odd ? cmul(v[e], twid<kFwd>(tw, t + T * e)) : v[e];
       }
       __syncwarp();
     }
