@@ -11,6 +11,7 @@
 // last pass of each product.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 
 #include "l3es_internal.h"
@@ -125,9 +126,12 @@ static int adj_prepare(l3es_plan* p) {
   if (w.Ua) return L3ES_OK;
   const Ctx& c = p->ctx;
   const size_t spec = sizeof(float2) * 3 * (size_t)c.cs * c.batch;
+  // Wm takes the cotangent's lines in rows of kt (ds per component) and, for ekin_tot, a
+  // whole spectrum; kt exceeds the half axis, and ds cs, at N = 8 alone
+  const size_t lines = sizeof(float2) * 3 * (size_t)std::max(c.cs, c.ds) * c.batch;
   float2** bufs[] = {&w.Ua, &w.Ub, &w.Uc, &w.Wm, &w.LAM, &w.G};
   for (float2** b : bufs) {
-    cudaError_t e = cudaMalloc((void**)b, spec);
+    cudaError_t e = cudaMalloc((void**)b, b == &w.Wm ? lines : spec);
     if (e != cudaSuccess) {
       cudaGetLastError();
       for (void* a : w.allocs) cudaFree(a);

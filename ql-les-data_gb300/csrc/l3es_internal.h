@@ -184,7 +184,7 @@ struct DnsTable {
   void (*irfftn)(const Ctx&, const float2* uh, float* u, cudaStream_t s);
   void (*rfftn)(const Ctx&, const float* u, float2* uh, cudaStream_t s);
   // vector-Jacobian product of the RHS at a.us with cotangent a.gscale * a.g, folded
-  // into the RK4 reverse recursion (AdjEpi); Wm: [batch][3][cs], Y6: [batch][6][cs]
+  // into the RK4 reverse recursion (AdjEpi); Wm: [batch][3][ds], Y6: [batch][6][cs]
   void (*vjp)(const Ctx&, const AdjEpi& a, float2* Wm, float2* Y6, cudaStream_t s);
 };
 
@@ -193,7 +193,7 @@ struct AdjWork {
   float2* Ua = nullptr;   // [batch][3][cs] RK stage states recomputed from the checkpoint
   float2* Ub = nullptr;
   float2* Uc = nullptr;
-  float2* Wm = nullptr;   // [batch][3][cs] projected cotangent lines
+  float2* Wm = nullptr;   // [batch][3][ds] projected cotangent lines; ekin_tot: a spectrum
   float2* Y6 = nullptr;   // [batch][6][cs] product spectra
   float2* LAM = nullptr;  // [batch][3][cs] accumulated cotangent
   float2* G = nullptr;    // [batch][3][cs] stage cotangent
