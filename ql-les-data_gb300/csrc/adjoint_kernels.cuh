@@ -23,11 +23,11 @@
 
 namespace l3es {
 
-// Constant-power band force derivative terms of one stage field, by all threads of
-// one block (blockDim a multiple of 32, at most 1024):
+// Constant-power band force derivative terms of one stage field, by all THREADS threads of
+// one block (8 and 16 at N = 8 and 16):
 //   s = eps / (2 E_f + tiny), c = -2 eps beta / (2 E_f + tiny)^2 / N^(2d),
 //   E_f = sum_band wt |us|^2 / (2 N^(2d)), beta = Re sum_band conj(gscale g) us.
-template <int DIM>
+template <int DIM, int THREADS>
 __device__ __forceinline__ void band_adj_terms(const float2* __restrict__ us, const float2* __restrict__ g,
                                                long long cs, float gscale, int N, int kf, double inv_n2d,
                                                double eps_inj, double* out) {
@@ -45,10 +45,8 @@ __device__ __forceinline__ void band_adj_terms(const float2* __restrict__ us, co
       beta += (double)gscale * ((double)gv.x * v.x + (double)gv.y * v.y);
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    e += __shfl_xor_sync(0xffffffffu, e, o);
-    beta += __shfl_xor_sync(0xffffffffu, beta, o);
-  }
+  e = lanes_sum<THREADS>(e);
+  beta = lanes_sum<THREADS>(beta);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   __syncthreads();
   if (lane == 0) {
@@ -58,7 +56,7 @@ __device__ __forceinline__ void band_adj_terms(const float2* __restrict__ us, co
   __syncthreads();
   if (threadIdx.x == 0) {
     double E = 0.0, B = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
+    for (int i = 0; i < (THREADS + 31) / 32; ++i) {
       E += red_e[i];
       B += red_b[i];
     }
@@ -91,7 +89,7 @@ kx_inv_adjproj(const float2* __restrict__ g, long long cs, float gscale, int kd,
   const int mid = km < 0 ? km + N : km;
   const long long bg = (long long)blockIdx.z * 3 * cs;
   if (band_kf > 0 && blockIdx.x == 0 && blockIdx.y == 0)
-    band_adj_terms<DIM>(us + bg, g + bg, cs, gscale, N, band_kf, inv_n2d, eps_inj, band_out + 2 * blockIdx.z);
+    band_adj_terms<DIM, TW * T>(us + bg, g + bg, cs, gscale, N, band_kf, inv_n2d, eps_inj, band_out + 2 * blockIdx.z);
   const float inv_wt = (kh == 0 || kh == N / 2) ? gscale : 0.5f * gscale;
   // band membership as unsigned offsets: -kd <= k <= kd  <=>  (unsigned)(k + kd) <= 2 kd
   // (the signed two-sided form was observed to keep out-of-band rows on the GPU)

@@ -112,7 +112,7 @@ struct XLin {
   double* band_scale;
 };
 
-template <int DIM>
+template <int DIM, int THREADS>
 __device__ __forceinline__ void band_coefficient(const float2* __restrict__ ub, long long cs, int N, int kf,
                                                  double inv_n2d, double eps_inj, double tiny, double* out);
 
@@ -226,8 +226,8 @@ kx_inv(const float2* __restrict__ uh, long long cs, float2* __restrict__ w, long
   const long long bofs = (long long)blockIdx.y * 3 * cs;  // batch of trajectories
   if constexpr (LINF) {
     if (xl.band_kf > 0 && blockIdx.x == 0)
-      band_coefficient<DIM>(uh + bofs, cs, N, xl.band_kf, xl.inv_n2d, xl.eps_inj, 1e-30,
-                            xl.band_scale + blockIdx.y);
+      band_coefficient<DIM, XW * T>(uh + bofs, cs, N, xl.band_kf, xl.inv_n2d, xl.eps_inj, 1e-30,
+                                    xl.band_scale + blockIdx.y);
   }
   float2 a[3][E];
 #pragma unroll
@@ -1148,9 +1148,21 @@ __device__ __forceinline__ int band_count(int kf) {
   return DIM == 3 ? (2 * kf + 1) * (2 * kf + 1) * (kf + 1) : (2 * kf + 1) * (kf + 1);
 }
 
+// Sum of v over the lanes of a warp, in every lane. A block smaller than a warp (its THREADS
+// a power of two) has no other lanes: neither named in the mask nor read.
+template <int THREADS>
+__device__ __forceinline__ double lanes_sum(double v) {
+  constexpr int L = THREADS < 32 ? THREADS : 32;
+  static_assert((L & (L - 1)) == 0 && THREADS % L == 0, "whole warps, or a power of two below one");
+  constexpr unsigned mask = L == 32 ? 0xffffffffu : (1u << L % 32) - 1u;
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+  return v;
+}
+
 // Constant-power band forcing coefficient eps / (2 E_f + tiny) of a stage field
-// (extension), computed by all threads of one block; thread 0 stores it.
-template <int DIM>
+// (extension), computed by all THREADS threads of one block; thread 0 stores it.
+template <int DIM, int THREADS>
 __device__ __forceinline__ void band_coefficient(const float2* __restrict__ ub, long long cs, int N, int kf,
                                                  double inv_n2d, double eps_inj, double tiny, double* out) {
   __shared__ double red_band[32];
@@ -1165,14 +1177,14 @@ __device__ __forceinline__ void band_coefficient(const float2* __restrict__ ub, 
       lo += wg * ((double)v.x * v.x + (double)v.y * v.y);
     }
   }
-  for (int o = 16; o > 0; o >>= 1) lo += __shfl_xor_sync(0xffffffffu, lo, o);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  lo = lanes_sum<THREADS>(lo);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   __syncthreads();
   if (lane == 0) red_band[wid] = lo;
   __syncthreads();
   if (threadIdx.x == 0) {
     double L = 0.0;
-    for (int i = 0; i < nw; ++i) L += red_band[i];
+    for (int i = 0; i < (THREADS + 31) / 32; ++i) L += red_band[i];
     *out = eps_inj / (2.0 * (0.5 * L * inv_n2d) + tiny);
   }
 }
@@ -1468,8 +1480,8 @@ kx_fwd_band(const float2* __restrict__ du, long long dcs, int kt, int kd, float2
   const int batch = blockIdx.z;
   const long long bd = (long long)batch * 3 * dcs, bp = (long long)batch * 3 * pcs;
   if (band_kf > 0 && blockIdx.x == 0 && blockIdx.y == 0)
-    band_coefficient<DIM>(us + (long long)batch * 3 * cs, cs, N, band_kf, inv_n2d, eps_inj, 1e-30,
-                          band_scale + batch);
+    band_coefficient<DIM, XW * T>(us + (long long)batch * 3 * cs, cs, N, band_kf, inv_n2d, eps_inj, 1e-30,
+                                  band_scale + batch);
   float2 d[3][E];
 #pragma unroll
   for (int c = 0; c < 3; ++c)
@@ -1499,7 +1511,7 @@ kx_fwd_band_tma(const __grid_constant__ CUtensorMap dmap, int kt, int kd, float2
   const int batch = blockIdx.y;
   const int ntx = kt / TW, nb = 2 * kd + 1, ntiles = ntx * nb;
   if (band_kf > 0 && blockIdx.x == 0)
-    band_coefficient<3>(us + (long long)batch * 3 * cs, cs, N, band_kf, inv_n2d, eps_inj, 1e-30, band_scale + batch);
+    band_coefficient<3, TW * T>(us + (long long)batch * 3 * cs, cs, N, band_kf, inv_n2d, eps_inj, 1e-30, band_scale + batch);
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
     mbar_init_fence();

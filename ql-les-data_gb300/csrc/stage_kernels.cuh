@@ -784,8 +784,8 @@ __global__ void __launch_bounds__(256)
 k_band_coefficient(const float2* __restrict__ us, long long cs, int N, int kf, double inv_n2d, double eps_inj,
                    double* __restrict__ band_scale) {
   pdl_begin();
-  band_coefficient<DIM>(us + (long long)blockIdx.x * 3 * cs, cs, N, kf, inv_n2d, eps_inj, 1e-30,
-                        band_scale + blockIdx.x);
+  band_coefficient<DIM, 256>(us + (long long)blockIdx.x * 3 * cs, cs, N, kf, inv_n2d, eps_inj, 1e-30,
+                             band_scale + blockIdx.x);
 }
 
 }  // namespace l3es

@@ -63,3 +63,29 @@ def _check(dim, n, batch, forcing):
 @pytest.mark.parametrize("dim", [2, 3])
 def test_vjp_and_step_match_the_oracle(dim, n, batch, forcing):
     _check(dim, n, batch, forcing)
+
+
+@pytest.mark.parametrize("batch", [1, 2])
+@pytest.mark.parametrize("n", [8, 16])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_constant_power_matches_the_oracle(dim, n, batch):
+    """The band sums of blocks smaller than a warp (8 and 16 threads)."""
+    _check(dim, n, batch, "const_power")
+
+
+@pytest.mark.parametrize("dim,n", [(2, 8), (2, 16), (2, 32), (2, 64), (3, 8), (3, 16)])
+def test_constant_power_rhs_of_small_blocks(dim, n):
+    """The right-hand side's band coefficient by blocks of 4 to 16 threads (2D: tiles of 2 and
+    of 8 columns)."""
+    axes = (1, 2, 3) if dim == 3 else (1, 2)
+    uh = _state(dim, n, 5)
+    _, kkk2, _, _ = R.wavenumbers(n, dim)
+    ref = R.rhs_wrapper(n, 5e-3, axes, const_power=(0.1, ((kkk2 > 0) & (kkk2 <= 4)).astype(float)))(None, uh, 1)
+    p = _native.Plan(dim=dim, n=n, nu=5e-3, dt=1e-3, forcing="const_power", kf=2, eps_inj=0.1)
+    for x_bulk in (1, 0):
+        p.set_schedule({"x_bulk": x_bulk})
+        u = _c64(uh)
+        du = torch.empty_like(u)
+        p.rhs(u, du)
+        # 2e-5: the bound of the repository's step tests (FP32 transforms)
+        assert np.abs(du.cpu().numpy() - ref).max() < 2e-5 * np.abs(ref).max(), x_bulk
