@@ -480,15 +480,95 @@ k_yz_plane(const float2* __restrict__ w, const float2* __restrict__ wx, long lon
 
 // ------------------------------------------------------------------------------
 // k_yz_plane with a plane shared by two CTAs, one for the even rows y and one for the odd: the
-// inverse y transform gives a CTA its rows from one N/2-point transform of the folded columns
-// (V[k] + V[k + N/2], or their difference turned by exp(2 pi i k / N)), the lines of its rows
-// need nothing else, and the halves of the forward transform meet where kx_stage reads them:
+// inverse y transform gives a CTA its rows from the folded columns (V[k] + V[k + N/2] or their
+// difference: half_rows_inv), the lines of its rows need nothing else, and the halves of the
+// forward transform (half_rows_fwd) meet where kx_stage reads them:
 //   X[k] = E[k] + exp(-2 pi i k / N) O[k],  X[k + N/2] = E[k] - exp(-2 pi i k / N) O[k],
 // E and the turned O in rows k and N/2 + k of du. Twice the CTAs, for launches that leave SMs
 // idle. Bound by latency: the 16 loads of a column stay unbranched so that
 // they are in flight together, and a CTA has twice the warps that the lines need, for the
 // columns (ten 64^3 steps 705 us with half of them, 532 us; 676 us by k_yz_plane).
+//
+// The halves are the halves of an N-point transform of radix 8 and N/8 (8 x 8, 8 x 4): the fold
+// is the first level of its radix-8 butterflies, whose outputs of one parity are four of
+// eight, and the turn by exp(2 pi i k / N) goes into the twiddles between its stages and the
+// eighth turns of the butterfly. A turn of its own beside an N/2-point transform took one
+// more rounding per value: the error of 64^3 and 32^3 steps against 64 bits was 0.7 and 1.2 %
+// above the unsplit transforms' in nearly every field, now it is level with theirs, and ten
+// 64^3 steps take 517 us instead of 532 (32^3 322 and 324).
 // ------------------------------------------------------------------------------
+// x times the k-th eighth turn, exp(DIR 2 pi i k / 8), k = 0..3
+template <int DIR>
+__device__ __forceinline__ float2 turn8(float2 x, int k) {
+  const float c = 0.70710678118654752f;
+  return k == 0 ? x : k == 2 ? mul_i<DIR>(x) : cmul(x, make_float2(k == 1 ? c : -c, DIR * c));
+}
+
+// Rows 2 m + odd (m = t + T e of N/2) of the inverse N-point transform, T = N / 16 lanes; v, b:
+// its inputs k = t + T e and k + N/2. XC interleaved columns; sm: N/2 + N/8 slots of them.
+template <int N, int XC>
+__device__ __forceinline__ void half_rows_inv(const float2 (&v)[8], const float2 (&b)[8], int odd, float2 (&z)[8],
+                                              float2* sm, int t, const float2* __restrict__ tw) {
+  constexpr int T = N / 16, R2 = N / 8, B2 = 8 / R2;
+  // one slot of padding in four: the lanes' writes, four slots apart, fall into different banks
+  auto slot = [&](int n) { return sm + (n + n / 4) * XC; };
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    float2 x[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int e = q + 2 * r;
+      x[r] = odd ? turn8<kInv>(csub(v[e], b[e]), r) : cadd(v[e], b[e]);
+    }
+    Dft<4, kInv, true>::run(x);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) *slot(4 * (t + T * q) + r) = x[r];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < B2; ++q) {
+    const int j = t + T * q;
+    float2 x[R2];
+#pragma unroll
+    for (int r = 0; r < R2; ++r) {
+      x[r] = *slot(j + 4 * r);
+      if (r > 0) x[r] = cmul(x[r], twid<kInv>(tw, r * (2 * j + odd)));
+    }
+    Dft<R2, kInv, true>::run(x);
+#pragma unroll
+    for (int r = 0; r < R2; ++r) z[q + r * B2] = x[r];
+  }
+}
+
+// The half of the forward N-point transform that rows 2 m + odd give, m = t + T e of N/2, in
+// place: outputs k = t + T e < N/2, those of the odd rows turned by exp(-2 pi i k / N).
+template <int N, int XC>
+__device__ __forceinline__ void half_rows_fwd(float2 (&v)[8], int odd, float2* sm, int t,
+                                              const float2* __restrict__ tw) {
+  constexpr int T = N / 16, R1 = N / 8, B1 = 8 / R1;
+  auto slot = [&](int n) { return sm + (n + n / 8) * XC; };
+#pragma unroll
+  for (int q = 0; q < B1; ++q) {
+    float2 x[R1];
+#pragma unroll
+    for (int r = 0; r < R1; ++r) x[r] = v[q + r * B1];
+    Dft<R1, kFwd, true>::run(x);
+#pragma unroll
+    for (int r = 0; r < R1; ++r) *slot((t + T * q) * R1 + r) = x[r];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int j = t + T * q;
+    float2 x[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) x[r] = cmul(*slot(j + R1 * r), twid<kFwd>(tw, j * (2 * r + odd)));
+    Dft<4, kFwd, true>::run(x);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[q + 2 * r] = odd ? turn8<kFwd>(x[r], r) : x[r];
+  }
+}
+
 template <int N, int CTAS>
 struct YzHalfCfg {
   static constexpr int R = N / 2;                 // rows of a half
@@ -498,7 +578,7 @@ struct YzHalfCfg {
   static constexpr int THREADS = YzCfg<N>::THREADS;  // at least a slot per row in the lines
   static constexpr int WARPS = THREADS / 32;
   static constexpr int FIELD = ROWS * YzCfg<N>::LD;
-  static constexpr int XSC = XC * xpad_len<XC>(R);
+  static constexpr int XSC = XC * (R + R / 4);
   static constexpr int XS = YzCfg<N>::XS1 > XSC ? YzCfg<N>::XS1 : XSC;
   static constexpr int SMEM = (6 * FIELD + WARPS * XS) * (int)sizeof(float2);
 };
@@ -550,12 +630,8 @@ k_yz_half(const float2* __restrict__ w, const float2* __restrict__ wx, long long
       }
 #pragma unroll
       for (int h = 0; h < 3 - CTAS; ++h) {
-        const int odd = first + h;
         float2 z[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-          z[e] = odd ? cmul(csub(v[e], b[e]), twid<kInv>(tw, t + T * e)) : cadd(v[e], b[e]);
-        block_fft<R, 8, kInv, XC, kSyncWarp>(z, xs + p, t, tw, 2);
+        half_rows_inv<N, XC>(v, b, first + h, z, xs + p, t, tw);
         if (ok) {
 #pragma unroll
           for (int e = 0; e < 8; ++e) s_yz[f * C::FIELD + (h * R + t + T * e) * LD + col] = z[e];
@@ -578,12 +654,10 @@ k_yz_half(const float2* __restrict__ w, const float2* __restrict__ wx, long long
 #pragma unroll
       for (int e = 0; e < 8; ++e)
         v[e] = ok ? s_yz[c * C::FIELD + (h * R + t + T * e) * LD + col] : make_float2(0.f, 0.f);
-      block_fft<R, 8, kFwd, XC, kSyncWarp>(v, xs + p, t, tw, 2);
+      half_rows_fwd<N, XC>(v, odd, xs + p, t, tw);
       if (ok) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          db[c * ds + (long long)(odd * R + t + T * e) * kt + col] =
-              odd ? cmul(v[e], twid<kFwd>(tw, t + T * e)) : v[e];
+        for (int e = 0; e < 8; ++e) db[c * ds + (long long)(odd * R + t + T * e) * kt + col] = v[e];
       }
       __syncwarp();
     }
