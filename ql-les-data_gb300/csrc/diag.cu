@@ -1,7 +1,8 @@
 // Diagnostics of the drivers (l3es/spectral_solver.py:123-127, :318-320;
 // l3es/utils.py:35-97, :300-315) with FP64 partial sums. Each point's or mode's
-// contribution is formed in FP32 and accumulated in float-float (Ff, ~48 bits); FP64
-// arithmetic is scarce on this GPU and only combines the threads' sums.
+// contribution is formed in FP32 and accumulated in float-float (Ff, ~48 bits: energy and
+// dissipation) or in F3 (at least FP64's bits: statistics and spectrum); FP64 arithmetic is
+// scarce on this GPU and only combines the threads' sums.
 //   l3es_field_stats      max |u_c| per component and 0.5 mean sum u^2 of a physical field
 //   l3es_dissipation      nu <|curl u|^2> by Parseval on the half spectrum
 //   l3es_energy_spectrum  shell sums E(k), shells int(|k| + 0.5)
@@ -13,19 +14,42 @@
 
 namespace l3es {
 
-// Sum of M non-negative FP32 terms in FP64: float-float, or FP64 throughout where that is
-// not finite (its error terms turn an infinite or overflowing sum into NaN).
-template <int M>
-__device__ __forceinline__ double ff_sum(const float (&e)[M]) {
-  Ff a{e[0], 0.f};
-#pragma unroll
-  for (int i = 1; i < M; ++i) a = ff_add(a, e[i]);
-  double s = (double)a.hi + (double)a.lo;
-  if (!isfinite(a.hi)) {
-    s = 0.0;
-    for (int i = 0; i < M; ++i) s += (double)e[i];
+// Sum of non-negative FP32 terms that loses less than an FP64 one: every addition's rounding
+// error goes to b and that addition's to c (TwoSum), so only c rounds, at 2^-72 of the sum.
+// Thirteen FP32 instructions a term; FP64 runs at two a clock and SM. An infinite or overflowing
+// sum has NaN error terms: where a is not finite the caller adds in FP64.
+struct F3 {
+  float a, b, c;
+  // (c is zero unless the terms' sizes differ by 2^24, and converting it costs as much as the
+  // others)
+  __device__ __forceinline__ double value() const {
+    double lo = (double)b;
+    if (c != 0.f) lo += (double)c;
+    return lo + (double)a;
   }
+};
+__device__ __forceinline__ float two_sum(float x, float y, float& err) {
+  const float s = x + y, q = s - x;
+  err = (x - (s - q)) + (y - q);
   return s;
+}
+__device__ __forceinline__ F3 f3_add(F3 s, F3 t) {
+  float e0, e1, e2;
+  s.a = two_sum(s.a, t.a, e0);
+  s.b = two_sum(two_sum(s.b, t.b, e1), e0, e2);
+  s.c += t.c + (e1 + e2);
+  return s;
+}
+// the sum of M terms over pairs, pairs of pairs, ...
+template <int M>
+__device__ __forceinline__ F3 f3_tree(const float* e) {
+  if constexpr (M == 2) {
+    F3 s{0.f, 0.f, 0.f};
+    s.a = two_sum(e[0], e[1], s.b);
+    return s;
+  } else {
+    return f3_add(f3_tree<M / 2>(e), f3_tree<M / 2>(e + M / 2));
+  }
 }
 
 // Eight floats from p + i on (VEC: two 16-byte loads), zeros from n on.
@@ -41,9 +65,10 @@ __device__ __forceinline__ void load8(const float* __restrict__ p, unsigned i, u
 }
 
 // per block: max |u_c| for c = 0..2 and sum_c u_c^2, over ps values per component; eight
-// neighbouring points per thread and turn, the sum in float-float (where that is not finite,
-// again in FP64). VEC: u is 16-byte aligned and ps a multiple of 4. With one point in flight
-// and an FP64 addition per point a 256^3 field took 68 us.
+// neighbouring points per thread and turn, the sum in F3 (where that is not finite, again in
+// FP64). VEC: u is 16-byte aligned and ps a multiple of 4. Bound by the reads: both launches
+// take 35.8 us on a 256^3 field, 201 MB (35.3 with the sum in float-float, which keeps 48 bits;
+// 68 with one point in flight and an FP64 addition per point).
 template <bool VEC>
 __global__ void __launch_bounds__(256)
 k_field_stats(const float* __restrict__ u, long long ps, int nblk, double* __restrict__ partial) {
@@ -51,23 +76,24 @@ k_field_stats(const float* __restrict__ u, long long ps, int nblk, double* __res
   const int batch = blockIdx.y;
   const float* ub = u + (long long)batch * 3 * ps;
   float mx[3] = {0.f, 0.f, 0.f};
-  Ff acc{0.f, 0.f};
+  F3 acc{0.f, 0.f, 0.f};
   const unsigned n = (unsigned)ps, step = 8u * (unsigned)nblk * blockDim.x;  // ps <= 512^3
   const unsigned first = 8u * (blockIdx.x * blockDim.x + threadIdx.x);
   auto energy = [](float x, float y, float z) { return fmaf(z, z, fmaf(y, y, x * x)); };
   for (unsigned i = first; i < n; i += step) {
-    float v[3][8];
+    float v[3][8], e[8];
 #pragma unroll
     for (int c = 0; c < 3; ++c) load8<VEC>(ub + c * ps, i, n, v[c]);
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) mx[c] = fmaxf(mx[c], fabsf(v[c][q]));
-      acc = ff_add(acc, energy(v[0][q], v[1][q], v[2][q]));
+      e[q] = energy(v[0][q], v[1][q], v[2][q]);
     }
+    acc = f3_add(acc, f3_tree<8>(e));
   }
-  double s = (double)acc.hi + (double)acc.lo;
-  if (!isfinite(acc.hi)) {
+  double s = acc.value();
+  if (!isfinite(acc.a)) {
     s = 0.0;
     for (unsigned i = first; i < n; i += step)
       for (unsigned j = i; j < i + 8 && j < n; ++j) s += (double)energy(ub[j], ub[ps + j], ub[2 * ps + j]);
@@ -207,10 +233,11 @@ constexpr int kSpecThreads = 128;
 // the mode count and of weight * |u_hat|^2, merged with FP64 atomics into
 // acc[batch][2][n]. The shell depends on the magnitudes of the wavenumbers only, so a warp
 // takes all rows (+-a, +-b) and (+-b, +-a) of one pair a >= b (2D: +-a) at once, sums a
-// mode's energies over them in float-float (up to 8 rows, 24 loads in flight per lane) and
+// mode's energies over them in F3 (up to 8 rows, 24 loads in flight per lane) and
 // makes one shared FP64 addition for the lot: those atomics are a compare-and-swap loop,
 // and two per mode into one histogram per block took 289 us on a 256^3 spectrum (76 us with
-// one addition per 8 modes, 57 us with a histogram per warp). shell int(|k| + 0.5): |k|^2 is an
+// one addition per 8 modes, 57 us with a histogram per warp, 52 us with the count's addition
+// before the energies, while the loads are in flight). shell int(|k| + 0.5): |k|^2 is an
 // integer below 3 (n/2)^2, whose square root is never within 1/(8|k|) of a half integer,
 // far more than the FP32 rounding.
 template <int DIM>
@@ -258,6 +285,9 @@ k_spectrum(const float2* __restrict__ uh, long long cs, int n, int nblk, double 
       for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int c = 0; c < 3; ++c) v[r][c] = r < rows ? __ldg(ub + c * cs + off[r] + kh) : make_float2(0.f, 0.f);
+      const int k2 = a * a + b * b + kh * kh;
+      const int shell = (int)(sqrtf((float)k2) + 0.5f), w = (kh == 0 || kh == n / 2) ? 1 : 2;
+      if (shell < n) atomicAdd(cnt + shell, (unsigned)(w * rows));  // while the loads are in flight
       float e[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
@@ -265,12 +295,14 @@ k_spectrum(const float2* __restrict__ uh, long long cs, int n, int nblk, double 
 #pragma unroll
         for (int c = 0; c < 3; ++c) e[r] = fmaf(v[r][c].x, v[r][c].x, fmaf(v[r][c].y, v[r][c].y, e[r]));
       }
-      const int k2 = a * a + b * b + kh * kh;
-      const int shell = (int)(sqrtf((float)k2) + 0.5f);
       if (shell < n) {
-        const int w = (kh == 0 || kh == n / 2) ? 1 : 2;
-        atomicAdd(cnt + shell, (unsigned)(w * rows));
-        atomicAdd(hist + shell, (w * scale) * ff_sum(e));
+        const F3 f = f3_tree<R>(e);
+        double s = f.value();
+        if (!isfinite(f.a)) {
+          s = 0.0;
+          for (int r = 0; r < R; ++r) s += (double)e[r];
+        }
+        atomicAdd(hist + shell, (w * scale) * s);
       }
     }
   }
