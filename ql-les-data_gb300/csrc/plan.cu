@@ -535,8 +535,9 @@ static int rk4_step(l3es_plan* plan, float2* S, int most, bool first, bool last,
     q.band_rk = band;
   }
   if (one_visit && c.dim == 2 && c.n <= kStep2dMax) {  // (kd, kt of these N are Step2dCfg's)
-    plan->tab.steps2d(c, S, prm, most, s);
-    return most;
+    const int made = std::min(most, kStep2dSteps);
+    plan->tab.steps2d(c, S, prm, made, s);
+    return made;
   }
   if (one_visit) {
     plan->tab.step(c, S, prm, first, last, s);

@@ -667,14 +667,18 @@ k_yz_half(const float2* __restrict__ w, const float2* __restrict__ wx, long long
 // ------------------------------------------------------------------------------
 // Whole RK4 steps of a 2D grid up to 32^2, one CTA per trajectory: the six fields of a
 // stage (31 KB at 32^2), its field and the accumulator on the band fit shared memory, and a
-// thread keeps the step's initial state of its modes in registers, so nsteps steps are one
-// launch that reads and writes the state once. A stage is the transforms and the combination
-// of kx_stage and the lines of k_yz_plane (the plane's rows are x here, its columns the half
-// axis), four block barriers in place of two launches. Ten steps at 32^2 x 9 took 266 us by
+// thread keeps the step's initial state of its modes in registers, so nsteps steps (up to
+// kStep2dSteps) are one launch that reads and writes the state once. A stage is the transforms
+// and the combination of kx_stage and the lines of k_yz_plane (the plane's rows are x here, its
+// columns the half axis), four block barriers in place of two launches. Ten steps at 32^2 x 9 took 266 us by
 // kx_stage and 82 us a single step from the start of plain launches; here 152 and 18 us. At
 // 64^2 one SM's issue rate is the bound (46 us a step; kx_stage over 17 SMs 33 us).
 // ------------------------------------------------------------------------------
 constexpr int kStep2dMax = 32;
+// Steps of one launch: 1024 take some 15 ms, so that a long run is not one kernel that nothing
+// else gets in between, and the stages' count stays far from overflow; the state's trip through
+// memory per launch is nothing beside them.
+constexpr int kStep2dSteps = 1024;
 
 template <int N>
 struct Step2dCfg {
