@@ -112,8 +112,8 @@ int64_t l3es_plan_workspace_bytes(const l3es_plan* plan);
  *       0 the packed half-length one,
  *   [3] the persistent bulk-copy band x pass (else one tile per CTA); plans start with 1 at
  *       N = 256.
- * The step of 2D grids and of 3D grids up to 64^3 has stage kernels of its own in the
- * forms it starts with; of these choices only [2] reaches them (2D, N = 256).
+ * The step of 2D grids and of 3D grids up to 64^3 has stage kernels of its own in form 2,
+ * which plans start with; of these choices only [2] reaches them (2D, N = 256).
  * Every schedule computes the same step; only speed differs. */
 int l3es_plan_get_schedule(const l3es_plan* plan, int32_t* sched4);
 int l3es_plan_set_schedule(l3es_plan* plan, const int32_t* sched4);
@@ -127,8 +127,8 @@ int l3es_plan_set_schedule(l3es_plan* plan, const int32_t* sched4);
  *     opens the next; above, the band x pass combines the stages in place on the band and
  *     every other mode is scaled by its closed form inside the next stage's x inverse (no
  *     elementwise pass).
- * Plans start with form 2 in 3D and form 1 in 2D; in 2D forms 1 and 2 are the same kernels,
- * the stage combination inside the x passes (and nsteps steps in one launch up to 32^2).
+ * A plan that was given no form takes form 2 (in 2D up to 32^2 up to 1024 steps share a
+ * launch). It reports 2 in 3D and 1 in 2D, where setting 1 selects the elementwise update.
  * Forms 1 and 2 apply when the forcing lies inside the band (constant-power kf <= kd,
  * Kolmogorov wavenumber < kt); otherwise, and for the integrating-factor scheme, the
  * step takes form 0. */

@@ -133,6 +133,8 @@ struct Schedule {
   int band_bulk = -1; // persistent bulk-copy band pass (-1: at N = 256, the measured default)
 };
 
+constexpr int kFormStart = -1;  // no step form set
+
 // Geometry + scratch of one plan, handed to the per-N launch wrappers.
 struct Ctx {
   int dim = 3, n = 0, h = 0, batch = 1;
@@ -160,10 +162,10 @@ struct Ctx {
   double* einj = nullptr;      // [batch] scratch e_inj
   float* nu_b = nullptr;       // [batch] viscosity per trajectory
   int* err = nullptr;          // device error word: nonzero after a kernel wait timed out
-  int step_form = 2;           // explicit RK4 step (run_steps): 0 per-mode update of the whole
-                               // spectrum, 1 closed-form stages outside the stage region (3D;
-                               // in 2D as 2), 2 the stage combination inside the x passes
-                               // (l3es_plan_set_step_form; plans start at 2 in 3D, 1 in 2D)
+  int step_form = kFormStart;  // explicit RK4 step (run_steps): 0 per-mode update of the whole
+                               // spectrum, 1 closed-form stages outside the stage region, 2 the
+                               // stage combination inside the x passes (l3es_plan_set_step_form);
+                               // a plan that was given none takes 2 (and reports 1 in 2D)
   Schedule sched;              // kernel variants of the step
   int kf = 0;                  // forcing band 0 < |k|^2 <= kf^2
   double eps_inj = 0.0;        // constant-power injection rate

@@ -242,8 +242,6 @@ int l3es_plan_create(const l3es_plan_desc* desc, l3es_plan** out) {
   // y pass: radix 16 at 256^3 (a step 2055 us against 2153 us with radix 8), radix 8 at
   // 128^3 (286 against 294 us) and 512^3 (19.67 against 19.97 ms)
   c.sched.y_var = dim == 3 && (n == 128 || n == 512);
-  // the stage combination inside the x passes (in 2D forms 1 and 2 both are kx_stage)
-  c.step_form = dim == 3 ? 2 : 1;
   c.nmid = dim == 3 ? n : 1;
   c.cs = c.nmid * n * c.h;
   c.fs = c.cs;
@@ -426,7 +424,8 @@ int l3es_plan_set_schedule(l3es_plan* plan, const int32_t* sched4) {
 
 int l3es_plan_get_step_form(const l3es_plan* plan, int32_t* form) {
   if (!plan || !form) return fail(L3ES_EINVAL, "l3es_plan_get_step_form: null argument");
-  *form = plan->ctx.step_form;
+  const Ctx& c = plan->ctx;
+  *form = c.step_form != kFormStart ? c.step_form : c.dim == 3 ? 2 : 1;
   return L3ES_OK;
 }
 
@@ -448,6 +447,9 @@ int l3es_plan_set_step_form(l3es_plan* plan, int32_t form) {
 // the step runs kernels that a knob does not reach (XStage, k_yz_plane, k_step2d) its two
 // settings time alike and either may be kept.
 // ---------------------------------------------------------------------------------
+// The form whose kernels the explicit step takes.
+static int form_taken(const Ctx& c) { return c.step_form == kFormStart ? 2 : c.step_form; }
+
 static std::string tune_key(const l3es_plan* p) {
   cudaDeviceProp prop{};
   cudaGetDeviceProperties(&prop, p->device);
@@ -456,7 +458,7 @@ static std::string tune_key(const l3es_plan* p) {
     if (ch == ' ') ch = '_';
   return name + "|sm" + std::to_string(prop.major) + std::to_string(prop.minor) + "|d" + std::to_string(p->ctx.dim) +
          "|n" + std::to_string(p->ctx.n) + "|b" + std::to_string(p->ctx.batch) + "|f" +
-         std::to_string(p->ctx.step_form);
+         std::to_string(form_taken(p->ctx));
 }
 
 static bool tune_cache_read(const char* path, const std::string& key, int32_t* v) {
@@ -499,6 +501,28 @@ static void tune_cache_write(const char* path, const std::string& key, const int
   std::fclose(f);
 }
 
+// Which kernels the plan's explicit RK4 step takes.
+struct StepRoute {
+  bool lin;        // closed-form stages outside the stage region (k_rk_update_lin)
+  bool band;       // the stage combination inside the x passes
+  bool one_visit;  // ... by kx_stage or k_step2d (else XLin and BandRk)
+};
+static StepRoute step_route(const l3es_plan* plan) {
+  const Ctx& c = plan->ctx;
+  const l3es_plan_desc& d = plan->desc;
+  const int form = form_taken(c);
+  // the closed form needs the explicit scheme and forcing terms inside the region (band
+  // forcing |k| <= kf, Kolmogorov mode kh = kolm_k); the combination inside the x passes needs
+  // the band inside the half axis too (kt <= N/2 + 1, i.e. N >= 16)
+  const int kf_band = d.forcing == L3ES_FORCING_CONST_POWER ? d.kf : 0;
+  StepRoute r;
+  r.lin = form >= 1 && d.scheme != L3ES_SCHEME_INTEGRATING_FACTOR && kf_band <= c.kd && kf_band < c.kt &&
+          (d.kolm_k <= 0 || d.kolm_k < c.kt);
+  r.band = r.lin && form >= 2 && c.kt <= c.h;
+  r.one_visit = r.band && step_by_kx_stage(c.dim, c.n);
+  return r;
+}
+
 // RK4 steps of the state S in the plan's step form (spectral_solver.py:65-80; the forcing
 // rescale of ekin_tot follows each step in run_steps), at most `most` of them; returns how
 // many it made. first / last: whether the x inverse of S has to be made, and whether the
@@ -508,16 +532,7 @@ static int rk4_step(l3es_plan* plan, float2* S, int most, bool first, bool last,
   const l3es_plan_desc& d = plan->desc;
   static const double a_rk4[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
   static const double b_rk4[3] = {0.5, 0.5, 1.0};
-  // closed-form stages outside the stage region (k_rk_update): explicit scheme, forcing
-  // terms inside the region (band forcing |k| <= kf, Kolmogorov mode kh = kolm_k)
-  const int kf_band = d.forcing == L3ES_FORCING_CONST_POWER ? d.kf : 0;
-  const int lin_ok = c.step_form >= 1 && d.scheme != L3ES_SCHEME_INTEGRATING_FACTOR && kf_band <= c.kd &&
-                     kf_band < c.kt && (d.kolm_k <= 0 || d.kolm_k < c.kt);
-  // the stage combination inside the x passes (form 2; in 2D, where the elementwise update
-  // is one launch of four per stage, form 1 as well); the band has to lie inside the half
-  // axis (kt <= N/2 + 1, i.e. N >= 16)
-  const bool band = lin_ok && c.step_form >= (c.dim == 3 ? 2 : 1) && c.kt <= c.h;
-  const bool one_visit = band && step_by_kx_stage(c.dim, c.n);
+  const StepRoute route = step_route(plan);
   EpiParams prm[4];
   for (int rk = 0; rk < 4; ++rk) {
     EpiParams& q = prm[rk];
@@ -531,22 +546,22 @@ static int rk4_step(l3es_plan* plan, float2* S, int most, bool first, bool last,
     q.rk = rk;
     q.if_h = d.scheme == L3ES_SCHEME_INTEGRATING_FACTOR ? (float)d.dt : 0.f;
     q.dt = (float)d.dt;
-    q.lin = lin_ok;
-    q.band_rk = band;
+    q.lin = route.lin;
+    q.band_rk = route.band;
   }
-  if (one_visit && c.dim == 2 && c.n <= kStep2dMax) {  // (kd, kt of these N are Step2dCfg's)
+  if (route.one_visit && c.dim == 2 && c.n <= kStep2dMax) {  // (kd, kt of these N are Step2dCfg's)
     const int made = std::min(most, kStep2dSteps);
     plan->tab.steps2d(c, S, prm, made, s);
     return made;
   }
-  if (one_visit) {
+  if (route.one_visit) {
     plan->tab.step(c, S, prm, first, last, s);
     return 1;
   }
   // the band-fused stages (XLin, BandRk) work in place, the accumulator in C in the band's
   // compact layout; the elementwise update keeps its stage field in T
   for (int rk = 0; rk < 4; ++rk)
-    plan->tab.stage(c, band || rk == 0 ? S : c.Tb, S, band ? S : c.Tb, rk, prm[rk], s);
+    plan->tab.stage(c, route.band || rk == 0 ? S : c.Tb, S, route.band ? S : c.Tb, rk, prm[rk], s);
   return 1;
 }
 

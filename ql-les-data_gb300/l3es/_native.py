@@ -344,9 +344,9 @@ class Plan:
     def step_form(self) -> int:
         """Form of the explicit RK4 step (l3es_plan_get_step_form): 0 one elementwise
         update of the whole spectrum per stage, 1 the closed form of the linear decay
-        outside the dealiased rows, 2 the stage combination inside the x passes (plans
-        start at 2 in 3D and at 1 in 2D, where 1 is the same as 2). All forms compute the
-        reference's RK4 step."""
+        outside the dealiased rows, 2 the stage combination inside the x passes. A plan
+        that was given none takes form 2; it reports 2 in 3D and 1 in 2D, where setting 1
+        selects the elementwise update. All forms compute the reference's RK4 step."""
         v = ctypes.c_int32()
         _check(self._lib.l3es_plan_get_step_form(self._h, ctypes.byref(v)), "l3es_plan_get_step_form")
         return int(v.value)
