@@ -136,9 +136,10 @@ int l3es_plan_get_step_form(const l3es_plan* plan, int32_t* form);
 int l3es_plan_set_step_form(l3es_plan* plan, int32_t form);
 
 /* Autotuner: times one RK4 step of the plan (its step form, on its own scratch) under
- * each schedule choice (one knob at a time) and keeps the fastest. cache_path
+ * each schedule choice that the step reaches (one knob at a time) and takes one that is
+ * 2 % faster than the present; other choices stay as they are. cache_path
  * (nullable) names a text file of earlier results, one line per GPU model, dim, N,
- * batch and step form; a hit skips the timing, a miss appends the result.
+ * batch, step form and set of kernels; a hit skips the timing, a miss appends the result.
  * Synchronises the stream; not while recording a graph. */
 int l3es_plan_autotune(l3es_plan* plan, const char* cache_path, void* stream);
 

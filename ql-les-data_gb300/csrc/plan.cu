@@ -443,12 +443,52 @@ int l3es_plan_set_step_form(l3es_plan* plan, int32_t form) {
 // radix-8 y passes, two-for-one or packed line pass, bulk-copy or one-tile band pass) by
 // timing one RK4 step in the plan's step form on its own scratch (coordinate descent, each
 // knob with the others at their current choice), and caches the result in a text file, one
-// line per (GPU, dim, N, batch, step form): "<key> x_bulk y_var line_pair band_bulk". Where
-// the step runs kernels that a knob does not reach (XStage, k_yz_plane, k_step2d) its two
-// settings time alike and either may be kept.
+// line per (GPU, dim, N, batch, step form, route): "<key> x_bulk y_var line_pair band_bulk".
+// A knob that the timed step does not reach stays as it is (its settings time alike, and a
+// pick by chance would go to the right-hand side, irfftn and the adjoint, which it does
+// reach), and a choice has to beat the present one by more than two timings of one setting
+// differ. The route's name tags the kernels that were timed: a line of other kernels, of
+// another forcing's or scheme's route or of a build before this tag is not read.
 // ---------------------------------------------------------------------------------
+constexpr float kTuneMargin = 0.98f;
+
 // The form whose kernels the explicit step takes.
 static int form_taken(const Ctx& c) { return c.step_form == kFormStart ? 2 : c.step_form; }
+
+// Which kernels the plan's explicit RK4 step takes.
+struct StepRoute {
+  bool lin;        // closed-form stages outside the stage region (k_rk_update_lin)
+  bool band;       // the stage combination inside the x passes
+  bool one_visit;  // ... by kx_stage or k_step2d (else XLin and BandRk)
+};
+static StepRoute step_route(const l3es_plan* plan) {
+  const Ctx& c = plan->ctx;
+  const l3es_plan_desc& d = plan->desc;
+  const int form = form_taken(c);
+  // the closed form needs the explicit scheme and forcing terms inside the region (band
+  // forcing |k| <= kf, Kolmogorov mode kh = kolm_k); the combination inside the x passes needs
+  // the band inside the half axis too (kt <= N/2 + 1, i.e. N >= 16)
+  const int kf_band = d.forcing == L3ES_FORCING_CONST_POWER ? d.kf : 0;
+  StepRoute r;
+  r.lin = form >= 1 && d.scheme != L3ES_SCHEME_INTEGRATING_FACTOR && kf_band <= c.kd && kf_band < c.kt &&
+          (d.kolm_k <= 0 || d.kolm_k < c.kt);
+  r.band = r.lin && form >= 2 && c.kt <= c.h;
+  r.one_visit = r.band && step_by_kx_stage(c.dim, c.n);
+  return r;
+}
+
+// The schedule knobs that the plan's step reaches, in l3es_plan_set_schedule's order (2D up to
+// 128^2 and 3D up to 64^3 have line passes of their own in form 2; the one-tile kernel always
+// makes the x inverse of a band-fused stage; the radix-16 and two-for-one line passes end at 256).
+static void tune_knobs(const l3es_plan* p, bool (&knob)[4]) {
+  const Ctx& c = p->ctx;
+  const StepRoute r = step_route(p);
+  const bool line = c.n >= 64 && c.n <= 256;
+  knob[0] = !r.band && (c.dim == 2 || c.n >= 64);
+  knob[1] = !r.one_visit && c.dim == 3 && c.n >= 128;
+  knob[2] = r.one_visit ? c.dim == 2 && c.n == 256 : line;
+  knob[3] = !r.one_visit && c.dim == 3 && c.n >= 64;
+}
 
 static std::string tune_key(const l3es_plan* p) {
   cudaDeviceProp prop{};
@@ -456,9 +496,10 @@ static std::string tune_key(const l3es_plan* p) {
   std::string name = prop.name;
   for (char& ch : name)
     if (ch == ' ') ch = '_';
+  const StepRoute route = step_route(p);
   return name + "|sm" + std::to_string(prop.major) + std::to_string(prop.minor) + "|d" + std::to_string(p->ctx.dim) +
          "|n" + std::to_string(p->ctx.n) + "|b" + std::to_string(p->ctx.batch) + "|f" +
-         std::to_string(form_taken(p->ctx));
+         std::to_string(form_taken(p->ctx)) + (route.one_visit ? "|stage2" : route.band ? "|band2" : "|elem2");
 }
 
 static bool tune_cache_read(const char* path, const std::string& key, int32_t* v) {
@@ -499,28 +540,6 @@ static void tune_cache_write(const char* path, const std::string& key, const int
   for (const auto& l : keep) std::fputs(l.c_str(), f);
   std::fprintf(f, "%s %d %d %d %d\n", key.c_str(), v[0], v[1], v[2], v[3]);
   std::fclose(f);
-}
-
-// Which kernels the plan's explicit RK4 step takes.
-struct StepRoute {
-  bool lin;        // closed-form stages outside the stage region (k_rk_update_lin)
-  bool band;       // the stage combination inside the x passes
-  bool one_visit;  // ... by kx_stage or k_step2d (else XLin and BandRk)
-};
-static StepRoute step_route(const l3es_plan* plan) {
-  const Ctx& c = plan->ctx;
-  const l3es_plan_desc& d = plan->desc;
-  const int form = form_taken(c);
-  // the closed form needs the explicit scheme and forcing terms inside the region (band
-  // forcing |k| <= kf, Kolmogorov mode kh = kolm_k); the combination inside the x passes needs
-  // the band inside the half axis too (kt <= N/2 + 1, i.e. N >= 16)
-  const int kf_band = d.forcing == L3ES_FORCING_CONST_POWER ? d.kf : 0;
-  StepRoute r;
-  r.lin = form >= 1 && d.scheme != L3ES_SCHEME_INTEGRATING_FACTOR && kf_band <= c.kd && kf_band < c.kt &&
-          (d.kolm_k <= 0 || d.kolm_k < c.kt);
-  r.band = r.lin && form >= 2 && c.kt <= c.h;
-  r.one_visit = r.band && step_by_kx_stage(c.dim, c.n);
-  return r;
 }
 
 // RK4 steps of the state S in the plan's step form (spectral_solver.py:65-80; the forcing
@@ -608,14 +627,13 @@ extern "C" int l3es_plan_autotune(l3es_plan* plan, const char* cache_path, void*
   if (rc == L3ES_OK) {
     l3es_plan_get_schedule(plan, v);
     l3es_plan_set_schedule(plan, v);
-    // knobs that change anything for this plan
-    const int n = c.n;
-    const bool knob[4] = {(c.dim == 3 && n >= 64) || c.dim == 2, c.dim == 3 && n >= 128, n >= 64 && n <= 256,
-                          c.dim == 3 && n >= 64};
-    const int nval[4] = {2, 2, n == 256 ? 4 : 2, 2};  // the line pass has two radix-16 forms at 256
-    float best = time_step(plan, s, e0, e1);
+    bool knob[4];
+    tune_knobs(plan, knob);
+    const int nval[4] = {2, 2, c.n == 256 ? 4 : 2, 2};  // the line pass has two radix-16 forms at 256
+    float best = 0.f;
     for (int k = 0; k < 4; ++k) {
       if (!knob[k]) continue;
+      if (best == 0.f) best = time_step(plan, s, e0, e1);
       const int keep = v[k];
       int pick = keep;
       for (int val = 0; val < nval[k]; ++val) {
@@ -623,7 +641,7 @@ extern "C" int l3es_plan_autotune(l3es_plan* plan, const char* cache_path, void*
         v[k] = val;
         l3es_plan_set_schedule(plan, v);
         const float t = time_step(plan, s, e0, e1);
-        if (t < best) {
+        if (t < kTuneMargin * best) {
           best = t;
           pick = val;
         }
