@@ -149,8 +149,9 @@ def _stream(stream=None) -> int:
     import torch
 
     # the current stream's handle without the Stream object around it, which took longer to
-    # make than a small grid's kernels to launch
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    # make than a small grid's kernels to launch; by the object where a torch has no such call
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return torch.cuda.current_stream().cuda_stream if raw is None else raw(torch.cuda.current_device())
 
 
 def _ptr(t) -> int:
