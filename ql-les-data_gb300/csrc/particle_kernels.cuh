@@ -275,6 +275,7 @@ k_dft_interp(const float2* __restrict__ hh, long long hcs, int c, const double* 
 // Grids that a one-thread-per-particle block of 128 could not serve (phase tables above
 // 227 KB) stay refused by the callers.
 inline bool dft_supported(int dim, int c) { return sizeof(float2) * dim * c * 128 <= 227 * 1024; }
+constexpr int kDftMaxC = 64;  // the largest of them, 2D and 3D
 
 // Launches k_dft_interp over np particles: two per lane while one round of two blocks per
 // SM takes them all (32^3 modes: 300 particles 74 against 103 us with four), four above, where
@@ -286,7 +287,10 @@ inline cudaError_t dft_launch(int dim, const float2* hh, long long hcs, int c, c
     const long long tiles = (np + K::TILE - 1) / K::TILE;
     const unsigned grid = (unsigned)(tiles < (1LL << 30) ? tiles : (1LL << 30));
     const size_t smem = K::smem(c);
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit of the largest c, whatever this one's: another thread may set it between this
+    // call and the launch
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::smem(kDftMaxC));
     if (e != cudaSuccess) return e;
     pdl_launch(kernel, grid, K::threads(c), smem, s, hh, hcs, c, r, np, u_r, dt, r_out);
     return cudaGetLastError();

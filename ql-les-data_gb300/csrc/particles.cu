@@ -530,6 +530,10 @@ k_herm_project(const float2* __restrict__ hb, long long hcs, int c, float cd, fl
 // 128 with per-particle 1D phase tables exp(-i k_d x_d) (FP64 recurrence, stored FP32);
 // tile sums in FP32, running total in FP64.
 // ------------------------------------------------------------------------------
+// Most shared memory of a launch (larger grids are refused); the kernel's limit on every call,
+// so that calls of several threads and grid sizes do not lower it for one another.
+constexpr int kP2gSmemMax = 200 * 1024;
+
 template <int DIM>
 __global__ void __launch_bounds__(128)
 k_p2g_dft(const double* __restrict__ r, const double* __restrict__ u_r, long long np, int ncomp, int n,
@@ -1159,14 +1163,14 @@ int l3es_interp_vjp(l3es_interp_plan* p, const double* r, int64_t np, const doub
     // S(k) = sum_j lam_j exp(-i k.r_j) on the c-grid (into p->g), then / c^dim
     const long long modes = dim == 3 ? (long long)c * c * c : (long long)c * c;
     const size_t smem = sizeof(float2) * 128 * dim * c;
-    if (smem > 200 * 1024) return fail(L3ES_EINVAL, "l3es_interp_vjp: ckp_N too large for the dft backend");
+    if (smem > kP2gSmemMax) return fail(L3ES_EINVAL, "l3es_interp_vjp: ckp_N too large for the dft backend");
     const float scale = (float)(1.0 / (double)modes);
     if (dim == 3) {
-      cudaFuncSetAttribute(k_p2g_dft<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_p2g_dft<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kP2gSmemMax);
       pdl_launch(k_p2g_dft<3>, (unsigned)((modes + 127) / 128), 128, smem, s, r, lam, np, 3, c, p->g, modes);
       pdl_launch(k_box_to_half_adj<3>, dim3(hbk, 3), 256, 0, s, p->g, modes, c, c, nullptr, scale, p->hb, p->hcs);
     } else {
-      cudaFuncSetAttribute(k_p2g_dft<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_p2g_dft<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kP2gSmemMax);
       pdl_launch(k_p2g_dft<2>, (unsigned)((modes + 127) / 128), 128, smem, s, r, lam, np, 2, c, p->g, modes);
       pdl_launch(k_box_to_half_adj<2>, dim3(hbk, 3), 256, 0, s, p->g, modes, c, c, nullptr, scale, p->hb, p->hcs);
     }
@@ -1220,12 +1224,12 @@ int l3es_interp_particles_to_grid(l3es_interp_plan* p, const double* r, const do
   const long long modes = p->dim == 3 ? (long long)c * c * c : (long long)c * c;
   // the NUFFT grid buffers (n = 2c) hold the c^dim spectrum and its real transform
   const size_t smem = sizeof(float2) * 128 * p->dim * c;
-  if (smem > 200 * 1024) return fail(L3ES_EINVAL, "l3es_interp_particles_to_grid: grid too large");
+  if (smem > kP2gSmemMax) return fail(L3ES_EINVAL, "l3es_interp_particles_to_grid: grid too large");
   if (p->dim == 3) {
-    cudaFuncSetAttribute(k_p2g_dft<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_p2g_dft<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kP2gSmemMax);
     pdl_launch(k_p2g_dft<3>, (unsigned)((modes + 127) / 128), 128, smem, s, r, u_r, np, 3, c, p->g, modes);
   } else {
-    cudaFuncSetAttribute(k_p2g_dft<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_p2g_dft<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kP2gSmemMax);
     pdl_launch(k_p2g_dft<2>, (unsigned)((modes + 127) / 128), 128, smem, s, r, u_r, np, 2, c, p->g, modes);
   }
   // u_grid = real(ifftn(S)) (ifftn carries 1/c^dim)
