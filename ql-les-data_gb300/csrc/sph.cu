@@ -24,7 +24,7 @@
 
 #include <cmath>
 #include <string>
-#include <vector>
+#include <type_traits>
 
 #include "l3es_internal.h"
 #include "particle_kernels.cuh"
@@ -590,23 +590,8 @@ struct l3es_sph_plan {
   float4* us = nullptr;    // [np_max] velocity per slot (forces)
   float4* rp = nullptr;    // [np_max] (rho, p, 1 / rho^2, -) per slot
   SphKept kept{};          // neighbour lists of np_max particles (null: searched twice)
-  std::vector<void*> allocs;
+  void* mem = nullptr;     // the one allocation behind all of them
 };
-
-static int sph_alloc(l3es_sph_plan* p, void** ptr, size_t bytes, const char* what) {
-  cudaError_t e = cudaMalloc(ptr, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return fail(L3ES_ENOMEM, std::string("cudaMalloc(") + what + "): " + cudaGetErrorString(e));
-  }
-  p->allocs.push_back(*ptr);
-  return L3ES_OK;
-}
-
-static void sph_free(l3es_sph_plan* p) {
-  for (void* a : p->allocs) cudaFree(a);
-  p->allocs.clear();
-}
 
 // cell list of r (+ dt u_pred when given); leaves xw, perm, xs (and us when u != null)
 static int sph_build(l3es_sph_plan* p, const double* r, const double* u_pred, double dt, const double* u,
@@ -709,35 +694,52 @@ int l3es_sph_plan_create(int32_t dim, int32_t n, double box, int64_t np_max, l3e
   p->g.inv_h = (float)(1.0 / p->dx);
   p->g.cut2 = (float)(9.0 * p->dx * p->dx);
   p->ncell = dim == 3 ? nc * nc * nc : nc * nc;
-  int rc = L3ES_OK;
+  // one allocation holds every array: a plan is made inside the first call of a relaxation
+  // function, and with one per array that call took 235 us for 80^2 particles (now 171), 355 for
+  // 32^3 (258)
   const size_t npm = (size_t)np_max;
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->xw, sizeof(double) * npm * dim, "xw");
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->cell, sizeof(int) * npm, "cell");
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->perm0, sizeof(int) * npm, "perm0");
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->perm, sizeof(int) * npm, "perm");
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->xs, sizeof(float4) * npm, "xs");
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->us, sizeof(float4) * npm, "us");
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->rp, sizeof(float4) * npm, "rp");
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->count, sizeof(int) * p->ncell, "count");
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->cursor, sizeof(int) * p->ncell, "cursor");
-  if (rc == L3ES_OK) rc = sph_alloc(p, (void**)&p->start, sizeof(int) * (p->ncell + 1), "start");
-  if (rc != L3ES_OK) {
-    sph_free(p);
-    delete p;
-    return rc;
-  }
-  // neighbour lists, where they and the slot numbers fit (128 np_max words' rows: whole blocks)
-  const size_t lanes = (npm * kSphLanes + kSphThreads - 1) / kSphThreads * kSphThreads;
+  const size_t lanes = (npm * kSphLanes + kSphThreads - 1) / kSphThreads * kSphThreads;  // whole blocks
   const int cap = dim == 3 ? kSphKept3d : kSphKept2d;
   const size_t words = lanes * (cap + 1);
-  if (nc >= 3 && np_max <= (1LL << kSphCodeShift) && words * sizeof(unsigned) <= kSphKeptBytes) {
-    unsigned* nb = nullptr;
-    if (cudaMalloc((void**)&nb, words * sizeof(unsigned)) == cudaSuccess) {
-      p->allocs.push_back(nb);
-      p->kept = SphKept{nb, reinterpret_cast<int*>(nb + lanes * cap), (long long)lanes, cap};
-    } else {
-      cudaGetLastError();  // without them the calls search twice
-    }
+  // neighbour lists, where they and the slot numbers fit
+  const bool keep = nc >= 3 && np_max <= (1LL << kSphCodeShift) && words * sizeof(unsigned) <= kSphKeptBytes;
+  size_t bytes = 0;
+  auto place = [&](auto*& ptr, size_t count) {
+    using T = std::remove_reference_t<decltype(*ptr)>;
+    if (p->mem) ptr = reinterpret_cast<T*>(static_cast<char*>(p->mem) + bytes);
+    bytes += (count * sizeof(T) + 255) / 256 * 256;
+  };
+  auto arrays = [&] {
+    bytes = 0;
+    place(p->xw, npm * dim);
+    place(p->cell, npm);
+    place(p->perm0, npm);
+    place(p->perm, npm);
+    place(p->xs, npm);
+    place(p->us, npm);
+    place(p->rp, npm);
+    place(p->count, p->ncell);
+    place(p->cursor, p->ncell);
+    place(p->start, p->ncell + 1);
+  };
+  arrays();
+  const size_t own = bytes;
+  cudaError_t e = keep ? cudaMalloc(&p->mem, own + words * sizeof(unsigned)) : cudaErrorMemoryAllocation;
+  const bool kept = e == cudaSuccess;
+  if (!kept) {  // without the lists the calls search twice
+    cudaGetLastError();
+    e = cudaMalloc(&p->mem, own);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    delete p;
+    return fail(L3ES_ENOMEM, std::string("cudaMalloc(particle arrays, ") + std::to_string(own) +
+                                 " B): " + cudaGetErrorString(e));
+  }
+  arrays();
+  if (kept) {
+    unsigned* nb = reinterpret_cast<unsigned*>(static_cast<char*>(p->mem) + own);
+    p->kept = SphKept{nb, reinterpret_cast<int*>(nb + lanes * cap), (long long)lanes, cap};
   }
   *out = p;
   return L3ES_OK;
@@ -745,7 +747,7 @@ int l3es_sph_plan_create(int32_t dim, int32_t n, double box, int64_t np_max, l3e
 
 int l3es_sph_plan_destroy(l3es_sph_plan* p) {
   if (!p) return L3ES_OK;
-  sph_free(p);
+  cudaFree(p->mem);
   delete p;
   return L3ES_OK;
 }
