@@ -60,7 +60,7 @@ struct DnsOps {
     if constexpr (N > kStageMax3d) {
       tma_band_fused_ctas = persistent_ctas(kx_fwd_band_tma<N, true>);
     }
-    if constexpr (N >= 16) stage_attrs<2>();
+    if constexpr (N > kStep2dMax) stage_attrs<2>();
     if constexpr (N >= 16 && N <= kStep2dMax) {
       cudaFuncSetAttribute(k_step2d<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, Step2dCfg<N>::SMEM);
       cudaGetLastError();
@@ -391,7 +391,7 @@ struct DnsOps {
                     pdl_launch(k_yz_plane<N>, dim3(N, c.batch), YzCfg<N>::THREADS, YzCfg<N>::SMEM, s, c.W, c.Wx, c.fs,
                                c.DU, c.ds, c.kt, c.kd, s2, c.tw, ct));
       }
-    } else if constexpr (DIM == 2 && N >= 16 && N <= 128) {
+    } else if constexpr (DIM == 2 && N > kStep2dMax && N <= 128) {
       const double A = 8.0 * 3.0 * c.cs * c.batch, Adu = 8.0 * 3.0 * c.ds * c.batch;
       const float scale = (float)(1.0 / ((double)N * N));
       constexpr int LPC = 128 / (N / 8);
@@ -407,7 +407,7 @@ struct DnsOps {
   // is not in W yet; last: nothing follows that needs the new state's.
   template <int DIM>
   static void step_dim(const Ctx& c, float2* S, const EpiParams* prm, bool first, bool last, cudaStream_t s) {
-    if constexpr (N >= 16 && (DIM == 2 || N <= kStageMax3d)) {
+    if constexpr (DIM == 2 ? N > kStep2dMax : N >= 16 && N <= kStageMax3d) {
       if (first) x_stage<DIM, -1, true>(c, S, prm[0], s);
       between<DIM>(c, s);
       x_stage<DIM, 0, true>(c, S, prm[0], s);

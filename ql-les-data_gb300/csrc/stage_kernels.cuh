@@ -60,7 +60,7 @@ struct XStageCfg {
   static constexpr int E = EE, T = N / E;
   static constexpr int G = XW * T;                       // threads per component
   static constexpr int THREADS = 3 * G;
-  static constexpr int SYNC = G % 32 == 0 ? kSyncGroup : kSyncCta;
+  static_assert(G % 32 == 0, "a component's barriers count whole warps");
   static constexpr int XS = xpad_len<XW>(N) * XW;        // exchange slots per component
   static constexpr int US = N * XW;                      // shared column values per component
   static constexpr int SMEM = 3 * (XS + US) * (int)sizeof(float2);
@@ -128,7 +128,7 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
           v[e] = mid < N / 2 ? cadd(v[e], o) : csub(v[e], o);
         }
       }
-      block_fft<N, E, kFwd, XW, K::SYNC>(v, sx + p, t, tw, 1);
+      block_fft<N, E, kFwd, XW, kSyncGroup>(v, sx + p, t, tw, 1);
 #pragma unroll
       for (int e = 0; e < E; ++e) su[g * K::US + (t + T * e) * XW + p] = v[e];
       __syncthreads();
@@ -202,14 +202,14 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
 #pragma unroll
     for (int e = 0; e < E; ++e) su[g * K::US + (t + T * e) * XW + p] = v[e];
     __syncthreads();
-    block_fft<N, E, kInv, XW, K::SYNC>(v, sx + p, t, tw, 1);
+    block_fft<N, E, kInv, XW, kSyncGroup>(v, sx + p, t, tw, 1);
     if (ok) {
       float2* dst = DIM == 3 && g > 0 ? wx + ((long long)batch * 2 + g - 1) * fs : w + ((long long)batch * 6 + g) * fs;
 #pragma unroll
       for (int e = 0; e < E; ++e) dst[(long long)(t + T * e) * MC + m] = v[e];
     }
     // curl component g = i (k x u)_g; in 3D the y pass forms the x component itself
-    if (DIM == 3 && g == 0 && K::SYNC == kSyncGroup) return;
+    if (DIM == 3 && g == 0) return;
     const int ga = g == 2 ? 0 : g + 1, gb = g == 0 ? 2 : g - 1;  // (k x u)_g = k_ga u_gb - k_gb u_ga
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -220,12 +220,9 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
       const float2 ua = su[ga * K::US + row * XW + p], ub = su[gb * K::US + row * XW + p];
       v[e] = mul_i<kInv>(make_float2(ka * ub.x - kb * ua.x, ka * ub.y - kb * ua.y));
     }
-    if constexpr (K::SYNC == kSyncGroup)
-      group_sync<K::G>();  // the exchange buffer's last reads are done
-    else
-      __syncthreads();
-    block_fft<N, E, kInv, XW, K::SYNC>(v, sx + p, t, tw, 1);
-    if (ok && !(DIM == 3 && g == 0)) {
+    group_sync<K::G>();  // the exchange buffer's last reads are done
+    block_fft<N, E, kInv, XW, kSyncGroup>(v, sx + p, t, tw, 1);
+    if (ok) {
       float2* dst = w + ((long long)batch * 6 + 3 + g) * fs;
 #pragma unroll
       for (int e = 0; e < E; ++e) dst[(long long)(t + T * e) * MC + m] = v[e];
@@ -234,7 +231,7 @@ kx_stage(const float2* __restrict__ du, long long dcs, float2* __restrict__ S, f
 }
 
 // ------------------------------------------------------------------------------
-// Half-axis line pass of 2D grids up to 128^2: one line per slot of T = N / 8 lanes, 32 / T
+// Half-axis line pass of 64^2 and 128^2 grids: one line per slot of T = N / 8 lanes, 32 / T
 // lines per warp, and the z products of two neighbouring slots in one transform that both
 // run (a slot doing two lines one after the other, as line_cross2 does, has a chain of 9
 // transforms instead of 5, on half as many warps: 8.1 us for 8 fields of 128^2). lines is
@@ -245,7 +242,7 @@ __global__ void __launch_bounds__(128)
 line_cross_slots(const float2* __restrict__ w, long long fs, float2* __restrict__ du, long long ds, int kt, int kd,
                  float s2, const float2* __restrict__ ct8, int lines) {
   pdl_begin();
-  static_assert(N >= 16 && N <= 128, "two lines per warp");
+  static_assert(N >= 64 && N <= 128, "two lines per warp");
   constexpr int T = N / 8, H = N / 2 + 1;
   __shared__ float2 s_x[128 / T * xpad_len<1>(N)];
   const int slot = threadIdx.x / T, t = threadIdx.x % T;
