@@ -31,13 +31,11 @@ struct DnsOps {
   // resident CTAs (all SMs) of a persistent kernel with K::SMEM dynamic shared memory
   template <typename F>
   static int persistent_ctas(F kernel) {
-    int nb = 0, dev = 0, sms = 0;
+    int nb = 0;
     const int smem = KxTma<N>::SMEM;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, TX, smem) == cudaSuccess &&
-        cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
-      return nb * sms;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, TX, smem) == cudaSuccess)
+      return nb * sm_count();
     cudaGetLastError();
     return 0;
   }
@@ -187,7 +185,7 @@ struct DnsOps {
           const long long tiles = (lines + L3::LPC - 1) / L3::LPC;
           if (c.sched.line_pair == 3 && lc3_staged_ok && lines % L3::LPC == 0)
             L3ES_LAUNCH(c, KK_LINE_CROSS, 2.0 * A + Adu, s,
-                        pdl_launch(tiles * c.batch <= 152 ? line_cross3<N, true, true> : line_cross3<N, true>,
+                        pdl_launch(tiles * c.batch <= c.sms ? line_cross3<N, true, true> : line_cross3<N, true>,
                                    dim3((unsigned)tiles, c.batch), L3::THREADS, L3::SMEM_STAGED, s, c.W, c.fs, c.DU,
                                    c.ds, c.kt, c.kd, s2, c.tw + line2_ct_offset<N>(),
                                    c.tw + line3_ct16_offset<N>(), (int)lines, c.err));
@@ -364,7 +362,7 @@ struct DnsOps {
   // doubled grid still has an SM per CTA. Ten steps with one CTA per plane and with two:
   // 64^3 664 and 532 us, 32^3 347 and 322, 32^3 x 2 423 and 371; above that two lose, 64^3 x 2
   // 808 and 916, 32^3 x 4 488 and 495.
-  static bool two_ctas(const Ctx& c) { return 2LL * N * c.batch <= 152; }
+  static bool two_ctas(const Ctx& c) { return 2LL * N * c.batch <= c.sms; }
 
   // W -> DU between two kx_stage launches: in 3D one kernel per x plane
   template <int DIM>

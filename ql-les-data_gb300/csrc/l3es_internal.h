@@ -138,6 +138,7 @@ constexpr int kFormStart = -1;  // no step form set
 // Geometry + scratch of one plan, handed to the per-N launch wrappers.
 struct Ctx {
   int dim = 3, n = 0, h = 0, batch = 1;
+  int sms = 0;          // SMs of the plan's device
   int kd = 0;           // largest kept |k| of the 2/3 cube mask (|k| < 2/3 (N/2+1))
   int kt = 0;           // stored half-axis columns of the nonlinear term (kd+1 -> multiple of TW)
   long long nmid = 1;   // middle-axis length (3D: N, 2D: 1)

@@ -295,7 +295,7 @@ inline cudaError_t dft_launch(int dim, const float2* hh, long long hcs, int c, c
     pdl_launch(kernel, grid, K::threads(c), smem, s, hh, hcs, c, r, np, u_r, dt, r_out);
     return cudaGetLastError();
   };
-  const bool small = np <= 2 * 152 * DftCfg<3, 2>::TILE;
+  const bool small = np <= 2LL * sm_count() * DftCfg<3, 2>::TILE;
   if (dim == 3) return small ? go(DftCfg<3, 2>{}, k_dft_interp<3, 2>) : go(DftCfg<3, 4>{}, k_dft_interp<3, 4>);
   return small ? go(DftCfg<2, 2>{}, k_dft_interp<2, 2>) : go(DftCfg<2, 4>{}, k_dft_interp<2, 4>);
 }

@@ -25,6 +25,16 @@ __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// SMs of the current device (GB300: 152), for the rules that compare a launch's blocks with
+// them; 0 if the device cannot tell.
+inline int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    cudaGetLastError();
+  return sms;
+}
+
 template <typename... P, typename... A>
 inline void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchAttribute at{};

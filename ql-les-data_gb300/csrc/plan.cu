@@ -232,6 +232,7 @@ int l3es_plan_create(const l3es_plan_desc* desc, l3es_plan** out) {
   p->desc = *desc;
   cudaGetDevice(&p->device);
   Ctx& c = p->ctx;
+  c.sms = sm_count();
   c.dim = dim;
   c.n = n;
   c.h = n / 2 + 1;
