@@ -360,8 +360,9 @@ struct DnsOps {
 
   // Whether two CTAs share a plane between two kx_stage launches (k_yz_half): while the
   // doubled grid still has an SM per CTA. Ten steps with one CTA per plane and with two:
-  // 64^3 664 and 532 us, 32^3 347 and 322, 32^3 x 2 423 and 371; above that two lose, 64^3 x 2
-  // 808 and 916, 32^3 x 4 488 and 495.
+  // 64^3 640 and 513 us, 32^3 342 and 320, 32^3 x 2 419 and 365; 64^3 x 2 802 and 901, 32^3 x 8
+  // 501 and 602 (between them 32^3 x 3 and x 4 would gain a little from two: 437 and 430, 484 and
+  // 428).
   static bool two_ctas(const Ctx& c) { return 2LL * N * c.batch <= c.sms; }
 
   // W -> DU between two kx_stage launches: in 3D one kernel per x plane

@@ -37,7 +37,7 @@ enum KernelKind {
   KK_ADJ_LINE,      // line_cross_adj (both adjoint products)
   KK_ADJ_EPI,       // k_adj_epi / kx_fwd_adj (vjp assembly + RK4 reverse recursion)
   KK_X_STAGE,       // kx_stage (closes an RK stage on the x pencils, opens the next)
-  KK_YZ_PLANE,      // k_yz_plane (small 3D grids: everything between two x passes)
+  KK_YZ_PLANE,      // k_yz_plane / k_yz_half (small 3D grids: everything between two x passes)
   KK_COUNT
 };
 const char* kernel_kind_name(int k);

@@ -13,8 +13,8 @@
 // Limits and sharing rules:
 //  - the scratch holds kNoallocScratchElems complex64 values (417,792 bytes), the
 //    coarse spectrum of ckp_N = 32 in 3D; requests above ckp_N = 32 in 3D or
-//    ckp_N = 64 in 2D (where the kernel's per-block phase tables reach the shared
-//    memory limit) are rejected with L3ES_EINVAL;
+//    ckp_N = 64 in 2D (the largest grid of the exact sum, kDftMaxC) are rejected with
+//    L3ES_EINVAL;
 //  - every GPU that loads the library keeps this array for the life of the
 //    process;
 //  - all calls share the one array and it keeps the previous call's contents.
@@ -96,7 +96,7 @@ extern "C" int l3es_interp_dft_noalloc(int32_t dim, int32_t n_fine, int32_t ckp_
     return fail(L3ES_EINVAL, "l3es_interp_dft_noalloc: need powers of two with 2 <= ckp_N <= N");
   if (np < 0) return fail(L3ES_EINVAL, "l3es_interp_dft_noalloc: np < 0");
   if (np > kNoallocMaxParticles)
-    return fail(L3ES_EINVAL, "l3es_interp_dft_noalloc: np above 128 (2^31 - 1), the one-thread-per-particle grid limit");
+    return fail(L3ES_EINVAL, "l3es_interp_dft_noalloc: np above 128 (2^31 - 1)");
   const int c = ckp_n, hc = c / 2 + 1;
   const long long hcs = dim == 3 ? (long long)c * c * hc : (long long)c * hc;
   if (3 * hcs > kNoallocScratchElems || (dim == 2 && c > 64))

@@ -28,7 +28,7 @@ namespace l3es {
 // 98.3 -> 69.7 us, 128^2 x 8 98.4 -> 70.6 us, 512^2 122.9 -> 97.7 us; 3D, dependent launches
 // on both sides, 64^3 89 -> 71 us, 64^3 x 6 222 -> 208 us, 64^3 x 12 425 -> 423 us; from
 // plain launches 32^3 121 -> 35 us, 16^3 130 -> 41 us. (With dependent launches, paired adds
-// and the line passes of their size those steps now take 47, 42 and 53 us.) With kx_stage 128^3 takes 38 instead
+// and the line passes of their size those steps now take 47, 42 and 51 us.) With kx_stage 128^3 takes 38 instead
 // of 32.6 us for one stage's x passes and 256^3 267 instead of 195 us: there the chip is full
 // and the barriers of the three groups cost more than the saved round trip. Larger 3D grids
 // keep kx_inv and the band-fused kx_fwd_band.
@@ -492,7 +492,7 @@ k_yz_plane(const float2* __restrict__ w, const float2* __restrict__ wx, long lon
 // eighth turns of the butterfly. A turn of its own beside an N/2-point transform took one
 // more rounding per value: the error of 64^3 and 32^3 steps against 64 bits was 0.7 and 1.2 %
 // above the unsplit transforms' in nearly every field, now it is level with theirs, and ten
-// 64^3 steps take 517 us instead of 532 (32^3 322 and 324).
+// 64^3 steps take 513 us instead of 532 (32^3 320 and 324).
 // ------------------------------------------------------------------------------
 // x times the k-th eighth turn, exp(DIR 2 pi i k / 8), k = 0..3
 template <int DIR>

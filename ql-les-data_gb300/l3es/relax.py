@@ -2,7 +2,7 @@
 
 The reference builds a JAX-SPH neighbour list, quintic kernel and Tait EoS and returns
 two jitted functions (relax.py:16-178). Here both run as CUDA kernels behind
-``l3es_sph_*`` (cell list rebuilt per call, one thread per particle in cell order).
+``l3es_sph_*`` (cell list rebuilt per call, eight lanes per particle in cell order).
 Positions and velocities are float64 (np, dim) torch CUDA tensors (numpy arrays are
 accepted and copied to the device).
 """
